@@ -48,7 +48,7 @@ void free_all(wg::Problem& P) {
       e = nullptr;
     }
   wg::gummel_free(P);
-  void* ptrs[] = {P.phi, P.kvec, P.xi_edge, P.kap, P.betai, P.pre_dinv, P.pre_h, P.kmap_a, P.kmap_s, P.cosm, P.pinv, P.pp, P.flr, P.fxi, P.qd, P.beta, P.xq, P.pot_x,
+  void* ptrs[] = {P.phi, P.phi_t, P.kvec, P.xi_edge, P.kap, P.betai, P.pre_dinv, P.pre_h, P.kmap_a, P.kmap_s, P.cosm, P.pinv, P.pp, P.flr, P.fxi, P.qd, P.beta, P.xq, P.pot_x,
                   P.pot_v, P.vslope, P.m_nodes, P.rhs, P.tr_b, P.x, P.w, P.z, P.r, P.V, P.xh, P.yh, P.H, P.cs, P.sn, P.g, P.hcol,
                   P.ycoef, P.partial, P.nrm_partial, P.nrm, P.nrm_keep, P.inv64, P.target, P.active, P.reorth, P.res_mask, P.res_digits, P.md_count, P.gs_count, P.kused, P.any_active};
   for (void* p : ptrs)
@@ -247,6 +247,8 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
   };
   A(cudaStreamCreateWithFlags(&P.stream, cudaStreamNonBlocking));
   A(dalloc(&P.phi, (size_t)s.nxi * s.nk, bytes));
+  const int hs = (s.nxi + 1) / 2, hk = (s.nk + 1) / 2;
+  A(dalloc(&P.phi_t, (size_t)hs * hk, bytes));
   A(dalloc(&P.kvec, s.nk, bytes));
   A(dalloc(&P.xi_edge, s.nxi + 1, bytes));
   A(dalloc(&P.kap, (size_t)nK * nK * wg::kNqx, bytes));
@@ -320,6 +322,10 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
     for (int i = 0; i <= s.nxi; ++i)
       betai[(size_t)ac * (s.nxi + 1) + i] = -(s.delta_xi / 4 * s.mpc) * s.kap_sum[ac] * s.cap[i];
   API_CK(&P, cudaMemcpyAsync(P.phi, phi.data(), sizeof(double2) * phi.size(), cudaMemcpyHostToDevice, P.stream));
+  std::vector<double2> phi_t((size_t)hs * hk);
+  for (int j = 0; j < hk; ++j)
+    for (int i = 0; i < hs; ++i) phi_t[(size_t)j * hs + i] = phi[(size_t)i * s.nk + j];
+  API_CK(&P, cudaMemcpyAsync(P.phi_t, phi_t.data(), sizeof(double2) * phi_t.size(), cudaMemcpyHostToDevice, P.stream));
   API_CK(&P, cudaMemcpyAsync(P.kvec, s.k.data(), sizeof(double) * s.nk, cudaMemcpyHostToDevice, P.stream));
   API_CK(&P, cudaMemcpyAsync(P.xi_edge, s.xi_edge.data(), sizeof(double) * (s.nxi + 1), cudaMemcpyHostToDevice, P.stream));
   API_CK(&P, cudaMemcpyAsync(P.kap, s.kap.data(), sizeof(double) * s.kap.size(), cudaMemcpyHostToDevice, P.stream));

@@ -4,9 +4,10 @@
 // get_SysM.m:1-16 = get_Diff.m:66-84 + get_Drift_accel_trial_permutedShell.m:64-333):
 //   1. flux_kernel       upwind x-flux times diag(k): per k a block-bidiagonal
 //                        stencil over elements (HBM-bound streaming kernel)
-//   2. zgemm_kernel      X^ = Phi X over every DG node of the batch (one GEMM),
+//   2. paired_kernel     X^ = Phi X over every DG node of the batch (one product),
 //      stencil_kernel    Y^_{e,a} = sum_b T(beta_{e,ab}) X^_{e,b} (xi-tridiagonal),
-//      zgemm_kernel      y += i Phi^H Y^ (second GEMM, accumulating epilogue)
+//      paired_kernel     y += i Phi^H Y^ (second product, accumulating epilogue)
+//      (zgemm_kernel where the caller owns Phi: the allocation-free apply)
 // plus the k-line preconditioner, the Vw(x,k) rebuild and the observables.
 #include <cuda_runtime.h>
 
@@ -135,7 +136,128 @@ __global__ void __launch_bounds__(kFluxThreads) flux_kernel(const double2* __res
 }
 
 // ---------------------------------------------------------------------------
-// 2a. Complex FP64 GEMM  C(M x Ncol) = op(A)(M x K) * B(K x Ncol), column-major
+// 2a. Transforms with the plane-wave basis, FP64.  Phi(s, j) = exp(i k_j xi_s) / sqrt(L) on grids that
+// are symmetric about 0 in both k and xi, so with the mirror pairs (p, p') of the input and c + i d =
+// Phi(m, p), the output pair (m, m') is
+//   X^(m) = A + i B,  X^(m') = A - i B,   A = sum_p c (x_p + x_p'),  B = sum_p d (x_p - x_p'),
+// a real matrix times complex columns: 4 FMAs per (m, p) pair, K M FMAs per column instead of the 4 K M
+// of the complex product.  The adjoint i Phi^H is the same with the pair (A - i B, A + i B).
+//   MODE 0: Y  = Phi X          tab = phi_t[p][m] (p a wave number, m a xi row)
+//   MODE 1: Y += i Phi^H X      tab = phi [p][m]  (p a xi row, m a wave number)
+// Bound by the FP64 pipe (2 FMAs per clock and SM: a warp's FMA takes 64 cycles of its quarter, so
+// loads, address arithmetic and shared-memory reads hide behind it).  What matters is that
+// the 608 pipe quarters get equal shares: one warp takes TS rows x 32/TS columns, blocks of 4 warps, and TS
+// (8, 16, 32) is the one that pads the rows least (table_rows).  C2 operator, 1,920 columns,
+// 256 x 256: 1,055 us a product with the 64 x 64 complex tiles (120 tiles), 225 us here (1.12 of 1.25 TFLOP/s);
+// 36 columns of 32 x 32 (one tile on one SM before): 136 us -> 10 us.
+// ---------------------------------------------------------------------------
+constexpr int kPairThreads = 128, kPairChunk = 32;
+
+template <int MODE, int TS>
+__global__ void __launch_bounds__(kPairThreads) paired_kernel(const double2* __restrict__ tab, int ldt,
+                                                              const double2* __restrict__ X,
+                                                              double2* __restrict__ Y, int K, int M,
+                                                              long long ncol) {
+  constexpr int CW = 32 / TS, CB = CW * (kPairThreads / 32), PC = kPairChunk, LD = CB * PC / kPairThreads;
+  __shared__ double2 es[2][CB][PC + 1], os[2][CB][PC + 1];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int hk = (K + 1) / 2, hm = (M + 1) / 2;
+  const int m = blockIdx.y * TS + lane % TS;
+  const int cl = (tid >> 5) * CW + lane / TS;
+  const long long c0 = (long long)blockIdx.x * CB;
+  const double2* tm = tab + (m < hm ? m : hm - 1);
+  double2 xa[LD], xb[LD];
+  auto fetch = [&](int p0) {
+#pragma unroll
+    for (int r = 0; r < LD; ++r) {
+      const int idx = tid + r * kPairThreads, p = p0 + idx % PC;
+      const long long c = c0 + idx / PC;
+      const bool in = p < hk && c < ncol;
+      xa[r] = in ? X[c * K + p] : make_double2(0.0, 0.0);
+      xb[r] = in && p != K - 1 - p ? X[c * K + (K - 1 - p)] : make_double2(0.0, 0.0);
+    }
+  };
+  auto stage = [&](int buf, int p0) {
+#pragma unroll
+    for (int r = 0; r < LD; ++r) {
+      const int idx = tid + r * kPairThreads, p = p0 + idx % PC;
+      const bool mid = p == K - 1 - p;   // the unpaired middle entry: sum x, difference 0
+      es[buf][idx / PC][idx % PC] = make_double2(xa[r].x + xb[r].x, xa[r].y + xb[r].y);
+      os[buf][idx / PC][idx % PC] = mid ? make_double2(0.0, 0.0)
+                                        : make_double2(xa[r].x - xb[r].x, xa[r].y - xb[r].y);
+    }
+  };
+  double2 A = make_double2(0.0, 0.0), B = make_double2(0.0, 0.0);
+  fetch(0);
+  stage(0, 0);
+  __syncthreads();
+  for (int p0 = 0, buf = 0; p0 < hk; p0 += PC, buf ^= 1) {
+    const bool more = p0 + PC < hk;
+    if (more) fetch(p0 + PC);
+    const int np = min(PC, hk - p0);
+    const double2* tp = tm + (long long)p0 * ldt;
+    int p = 0;
+    for (; p + 8 <= np; p += 8) {
+      double2 t[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) t[u] = __ldg(tp + (long long)(p + u) * ldt);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const double2 e = es[buf][cl][p + u], o = os[buf][cl][p + u];
+        A.x = fma(t[u].x, e.x, A.x);
+        A.y = fma(t[u].x, e.y, A.y);
+        B.x = fma(t[u].y, o.x, B.x);
+        B.y = fma(t[u].y, o.y, B.y);
+      }
+    }
+    for (; p < np; ++p) {
+      const double2 t = __ldg(tp + (long long)p * ldt), e = es[buf][cl][p], o = os[buf][cl][p];
+      A.x = fma(t.x, e.x, A.x);
+      A.y = fma(t.x, e.y, A.y);
+      B.x = fma(t.y, o.x, B.x);
+      B.y = fma(t.y, o.y, B.y);
+    }
+    if (more) stage(buf ^ 1, p0 + PC);
+    __syncthreads();
+  }
+  const long long c = c0 + cl;
+  if (m >= hm || c >= ncol) return;
+  const int mr = M - 1 - m;
+  double2* y = Y + c * M;
+  if (MODE == 0) {
+    y[m] = make_double2(A.x - B.y, A.y + B.x);
+    if (mr != m) y[mr] = make_double2(A.x + B.y, A.y - B.x);
+  } else {   // t = A -+ i B, y += i t
+    double2 o = y[m];
+    y[m] = make_double2(o.x - (A.y - B.x), o.y + (A.x + B.y));
+    if (mr != m) {
+      o = y[mr];
+      y[mr] = make_double2(o.x - (A.y + B.x), o.y + (A.x - B.y));
+    }
+  }
+}
+
+// Rows per warp: the fewest padded rows over ceil(rows / TS) tiles, the wider tile on a tie (33 rows, Nk = 65:
+// 40 padded rows with 8 a tile, 64 with 32).
+int table_rows(int half) {
+  int best = 32;
+  for (int ts = 16; ts >= 8; ts /= 2)
+    if ((half + ts - 1) / ts * ts < (half + best - 1) / best * best) best = ts;
+  return best;
+}
+
+template <int MODE>
+void paired_launch(const double2* tab, int ldt, const double2* X, double2* Y, int K, int M, long long ncol,
+                   cudaStream_t st) {
+  const int half = (M + 1) / 2, ts = table_rows(half), cb = kPairThreads / ts;
+  const dim3 grid((unsigned)((ncol + cb - 1) / cb), (unsigned)((half + ts - 1) / ts));
+  if (ts == 32) paired_kernel<MODE, 32><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol);
+  else if (ts == 16) paired_kernel<MODE, 16><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol);
+  else paired_kernel<MODE, 8><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol);
+}
+
+// ---------------------------------------------------------------------------
+// 2a'. The same products with a caller's Phi (any matrix).  Complex FP64 GEMM  C(M x Ncol) = op(A)(M x K) * B(K x Ncol), column-major
 // B and C with leading dimensions ldb = K, ldc = M.
 //   MODE 0: A(m,k) = phi[m*lda + k]        C  = acc        (X^ = Phi X)
 //   MODE 1: A(m,k) = conj(phi[k*lda + m])  C += i * acc    (y += i Phi^H Y^)
@@ -341,21 +463,19 @@ void stencil_launch(const double2* xh, double2* yh, const double* beta, const do
 template <int NK>
 cudaError_t apply_nk(Problem& P, const double2* x, double2* y) {
   const double BN = (double)P.N * P.batch, ncols = (double)P.ncols, nxi = P.s.nxi, nk = P.s.nk;
-  const double gemm_flops = 8.0 * nxi * nk * ncols;
+  const double gemm_flops = 2.0 * nxi * nk * ncols;   // paired rows and columns: a quarter of the complex product
   cudaEvent_t ev = prof_begin(P, PROF_FLUX64, 1, 32.0 * BN, 8.0 * NK * BN);
   flux_launch<NK>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream);
   prof_end(P, PROF_FLUX64, ev);
-  dim3 g1((unsigned)((P.ncols + GBN - 1) / GBN), (P.s.nxi + GBM - 1) / GBM);
   ev = prof_begin(P, PROF_GEMM_F64, 1, 16.0 * (BN + nxi * ncols), gemm_flops);
-  zgemm_kernel<0><<<g1, 256, 0, P.stream>>>(P.phi, P.s.nk, x, P.xh, P.s.nxi, P.s.nk, P.ncols);
+  paired_launch<0>(P.phi_t, (P.s.nxi + 1) / 2, x, P.xh, P.s.nk, P.s.nxi, P.ncols, P.stream);
   prof_end(P, PROF_GEMM_F64, ev);
   ev = prof_begin(P, PROF_STENCIL64, 1, 32.0 * nxi * ncols + 8.0 * P.batch * P.s.n_el * NK * NK * (nxi + 1),
                   16.0 * NK * nxi * ncols);
   stencil_launch<NK>(P.xh, P.yh, P.beta, P.betai, P.batch, P.s.n_el, P.s.nxi, P.stream);
   prof_end(P, PROF_STENCIL64, ev);
-  dim3 g2((unsigned)((P.ncols + GBN - 1) / GBN), (P.s.nk + GBM - 1) / GBM);
   ev = prof_begin(P, PROF_GEMM_F64, 1, 16.0 * (2 * BN + nxi * ncols), gemm_flops);
-  zgemm_kernel<1><<<g2, 256, 0, P.stream>>>(P.phi, P.s.nk, P.yh, y, P.s.nk, P.s.nxi, P.ncols);
+  paired_launch<1>(P.phi, P.s.nk, P.yh, y, P.s.nxi, P.s.nk, P.ncols, P.stream);
   prof_end(P, PROF_GEMM_F64, ev);
   return cudaGetLastError();
 }
@@ -540,8 +660,7 @@ cudaError_t launch_precondition(Problem& P, const double2* r, long long r_stride
 
 cudaError_t launch_rho_xi(Problem& P, int b, double2* out) {
   const long long ncol = (long long)P.s.n_el * P.s.nK;
-  dim3 g1((unsigned)((ncol + GBN - 1) / GBN), (P.s.nxi + GBM - 1) / GBM);
-  zgemm_kernel<0><<<g1, 256, 0, P.stream>>>(P.phi, P.s.nk, P.x + (long long)b * P.N, out, P.s.nxi, P.s.nk, ncol);
+  paired_launch<0>(P.phi_t, (P.s.nxi + 1) / 2, P.x + (long long)b * P.N, out, P.s.nk, P.s.nxi, ncol, P.stream);
   return cudaGetLastError();
 }
 

@@ -223,6 +223,7 @@ struct Problem {
   cudaStream_t stream = nullptr;
   // constant device data
   double2* phi = nullptr;        // nxi x nk row-major
+  double2* phi_t = nullptr;      // [ceil(nk/2)][ceil(nxi/2)]: phi_t[j][s] = phi[s][j] of the lower halves
   double* kvec = nullptr;        // nk
   double* xi_edge = nullptr;     // nxi + 1
   double* kap = nullptr;         // nK*nK*10
