@@ -217,6 +217,10 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
   P.nx = s.n_el * (nK - 1) + 1;
   P.nchunk = (int)std::max<long long>(1, (P.N + 2047) / 2048);
   P.nblk = (int)std::max<long long>(1, (P.N + 255) / 256);
+  // FP64 multi-dot: two blocks per SM at six vector groups (24 vectors) of one problem, 256 elements per block at
+  // least; a rule on N alone, so that a problem's sums do not depend on the batch it is in
+  for (P.md_e = 8; P.md_e > 1 && (P.N + 256 * P.md_e - 1) / (256 * P.md_e) * 6 < 2 * 152;) P.md_e /= 2;
+  P.md_chunk = (int)((P.N + 256 * P.md_e - 1) / (256 * P.md_e));
   const long long BN = P.N * batch;
   const int mp1 = P.restart + 1;
   const int pst = P.restart_max + 1;
@@ -292,7 +296,7 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
   A(dalloc(&P.g, (size_t)batch * pst, bytes));
   A(dalloc(&P.hcol, (size_t)batch * pst, bytes));
   A(dalloc(&P.ycoef, (size_t)batch * P.restart_max, bytes));
-  A(dalloc(&P.partial, (size_t)batch * pst * P.nchunk, bytes));
+  A(dalloc(&P.partial, (size_t)batch * pst * std::max(P.nchunk, P.precision == WG_PREC_MIXED ? 0 : P.md_chunk), bytes));
   A(dalloc(&P.nrm_partial, (size_t)batch * std::max(P.nchunk, P.nblk), bytes));
   A(dalloc(&P.nrm, batch, bytes));
   A(dalloc(&P.nrm_keep, batch, bytes));

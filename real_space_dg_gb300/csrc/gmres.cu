@@ -38,17 +38,32 @@ __device__ __forceinline__ double2 ld2(const float2& v) { return make_double2(v.
 __device__ __forceinline__ void st2(double2& d, double2 v) { d = v; }
 __device__ __forceinline__ void st2(float2& d, double2 v) { d = make_float2((float)v.x, (float)v.y); }
 
-// Basis loads of the FP32 inner solve: two consecutive complex values (16 bytes of an FP32
-// basis, 8 bytes of an FP16 one) as one float4; one complex value as float2.
-__device__ __forceinline__ float4 ld_pair(const float2* v, long long n4) {
-  return reinterpret_cast<const float4*>(v)[n4];
-}
-__device__ __forceinline__ float4 ld_pair(const __half2* v, long long n4) {
-  const uint2 u = reinterpret_cast<const uint2*>(v)[n4];
-  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
-  const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-  return make_float4(a.x, a.y, b.x, b.y);
-}
+// Basis loads of the FP32 inner solve: four consecutive complex values (32 bytes of an FP32 basis,
+// 16 bytes of an FP16 one; N is a multiple of 4 there) as they come, and their value as floats.
+template <typename VB> struct Quad;
+template <> struct Quad<float2> {
+  float4 u, v;
+  __device__ __forceinline__ void load(const float2* p, long long n4) {
+    u = __ldg(reinterpret_cast<const float4*>(p) + 2 * n4);
+    v = __ldg(reinterpret_cast<const float4*>(p) + 2 * n4 + 1);
+  }
+  __device__ __forceinline__ void zero() { u = v = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ float2 get(int i) const {
+    return i == 0 ? make_float2(u.x, u.y) : i == 1 ? make_float2(u.z, u.w)
+                                                   : i == 2 ? make_float2(v.x, v.y) : make_float2(v.z, v.w);
+  }
+};
+template <> struct Quad<__half2> {
+  uint4 u;
+  __device__ __forceinline__ void load(const __half2* p, long long n4) {
+    u = __ldg(reinterpret_cast<const uint4*>(p) + n4);
+  }
+  __device__ __forceinline__ void zero() { u = make_uint4(0u, 0u, 0u, 0u); }
+  __device__ __forceinline__ float2 get(int i) const {
+    const unsigned w = i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w;
+    return __half22float2(*reinterpret_cast<const __half2*>(&w));
+  }
+};
 __device__ __forceinline__ float2 ld_one(const float2& v) { return v; }
 __device__ __forceinline__ double2 ld_one(const double2& v) { return v; }
 __device__ __forceinline__ float2 ld_one(const __half2& v) { return __half22float2(v); }
@@ -67,10 +82,10 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 struct Acc64 {
   double2 v = make_double2(0.0, 0.0);
   __device__ __forceinline__ void add_cdot(const double2& a, const double2& x) {  // += conj(a) x
-    v.x += a.x * x.x + a.y * x.y;
-    v.y += a.x * x.y - a.y * x.x;
+    v.x = fma(a.x, x.x, fma(a.y, x.y, v.x));
+    v.y = fma(a.x, x.y, fma(-a.y, x.x, v.y));
   }
-  __device__ __forceinline__ void add_norm(const double2& a) { v.x += a.x * a.x + a.y * a.y; }
+  __device__ __forceinline__ void add_norm(const double2& a) { v.x = fma(a.x, a.x, fma(a.y, a.y, v.x)); }
   __device__ __forceinline__ void warp_reduce() {
     for (int o = 16; o > 0; o >>= 1) {
       v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
@@ -89,10 +104,9 @@ struct Acc64 {
 
 struct AccF32 {
   float re = 0.f, im = 0.f;
-  // two consecutive complex values per float4
-  __device__ __forceinline__ void add_cdot4(const float4& a, const float4& x) {
-    re = fmaf(a.x, x.x, fmaf(a.y, x.y, fmaf(a.z, x.z, fmaf(a.w, x.w, re))));
-    im = fmaf(a.x, x.y, fmaf(-a.y, x.x, fmaf(a.z, x.w, fmaf(-a.w, x.z, im))));
+  __device__ __forceinline__ void add_cdot(const float2& a, const float2& x) {
+    re = fmaf(a.x, x.x, fmaf(a.y, x.y, re));
+    im = fmaf(a.x, x.y, fmaf(-a.y, x.x, im));
   }
   __device__ __forceinline__ void add_norm(const float2& a) { re = fmaf(a.x, a.x, fmaf(a.y, a.y, re)); }
   __device__ __forceinline__ void warp_reduce() {
@@ -123,8 +137,8 @@ template <> struct AccFor<float2> { using type = AccF32; };
 
 // Complex multiply-subtract in the vector's own precision: w -= v h.
 __device__ __forceinline__ void cms(double2& w, const double2& v, const double2& h) {
-  w.x -= v.x * h.x - v.y * h.y;
-  w.y -= v.x * h.y + v.y * h.x;
+  w.x = fma(-v.x, h.x, fma(v.y, h.y, w.x));
+  w.y = fma(-v.x, h.y, fma(-v.y, h.x, w.y));
 }
 __device__ __forceinline__ void cms(float2& w, const float2& v, const float2& h) {
   w.x = fmaf(-v.x, h.x, fmaf(v.y, h.y, w.x));
@@ -161,7 +175,7 @@ __device__ __forceinline__ bool last_block_of_problem(int* __restrict__ count, i
   __shared__ int last;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&count[b], 1) == (int)gridDim.x - 1;
+  if (threadIdx.x == 0) last = atomicAdd(&count[b], 1) == (int)(gridDim.x * gridDim.z) - 1;
   __syncthreads();
   if (last) __threadfence();
   return last;
@@ -211,56 +225,79 @@ __device__ void dot_reduce_block(const double2* __restrict__ partial, double2* _
 // Givens step k of problem b (one warp): rotate the new Hessenberg column by the
 // previous rotations, make the next rotation, update g and deactivate the problem
 // once the residual estimate |g[k+1]| reaches its target.  H is column-major per
-// problem (H[b][col*(m+1)+row]), cs/sn/g per problem; staging in shared memory.
+// problem (H[b][col*(m+1)+row]), cs/sn/g per problem; h_next = H[k+1][k].
+// Rotation i maps (t_i, h_{i+1}) to (r_i, t_{i+1}) with r_i = c t + s h and t_{i+1} = -conj(s) t + conj(c) h:
+// t is a first-order recurrence, so a warp scan of its affine maps (|factor| <= 1) gives 32 rotations in
+// about 55 FP64 instructions instead of 14 per rotation in sequence (each takes a quarter's FP64 pipe for
+// 64 cycles whatever the number of lanes).  This tail runs after the last block of an update, so it is on
+// the critical path of every Arnoldi step: the update launches of a 1,152-unknown solve (k up to 50)
+// took 28.1 us on average with the sequential rotations, 21.5 us with the scan.
 __device__ void givens_warp(double2* __restrict__ H, double2* __restrict__ cs, double2* __restrict__ sn,
                             double2* __restrict__ g, int* __restrict__ active, int* __restrict__ kused,
-                            const double* __restrict__ target, int b, int k, int pstride, int m, double2* col_s,
-                            double2* c_s, double2* s_s) {
+                            const double* __restrict__ target, int b, int k, int pstride, int m, double h_next) {
   const int lane = threadIdx.x & 31;
   double2* col = H + (long long)b * pstride * m + (long long)k * pstride;
   double2* c = cs + b * m;
   double2* s = sn + b * m;
-  for (int i = lane; i <= k + 1; i += 32) col_s[i] = col[i];
-  for (int i = lane; i < k; i += 32) {
-    c_s[i] = c[i];
-    s_s[i] = s[i];
+  double2* gg = g + b * pstride;
+  const double2 gk = gg[k];
+  const double tg = target[b];
+  double2 t = col[0];
+  for (int i0 = 0; i0 < k; i0 += 32) {
+    const int i = i0 + lane;
+    const bool in = i < k;
+    const double2 zero = make_double2(0.0, 0.0);
+    const double2 ci = in ? c[i] : zero, si = in ? s[i] : zero, hn = in ? col[i + 1] : zero;
+    double2 A = in ? make_double2(-si.x, si.y) : make_double2(1.0, 0.0);
+    double2 Bv = make_double2(fma(ci.x, hn.x, ci.y * hn.y), fma(ci.x, hn.y, -ci.y * hn.x));
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      double2 Ap, Bp;
+      Ap.x = __shfl_up_sync(0xffffffffu, A.x, o);
+      Ap.y = __shfl_up_sync(0xffffffffu, A.y, o);
+      Bp.x = __shfl_up_sync(0xffffffffu, Bv.x, o);
+      Bp.y = __shfl_up_sync(0xffffffffu, Bv.y, o);
+      if (lane >= o) {
+        Bv = make_double2(fma(A.x, Bp.x, fma(-A.y, Bp.y, Bv.x)), fma(A.x, Bp.y, fma(A.y, Bp.x, Bv.y)));
+        A = make_double2(fma(A.x, Ap.x, -A.y * Ap.y), fma(A.x, Ap.y, A.y * Ap.x));
+      }
+    }
+    const double2 tn = make_double2(fma(A.x, t.x, fma(-A.y, t.y, Bv.x)), fma(A.x, t.y, fma(A.y, t.x, Bv.y)));
+    double2 ti;   // t_i: the previous lane's t_{i+1}
+    ti.x = __shfl_up_sync(0xffffffffu, tn.x, 1);
+    ti.y = __shfl_up_sync(0xffffffffu, tn.y, 1);
+    if (lane == 0) ti = t;
+    if (in)
+      col[i] = make_double2(fma(ci.x, ti.x, fma(-ci.y, ti.y, fma(si.x, hn.x, -si.y * hn.y))),
+                            fma(ci.x, ti.y, fma(ci.y, ti.x, fma(si.x, hn.y, si.y * hn.x))));
+    t.x = __shfl_sync(0xffffffffu, tn.x, 31);
+    t.y = __shfl_sync(0xffffffffu, tn.y, 31);
   }
-  __syncwarp();
+  const double d2 = fma(t.x, t.x, fma(t.y, t.y, h_next * h_next));
+  double2 cc = make_double2(1.0, 0.0);
+  double ss = 0.0, den = 0.0;
+  if (d2 > 0.0) {
+    const double inv = rsqrt(d2);
+    den = d2 * inv;
+    cc = make_double2(t.x * inv, -t.y * inv);
+    ss = h_next * inv;
+  } else if (d2 != 0.0) {   // NaN: passed on, the problem stops below
+    den = d2;
+    cc = make_double2(d2, d2);
+    ss = d2;
+  }
+  const double2 gn = make_double2(-ss * gk.x, -ss * gk.y);
   if (lane == 0) {
-    double2* gg = g + b * pstride;
-    double2 hi = col_s[0];
-    for (int i = 0; i < k; ++i) {
-      const double2 hj = col_s[i + 1];
-      const double2 ci = c_s[i], si = s_s[i];
-      col_s[i] = make_double2(ci.x * hi.x - ci.y * hi.y + si.x * hj.x - si.y * hj.y,
-                              ci.x * hi.y + ci.y * hi.x + si.x * hj.y + si.y * hj.x);
-      hi = make_double2(-(si.x * hi.x + si.y * hi.y) + (ci.x * hj.x + ci.y * hj.y),
-                        -(si.x * hi.y - si.y * hi.x) + (ci.x * hj.y - ci.y * hj.x));
-    }
-    const double2 a = hi, bb = col_s[k + 1];
-    const double den = sqrt(a.x * a.x + a.y * a.y + bb.x * bb.x + bb.y * bb.y);
-    double2 cc, ss;
-    if (den == 0.0) {
-      cc = make_double2(1.0, 0.0);
-      ss = make_double2(0.0, 0.0);
-    } else {
-      const double inv = 1.0 / den;
-      cc = make_double2(a.x * inv, -a.y * inv);
-      ss = make_double2(bb.x * inv, -bb.y * inv);
-    }
     c[k] = cc;
-    s[k] = ss;
-    col_s[k] = make_double2(den, 0.0);
-    col_s[k + 1] = make_double2(0.0, 0.0);
-    const double2 gk = gg[k];
-    gg[k + 1] = make_double2(-(ss.x * gk.x + ss.y * gk.y), -(ss.x * gk.y - ss.y * gk.x));
-    gg[k] = make_double2(cc.x * gk.x - cc.y * gk.y, cc.x * gk.y + cc.y * gk.x);
+    s[k] = make_double2(ss, 0.0);
+    col[k] = make_double2(den, 0.0);
+    col[k + 1] = make_double2(0.0, 0.0);
+    gg[k + 1] = gn;
+    gg[k] = make_double2(fma(cc.x, gk.x, -cc.y * gk.y), fma(cc.x, gk.y, cc.y * gk.x));
     kused[b] = k + 1;
-    const double res = sqrt(gg[k + 1].x * gg[k + 1].x + gg[k + 1].y * gg[k + 1].y);
-    if (!(res > target[b]) || bb.x == 0.0 || !isfinite(res)) active[b] = 0;
+    const double res2 = fma(gn.x, gn.x, gn.y * gn.y);
+    if (!(res2 > tg * tg) || h_next == 0.0 || !isfinite(res2)) active[b] = 0;
   }
-  __syncwarp();
-  for (int i = lane; i <= k + 1; i += 32) col[i] = col_s[i];
 }
 
 // Arguments of the per-problem tail work done by the last block of a launch.
@@ -283,244 +320,270 @@ struct KrylovTail {
   int k, pstride, m, first;
 };
 
-// Multi-dot: partial[b][i][c] = sum over chunk c of conj(V_i) . w for every i < nv.
-// One block per (chunk of 256*E elements, problem): w stays in registers, each V_i
-// chunk is read once, warps drop their partial sums in shared memory and the
-// block adds them at the end (no block barrier per coefficient).
-constexpr int kMdE = 8;
-template <typename T, typename VB = T>
-__global__ void __launch_bounds__(256) multidot_kernel(const VB* __restrict__ V, const T* __restrict__ w,
-                                                       double2* __restrict__ partial, const int* __restrict__ active,
-                                                       long long N, int nv, int mp1, int pstride, int nchunk,
-                                                       KrylovTail tl) {
-  extern __shared__ double red[];  // [nv][8 warps][4 doubles]
+// Sums over a warp of 8 values per lane: 9 shuffles and additions instead of 40 (each step exchanges half of
+// the values still held).  Lane l returns the sum of v[l >> 2].
+template <typename R>
+__device__ __forceinline__ R warp_sum8(R (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 4; h >= 1; h /= 2) {
+    const bool up = lane & (4 * h);
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const R give = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * h);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
+}
+
+// Multi-dot: partial[b][i][c] = sum over chunk c of conj(V_i) . w for every i < nv; the last block of problem b
+// reduces the partials into the Hessenberg column.  The warps drop their sums of four vectors (real and
+// imaginary parts: 8 values) in shared memory and the block adds them at the end.
+//
+// FP32 vectors, basis of VB (FP16 or FP32): one block per (2,048 elements, problem); w stays in
+// registers, four basis vectors per pass with their loads in flight together (16 bytes each).  Bound by HBM.
+// 16 problems of 245,760 unknowns, 20 vectors (346 MB): 82 -> 75 us against 8-byte loads and 40 shuffles per sum.
+constexpr int kMdChunk = 2048;
+template <typename VB>
+__global__ void __launch_bounds__(256, 3) multidot32_kernel(const VB* __restrict__ V, const float2* __restrict__ w,
+                                                            double2* __restrict__ partial,
+                                                            const int* __restrict__ active, long long N, int nv,
+                                                            int mp1, int pstride, int nchunk, KrylovTail tl) {
+  extern __shared__ float red32[];  // [nv rounded up to 4][2][8 warps]
   const int b = blockIdx.y, c = blockIdx.x;
   if (!active[b]) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if constexpr (std::is_same<T, float2>::value) {
-    // two complex values per 16-byte load (N is even for the mixed form)
-    constexpr int E4 = kMdE / 2;
-    const long long base4 = (long long)c * 256 * E4 + threadIdx.x, N4 = N / 2;
-    const float4* wb = reinterpret_cast<const float4*>(w + (long long)b * N);
-    float4 wv[E4];
+  const long long N4 = N / 4, n0 = (long long)c * (kMdChunk / 4) + threadIdx.x, n1 = n0 + 256;
+  const bool in0 = n0 < N4, in1 = n1 < N4;
+  Quad<float2> w0, w1;
+  w0.zero();
+  w1.zero();
+  if (in0) w0.load(w + (long long)b * N, n0);
+  if (in1) w1.load(w + (long long)b * N, n1);
+  const VB* v = V + (long long)b * mp1 * N;
+  for (int i = 0; i < nv; i += 4) {
+    Quad<VB> a0[4], a1[4];
 #pragma unroll
-    for (int j = 0; j < E4; ++j) {
-      const long long n = base4 + (long long)j * 256;
-      wv[j] = n < N4 ? wb[n] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < 4; ++u) {
+      a0[u].zero();
+      a1[u].zero();
+      if (i + u < nv && in0) a0[u].load(v + (long long)(i + u) * N, n0);
+      if (i + u < nv && in1) a1[u].load(v + (long long)(i + u) * N, n1);
     }
-    int i = 0;
-    // four basis vectors per pass: 16 loads in flight per thread between two reductions
-    for (; i + 3 < nv; i += 4) {
-      const VB* v0 = V + ((long long)b * mp1 + i) * N;
-      float4 a[4][E4];
+    float s[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < 4; ++u) {
+      AccF32 t;
 #pragma unroll
-        for (int j = 0; j < E4; ++j) {
-          const long long n = base4 + (long long)j * 256;
-          a[u][j] = n < N4 ? ld_pair(v0 + (long long)u * N, n) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      AccF32 s4[4];
+      for (int q = 0; q < 4; ++q) t.add_cdot(a0[u].get(q), w0.get(q));
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-#pragma unroll
-        for (int j = 0; j < E4; ++j) s4[u].add_cdot4(a[u][j], wv[j]);
-        s4[u].warp_reduce();
-      }
-      if (lane == 0)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) s4[u].stage(red + ((i + u) * 8 + warp) * 4);
+      for (int q = 0; q < 4; ++q) t.add_cdot(a1[u].get(q), w1.get(q));
+      s[2 * u] = t.re;
+      s[2 * u + 1] = t.im;
     }
-    for (; i + 1 < nv; i += 2) {
-      const VB* v0 = V + ((long long)b * mp1 + i) * N;
-      const VB* v1 = v0 + N;
-      float4 a0[E4], a1[E4];
-#pragma unroll
-      for (int j = 0; j < E4; ++j) {
-        const long long n = base4 + (long long)j * 256;
-        a0[j] = n < N4 ? ld_pair(v0, n) : make_float4(0.f, 0.f, 0.f, 0.f);
-        a1[j] = n < N4 ? ld_pair(v1, n) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      AccF32 s0, s1;
-#pragma unroll
-      for (int j = 0; j < E4; ++j) {
-        s0.add_cdot4(a0[j], wv[j]);
-        s1.add_cdot4(a1[j], wv[j]);
-      }
-      s0.warp_reduce();
-      s1.warp_reduce();
-      if (lane == 0) {
-        s0.stage(red + (i * 8 + warp) * 4);
-        s1.stage(red + ((i + 1) * 8 + warp) * 4);
-      }
-    }
-    if (i < nv) {
-      const VB* v0 = V + ((long long)b * mp1 + i) * N;
-      AccF32 s0;
-#pragma unroll
-      for (int j = 0; j < E4; ++j) {
-        const long long n = base4 + (long long)j * 256;
-        if (n < N4) s0.add_cdot4(ld_pair(v0, n), wv[j]);
-      }
-      s0.warp_reduce();
-      if (lane == 0) s0.stage(red + (i * 8 + warp) * 4);
-    }
-  } else {
-    const long long base = (long long)c * 256 * kMdE + threadIdx.x;
-    const T* wb = w + (long long)b * N;
-    T wv[kMdE];
-#pragma unroll
-    for (int j = 0; j < kMdE; ++j) {
-      const long long n = base + (long long)j * 256;
-      if (n < N) wv[j] = wb[n];
-      else { wv[j].x = 0; wv[j].y = 0; }
-    }
-    for (int i = 0; i < nv; ++i) {
-      const VB* v = V + ((long long)b * mp1 + i) * N;
-      typename AccFor<T>::type a;
-#pragma unroll
-      for (int j = 0; j < kMdE; ++j) {
-        const long long n = base + (long long)j * 256;
-        if (n < N) a.add_cdot(v[n], wv[j]);
-      }
-      a.warp_reduce();
-      if (lane == 0) a.stage(red + (i * 8 + warp) * 4);
-    }
+    const float r = warp_sum8(s);
+    if ((lane & 3) == 0) red32[(2 * i + (lane >> 2)) * 8 + warp] = r;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nv; i += blockDim.x)
-    partial[((long long)b * pstride + i) * nchunk + c] = AccFor<T>::type::combine(red + i * 8 * 4, 8);
-  // the last chunk of problem b reduces the partials into the Hessenberg column
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+    double2 r = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      r.x += (double)red32[16 * i + q];
+      r.y += (double)red32[16 * i + 8 + q];
+    }
+    partial[((long long)b * pstride + i) * nchunk + c] = r;
+  }
   if (!last_block_of_problem(tl.md_count, b)) return;
   dot_reduce_block(partial, tl.hcol, tl.hcol32, tl.H, b, nv, tl.k, pstride, tl.m, nchunk, tl.first);
   if (threadIdx.x == 0) tl.md_count[b] = 0;
 }
 
+// FP64: one block per (256 E elements, problem, four vectors).  Bound by the FP64 pipe (4 FMAs per element and
+// vector), so the vectors are split over blocks: the 608 pipe quarters fill evenly at any nv, and a small
+// problem is not one block that takes its vectors one after another.  E (Problem::md_e) is the largest of
+// 8, 4, 2, 1 that still gives a few blocks per SM.
+// 2 problems of 245,760 unknowns, 25 vectors: 214 -> 111 us against whole problems per block and a multiply, FMA
+// and add per product (0.81 TFLOP/s); 1,152 unknowns: 109 -> 13 us.
+template <int E>
+__global__ void __launch_bounds__(256) multidot64_kernel(const double2* __restrict__ V, const double2* __restrict__ w,
+                                                         double2* __restrict__ partial,
+                                                         const int* __restrict__ active, long long N, int nv, int mp1,
+                                                         int pstride, int nchunk, KrylovTail tl) {
+  __shared__ double red[8][8];
+  const int b = blockIdx.y, c = blockIdx.x, i0 = 4 * blockIdx.z;
+  if (!active[b]) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long base = (long long)c * 256 * E + threadIdx.x;
+  const double2* wb = w + (long long)b * N;
+  const double2* v = V + ((long long)b * mp1 + i0) * N;
+  Acc64 acc[4];
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    const long long n = base + (long long)j * 256;
+    if (n < N) {
+      const double2 x = __ldg(wb + n);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i0 + u < nv) acc[u].add_cdot(__ldg(v + (long long)u * N + n), x);
+    }
+  }
+  double s[8];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    s[2 * u] = acc[u].v.x;
+    s[2 * u + 1] = acc[u].v.y;
+  }
+  const double r = warp_sum8(s);
+  if ((lane & 3) == 0) red[lane >> 2][warp] = r;
+  __syncthreads();
+  if (threadIdx.x < 4 && i0 + (int)threadIdx.x < nv) {
+    double2 t = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      t.x += red[2 * threadIdx.x][q];
+      t.y += red[2 * threadIdx.x + 1][q];
+    }
+    partial[((long long)b * pstride + i0 + threadIdx.x) * nchunk + c] = t;
+  }
+  if (!last_block_of_problem(tl.md_count, b)) return;
+  dot_reduce_block(partial, tl.hcol, tl.hcol32, tl.H, b, nv, tl.k, pstride, tl.m, nchunk, tl.first);
+  if (threadIdx.x == 0) tl.md_count[b] = 0;
+}
 
+// What follows the update w -= sum_i V_i hcol_i: nrm_partial[b][block] = sum |w|^2 (a: the thread's share), and
+// the last block of problem b finishes the step.  MODE 1 runs the DGKS test (reorth[b]) and, when no second
+// pass is needed, MODE 2's work: |w|, H[k+1][k], inverse norm, Givens step.
+template <int MODE, typename Acc>
+__device__ void update_tail(Acc& a, const int b, double* __restrict__ nrm_partial, int nv, int pstride, int nblk,
+                            const KrylovTail& tl) {
+  __shared__ double wsum[8 * 4];
+  a.warp_reduce();
+  if ((threadIdx.x & 31) == 0) a.stage(wsum + (threadIdx.x >> 5) * 4);
+  __syncthreads();
+  if (threadIdx.x == 0)
+    nrm_partial[(long long)b * nblk + blockIdx.x] = Acc::combine(wsum, blockDim.x >> 5).x;
+  if (!last_block_of_problem(tl.gs_count, b)) return;
+  // the whole last block adds the partial norms (independent loads), warp 0 finishes the step
+  double w2p = 0;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < nblk; c += blockDim.x) w2p += __ldcg(&nrm_partial[(long long)b * nblk + c]);
+  const double w2b = block_sum1(w2p);
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const double w2 = __shfl_sync(0xffffffffu, w2b, 0);
+    bool finish = true;
+    if (MODE == 1) {
+      double h2 = 0;
+      for (int i = lane; i < nv; i += 32) {
+        const double2 h = tl.hcol[(long long)b * pstride + i];
+        h2 += h.x * h.x + h.y * h.y;
+      }
+      h2 = warp_sum(h2);
+      const int re = w2 < tl.eta2 * (w2 + h2) ? 1 : 0;
+      if (lane == 0) tl.reorth[b] = re;
+      finish = !re;
+    }
+    if (finish) {
+      const double inv = w2 > 0 ? rsqrt(w2) : 0.0;
+      const double v = w2 > 0 ? w2 * inv : w2;   // NaN passes on
+      if (lane == 0) {
+        tl.nrm[b] = v;
+        if (tl.inv64) tl.inv64[b] = inv;
+        if (tl.inv32) tl.inv32[b] = (float)inv;
+      }
+      givens_warp(tl.H, tl.cs, tl.sn, tl.g, tl.active, tl.kused, tl.target, b, tl.k, pstride, tl.m, v);
+    }
+  }
+  if (threadIdx.x == 0) tl.gs_count[b] = 0;
+}
 
-// w -= sum_i V_i hcol_i.  FP64 vectors: grid (ceil(N/256), B), one complex value per
-// thread; FP32 vectors: grid (ceil(N/(256 kGsPairs)), B), 128 threads of kGsPairs 16-byte
-// accesses (two complex values each); the coefficients are staged in shared memory.
-// MODE 0: update only.  MODE >= 1: also nrm_partial[b][block] = sum |w|^2, and the last
-// block of problem b finishes the step: MODE 1 runs the DGKS test (reorth[b]) and, when
-// no second pass is needed, MODE 2's work: |w|, H[k+1][k], inverse norm, Givens step.
-constexpr int kGsPairs = 2;
-template <typename T, int MODE, typename VB = T>
-__global__ void __launch_bounds__(256) gs_update_kernel(const VB* __restrict__ V, T* __restrict__ w,
-                                                        const T* __restrict__ hcol, const int* __restrict__ mask,
-                                                        double* __restrict__ nrm_partial, long long N, int nv, int mp1,
-                                                        int pstride, int nblk, KrylovTail tl) {
+// w -= sum_i V_i hcol_i, FP32 vectors: 128 threads of four consecutive complex values, the loads of eight
+// basis vectors in flight per thread (16 bytes each of an FP16 basis).  Bound by HBM.  The problems are taken
+// in the reverse of the multi-dot's order: the basis vectors that one of the two reads last are the first of
+// the other, so the part that fits the L2 (129 MB) is not read from memory again.
+// 16 problems of 245,760 unknowns, 20 vectors: 105 -> 65 us (5.5 TB/s) against 8-byte loads in batches of four.
+constexpr int kUp32Threads = 128, kUp32Elems = 4 * kUp32Threads;
+template <int MODE, typename VB>
+__global__ void __launch_bounds__(kUp32Threads, 8) gs_update32_kernel(const VB* __restrict__ V,
+                                                                      float2* __restrict__ w,
+                                                                      const float2* __restrict__ hcol,
+                                                                      const int* __restrict__ mask,
+                                                                      double* __restrict__ nrm_partial, long long N,
+                                                                      int nv, int mp1, int pstride, int nblk,
+                                                                      KrylovTail tl) {
+  const int b = gridDim.y - 1 - blockIdx.y;
+  if (!mask[b]) return;
+  __shared__ float2 hs[kMaxRestart + 8];
+  for (int i = threadIdx.x; i < ((nv + 7) & ~7); i += kUp32Threads)
+    hs[i] = i < nv ? hcol[b * pstride + i] : make_float2(0.f, 0.f);
+  const long long N4 = N / 4, n4 = (long long)blockIdx.x * kUp32Threads + threadIdx.x;
+  const bool in = n4 < N4;
+  float4* wp = reinterpret_cast<float4*>(w + (long long)b * N) + 2 * n4;
+  float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
+  if (in) {
+    x0 = wp[0];
+    x1 = wp[1];
+  }
+  float2 acc[4] = {make_float2(x0.x, x0.y), make_float2(x0.z, x0.w), make_float2(x1.x, x1.y),
+                   make_float2(x1.z, x1.w)};
+  const VB* v = V + (long long)b * mp1 * N;
+  __syncthreads();
+  constexpr int U = sizeof(VB) == 4 ? 8 : 4;
+  for (int i0 = 0; i0 < nv; i0 += U) {
+    Quad<VB> q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      q[u].zero();
+      if (in && i0 + u < nv) q[u].load(v + (long long)(i0 + u) * N, n4);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float2 h = hs[i0 + u];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) cms(acc[r], q[u].get(r), h);
+    }
+  }
+  AccF32 a;
+  if (in) {
+    wp[0] = make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
+    wp[1] = make_float4(acc[2].x, acc[2].y, acc[3].x, acc[3].y);
+    if (MODE)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) a.add_norm(acc[r]);
+  }
+  if constexpr (MODE >= 1) update_tail<MODE>(a, b, nrm_partial, nv, pstride, nblk, tl);
+}
+
+// The same in FP64: one complex value per thread, bound by the FP64 pipe (4 FMAs per element and vector).
+// Explicit FMAs: w -= v h had compiled to a multiply, an FMA and a subtraction per component.  2 problems of
+// 245,760 unknowns, 25 vectors: 156 -> 96 us (0.94 TFLOP/s).
+template <int MODE>
+__global__ void __launch_bounds__(256) gs_update64_kernel(const double2* __restrict__ V, double2* __restrict__ w,
+                                                          const double2* __restrict__ hcol,
+                                                          const int* __restrict__ mask,
+                                                          double* __restrict__ nrm_partial, long long N, int nv,
+                                                          int mp1, int pstride, int nblk, KrylovTail tl) {
   const int b = blockIdx.y;
   if (!mask[b]) return;
-  __shared__ T hs[kMaxRestart + 1];
+  __shared__ double2 hs[kMaxRestart + 1];
   for (int i = threadIdx.x; i < nv; i += blockDim.x) hs[i] = hcol[b * pstride + i];
+  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long t = (long long)b * N + n;
+  double2 acc = n < N ? w[t] : make_double2(0.0, 0.0);
   __syncthreads();
-  typename AccFor<T>::type a;
-  if constexpr (std::is_same<T, float2>::value) {
-    // kGsPairs float4 (two complex values each) per thread, 128 apart: the grid of a handle
-    // fits one wave of resident blocks and every basis pass has kGsPairs loads per thread
-    const long long N4 = N / 2;
-    const long long n40 = (long long)blockIdx.x * (128 * kGsPairs) + threadIdx.x;
-    float4* wp = reinterpret_cast<float4*>(w + (long long)b * N);
-    float4 acc[kGsPairs];
-#pragma unroll
-    for (int g = 0; g < kGsPairs; ++g) {
-      const long long n4 = n40 + 128 * g;
-      acc[g] = n4 < N4 ? wp[n4] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    const VB* v = V + (long long)b * mp1 * N;
-    // the loads of four basis vectors are issued before their updates are applied
-    constexpr int U = 4;
-    for (int i0 = 0; i0 < nv; i0 += U) {
-      float4 x[U][kGsPairs];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int g = 0; g < kGsPairs; ++g) {
-          const long long n4 = n40 + 128 * g;
-          x[u][g] = (i0 + u < nv && n4 < N4) ? ld_pair(v, (long long)(i0 + u) * N4 + n4)
-                                             : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        // past nv the coefficient is zero and the (zero) loads change nothing
-        const float2 h = i0 + u < nv ? hs[i0 + u] : make_float2(0.f, 0.f);
-#pragma unroll
-        for (int g = 0; g < kGsPairs; ++g) {
-          acc[g].x = fmaf(-x[u][g].x, h.x, fmaf(x[u][g].y, h.y, acc[g].x));
-          acc[g].y = fmaf(-x[u][g].x, h.y, fmaf(-x[u][g].y, h.x, acc[g].y));
-          acc[g].z = fmaf(-x[u][g].z, h.x, fmaf(x[u][g].w, h.y, acc[g].z));
-          acc[g].w = fmaf(-x[u][g].z, h.y, fmaf(-x[u][g].w, h.x, acc[g].w));
-        }
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < kGsPairs; ++g) {
-      const long long n4 = n40 + 128 * g;
-      if (n4 < N4) {
-        wp[n4] = acc[g];
-        if (MODE) {
-          a.add_norm(make_float2(acc[g].x, acc[g].y));
-          a.add_norm(make_float2(acc[g].z, acc[g].w));
-        }
-      }
-    }
-  } else {
-    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n < N) {
-      const long long t = (long long)b * N + n;
-      T acc = w[t];
-      const VB* v = V + (long long)b * mp1 * N + n;
-#pragma unroll 4
-      for (int i = 0; i < nv; ++i) cms(acc, v[(long long)i * N], hs[i]);
-      w[t] = acc;
-      if (MODE) a.add_norm(acc);
-    }
-  }
-  if constexpr (MODE >= 1) {
-    __shared__ double wsum[8 * 4];
-    a.warp_reduce();
-    if ((threadIdx.x & 31) == 0) a.stage(wsum + (threadIdx.x >> 5) * 4);
-    __syncthreads();
-    if (threadIdx.x == 0)
-      nrm_partial[(long long)b * nblk + blockIdx.x] = AccFor<T>::type::combine(wsum, blockDim.x >> 5).x;
-    if (!last_block_of_problem(tl.gs_count, b)) return;
-    // the whole last block adds the partial norms (independent loads), warp 0 finishes the step
-    double w2p = 0;
+  Acc64 a;
+  if (n < N) {
+    const double2* v = V + (long long)b * mp1 * N + n;
 #pragma unroll 8
-    for (int c = threadIdx.x; c < nblk; c += blockDim.x) w2p += __ldcg(&nrm_partial[(long long)b * nblk + c]);
-    const double w2b = block_sum1(w2p);
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
-      const double w2 = w2b;
-      bool finish = true;
-      if (MODE == 1) {
-        double h2 = 0;
-        for (int i = lane; i < nv; i += 32) {
-          const double2 h = tl.hcol[(long long)b * pstride + i];
-          h2 += h.x * h.x + h.y * h.y;
-        }
-        h2 = warp_sum(h2);
-        const int re = w2 < tl.eta2 * (w2 + h2) ? 1 : 0;
-        if (lane == 0) tl.reorth[b] = re;
-        finish = !re;
-      }
-      if (finish) {
-        __shared__ double2 col_s[kMaxRestart + 1], c_s[kMaxRestart], s_s[kMaxRestart];
-        if (lane == 0) {
-          const double v = sqrt(w2);
-          tl.nrm[b] = v;
-          if (tl.inv64) tl.inv64[b] = v > 0 ? 1.0 / v : 0.0;
-          if (tl.inv32) tl.inv32[b] = v > 0 ? (float)(1.0 / v) : 0.f;
-          tl.H[(long long)b * pstride * tl.m + (long long)tl.k * pstride + tl.k + 1] = make_double2(v, 0.0);
-        }
-        __syncwarp();
-        givens_warp(tl.H, tl.cs, tl.sn, tl.g, tl.active, tl.kused, tl.target, b, tl.k, pstride, tl.m, col_s, c_s,
-                    s_s);
-      }
-    }
-    if (threadIdx.x == 0) tl.gs_count[b] = 0;
+    for (int i = 0; i < nv; ++i) cms(acc, __ldg(v + (long long)i * N), hs[i]);
+    w[t] = acc;
+    if (MODE) a.add_norm(acc);
   }
+  if constexpr (MODE >= 1) update_tail<MODE>(a, b, nrm_partial, nv, pstride, nblk, tl);
 }
 
 template <typename T>
@@ -704,9 +767,6 @@ inline unsigned blocks_for(long long n) { return (unsigned)((n + 255) / 256); }
 // One Arnoldi step k on basis V (stride (m+1) N per problem): z = M^-1 V_k,
 // w = A z, CGS2 against V_0..V_k, V_{k+1} = w / |w|, Givens.  `prec` and `apply`
 // are the operator pair of the basis precision.
-template <typename T> T* coef_col(Problem& P);
-template <> double2* coef_col<double2>(Problem& P) { return P.hcol; }
-template <> float2* coef_col<float2>(Problem& P) { return P.mx.hcol; }
 template <typename T> float2* coef_col32(Problem& P);
 template <> float2* coef_col32<double2>(Problem&) { return nullptr; }
 template <> float2* coef_col32<float2>(Problem& P) { return P.mx.hcol; }
@@ -732,8 +792,8 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, Prec prec, Apply apply) 
   WG_CK(apply());
   const int nv = k + 1;
   const double vec = (double)N * B * sizeof(T), vecb = (double)N * B * sizeof(VB);
-  // the FP32 update covers 256 kGsPairs complex values per block of 128 threads
-  const long long per_blk = sizeof(T) == sizeof(float2) ? 256LL * kGsPairs : 256LL;
+  constexpr bool f32 = std::is_same<T, float2>::value;
+  const long long per_blk = f32 ? kUp32Elems : 256;
   const dim3 gu((unsigned)((N + per_blk - 1) / per_blk), B);
   const int nblk = (int)gu.x;
   // classical Gram-Schmidt; the second pass runs for the problems that fail the DGKS
@@ -745,27 +805,32 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, Prec prec, Apply apply) 
   KrylovTail tl{P.md_count, P.gs_count, P.partial, P.hcol, coef_col32<T>(P), P.H, P.cs, P.sn, P.g, P.active,
                 P.kused, P.reorth, P.target, P.nrm, sizeof(T) == sizeof(float2) ? nullptr : P.inv64,
                 sizeof(T) == sizeof(float2) ? P.mx.inv : nullptr, eta * eta, k, ps, mm, 1};
-  const unsigned gthreads = sizeof(T) == sizeof(float2) ? 128 : 256;
   // the DGKS flags are written only for problems that take part in the first pass
   if (passes == 2 && eta < 1) WG_CK(cudaMemsetAsync(P.reorth, 0, sizeof(int) * B, P.stream));
   for (int pass = 0; pass < passes; ++pass) {
     const int* mask = (pass == 0 || eta >= 1) ? P.active : P.reorth;
     tl.first = pass == 0;
     cudaEvent_t ev = prof_begin(P, PROF_MULTIDOT, 1, nv * vecb + vec, 8.0 * nv * N * B, mask);
-    multidot_kernel<T, VB><<<dim3(P.nchunk, B), 256, sizeof(double) * 32 * nv, P.stream>>>(V, w, P.partial, mask,
-                                                                                          N, nv, mp1, ps, P.nchunk,
-                                                                                          tl);
+    if constexpr (f32) {
+      multidot32_kernel<VB><<<dim3(P.nchunk, B), 256, sizeof(float) * 16 * ((nv + 3) & ~3), P.stream>>>(
+          V, w, P.partial, mask, N, nv, mp1, ps, P.nchunk, tl);
+    } else {
+      const dim3 gm(P.md_chunk, B, (nv + 3) / 4);
+      auto md = P.md_e == 8 ? multidot64_kernel<8> : P.md_e == 4 ? multidot64_kernel<4>
+                                                   : P.md_e == 2 ? multidot64_kernel<2> : multidot64_kernel<1>;
+      md<<<gm, 256, 0, P.stream>>>(V, w, P.partial, mask, N, nv, mp1, ps, P.md_chunk, tl);
+    }
     prof_end(P, PROF_MULTIDOT, ev);
     ev = prof_begin(P, PROF_GSUPDATE, 1, nv * vecb + 2 * vec, 8.0 * nv * N * B, mask);
-    if (pass == passes - 1)
-      gs_update_kernel<T, 2, VB><<<gu, gthreads, 0, P.stream>>>(V, w, coef_col<T>(P), mask, P.nrm_partial, N, nv,
-                                                                 mp1, ps, nblk, tl);
-    else if (eta < 1)
-      gs_update_kernel<T, 1, VB><<<gu, gthreads, 0, P.stream>>>(V, w, coef_col<T>(P), mask, P.nrm_partial, N, nv,
-                                                                 mp1, ps, nblk, tl);
-    else
-      gs_update_kernel<T, 0, VB><<<gu, gthreads, 0, P.stream>>>(V, w, coef_col<T>(P), mask, P.nrm_partial, N, nv,
-                                                                 mp1, ps, nblk, tl);
+    const int mode = pass == passes - 1 ? 2 : (eta < 1 ? 1 : 0);
+    if constexpr (f32) {
+      auto up = mode == 2 ? gs_update32_kernel<2, VB> : mode == 1 ? gs_update32_kernel<1, VB>
+                                                                  : gs_update32_kernel<0, VB>;
+      up<<<gu, kUp32Threads, 0, P.stream>>>(V, w, P.mx.hcol, mask, P.nrm_partial, N, nv, mp1, ps, nblk, tl);
+    } else {
+      auto up = mode == 2 ? gs_update64_kernel<2> : mode == 1 ? gs_update64_kernel<1> : gs_update64_kernel<0>;
+      up<<<gu, 256, 0, P.stream>>>(V, w, P.hcol, mask, P.nrm_partial, N, nv, mp1, ps, nblk, tl);
+    }
     prof_end(P, PROF_GSUPDATE, ev);
   }
   // V_{k+1} = w / |w| is written by the next step's preconditioner

@@ -285,6 +285,7 @@ struct Problem {
   int* kused = nullptr;          // [B] iterations used in this cycle
   int* any_active = nullptr;     // [1]
   int nchunk = 0;  // 2048-element chunks of one problem vector (multi-dot partials)
+  int md_e = 8, md_chunk = 0;   // FP64 multi-dot: elements per thread, chunks of 256 md_e elements per vector
   int nblk = 0;    // 256-element blocks of one problem vector (norm partials)
   // host mirrors
   std::vector<double> h_nrm;

@@ -1,0 +1,68 @@
+"""Transform and Gram-Schmidt kernels of the 1D path at the sizes where their tiles end."""
+import numpy as np
+import pytest
+
+from conftest import small_rtd
+from oracle import dg1d, krylov
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_el,nk,nxi,order", [
+    (2, 8, 8, 1), (2, 15, 15, 1), (3, 16, 17, 2), (3, 17, 18, 1), (5, 31, 40, 3), (2, 63, 63, 2), (3, 64, 66, 1),
+    (2, 65, 65, 3), (3, 127, 129, 1), (2, 130, 131, 2)])
+def test_paired_transforms(built_lib, n_el, nk, nxi, order):
+    """Phi rho and the operator (both transforms) with odd and even Nk and N_xi around the tiles of 8, 16 and 32
+    rows and the chunks of 32 pairs.  A sum of nk terms of size |x| / sqrt(L) carries at most nk eps of their
+    absolute sum, and the phases k xi (up to pi nk / 2) another pi nk / 2 eps."""
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order, n_xi=nxi)
+    p = dg1d.init_params(mat, efl, efr, E, m)
+    rng = np.random.default_rng(nk)
+    with Problem1D(n_el=n_el, n_local=order + 1, nk=nk, n_xi=nxi, l_xi=spec.l_xi_m) as P:
+        P.set_potential(0, mat["x"], E, m, spec.m_rel, spec.temp_k, efl, efr)
+        x = rng.normal(size=P.N) + 1j * rng.normal(size=P.N)
+        P.set_rho(0, x)
+        X = x.reshape(-1, nk)
+        bound = 2.3e-16 * (1 + np.pi / 2) * nk * np.abs(X).sum(1) / np.sqrt(spec.l_xi_m)
+        assert np.all(np.abs(P.rho_xi(0) - X @ p["phi"].T) <= bound[:, None])
+        want = krylov.Operator1D(mat, p, E).apply(x)
+        assert np.linalg.norm(P.apply(x) - want) <= 1e-12 * np.linalg.norm(want)
+
+
+def _residual(P, rho):
+    b = P.rhs()
+    return np.linalg.norm(b - P.apply(rho)) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("reorth", [0.0, 1.0, -1.0])
+@pytest.mark.parametrize("n_el,nk,order", [(5, 17, 1), (40, 65, 2), (100, 96, 3), (140, 96, 3), (272, 96, 3)])
+def test_gram_schmidt_fp64(built_lib, n_el, nk, order, reorth):
+    """The FP64 Arnoldi at sizes below one block, with 1, 2, 4 and 8 elements per thread of the multi-dot, with
+    one, a tested and two Gram-Schmidt passes: the solution meets the tolerance by its own residual.  The
+    residual of the solver and the one formed here differ by the operator's rounding (1e-13 of |b| allowed)."""
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order, bias=0.05)
+    with Problem1D(n_el=n_el, n_local=order + 1, nk=nk, l_xi=spec.l_xi_m, reorth=reorth, restart=37) as P:
+        P.set_potential(0, mat["x"], E, m, spec.m_rel, spec.temp_k, efl, efr)
+        st, info = P.solve(tol=1e-10, maxit=60)
+        assert st == 0 and _residual(P, P.rho(0)) <= 1.001e-10
+
+
+@pytest.mark.parametrize("basis32", [False, True])
+@pytest.mark.parametrize("inner_reorth", [0.0, 0.7, 1.0])
+@pytest.mark.parametrize("n_el,nk,order,batch", [(5, 36, 2, 1), (2, 32, 1, 3), (16, 64, 1, 2), (31, 68, 3, 3)])
+def test_gram_schmidt_mixed(built_lib, n_el, nk, order, batch, inner_reorth, basis32):
+    """The inner FP32 Arnoldi (FP16 and FP32 basis) around its blocks of 512 and 2,048 elements, with one, a tested
+    and two passes: every problem of the batch meets the tolerance by its own FP64 residual."""
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order, bias=0.05)
+    with Problem1D(n_el=n_el, n_local=order + 1, nk=nk, l_xi=spec.l_xi_m, batch=batch, precision="mixed",
+                   inner_reorth=inner_reorth, inner_basis_fp32=basis32, inner_restart=29) as P:
+        for b in range(batch):
+            P.set_potential(b, mat["x"], E * (1 + 0.02 * b), m, spec.m_rel, spec.temp_k, efl, efr)
+        st, info = P.solve(tol=1e-10, maxit=60)
+        rho = np.concatenate([P.rho(b) for b in range(batch)])
+        r = (P.rhs() - P.apply(rho)).reshape(batch, -1)
+        assert st == 0
+        assert np.all(np.linalg.norm(r, axis=1) <= 1.001e-10 * np.linalg.norm(P.rhs().reshape(batch, -1), axis=1))
