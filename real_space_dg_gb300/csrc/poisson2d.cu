@@ -11,19 +11,22 @@
 //
 // Unique nodes k = ix + iy nx (x fastest, MATLAB's order), iy < nu (nu = Ny - 1 when periodic).
 // The update solves J d = -F(free) with J = A_ff (direct) or A_ff - diag(q^2 n / (kB T)) (Newton),
-// ordered by x columns: J is block tridiagonal, the column blocks D_ix (the Y stencil, a ring
-// when periodic, plus the diagonal) coupled to the neighbour columns by diagonal matrices
-// L_ix, U_ix (the X faces).  Block LU without pivoting (J is diagonally dominant; Dirichlet
-// nodes stay in as identity rows with a zero right-hand side):
-//   S_0 = D_0,  S_ix = D_ix - L_ix S_{ix-1}^-1 U_{ix-1},  g_ix = S_ix^-1 (r_ix - L_ix g_{ix-1}),
-//   d_{nx-1} = g_{nx-1},  d_ix = g_ix - S_ix^-1 U_ix d_{ix+1}.
-// Row a of S_ix needs row a of S_{ix-1}^-1 only, so one warp runs the sweep with lane a holding
-// row a in registers (NU = 4/8/12/16/24/32, padded with identity rows); the Gauss-Jordan inversion of
-// each S_ix broadcasts the pivot row by shuffles.  The inverses go to a scratch [nx][NU][NU]
-// for the backward sweep.  One warp per problem (a batch of bias points runs as a grid);
-// projection, residuals and diagnostics run in the same warp with fixed-order reductions.
+// ordered by x columns: J is block tridiagonal, the column blocks D (the Y stencil, a ring when periodic, plus
+// the diagonal) coupled to the neighbour columns by diagonal matrices L, U (the X faces).  J is diagonally dominant
+// and so are the Schur complements below, so blocks are eliminated without pivoting; Dirichlet nodes stay in as
+// identity rows with a zero right-hand side.
+//
+// Block cyclic reduction over x: level by level every second remaining column is eliminated,
+//   D_c' = D_c - L_c D_l^-1 U_l - U_c D_r^-1 L_r,  L_c' = -L_c D_l^-1 L_l,  U_c' = -U_c D_r^-1 U_r,
+//   r_c' = r_c - L_c D_l^-1 r_l - U_c D_r^-1 r_r            (l, r: the eliminated neighbours of kept column c),
+// all columns of a level at once, one block each (poisson2d_reduce_kernel), then the levels are substituted back.
+// log2(nx) + 1 dependent steps instead of a sweep over nx columns: the sweep (one warp per bias point) was
+// a chain of nx inversions, 20 us each.  Measured with a 361 x 13 periodic grid, projection and update of 16 bias points:
+// 7.4 ms with the sweep, 0.44 ms here (one point, 97 x 11: 1.9 -> 0.18 ms).
+// Every reduction over nodes has a fixed order that does not depend on the batch.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <string>
@@ -58,221 +61,397 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// (A u)_k on the unique nodes: free rows the stencil (periodic Y ring), fixed rows the identity.
-__device__ __forceinline__ double stencil(const P2Dev& P, const double* u, int ix, int iy) {
-  const int k = ix + iy * P.nx;
-  if (P.fixed[k]) return u[k];
-  double s = P.diag[k] * u[k];
-  if (ix > 0) s += P.cxm[k] * u[k - 1];
-  if (ix < P.nx - 1) s += P.cxp[k] * u[k + 1];
-  if (iy > 0 || P.periodic) s += P.cym[k] * u[(iy > 0 ? iy - 1 : P.nu - 1) * P.nx + ix];
-  if (iy < P.nu - 1 || P.periodic) s += P.cyp[k] * u[(iy < P.nu - 1 ? iy + 1 : 0) * P.nx + ix];
-  return s;
+// Sum and maximum over a block of 256 threads, fixed order; the results are valid in every thread.
+__device__ double block_sum(double v, double* s) {
+  v = warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) t += s[i];
+  return t;
+}
+__device__ double block_max(double v, double* s) {
+  v = warp_max(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = s[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) t = fmax(t, s[i]);
+  return t;
 }
 
-template <int NU>
-__global__ void __launch_bounds__(32) poisson2d_step_kernel(
-    P2Dev P, const double* __restrict__ src, int src_is_dg, const double* __restrict__ phi0,
-    const double* __restrict__ bc, int newton, double q_kt, double alpha, double* __restrict__ phi,
-    double* __restrict__ density, double* __restrict__ work, double* __restrict__ sinv_all,
-    wg_poisson2d_info* __restrict__ info) {
-  const int b = blockIdx.x, lane = threadIdx.x;
-  const int nx = P.nx, ny = P.ny, nu = P.nu, nun = nu * nx;
-  const size_t full = (size_t)nx * ny;
+// Buffers of one step (all problems): n, v, F [B][nun]; r, y, d [B][nx][NU]; the blocks of the reduction and
+// the block partials of the reductions over nodes.
+struct P2Work {
+  double *n, *v, *F, *r, *y, *d;
+  double *D, *L, *U;      // [B][nx / 2][NU][NU]: the odd columns' blocks of the current level
+  double *XL, *XU;        // [B][nx / 2][NU][NU]: D^-1 L and D^-1 U of the columns eliminated above level 0
+  double* Dinv;           // [B][(nx + 1) / 2][NU][NU]: D^-1 of the even columns (eliminated at level 0)
+  double* part;           // [B][kP2Part][blocks]
+  int* count;             // [B] tickets of the last step kernel (zero between launches)
+};
+constexpr int kP2Threads = 256, kP2Part = 14;
+
+// 1. The density on the unique nodes (DG integrals over the dual volumes, or given), v = phi0 with the contacts
+// set, F = A v - charge, r = -F on the free nodes, and the block partials of the scale and the integrals.
+__global__ void __launch_bounds__(kP2Threads) poisson2d_assemble_kernel(P2Dev P, P2Work w, int NU,
+                                                                        const double* __restrict__ src, int src_is_dg,
+                                                                        const double* __restrict__ phi0,
+                                                                        const double* __restrict__ bc) {
+  __shared__ double red[8];
+  const int b = blockIdx.y, nx = P.nx, nu = P.nu, nun = nu * nx;
+  const size_t full = (size_t)nx * P.ny;
   src += (size_t)b * (src_is_dg ? (size_t)P.ndx * P.ndy : full);
   phi0 += (size_t)b * full;
   bc += (size_t)b * nun;
-  phi += (size_t)b * full;
-  density += (size_t)b * full;
-  double* n = work + (size_t)b * 6 * nun;      // density on the unique nodes
-  double* v = n + nun;                          // v = phi0, contacts set
-  double* F = v + nun;                          // A v - charge
-  double* g = F + nun;                          // forward-sweep vectors, then the update d
-  double* r = g + nun;                          // -F on free nodes
-  double* t = r + nun;                          // scratch
-  double* Sinv = sinv_all + (size_t)b * nx * NU * NU;
-
-  // 1. the density on the unique nodes: DG integrals over the dual volumes, or given
-  double src_int = 0.0, tgt_int = 0.0;
-  if (src_is_dg) {
-    for (int k = lane; k < nun; k += 32) {
-      const int ix = k % nx, iy = k / nx;
+  const int k = blockIdx.x * kP2Threads + threadIdx.x;
+  double src_int = 0.0, tgt_int = 0.0, m_qn = 0.0, m_qnet = 0.0, m_av = 0.0, m_f = 0.0;
+  auto vat = [&](int q) { return P.fixed[q] ? bc[q] : phi0[q]; };
+  if (k < nun) {
+    const int ix = k % nx, iy = k / nx;
+    double nk;
+    if (src_is_dg) {
       double acc = 0.0;
       for (int p = P.tx_rp[ix]; p < P.tx_rp[ix + 1]; ++p) {
-        const double tx = P.tx_val[p];
         const double* row = src + P.tx_col[p];
         double s = 0.0;
         for (int q = P.ty_rp[iy]; q < P.ty_rp[iy + 1]; ++q) s += P.ty_val[q] * row[(size_t)P.ty_col[q] * P.ndx];
-        acc += tx * s;
+        acc += P.tx_val[p] * s;
       }
-      tgt_int += acc;
-      n[k] = acc / (P.wx[ix] * P.wy[iy]);
+      tgt_int = acc;
+      nk = acc / (P.wx[ix] * P.wy[iy]);
+    } else {
+      nk = src[k];
     }
-    for (int e = lane; e < P.ndx * P.ndy; e += 32) src_int += P.srcx[e % P.ndx] * src[e] * P.srcy[e / P.ndx];
-    src_int = warp_sum(src_int);
-    tgt_int = warp_sum(tgt_int);
-  } else {
-    for (int k = lane; k < nun; k += 32) n[k] = src[(size_t)(k / nx) * nx + k % nx];
-  }
-  // 2. v, A v, F = A v - charge and the residual scale (free nodes)
-  for (int k = lane; k < nun; k += 32) v[k] = P.fixed[k] ? bc[k] : phi0[k];
-  __syncwarp();
-  double m_qn = 0.0, m_qnet = 0.0, m_av = 0.0, m_f = 0.0;
-  for (int k = lane; k < nun; k += 32) {
-    const double av = stencil(P, v, k % nx, k / nx);
-    const double ch = kQ * (n[k] - P.net[k]);
-    F[k] = av - ch;
-    if (!P.fixed[k]) {
-      m_qn = fmax(m_qn, fabs(kQ * n[k]));
-      m_qnet = fmax(m_qnet, fabs(kQ * P.net[k]));
-      m_av = fmax(m_av, fabs(av));
-      m_f = fmax(m_f, fabs(F[k]));
+    const double v = vat(k);
+    double av = v;
+    const bool fx = P.fixed[k];
+    if (!fx) {
+      av = P.diag[k] * v;
+      if (ix > 0) av += P.cxm[k] * vat(k - 1);
+      if (ix < nx - 1) av += P.cxp[k] * vat(k + 1);
+      if (iy > 0 || P.periodic) av += P.cym[k] * vat((iy > 0 ? iy - 1 : nu - 1) * nx + ix);
+      if (iy < nu - 1 || P.periodic) av += P.cyp[k] * vat((iy < nu - 1 ? iy + 1 : 0) * nx + ix);
     }
-    r[k] = P.fixed[k] ? 0.0 : -F[k];
+    const double f = av - kQ * (nk - P.net[k]);
+    if (!fx) {
+      m_qn = fabs(kQ * nk);
+      m_qnet = fabs(kQ * P.net[k]);
+      m_av = fabs(av);
+      m_f = fabs(f);
+    }
+    const size_t g = (size_t)b * nun + k;
+    w.n[g] = nk;
+    w.v[g] = v;
+    w.F[g] = f;
+    w.r[((size_t)b * nx + ix) * NU + iy] = fx ? 0.0 : -f;
   }
-  m_qn = warp_max(m_qn);
-  m_qnet = warp_max(m_qnet);
-  m_av = warp_max(m_av);
-  m_f = warp_max(m_f);
-  const double scale = fmax(fmax(m_qn, m_qnet), fmax(m_av, kQ));
-  __syncwarp();
+  // rows nu .. NU-1 of every column are identity padding with a zero right-hand side
+  for (int q = k; q < nx * (NU - nu); q += gridDim.x * kP2Threads)
+    w.r[((size_t)b * nx + q % nx) * NU + nu + q / nx] = 0.0;
+  if (src_is_dg)
+    for (int e = k; e < P.ndx * P.ndy; e += gridDim.x * kP2Threads)
+      src_int += P.srcx[e % P.ndx] * src[e] * P.srcy[e / P.ndx];
+  const double out[6] = {block_sum(src_int, red), block_sum(tgt_int, red), block_max(m_qn, red),
+                         block_max(m_qnet, red), block_max(m_av, red), block_max(m_f, red)};
+  if (threadIdx.x == 0)
+    for (int i = 0; i < 6; ++i) w.part[((size_t)b * kP2Part + i) * gridDim.x + blockIdx.x] = out[i];
+}
 
-  // 3. forward block sweep: lane a holds row a of S_ix and then of S_ix^-1 (rows nu..NU-1
-  //    are identity padding; lanes NU..31 carry zero rows and store nothing)
-  const bool live = lane < nu;
-  double row[NU];
+// Entry (i, j) of column c's diagonal block of J; rows of fixed nodes (and the padding) are identity rows, and
+// couplings to fixed nodes are dropped (their update is zero).
+__device__ __forceinline__ double block_entry(const P2Dev& P, const double* __restrict__ n, int newton, double q_kt,
+                                              int c, int i, int j) {
+  if (i >= P.nu || j >= P.nu) return i == j ? 1.0 : 0.0;
+  const int k = c + i * P.nx;
+  if (P.fixed[k]) return i == j ? 1.0 : 0.0;
+  if (i == j) return P.diag[k] - (newton ? q_kt * n[k] : 0.0);
+  if (P.fixed[c + j * P.nx]) return 0.0;
+  const int jm = i > 0 ? i - 1 : (P.periodic ? P.nu - 1 : -1);
+  const int jp = i < P.nu - 1 ? i + 1 : (P.periodic ? 0 : -1);
+  return (j == jm ? P.cym[k] : 0.0) + (j == jp ? P.cyp[k] : 0.0);
+}
+// Couplings of row i of column c to the same row of the columns c - 1 and c + 1.
+__device__ __forceinline__ double left_entry(const P2Dev& P, int c, int i) {
+  const int k = c + i * P.nx;
+  return i < P.nu && c > 0 && !P.fixed[k] && !P.fixed[k - 1] ? P.cxm[k] : 0.0;
+}
+__device__ __forceinline__ double right_entry(const P2Dev& P, int c, int i) {
+  const int k = c + i * P.nx;
+  return i < P.nu && c < P.nx - 1 && !P.fixed[k] && !P.fixed[k + 1] ? P.cxp[k] : 0.0;
+}
+
+// 2. One level of the cyclic reduction over x (see the head of this file).  The columns of level l are c_k =
+// (k + 1) s - 1, k < K = nx / s, s = 2^l; the block of kept column k = 2 blockIdx.x + 1 eliminates its two
+// neighbours k - 1 and k + 1 (both halves of the threads at once), by Gauss-Jordan elimination of [D | L U r]
+// (level 0: [D | I r], the couplings there being diagonal), and folds them into its own D, L, U and r.  A column
+// between two kept ones is eliminated by both blocks (9 instead of 7 NU^3 FMAs per kept column), which saves a
+// launch per level.  Thread (nb, i, q) keeps row i, columns q + t TPR of neighbour nb in registers; only the pivot
+// row, column and its reciprocal go through shared memory (one barrier per pivot, two buffers).
+template <int NU, bool FIRST>
+struct ReduceShape {
+  static constexpr int W = (FIRST ? 2 : 3) * NU + 1;          // augmented width
+  static constexpr int CPT = NU >= 24 ? 8 : 4;                // columns per thread
+  static constexpr int TPR = (W + CPT - 1) / CPT;             // threads per row
+  static constexpr int THREADS = (2 * NU * TPR + 31) / 32 * 32;
+};
+
+template <int NU, bool FIRST>
+__global__ void __launch_bounds__(ReduceShape<NU, FIRST>::THREADS)
+    poisson2d_reduce_kernel(P2Dev P, P2Work w, int newton, double q_kt, int s, int K) {
+  using S = ReduceShape<NU, FIRST>;
+  constexpr int W = S::W, CPT = S::CPT, TPR = S::TPR, WX = W - NU, BB = NU * NU;
+  __shared__ double rowb[2][2][W], colb[2][2][NU], pinv[2][NU], X[2][NU][WX], E[NU][NU + 1];
+  const int b = blockIdx.y, nx = P.nx, nh = nx / 2, tid = threadIdx.x;
+  const int nb = tid / (NU * TPR), i = tid % (NU * TPR) / TPR, q = tid % TPR;
+  const bool on = nb < 2;
+  const int kk = 2 * blockIdx.x + 1;                    // the kept column (none when K == 1)
+  const bool kept = kk < K, has_r = kk + 1 < K;
+  const int c = (kk + 1) * s - 1;                       // its x index
+  const int ce = nb == 0 ? c - s : c + s;               // the neighbour of this half
+  const bool live = on && (nb == 0 || has_r);
+  const double* n = w.n + (size_t)b * P.nu * nx;
+  double* r = w.r + (size_t)b * nx * NU;
+  double* y = w.y + (size_t)b * nx * NU;
+  auto blk = [&](double* base, int col) { return base + ((size_t)b * nh + col / 2) * BB; };   // col is odd here
+  double a[CPT];
 #pragma unroll
-  for (int j = 0; j < NU; ++j) row[j] = 0.0;
-  double uprev = 0.0, gprev = 0.0;   // u_{ix-1} and g_{ix-1} of this lane's row
-  for (int ix = 0; ix < nx; ++ix) {
-    const int k = ix + lane * nx;
-    const bool fx = !live || P.fixed[k];
-    const double l = fx ? 0.0 : P.cxm[k];
-    const double u = fx ? 0.0 : P.cxp[k];
-    // S row a = D row a - l_a Sinv_prev[a][j] u_prev[j], built in place over Sinv_prev's row
-    const double dg = fx ? 1.0 : P.diag[k] - (newton ? q_kt * n[k] : 0.0);
-    const int jm = fx ? -1 : (lane > 0 ? lane - 1 : (P.periodic ? nu - 1 : -1));
-    const int jp = fx ? -1 : (lane < nu - 1 ? lane + 1 : (P.periodic ? 0 : -1));
-    const double cm = fx ? 0.0 : P.cym[k], cp = fx ? 0.0 : P.cyp[k];
-#pragma unroll
-    for (int j = 0; j < NU; ++j) {
-      const double uj = __shfl_sync(0xffffffffu, uprev, j);
-      const double dj = (j == lane && lane < NU ? dg : 0.0) + (j == jm ? cm : 0.0) + (j == jp ? cp : 0.0);
-      row[j] = dj - (ix > 0 ? l * row[j] * uj : 0.0);
+  for (int t = 0; t < CPT; ++t) {
+    const int j = q + t * TPR;
+    a[t] = 0.0;
+    if (live && j < W) {
+      if (FIRST)
+        a[t] = j < NU ? block_entry(P, n, newton, q_kt, ce, i, j) : j < 2 * NU ? (j - NU == i ? 1.0 : 0.0)
+                                                                              : r[(size_t)ce * NU + i];
+      else
+        a[t] = j < NU ? blk(w.D, ce)[i * NU + j]
+                      : j < 2 * NU ? blk(w.L, ce)[i * NU + j - NU]
+                                   : j < 3 * NU ? blk(w.U, ce)[i * NU + j - 2 * NU] : r[(size_t)ce * NU + i];
     }
-    // t = r_ix - L_ix g_{ix-1}
-    const double tk = (live ? r[k] : 0.0) - l * gprev;
-    // Gauss-Jordan inversion in place (no pivoting: S is diagonally dominant)
+  }
 #pragma unroll
-    for (int p = 0; p < NU; ++p) {
-      const double pinv = 1.0 / __shfl_sync(0xffffffffu, row[p], p);
-      if (lane == p) {
-        row[p] = 1.0;
+  for (int p = 0; p < NU; ++p) {
+    const int bf = p & 1;
+    if (live) {
+      if (i == p)
 #pragma unroll
-        for (int j = 0; j < NU; ++j) row[j] *= pinv;
+        for (int t = 0; t < CPT; ++t)
+          if (q + t * TPR < W) rowb[bf][nb][q + t * TPR] = a[t];
+      if (q == p % TPR) {
+        colb[bf][nb][i] = a[p / TPR];
+        if (i == p) pinv[nb][p] = 1.0 / a[p / TPR];
       }
-      const double f = row[p];
+    }
+    __syncthreads();
+    if (live && i != p) {
+      const double f = colb[bf][nb][i] * pinv[nb][p];
 #pragma unroll
-      for (int j = 0; j < NU; ++j) {
-        const double pj = __shfl_sync(0xffffffffu, row[j], p);
-        if (lane != p) row[j] = j == p ? -f * pj : row[j] - f * pj;
+      for (int t = 0; t < CPT; ++t)
+        if (p < (t + 1) * TPR - 1 && q + t * TPR < W)   // columns up to p are done with
+          a[t] = fma(-f, rowb[bf][nb][q + t * TPR], a[t]);
+    }
+  }
+  if (live) {
+    const bool store = nb == 0 || kk + 1 == K - 1;      // a shared neighbour is stored by the block on its right
+#pragma unroll
+    for (int t = 0; t < CPT; ++t) {
+      const int j = q + t * TPR - NU;
+      if (j < 0 || j >= WX) continue;
+      const double x = a[t] * pinv[nb][i];
+      X[nb][i][j] = x;
+      if (!store) continue;
+      if (j == WX - 1) y[(size_t)ce * NU + i] = x;
+      else if (FIRST) w.Dinv[((size_t)b * ((nx + 1) / 2) + ce / 2) * BB + i * NU + j] = x;
+      else (j < NU ? blk(w.XL, ce) : blk(w.XU, ce))[i * NU + j % NU] = x;
+    }
+  }
+  if (!kept) return;
+  __syncthreads();
+  if (FIRST) {
+    // couplings are diagonal: L' = -l Dinv_left diag(l_left), ...
+    for (int e = tid; e < BB; e += S::THREADS) {
+      const int ii = e / NU, j = e % NU;
+      const double l = left_entry(P, c, ii), u = right_entry(P, c, ii);
+      const double gl = -l * X[0][ii][j], gr = has_r ? -u * X[1][ii][j] : 0.0;
+      blk(w.D, c)[e] = block_entry(P, n, newton, q_kt, c, ii, j) + gl * right_entry(P, c - 1, j) +
+                       (has_r ? gr * left_entry(P, c + 1, j) : 0.0);
+      blk(w.L, c)[e] = gl * left_entry(P, c - 1, j);
+      blk(w.U, c)[e] = has_r ? gr * right_entry(P, c + 1, j) : 0.0;
+      if (j == 0)
+        r[(size_t)c * NU + ii] += -l * X[0][ii][WX - 1] + (has_r ? -u * X[1][ii][WX - 1] : 0.0);
+    }
+    return;
+  }
+  // products of this half's coupling block with [XL | XU | y] of its neighbour
+  constexpr int KX = (WX + TPR - 1) / TPR;
+  double acc[KX];
+#pragma unroll
+  for (int t = 0; t < KX; ++t) acc[t] = 0.0;
+  if (live) {
+    const double* C = (nb == 0 ? blk(w.L, c) : blk(w.U, c)) + i * NU;
+#pragma unroll 4
+    for (int m = 0; m < NU; ++m) {
+      const double cm = C[m];
+#pragma unroll
+      for (int t = 0; t < KX; ++t)
+        if (q + t * TPR < WX) acc[t] = fma(cm, X[nb][m][q + t * TPR], acc[t]);
+    }
+  }
+  __syncthreads();   // every thread has read its coupling row before L and U are overwritten
+  if (on && nb == 1)
+#pragma unroll
+    for (int t = 0; t < KX; ++t) {
+      const int j = q + t * TPR;
+      if (j < NU) E[i][j] = acc[t];
+      else if (j < 2 * NU) blk(w.U, c)[i * NU + j - NU] = -acc[t];
+      else if (j == 2 * NU) E[i][NU] = acc[t];
+    }
+  __syncthreads();
+  if (on && nb == 0)
+#pragma unroll
+    for (int t = 0; t < KX; ++t) {
+      const int j = q + t * TPR;
+      if (j < NU) blk(w.L, c)[i * NU + j] = -acc[t];
+      else if (j < 2 * NU) blk(w.D, c)[i * NU + j - NU] -= acc[t] + E[i][j - NU];
+      else if (j == 2 * NU) r[(size_t)c * NU + i] -= acc[t] + E[i][NU];
+    }
+}
+
+// 3. Back substitution of levels hi .. lo (2^lo = s_lo): d_c = y_c - XL_c d_{c-s} - XU_c d_{c+s}.  With
+// gridDim.x == 1 the block takes every column of these levels; otherwise lo == 0 and block x takes the columns of
+// [8 x, 8 x + 8), whose ends above level 2 are known, in levels 2, 1, 0.  One thread per row of a column.
+template <int NU>
+__global__ void __launch_bounds__(kP2Threads) poisson2d_back_kernel(P2Dev P, P2Work w, int s_hi, int s_lo,
+                                                                    int grouped) {
+  const int b = blockIdx.y, nx = P.nx, nh = nx / 2;
+  const double* y = w.y + (size_t)b * nx * NU;
+  double* d = w.d + (size_t)b * nx * NU;
+  const int c0 = grouped ? 8 * blockIdx.x : 0, c1 = grouped ? min(nx, c0 + 8) : nx;
+  for (int s = s_hi; s >= s_lo; s /= 2) {
+    // columns eliminated at stride s: c = s - 1 + 2 s m
+    const int cnt = c1 - c0 >= s ? (c1 - c0 - s) / (2 * s) + 1 : 0;
+    for (int e = threadIdx.x; e < cnt * NU; e += kP2Threads) {
+      const int c = c0 + s - 1 + 2 * s * (e / NU), i = e % NU;
+      const bool hl = c - s >= 0, hr = c + s < nx;
+      const double* dl = d + (size_t)(c - s) * NU;
+      const double* dr = d + (size_t)(c + s) * NU;
+      double v0 = y[(size_t)c * NU + i], v1 = 0.0;
+      if (s == 1) {
+        const double* m = w.Dinv + (((size_t)b * ((nx + 1) / 2) + c / 2) * NU + i) * NU;
+#pragma unroll 4
+        for (int j = 0; j < NU; ++j) {
+          if (hl) v0 -= m[j] * (left_entry(P, c, j) * dl[j]);
+          if (hr) v1 -= m[j] * (right_entry(P, c, j) * dr[j]);
+        }
+      } else {
+        const size_t o = (((size_t)b * nh + c / 2) * NU + i) * NU;
+        if (hl)
+#pragma unroll 4
+          for (int j = 0; j < NU; ++j) v0 -= w.XL[o + j] * dl[j];
+        if (hr)
+#pragma unroll 4
+          for (int j = 0; j < NU; ++j) v1 -= w.XU[o + j] * dr[j];
       }
+      d[(size_t)c * NU + i] = v0 + v1;
     }
-    // g_ix = S^-1 t
-    double gk = 0.0;
-#pragma unroll
-    for (int j = 0; j < NU; ++j) gk += row[j] * __shfl_sync(0xffffffffu, tk, j);
-    if (lane < NU) {
-      double* so = Sinv + ((size_t)ix * NU + lane) * NU;
-#pragma unroll
-      for (int j = 0; j < NU; ++j) so[j] = row[j];
-    }
-    if (live) g[k] = gk;
-    gprev = gk;
-    uprev = u;
+    __syncthreads();
   }
-  __syncwarp();
-  // 4. backward sweep: d_ix = g_ix - S_ix^-1 U_ix d_{ix+1}
-  double dnext = 0.0;
-  for (int ix = nx - 1; ix >= 0; --ix) {
-    const int k = ix + lane * nx;
-    const bool fx = !live || P.fixed[k];
-    const double u = fx ? 0.0 : P.cxp[k];
-    const double w = u * dnext;
-    const double* so = Sinv + ((size_t)ix * NU + (lane < NU ? lane : 0)) * NU;
-    double s = 0.0;
-#pragma unroll
-    for (int j = 0; j < NU; ++j) s += (lane < NU ? so[j] : 0.0) * __shfl_sync(0xffffffffu, w, j);
-    const double d = (live ? g[k] : 0.0) - (ix < nx - 1 ? s : 0.0);
-    if (live) g[k] = d;
-    dnext = d;
-  }
-  __syncwarp();
-  // 5. the linear residual J d + F, the update, iter_err, the step size
-  double m_lin = 0.0, e2 = 0.0, m_d = 0.0;
-  for (int k = lane; k < nun; k += 32) {
-    t[k] = P.fixed[k] ? 0.0 : g[k];
-  }
-  __syncwarp();
-  for (int k = lane; k < nun; k += 32) {
-    if (P.fixed[k]) continue;
-    const double jd = stencil(P, t, k % nx, k / nx) - (newton ? q_kt * n[k] * t[k] : 0.0);
-    m_lin = fmax(m_lin, fabs(jd + F[k]));
-    m_d = fmax(m_d, fabs(t[k]));
-  }
-  __syncwarp();
-  for (int k = lane; k < nun; k += 32) {
-    const double up = P.fixed[k] ? v[k] : v[k] + alpha * t[k];
-    if (!P.fixed[k]) {
-      const double dd = up - phi0[k];
-      e2 += dd * dd;
-    }
-    r[k] = up;   // updated
-  }
-  __syncwarp();
-  // 6. the residual after the update and the charge diagnostics
-  double m_after = 0.0, qnet = 0.0, qabs_net = 0.0, qabs_n = 0.0;
-  bool finite = true;
-  for (int k = lane; k < nun; k += 32) {
+}
+
+// 4. The linear residual J d + F, the update, the residual after it, the diagnostics, and phi and the density
+// on the full grid (the duplicate Y column when periodic).  The last block of a problem adds the partials.
+__global__ void __launch_bounds__(kP2Threads) poisson2d_finish_kernel(P2Dev P, P2Work w, int NU,
+                                                                      const double* __restrict__ phi0, int newton,
+                                                                      double q_kt, double alpha,
+                                                                      double* __restrict__ phi,
+                                                                      double* __restrict__ density,
+                                                                      wg_poisson2d_info* __restrict__ info) {
+  __shared__ double red[8];
+  __shared__ int last;
+  const int b = blockIdx.y, nx = P.nx, nu = P.nu, nun = nu * nx;
+  const size_t full = (size_t)nx * P.ny;
+  const double* n = w.n + (size_t)b * nun;
+  const double* v = w.v + (size_t)b * nun;
+  const double* F = w.F + (size_t)b * nun;
+  const double* d = w.d + (size_t)b * nx * NU;
+  const int k = blockIdx.x * kP2Threads + threadIdx.x;
+  double m_lin = 0.0, m_d = 0.0, e2 = 0.0, m_after = 0.0, qnet = 0.0, qabs_net = 0.0, qabs_n = 0.0, bad = 0.0;
+  if (k < nun) {
     const int ix = k % nx, iy = k / nx;
+    auto dat = [&](int x, int yy) { return P.fixed[x + yy * nx] ? 0.0 : d[(size_t)x * NU + yy]; };
+    const double t = dat(ix, iy), up = P.fixed[k] ? v[k] : v[k] + alpha * t;
     const double ch = kQ * (n[k] - P.net[k]);
-    if (!P.fixed[k]) m_after = fmax(m_after, fabs(stencil(P, r, ix, iy) - ch));
+    if (!P.fixed[k]) {
+      double jd = P.diag[k] * t, au = P.diag[k] * up;
+      auto nbr = [&](double cf, int x, int yy) {
+        const double dn = dat(x, yy);
+        jd += cf * dn;
+        au += cf * (P.fixed[x + yy * nx] ? v[x + yy * nx] : v[x + yy * nx] + alpha * dn);
+      };
+      if (ix > 0) nbr(P.cxm[k], ix - 1, iy);
+      if (ix < nx - 1) nbr(P.cxp[k], ix + 1, iy);
+      if (iy > 0 || P.periodic) nbr(P.cym[k], ix, iy > 0 ? iy - 1 : nu - 1);
+      if (iy < nu - 1 || P.periodic) nbr(P.cyp[k], ix, iy < nu - 1 ? iy + 1 : 0);
+      m_lin = fabs(jd - (newton ? q_kt * n[k] * t : 0.0) + F[k]);
+      m_d = fabs(t);
+      const double dd = up - phi0[(size_t)b * full + k];
+      e2 = dd * dd;
+      m_after = fabs(au - ch);
+    }
     const double vol = P.vx[ix] * P.vy[iy];
-    qnet += vol * ch;
-    qabs_net += vol * fabs(P.net[k]);
-    qabs_n += vol * fabs(n[k]);
-    if (!isfinite(r[k])) finite = false;
+    qnet = vol * ch;
+    qabs_net = vol * fabs(P.net[k]);
+    qabs_n = vol * fabs(n[k]);
+    bad = isfinite(up) ? 0.0 : 1.0;
+    phi[b * full + k] = up;
+    density[b * full + k] = n[k];
+    if (P.periodic && iy == 0) {
+      phi[b * full + (size_t)nu * nx + ix] = up;
+      density[b * full + (size_t)nu * nx + ix] = n[k];
+    }
   }
-  m_lin = warp_max(m_lin);
-  m_d = warp_max(m_d);
-  e2 = warp_sum(e2);
-  m_after = warp_max(m_after);
-  qnet = warp_sum(qnet);
-  qabs_net = warp_sum(qabs_net);
-  qabs_n = warp_sum(qabs_n);
-  finite = __all_sync(0xffffffffu, finite);
-  // 7. phi and the density on the full grid (the duplicate Y column when periodic)
-  for (size_t k = lane; k < full; k += 32) {
-    const int ix = (int)(k % nx), iy = (int)(k / nx);
-    const int ku = (iy < nu ? iy : 0) * nx + ix;
-    phi[k] = r[ku];
-    density[k] = n[ku];
+  const double out[8] = {block_sum(e2, red),      block_sum(qnet, red),    block_sum(qabs_net, red),
+                         block_sum(qabs_n, red),  block_max(m_lin, red),   block_max(m_d, red),
+                         block_max(m_after, red), block_max(bad, red)};
+  double* part = w.part + (size_t)b * kP2Part * gridDim.x;   // 0 .. 5 are the assembly's
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 8; ++i) part[(6 + i) * gridDim.x + blockIdx.x] = out[i];
+    __threadfence();
+    last = atomicAdd(&w.count[b], 1) == (int)gridDim.x - 1;
   }
-  if (lane == 0) {
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double all[kP2Part];
+  for (int i = 0; i < kP2Part; ++i) {
+    const bool sum = i < 2 || (i >= 6 && i < 10);
+    double t = 0.0;
+    for (int q = threadIdx.x; q < (int)gridDim.x; q += kP2Threads) {
+      const double x = __ldcg(&part[i * gridDim.x + q]);
+      t = sum ? t + x : fmax(t, x);
+    }
+    all[i] = sum ? block_sum(t, red) : block_max(t, red);
+  }
+  if (threadIdx.x == 0) {
+    w.count[b] = 0;
+    const double m_f = all[5], scale = fmax(fmax(all[2], all[3]), fmax(all[4], kQ));
     wg_poisson2d_info& o = info[b];
-    const double lin = m_lin / fmax(m_f, kQ);
-    o.converged = finite && isfinite(lin) && lin < 1e-8;
+    const double lin = all[10] / fmax(m_f, kQ);
+    o.converged = all[13] == 0.0 && isfinite(lin) && lin < 1e-8;
     o.linear_relres = lin;
     o.physical_relres_before = m_f / scale;
-    o.physical_relres_after = m_after / scale;
+    o.physical_relres_after = all[12] / scale;
     o.physical_residual_before = m_f;
     o.residual_scale = scale;
-    o.unmixed_step = m_d;
-    o.iter_err = sqrt(e2);
-    o.net_charge_per_length = -qnet;
-    o.relative_charge_imbalance = fabs(qnet) / fmax(kQ * fmax(qabs_net, qabs_n), DBL_MIN);
-    o.source_integral = src_int;
-    o.target_integral = tgt_int;
+    o.unmixed_step = all[11];
+    o.iter_err = sqrt(all[6]);
+    o.net_charge_per_length = -all[7];
+    o.relative_charge_imbalance = fabs(all[7]) / fmax(kQ * fmax(all[8], all[9]), DBL_MIN);
+    o.source_integral = all[0];
+    o.target_integral = all[1];
   }
 }
 
@@ -323,8 +502,8 @@ struct wg_poisson2d {
   P2Dev P{};
   cudaStream_t stream = nullptr;
   std::vector<void*> owned;
-  double *src = nullptr, *phi0 = nullptr, *bc = nullptr, *phi = nullptr, *dens = nullptr, *work = nullptr,
-         *sinv = nullptr;
+  double *src = nullptr, *phi0 = nullptr, *bc = nullptr, *phi = nullptr, *dens = nullptr, *work = nullptr;
+  P2Work w{};
   wg_poisson2d_info* info = nullptr;
   bool projection = false;
   std::string msg;
@@ -347,12 +526,28 @@ cudaError_t keep(wg_poisson2d* h, T** d, const std::vector<T>& v) {
 cudaError_t launch_step(wg_poisson2d* h, const double* src, int is_dg, const double* phi0, const double* bc,
                         int newton, double alpha, double* phi, double* dens, cudaStream_t st) {
   const double q_kt = kQ * kQ / (kKB * h->d.temp);
-  const int B = h->d.batch;
-  double* work = h->work;
-#define WG_P2_CASE(NU_)                                                                                      \
-  case NU_:                                                                                                  \
-    poisson2d_step_kernel<NU_><<<B, 32, 0, st>>>(h->P, src, is_dg, phi0, bc, newton, q_kt, alpha, phi, dens, \
-                                                 work, h->sinv, h->info);                                    \
+  const P2Dev& P = h->P;
+  const P2Work& w = h->w;
+  const unsigned B = (unsigned)h->d.batch;
+  const dim3 nodes((unsigned)((P.nu * P.nx + kP2Threads - 1) / kP2Threads), B);
+  int top = 1;
+  while (P.nx / (2 * top) >= 1) top *= 2;
+  poisson2d_assemble_kernel<<<nodes, kP2Threads, 0, st>>>(P, w, h->NU, src, is_dg, phi0, bc);
+#define WG_P2_CASE(NU_)                                                                                          \
+  case NU_:                                                                                                      \
+    for (int s = 1; s <= top; s *= 2) {                                                                          \
+      const int K = P.nx / s;                                                                                    \
+      const dim3 grid((unsigned)std::max(1, K / 2), B);                                                          \
+      if (s == 1)                                                                                                \
+        poisson2d_reduce_kernel<NU_, true>                                                                       \
+            <<<grid, ReduceShape<NU_, true>::THREADS, 0, st>>>(P, w, newton, q_kt, s, K);                        \
+      else                                                                                                       \
+        poisson2d_reduce_kernel<NU_, false>                                                                      \
+            <<<grid, ReduceShape<NU_, false>::THREADS, 0, st>>>(P, w, newton, q_kt, s, K);                       \
+    }                                                                                                            \
+    if (top >= 8) poisson2d_back_kernel<NU_><<<dim3(1, B), kP2Threads, 0, st>>>(P, w, top, 8, 0);               \
+    poisson2d_back_kernel<NU_>                                                                                   \
+        <<<dim3((unsigned)((P.nx + 7) / 8), B), kP2Threads, 0, st>>>(P, w, std::min(top, 4), 1, 1);              \
     break;
   switch (h->NU) {
     WG_P2_CASE(4)
@@ -365,6 +560,7 @@ cudaError_t launch_step(wg_poisson2d* h, const double* src, int is_dg, const dou
       return cudaErrorInvalidValue;
   }
 #undef WG_P2_CASE
+  poisson2d_finish_kernel<<<nodes, kP2Threads, 0, st>>>(P, w, h->NU, phi0, newton, q_kt, alpha, phi, dens, h->info);
   return cudaGetLastError();
 }
 
@@ -500,8 +696,24 @@ int wg_poisson2d_create(const wg_poisson2d_desc* d, const double* eps_r, const u
   if (e == cudaSuccess) e = cudaMalloc(&h->bc, (size_t)B * nun * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&h->phi, sz);
   if (e == cudaSuccess) e = cudaMalloc(&h->dens, sz);
-  if (e == cudaSuccess) e = cudaMalloc(&h->work, (size_t)B * 6 * nun * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&h->sinv, (size_t)B * nx * h->NU * h->NU * sizeof(double));
+  {
+    const size_t bb = (size_t)h->NU * h->NU, half = (size_t)B * (nx / 2) * bb, even = (size_t)B * ((nx + 1) / 2) * bb,
+                 col = (size_t)B * nx * h->NU, un = (size_t)B * nun,
+                 part = (size_t)B * kP2Part * ((nun + kP2Threads - 1) / kP2Threads);
+    double** const ptr[] = {&h->w.n, &h->w.v, &h->w.F, &h->w.r, &h->w.y, &h->w.d,    &h->w.D,
+                            &h->w.L, &h->w.U, &h->w.XL, &h->w.XU, &h->w.Dinv, &h->w.part};
+    const size_t len[] = {un, un, un, col, col, col, half, half, half, half, half, even, part};
+    size_t total = 0;
+    for (size_t l : len) total += l;
+    if (e == cudaSuccess) e = cudaMalloc(&h->work, total * sizeof(double));
+    size_t at0 = 0;
+    for (int i = 0; i < 13; ++i) {
+      *ptr[i] = h->work + at0;
+      at0 += len[i];
+    }
+    if (e == cudaSuccess) e = cudaMalloc(&h->w.count, (size_t)B * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(h->w.count, 0, (size_t)B * sizeof(int));
+  }
   if (e == cudaSuccess) e = cudaMalloc(&h->info, (size_t)B * sizeof(wg_poisson2d_info));
   if (e != cudaSuccess) {
     wg_poisson2d_destroy(h);
@@ -517,7 +729,7 @@ int wg_poisson2d_destroy(wg_poisson2d* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : h->owned) cudaFree(p);
   for (void* p : {(void*)h->src, (void*)h->phi0, (void*)h->bc, (void*)h->phi, (void*)h->dens, (void*)h->work,
-                  (void*)h->sinv, (void*)h->info})
+                  (void*)h->w.count, (void*)h->info})
     if (p) cudaFree(p);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
