@@ -9,25 +9,32 @@
 // off-diagonal products T = D^-1 Ht D is symmetric tridiagonal for a diagonal D
 // (d_{i+1} / d_i = sqrt(Ht(i+1,i) / Ht(i,i+1))), with the same eigenvalues and the
 // eigenvectors v = D w.  Per slice:
-//   subband_slice_kernel    one warp per slice (problem, valley, x):
-//     1. Ht's diagonal a, T's off-diagonal b, b^2 and the ratios of D in shared memory;
-//     2. Sturm counts (signs of the LDL^T pivots of T - x) locate the eigenvalues with
-//        index in [n0 - nm, n0 + nm), n0 = #(< 0), by multisection: the nc candidates
-//        share the 32 lanes, g = 32 / nc lanes per candidate each counting at one of g
-//        interior points, so an interval shrinks (g + 1)-fold per step;
-//     3. the nm of smallest magnitude, a contiguous run around zero, ascending;
-//     4. one lane per mode: the eigenvector of T from the twisted factorisation of
-//        T - lambda (Dhillon and Parlett, "Orthogonal eigenvectors and relative gaps",
-//        SIAM J. Matrix Anal. Appl. 25 (2004) 858-899): top-down pivots D+, bottom-up
-//        pivots D-, the twist index r of smallest |gamma_r| = |D+_r + D-_r - (a_r - lambda)|,
-//        then w_r = 1 and the one-term recurrences out of r; v = D w normalised in the
-//        2-norm and signed by its last entry (solve_bandstructure.m:28-30).
+//   subband_coarse_kernel   one warp per slice (problem, valley, x), all in FP32: Sturm counts (signs of the LDL^T
+//     pivots of T - x) around 0, then multisection of the eigenvalues with index in [n0 - nm, n0 + nm),
+//     n0 = #(< 0), to 1e-5 of the spectral radius (the candidates share the 32 lanes, g lanes count at g interior
+//     points of a candidate's interval per step); the nm of smallest magnitude are a contiguous run around zero.
+//   subband_refine_kernel   one lane per (slice, mode), FP64: Rayleigh quotient steps of the twisted factorisation
+//     of T - lambda (Dhillon and Parlett, "Orthogonal eigenvectors and relative gaps", SIAM J. Matrix Anal.
+//     Appl. 25 (2004) 858-899): top-down pivots D+, bottom-up pivots D-, the twist index r of smallest |gamma_r|,
+//     z_r = 1 and the one-term recurrences out of r; lambda += gamma_r / |z|^2 converges cubically, so from 1e-5
+//     two steps reach rounding level and the third factorisation gives the vector.  The negative pivots
+//     count the eigenvalues below lambda: it is eigenvalue k, or the slice goes to
+//   subband_bisect_kernel   one warp per listed slice: FP64 multisection to the end and the vectors from it.  It
+//     takes what the others cannot vouch for: two eigenvalues closer than the FP32 bracket, a tie of |lambda| at the
+//     edge of the run, entries outside the FP32 range, invalid data (which it reports).
 //   subband_cleanup_kernel  one warp per (problem, x >= 1, mode) of valley 1: v -> -v when
 //                           its overlap with the same mode of slice 1 is below -1/2.
 // A handle solves a batch of independent problems (gate or bias points) in one launch.
-// The pivots live in a scratch [slice][i][mode] (lanes = modes, coalesced).  All FP64.
+// v = D w normalised in the 2-norm and signed by its last entry (solve_bandstructure.m:28-30).
+//
+// Bound by the FP64 pipe (a warp instruction takes a quarter's pipe for 64 cycles however many lanes are on):
+// the multisection needed ~20 FP64 sweeps with a division per row for each slice's own warp, the refinement takes
+// three factorisations with a 4-operation reciprocal for 32 modes (several slices) at once.
+// 25,664 slices of 71 rows, 8 modes: 34.0 -> 2.2 ms; one gate point of 234 slices, 67 rows, 4 modes (host call):
+// 0.93 -> 0.44 ms.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <string>
@@ -87,15 +94,303 @@ __device__ int sturm_count32(const SliceShared& s, int n, float x, float pivmin)
 
 __device__ __forceinline__ double hop(double t0, double ma, double mb) { return -2.0 * t0 / (ma + mb); }
 
-__global__ void __launch_bounds__(128) subband_slice_kernel(const double* __restrict__ me_y, const double* __restrict__ pot,
-                                                            double t0, int nslice, int nv, int nx, int ny, int nm,
-                                                            double* __restrict__ E, double* __restrict__ Vsub,
-                                                            double* __restrict__ dplus, double* __restrict__ dminus,
-                                                            int* __restrict__ err) {
-  extern __shared__ double smem[];
+// Slices left to the bisection: list[0 .. *count), each once (flag per slice).
+struct FallbackList {
+  int *count, *flag, *list;
+  __device__ void add(int slice) const {
+    if (atomicExch(&flag[slice], 1) == 0) list[atomicAdd(count, 1)] = slice;
+  }
+};
+
+// The count in FP32 with fast divisions: exact for a matrix a few FP32 ulps of the spectral radius away.
+__device__ __forceinline__ int coarse_count(const float* a, const float* b2, int n, float x, float pivmin) {
+  float q = a[0] - x;
+  q = fabsf(q) < pivmin ? -pivmin : q;
+  int c = q < 0.f;
+#pragma unroll 4
+  for (int i = 1; i < n; ++i) {
+    q = a[i] - x - __fdividef(b2[i - 1], q);
+    q = fabsf(q) < pivmin ? -pivmin : q;
+    c += q < 0.f;
+  }
+  return c;
+}
+
+// Shared memory of the coarse stage per warp: a, b^2 [ny] and up to 2 nm + 1 candidates.
+__host__ __device__ constexpr int coarse_floats(int ny) { return 2 * ny + 2 * kMaxModes + 2; }
+
+// Width of the FP32 brackets, and what two of them may be apart and still be confused, in units of the radius.
+constexpr float kCoarseTol = 1e-5f, kCoarseMargin = 2e-5f;
+
+// E[slice][k] <- the FP32 estimate of eigenvalue kfirst[slice] + k (kfirst = -1: left to the bisection).
+__global__ void __launch_bounds__(128) subband_coarse_kernel(const double* __restrict__ me_y,
+                                                             const double* __restrict__ pot, float t0, int nslice,
+                                                             int nv, int nx, int ny, int nm, double* __restrict__ E,
+                                                             int* __restrict__ kfirst, FallbackList fb) {
+  extern __shared__ float smf[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slice = blockIdx.x * (blockDim.x >> 5) + warp;   // slice = (problem * nv + v) * nx + x
   if (slice >= nslice) return;
+  float* a = smf + (size_t)warp * coarse_floats(ny);
+  float* b2 = a + ny;
+  float* lam = b2 + ny;   // up to 2 nm + 1 candidates
+  const double* m = me_y + (size_t)slice * ny;
+  const double* V = pot + ((size_t)(slice / (nv * nx)) * nx + slice % nx) * ny;
+  auto hopf = [&](int i) { return -2.f * t0 / ((float)m[i] + (float)m[i + 1]); };   // rows i, i + 1
+  bool bad = false;
+  float glo = INFINITY, ghi = -INFINITY, bmax = 0.f;
+  for (int i = lane; i < ny; i += 32) {
+    const int r = i == 0 ? 1 : (i == ny - 1 ? ny - 2 : i);
+    const float lo = hopf(r - 1), up = hopf(r);
+    a[i] = -(lo + up) + (float)V[r];
+    // Ht(i, i+1) Ht(i+1, i); rows 0 and ny - 1 copy rows 1 and ny - 2
+    const float p = i == ny - 1 ? 0.f : (i == 0 ? up : hopf(i)) * (i + 1 == ny - 1 ? hopf(ny - 3) : hopf(i));
+    b2[i] = p;
+    bad = bad || !isfinite(a[i]) || !isfinite(p) || (i < ny - 1 && !(p > 0.f));
+    bmax = fmaxf(bmax, p);
+  }
+  __syncwarp();
+  for (int i = lane; i < ny; i += 32) {
+    const float rad = sqrtf(b2[i]) + (i > 0 ? sqrtf(b2[i - 1]) : 0.f);
+    glo = fminf(glo, a[i] - rad);
+    ghi = fmaxf(ghi, a[i] + rad);
+  }
+  for (int o = 16; o; o >>= 1) {
+    glo = fminf(glo, __shfl_xor_sync(0xffffffffu, glo, o));
+    ghi = fmaxf(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
+    bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
+  }
+  const float gnorm = fmaxf(fabsf(glo), fabsf(ghi)), pivmin = FLT_MIN * fmaxf(1.f, bmax);
+  bad = __any_sync(0xffffffffu, bad || !(gnorm < 1e30f));
+  int first = -1;
+  if (!bad) {
+    glo -= 1e-5f * gnorm;
+    ghi += 1e-5f * gnorm;
+    // the counts a little below and above 0 bound n0 from both sides
+    const float zero = 4e-6f * gnorm;
+    const int cz = lane < 2 ? coarse_count(a, b2, ny, lane == 0 ? -zero : zero, pivmin) : 0;
+    const int na = __shfl_sync(0xffffffffu, cz, 0), nb = __shfl_sync(0xffffffffu, cz, 1);
+    const int c0 = max(0, na - nm), c1 = min(ny, nb + nm), nc = c1 - c0;
+    bad = nb - na > 1;
+    for (int cb = 0; cb < nc && !bad; cb += 32) {
+      const int n = min(32, nc - cb), g = 32 / n, c = lane / g, j = lane % g;
+      const bool mine = c < n;
+      const int k = c0 + cb + (mine ? c : 0);
+      const unsigned gmask = (g == 32 ? 0xffffffffu : ((1u << g) - 1u)) << (mine ? c * g : 0);
+      float lo = glo, hi = ghi;
+      for (int it = 0; it < 64; ++it) {
+        const bool open = mine && hi - lo > kCoarseTol * gnorm;
+        if (!__any_sync(0xffffffffu, open)) break;
+        const float step = (hi - lo) / (g + 1), p = lo + (j + 1) * step;
+        const bool above = open && (p >= hi || (p > lo && coarse_count(a, b2, ny, p, pivmin) > k));
+        const unsigned vote = __ballot_sync(0xffffffffu, above) & gmask;
+        if (open) {
+          const int jf = vote ? __ffs(vote) - 1 - c * g : g;
+          const float nlo = jf == 0 ? lo : fmaxf(lo, lo + jf * step);
+          const float nhi = jf == g ? hi : fminf(hi, lo + (jf + 1) * step);
+          lo = nlo;
+          hi = nhi;
+        }
+      }
+      if (mine && j == 0) lam[cb + c] = 0.5f * (lo + hi);
+    }
+    __syncwarp();
+    // the nm of smallest magnitude: grow a window outwards from the sign change
+    int lo = -1, hi = 0;
+    while (hi < nc && lam[hi] < 0.f) ++hi;
+    lo = hi - 1;
+    for (int t = 0; t < nm && !bad; ++t) {
+      if (hi < nc && (lo < 0 || fabsf(lam[hi]) <= fabsf(lam[lo]))) ++hi;
+      else --lo;
+    }
+    // the last one taken and the first one left out on the other side must not be a tie
+    if (!bad) {
+      if (lo >= 0 && hi - 1 > lo && fabsf(lam[lo]) - fabsf(lam[hi - 1]) < 2 * kCoarseMargin * gnorm) bad = true;
+      if (hi < nc && lo + 1 < hi && fabsf(lam[hi]) - fabsf(lam[lo + 1]) < 2 * kCoarseMargin * gnorm &&
+          lam[lo + 1] < 0.f)
+        bad = true;
+      first = c0 + lo + 1;
+      for (int k = lane; k < nm; k += 32) E[(size_t)slice * nm + k] = lam[lo + 1 + k];
+    }
+  }
+  if (lane == 0) {
+    kfirst[slice] = bad ? -1 : first;
+    if (bad) fb.add(slice);
+  }
+}
+
+// 1 / x to rounding level: the hardware's approximation (rcp.approx.ftz.f64, about 20 bits) and one third-order
+// Newton step r (1 + e + e^2), e = 1 - x r (error e^3).
+__device__ __forceinline__ double fast_rcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+
+// Shared memory of the refinement: per slice a, b^2, b [ny], and the slices a block of one warp takes (32 / nm
+// where their data fit in 40 KB).
+__host__ __device__ constexpr int refine_doubles(int ny) { return 3 * ny; }
+int refine_slices(int ny, int nm) {
+  return std::max(1, std::min(32 / nm, (int)(40 * 1024 / (sizeof(double) * refine_doubles(ny)))));
+}
+
+__global__ void __launch_bounds__(32) subband_refine_kernel(const double* __restrict__ me_y,
+                                                            const double* __restrict__ pot, double t0, int nslice,
+                                                            int nv, int nx, int ny, int nm, int sl,
+                                                            double* __restrict__ E, double* __restrict__ Vsub,
+                                                            double* __restrict__ dplus, double* __restrict__ dminus,
+                                                            const int* __restrict__ kfirst, FallbackList fb) {
+  extern __shared__ double smem[];
+  __shared__ double r0s[32], r1s[32], gns[32], pvs[32];
+  const int lane = threadIdx.x, s0 = blockIdx.x * sl;
+  // T of every slice of the block; rows 0 and ny - 1 of Ht copy rows 1 and ny - 2
+  for (int q = 0; q < sl && s0 + q < nslice; ++q) {
+    const int slice = s0 + q;
+    double* a = smem + (size_t)q * refine_doubles(ny);
+    double *b2 = a + ny, *b = b2 + ny;
+    const double* m = me_y + (size_t)slice * ny;
+    const double* V = pot + ((size_t)(slice / (nv * nx)) * nx + slice % nx) * ny;
+    for (int i = lane; i < ny; i += 32) b[i] = i < ny - 1 ? hop(t0, m[i], m[i + 1]) : 0.0;
+    __syncwarp();
+    const double u0 = b[1], l0 = b[0], u1 = b[ny - 2], l1 = b[ny - 3];
+    float g = 0.f, bm = 0.f;
+    for (int i = lane; i < ny; i += 32) {
+      const int r = i == 0 ? 1 : (i == ny - 1 ? ny - 2 : i);
+      const double h = b[i];
+      a[i] = -(b[r - 1] + b[r]) + V[r];
+      b2[i] = i == 0 ? u0 * l0 : i == ny - 2 ? u1 * l1 : h * h;
+      g = fmaxf(g, fabsf((float)a[i]) + 2.f * fmaxf(fabsf((float)b[r - 1]), fabsf((float)b[r])));
+      bm = fmaxf(bm, (float)b2[i]);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      b[0] = -sqrt(u0 * l0);
+      r0s[q] = sqrt(u0 / l0);          // v_0 = w_0 / (d_1 / d_0) in units of the interior's d
+    }
+    if (lane == 1) {
+      b[ny - 2] = -sqrt(u1 * l1);
+      r1s[q] = sqrt(l1 / u1);
+    }
+    for (int o = 16; o; o >>= 1) {
+      g = fmaxf(g, __shfl_xor_sync(0xffffffffu, g, o));
+      bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
+    }
+    if (lane == 0) {
+      gns[q] = g;
+      pvs[q] = DBL_MIN * fmax(1.0, 2.0 * (double)bm);
+    }
+    __syncwarp();
+  }
+  const int q = lane / nm, k = lane % nm, slice = s0 + q;
+  if (q >= sl || slice >= nslice) return;
+  const int kf = kfirst[slice];
+  if (kf < 0) return;
+  const double* a = smem + (size_t)q * refine_doubles(ny);
+  const double *b2 = a + ny, *b = b2 + ny;
+  const double gnorm = gns[q], pivmin = pvs[q], atol = 4.0 * DBL_EPSILON * gnorm;
+  const unsigned long long pivbits = abs_bits(pivmin);
+  const double lam0 = E[(size_t)slice * nm + k];
+  double* dp = dplus + (size_t)slice * ny * nm + k;    // 1 / D+, then the vector [i][mode]
+  double* dm = dminus + (size_t)slice * ny * nm + k;   // 1 / D-
+  double lam = lam0, z0 = 0.0, z1 = 0.0, nint = 0.0;
+  bool ok = false, sure = false;
+  for (int it = 0; it < 8; ++it) {
+    double qp = a[0] - lam;
+    if (abs_bits(qp) < pivbits) qp = -pivmin;
+    int neg = qp < 0.0;
+    double ri = fast_rcp(qp);
+    dp[0] = ri;
+#pragma unroll 4
+    for (int i = 1; i < ny; ++i) {
+      qp = fma(-b2[i - 1], ri, a[i] - lam);
+      if (abs_bits(qp) < pivbits) qp = -pivmin;
+      neg += (int)((unsigned long long)__double_as_longlong(qp) >> 63);
+      ri = fast_rcp(qp);
+      dp[(size_t)i * nm] = ri;
+    }
+    // gamma_i = D+_i + D-_i - (a_i - lambda) = D-_i - b2_{i-1} / D+_{i-1}
+    int r = ny - 1;
+    double gam = qp;
+    double qm = a[ny - 1] - lam;
+    if (abs_bits(qm) < pivbits) qm = -pivmin;
+    ri = fast_rcp(qm);
+    dm[(size_t)(ny - 1) * nm] = ri;
+#pragma unroll 4
+    for (int i = ny - 2; i >= 0; --i) {
+      qm = fma(-b2[i], ri, a[i] - lam);
+      if (abs_bits(qm) < pivbits) qm = -pivmin;
+      const double gi = i > 0 ? fma(-b2[i - 1], dp[(size_t)(i - 1) * nm], qm) : qm;
+      if (abs_bits(gi) < abs_bits(gam)) {
+        gam = gi;
+        r = i;
+      }
+      ri = fast_rcp(qm);
+      dm[(size_t)i * nm] = ri;
+    }
+    // the vector out of r; its two end entries are kept apart (they alone carry D)
+    z0 = r == 0 ? 1.0 : 0.0;
+    z1 = r == ny - 1 ? 1.0 : 0.0;
+    nint = r > 0 && r < ny - 1 ? 1.0 : 0.0;
+    double z = 1.0;
+#pragma unroll 4
+    for (int i = r - 1; i >= 1; --i) {
+      z *= -(b[i] * dp[(size_t)i * nm]);
+      nint = fma(z, z, nint);
+      dp[(size_t)i * nm] = z;
+    }
+    if (r > 0) {
+      z0 = -(b[0] * dp[0]) * z;
+      dp[0] = z0;
+    }
+    dp[(size_t)r * nm] = 1.0;
+    z = 1.0;
+#pragma unroll 4
+    for (int i = r + 1; i < ny - 1; ++i) {
+      z *= -(b[i - 1] * dm[(size_t)i * nm]);
+      nint = fma(z, z, nint);
+      dp[(size_t)i * nm] = z;
+    }
+    if (r < ny - 1) {
+      z1 = -(b[ny - 2] * dm[(size_t)(ny - 1) * nm]) * z;
+      dp[(size_t)(ny - 1) * nm] = z1;
+    }
+    const double delta = gam / fma(z0, z0, fma(z1, z1, nint));
+    if (!(fabs(delta) < kCoarseMargin * gnorm)) break;      // NaN included
+    // a step well above rounding says on which side of lambda the eigenvalue lies: for eigenvalue k the count is
+    // then k or k + 1 (a count at the converged lambda alone could also be that of a close neighbour)
+    if (fabs(delta) > 16.0 * atol) sure = neg == kf + k + (delta < 0.0 ? 1 : 0);
+    lam += delta;
+    if (!(fabs(lam - lam0) < 2 * kCoarseMargin * gnorm)) break;
+    if (fabs(delta) <= atol + 2.0 * DBL_EPSILON * fabs(lam)) {
+      ok = sure && (neg == kf + k || neg == kf + k + 1);
+      break;
+    }
+  }
+  // v = D w, signed by its last entry
+  const double v0 = z0 * r0s[q], v1 = z1 * r1s[q];
+  const double sc = (v1 > 0.0 ? 1.0 : (v1 < 0.0 ? -1.0 : 0.0)) / sqrt(fma(v0, v0, fma(v1, v1, nint)));
+  if (!ok || !isfinite(sc)) {
+    fb.add(slice);
+    return;
+  }
+  E[(size_t)slice * nm + k] = lam;
+  double* out = Vsub + ((size_t)slice * nm + k) * ny;
+  out[0] = sc * v0;
+#pragma unroll 4
+  for (int i = 1; i < ny - 1; ++i) out[i] = sc * dp[(size_t)i * nm];
+  out[ny - 1] = sc * v1;
+}
+
+// One slice by FP64 multisection and one twisted factorisation per mode (one warp).
+__device__ void bisect_slice(const double* __restrict__ me_y, const double* __restrict__ pot, double t0, int slice,
+                             int nv, int nx, int ny, int nm, double* __restrict__ E, double* __restrict__ Vsub,
+                             double* __restrict__ dplus, double* __restrict__ dminus, int* __restrict__ err) {
+  extern __shared__ double smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   SliceShared s = slice_shared(smem + (size_t)warp * slice_doubles(ny), ny);
   const double* m = me_y + (size_t)slice * ny;
   const double* V = pot + ((size_t)(slice / (nv * nx)) * nx + slice % nx) * ny;
@@ -292,6 +587,19 @@ __global__ void __launch_bounds__(128) subband_slice_kernel(const double* __rest
   }
 }
 
+__global__ void __launch_bounds__(128) subband_bisect_kernel(const double* __restrict__ me_y,
+                                                             const double* __restrict__ pot, double t0, int nv, int nx,
+                                                             int ny, int nm, double* __restrict__ E,
+                                                             double* __restrict__ Vsub, double* __restrict__ dplus,
+                                                             double* __restrict__ dminus, int* __restrict__ err,
+                                                             FallbackList fb) {
+  const int nw = blockDim.x >> 5, n = *fb.count;
+  for (int i = blockIdx.x * nw + (threadIdx.x >> 5); i < n; i += gridDim.x * nw) {
+    bisect_slice(me_y, pot, t0, fb.list[i], nv, nx, ny, nm, E, Vsub, dplus, dminus, err);
+    __syncwarp();
+  }
+}
+
 __global__ void __launch_bounds__(256) subband_cleanup_kernel(double* __restrict__ Vsub, int batch, int nv, int nx,
                                                               int ny, int nm) {
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -325,6 +633,8 @@ struct wg_subbands {
   cudaStream_t stream = nullptr;
   double *me_y = nullptr, *V = nullptr, *E = nullptr, *Vsub = nullptr, *dp = nullptr, *dm = nullptr;
   int* err = nullptr;
+  int* kfirst = nullptr;     // [slices] index of the first eigenvalue taken, -1: left to the bisection
+  int* fallback = nullptr;   // count, flag [slices], list [slices]
   std::string msg;
 };
 
@@ -352,8 +662,10 @@ int wg_subbands_create(int batch, int n_valleys, int nx, int ny, int n_modes, wg
   if (e == cudaSuccess) e = cudaMalloc(&h->dm, slices * n_modes * ny * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&h->err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&h->kfirst, slices * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&h->fallback, (2 * slices + 1) * sizeof(int));
   if (e == cudaSuccess && warps_per_block(ny) * slice_smem(ny) > 48 * 1024)
-    e = cudaFuncSetAttribute(subband_slice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(subband_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(warps_per_block(ny) * slice_smem(ny)));
   if (e != cudaSuccess) {
     wg_subbands_destroy(h);
@@ -369,7 +681,8 @@ int wg_subbands_destroy(wg_subbands* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (double* p : {h->me_y, h->V, h->E, h->Vsub, h->dp, h->dm})
     if (p) cudaFree(p);
-  if (h->err) cudaFree(h->err);
+  for (int* p : {h->err, h->kfirst, h->fallback})
+    if (p) cudaFree(p);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return WG_OK;
@@ -384,8 +697,15 @@ int wg_subbands_solve_device(wg_subbands* h, double dy_nm, const double* me_y, c
   const double hb = 6.626e-34 / 2 / M_PI;
   const double t0 = hb * hb / 2 / (9.109e-31 * dy_nm * dy_nm * 1.602e-19 * 1e-18);   // eval_transversal_Hamiltonian.m:20
   const int slices = h->batch * h->nv * h->nx, wpb = warps_per_block(h->ny);
-  subband_slice_kernel<<<(slices + wpb - 1) / wpb, 32 * wpb, wpb * slice_smem(h->ny), st>>>(
-      me_y, V, t0, slices, h->nv, h->nx, h->ny, h->nm, E, Vsub, h->dp, h->dm, h->err);
+  const FallbackList fb{h->fallback, h->fallback + 1, h->fallback + 1 + slices};
+  cudaMemsetAsync(h->fallback, 0, (1 + (size_t)slices) * sizeof(int), st);
+  subband_coarse_kernel<<<(slices + 3) / 4, 128, 4 * coarse_floats(h->ny) * sizeof(float), st>>>(
+      me_y, V, (float)t0, slices, h->nv, h->nx, h->ny, h->nm, E, h->kfirst, fb);
+  const int sl = refine_slices(h->ny, h->nm);
+  subband_refine_kernel<<<(slices + sl - 1) / sl, 32, sl * refine_doubles(h->ny) * sizeof(double), st>>>(
+      me_y, V, t0, slices, h->nv, h->nx, h->ny, h->nm, sl, E, Vsub, h->dp, h->dm, h->kfirst, fb);
+  subband_bisect_kernel<<<std::min((slices + wpb - 1) / wpb, 608), 32 * wpb, wpb * slice_smem(h->ny), st>>>(
+      me_y, V, t0, h->nv, h->nx, h->ny, h->nm, E, Vsub, h->dp, h->dm, h->err, fb);
   if (h->nx > 1) {
     const long long warps = (long long)h->batch * (h->nx - 1) * h->nm;
     subband_cleanup_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(Vsub, h->batch, h->nv, h->nx,
