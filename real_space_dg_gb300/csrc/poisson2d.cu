@@ -22,7 +22,7 @@
 // all columns of a level at once, one block each (poisson2d_reduce_kernel), then the levels are substituted back.
 // log2(nx) + 1 dependent steps instead of a sweep over nx columns: the sweep (one warp per bias point) was
 // a chain of nx inversions, 20 us each.  Measured with a 361 x 13 periodic grid, projection and update of 16 bias points:
-// 7.4 ms with the sweep, 0.44 ms here (one point, 97 x 11: 1.9 -> 0.18 ms).
+// 7.4 ms with the sweep, 0.35 ms here (one point, 97 x 11: 1.9 -> 0.15 ms).
 // Every reduction over nodes has a fixed order that does not depend on the batch.
 #include <cuda_runtime.h>
 
@@ -56,31 +56,36 @@ __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// of non-negative values, NaN ignored: as integers, which their bit patterns are ordered like
 __device__ __forceinline__ double warp_max(double v) {
-  for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  long long u = __double_as_longlong(v);
+  if (u > 0x7ff0000000000000ll) u = 0;
+  for (int o = 16; o; o >>= 1) {
+    const long long t = __shfl_xor_sync(0xffffffffu, u, o);
+    u = t > u ? t : u;
+  }
+  return __longlong_as_double(u);
 }
 
-// Sum and maximum over a block of 256 threads, fixed order; the results are valid in every thread.
-__device__ double block_sum(double v, double* s) {
-  v = warp_sum(v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
+// Sums of v[0 .. NS) and maxima of the non-negative v[NS .. N) over a block of 256 threads, fixed order; out[i] is
+// written by one thread each, without a barrier after it.
+template <int N, int NS>
+__device__ void block_reduce(const double (&v)[N], double (*red)[8], double* out, int stride) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) t += s[i];
-  return t;
-}
-__device__ double block_max(double v, double* s) {
-  v = warp_max(v);
+  for (int i = 0; i < N; ++i) {
+    double t = v[i];
+    if (i < NS) t = warp_sum(t);
+    else t = warp_max(t);
+    if (lane == 0) red[i][warp] = t;
+  }
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = s[0];
-#pragma unroll
-  for (int i = 1; i < 8; ++i) t = fmax(t, s[i]);
-  return t;
+  if (threadIdx.x < N) {
+    const int i = threadIdx.x;
+    double t = red[i][0];
+    for (int q = 1; q < 8; ++q) t = i < NS ? t + red[i][q] : fmax(t, red[i][q]);
+    out[(size_t)i * stride] = t;
+  }
 }
 
 // Buffers of one step (all problems): n, v, F [B][nun]; r, y, d [B][nx][NU]; the blocks of the reduction and
@@ -101,7 +106,7 @@ __global__ void __launch_bounds__(kP2Threads) poisson2d_assemble_kernel(P2Dev P,
                                                                         const double* __restrict__ src, int src_is_dg,
                                                                         const double* __restrict__ phi0,
                                                                         const double* __restrict__ bc) {
-  __shared__ double red[8];
+  __shared__ double red[6][8];
   const int b = blockIdx.y, nx = P.nx, nu = P.nu, nun = nu * nx;
   const size_t full = (size_t)nx * P.ny;
   src += (size_t)b * (src_is_dg ? (size_t)P.ndx * P.ndy : full);
@@ -155,10 +160,8 @@ __global__ void __launch_bounds__(kP2Threads) poisson2d_assemble_kernel(P2Dev P,
   if (src_is_dg)
     for (int e = k; e < P.ndx * P.ndy; e += gridDim.x * kP2Threads)
       src_int += P.srcx[e % P.ndx] * src[e] * P.srcy[e / P.ndx];
-  const double out[6] = {block_sum(src_int, red), block_sum(tgt_int, red), block_max(m_qn, red),
-                         block_max(m_qnet, red), block_max(m_av, red), block_max(m_f, red)};
-  if (threadIdx.x == 0)
-    for (int i = 0; i < 6; ++i) w.part[((size_t)b * kP2Part + i) * gridDim.x + blockIdx.x] = out[i];
+  const double v6[6] = {src_int, tgt_int, m_qn, m_qnet, m_av, m_f};
+  block_reduce<6, 2>(v6, red, w.part + (size_t)b * kP2Part * gridDim.x + blockIdx.x, gridDim.x);
 }
 
 // Entry (i, j) of column c's diagonal block of J; rows of fixed nodes (and the padding) are identity rows, and
@@ -184,178 +187,247 @@ __device__ __forceinline__ double right_entry(const P2Dev& P, int c, int i) {
   return i < P.nu && c < P.nx - 1 && !P.fixed[k] && !P.fixed[k + 1] ? P.cxp[k] : 0.0;
 }
 
-// 2. One level of the cyclic reduction over x (see the head of this file).  The columns of level l are c_k =
-// (k + 1) s - 1, k < K = nx / s, s = 2^l; the block of kept column k = 2 blockIdx.x + 1 eliminates its two
-// neighbours k - 1 and k + 1 (both halves of the threads at once), by Gauss-Jordan elimination of [D | L U r]
-// (level 0: [D | I r], the couplings there being diagonal), and folds them into its own D, L, U and r.  A column
-// between two kept ones is eliminated by both blocks (9 instead of 7 NU^3 FMAs per kept column), which saves a
-// launch per level.  Thread (nb, i, q) keeps row i, columns q + t TPR of neighbour nb in registers; only the pivot
-// row, column and its reciprocal go through shared memory (one barrier per pivot, two buffers).
-template <int NU, bool FIRST>
+// 2a. Level 0: D^-1 and y = D^-1 r of every even column (one block each).
+// 2b. Level l >= 1, s = 2^l: the columns c_k = (k + 1) s - 1, k < K = nx / s, are still there.  The block of c_k first
+// folds the neighbours c_k -+ s/2 that the level before eliminated into D, L, U and r (level 1: the couplings
+// are diagonal and come from the stencil), then an even k eliminates: [X_L X_U y] = D^-1 [L U r]; an odd k stores
+// the folded blocks.  Thread (i, q) keeps row i, columns q + t TPR of the augmented matrix in registers.
+//
+// A warp's FP64 instruction takes its SM quarter's pipe for 64 cycles and returns after as many, so a block is
+// four warps (one per quarter) at up to 16 rows, and what counts in a latter level, where a handful of blocks run,
+// is instructions per pivot: CPT updates, one product, and the reciprocal (4, by the pivot's warp alone).  Both
+// neighbours in one block (eliminating a shared one twice) and 1 / x by division took 93, 82 and 44 us at levels 0, 1
+// and 2 of 16 bias points on 361 columns of 12 rows, 436 us for the whole step; here the step takes 346 us (one
+// point on 97 columns of 11 rows: 179 -> 148 us).
+template <int NU, int NB>
 struct ReduceShape {
-  static constexpr int W = (FIRST ? 2 : 3) * NU + 1;          // augmented width
-  static constexpr int CPT = NU >= 24 ? 8 : 4;                // columns per thread
+  static constexpr int W = NB * NU + 1;                       // augmented width: NB blocks and r
+  static constexpr int CPT = NU >= 24 ? 8 : (NB == 2 && NU == 12 ? 3 : 4);   // columns per thread
   static constexpr int TPR = (W + CPT - 1) / CPT;             // threads per row
-  static constexpr int THREADS = (2 * NU * TPR + 31) / 32 * 32;
+  static constexpr int THREADS = (NU * TPR + 31) / 32 * 32;
 };
 
+// 1 / x to rounding level: the hardware's approximation (rcp.approx.ftz.f64, about 20 bits) and a third-order
+// Newton step r (1 + e + e^2), e = 1 - x r.
+__device__ __forceinline__ double fast_rcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// [D | rest] -> D^-1 rest in registers, no pivoting; dg[i]: 1 / the pivot of row i.
+template <int NU, int NB>
+__device__ void eliminate(double (&a)[ReduceShape<NU, NB>::CPT], int i, int q, bool on,
+                          double (*rowb)[ReduceShape<NU, NB>::W], double (*colb)[NU], double* dg) {
+  using S = ReduceShape<NU, NB>;
+#pragma unroll
+  for (int p = 0; p < NU; ++p) {
+    const int bf = p & 1;
+    if (on) {
+      if (q == p % S::TPR) {
+        colb[bf][i] = a[p / S::TPR];
+        if (i == p) dg[p] = fast_rcp(a[p / S::TPR]);
+      }
+      if (i == p)
+#pragma unroll
+        for (int t = 0; t < S::CPT; ++t)
+          if (q + t * S::TPR < S::W) rowb[bf][q + t * S::TPR] = a[t];
+    }
+    __syncthreads();
+    if (on && i != p) {
+      const double f = -colb[bf][i] * dg[p];
+#pragma unroll
+      for (int t = 0; t < S::CPT; ++t)
+        if (p < (t + 1) * S::TPR - 1 && q + t * S::TPR < S::W)   // columns up to p are done with
+          a[t] = fma(f, rowb[bf][q + t * S::TPR], a[t]);
+    }
+  }
+  if (on) {
+    const double d = dg[i];
+#pragma unroll
+    for (int t = 0; t < S::CPT; ++t) a[t] *= d;
+  }
+}
+
+template <int NU>
+__global__ void __launch_bounds__(ReduceShape<NU, 2>::THREADS)
+    poisson2d_invert_kernel(P2Dev P, P2Work w, int newton, double q_kt) {
+  using S = ReduceShape<NU, 2>;
+  __shared__ double rowb[2][S::W], colb[2][NU], dg[NU];
+  const int b = blockIdx.y, nx = P.nx, c = 2 * blockIdx.x;
+  const int i = threadIdx.x / S::TPR, q = threadIdx.x % S::TPR;
+  const bool on = i < NU;
+  const double* n = w.n + (size_t)b * P.nu * nx;
+  double a[S::CPT];
+#pragma unroll
+  for (int t = 0; t < S::CPT; ++t) {
+    const int j = q + t * S::TPR;
+    a[t] = !on || j >= S::W ? 0.0
+                            : j < NU ? block_entry(P, n, newton, q_kt, c, i, j)
+                                     : j < 2 * NU ? (j - NU == i ? 1.0 : 0.0) : w.r[((size_t)b * nx + c) * NU + i];
+  }
+  eliminate<NU, 2>(a, i, q, on, rowb, colb, dg);
+  if (on)
+#pragma unroll
+    for (int t = 0; t < S::CPT; ++t) {
+      const int j = q + t * S::TPR;
+      if (j == 2 * NU) w.y[((size_t)b * nx + c) * NU + i] = a[t];
+      else if (j >= NU && j < 2 * NU)
+        w.Dinv[(((size_t)b * ((nx + 1) / 2) + blockIdx.x) * NU + i) * NU + j - NU] = a[t];
+    }
+}
+
 template <int NU, bool FIRST>
-__global__ void __launch_bounds__(ReduceShape<NU, FIRST>::THREADS)
-    poisson2d_reduce_kernel(P2Dev P, P2Work w, int newton, double q_kt, int s, int K) {
-  using S = ReduceShape<NU, FIRST>;
-  constexpr int W = S::W, CPT = S::CPT, TPR = S::TPR, WX = W - NU, BB = NU * NU;
-  __shared__ double rowb[2][2][W], colb[2][2][NU], pinv[2][NU], X[2][NU][WX], E[NU][NU + 1];
-  const int b = blockIdx.y, nx = P.nx, nh = nx / 2, tid = threadIdx.x;
-  const int nb = tid / (NU * TPR), i = tid % (NU * TPR) / TPR, q = tid % TPR;
-  const bool on = nb < 2;
-  const int kk = 2 * blockIdx.x + 1;                    // the kept column (none when K == 1)
-  const bool kept = kk < K, has_r = kk + 1 < K;
-  const int c = (kk + 1) * s - 1;                       // its x index
-  const int ce = nb == 0 ? c - s : c + s;               // the neighbour of this half
-  const bool live = on && (nb == 0 || has_r);
+__global__ void __launch_bounds__(ReduceShape<NU, 3>::THREADS)
+    poisson2d_reduce_kernel(P2Dev P, P2Work w, int newton, double q_kt, int s) {
+  using S = ReduceShape<NU, 3>;
+  constexpr int BB = NU * NU, CPT = S::CPT, TPR = S::TPR;
+  __shared__ double rowb[2][S::W], colb[2][NU], dg[NU];
+  const int b = blockIdx.y, nx = P.nx, nh = nx / 2, k = blockIdx.x;
+  const int c = (k + 1) * s - 1, cl = c - s / 2, cr = c + s / 2;
+  const bool has_r = cr < nx;
+  const int i = threadIdx.x / TPR, q = threadIdx.x % TPR;
+  const bool on = i < NU;
   const double* n = w.n + (size_t)b * P.nu * nx;
   double* r = w.r + (size_t)b * nx * NU;
   double* y = w.y + (size_t)b * nx * NU;
   auto blk = [&](double* base, int col) { return base + ((size_t)b * nh + col / 2) * BB; };   // col is odd here
+  // 1. fold: D -= L XU_l + U XL_r, L = -L XL_l, U = -U XU_r, r -= L y_l + U y_r
+  // up to 16 rows the six blocks and the products L XL_l, L XU_l, U XL_r, U XU_r, L y_l, U y_r go through shared
+  // memory: one round of loads, and every lane of the products' FMAs is used
+  constexpr bool STAGED = !FIRST && NU <= 16;
+  constexpr int PR = 4 * BB + 2 * NU;
+  __shared__ double sb[STAGED ? 6 * BB + 2 * NU : 1], pr_s[STAGED ? PR : 1];
+  if constexpr (STAGED) {
+    const double* src[6] = {blk(w.L, c), blk(w.U, c), blk(w.XL, cl), blk(w.XU, cl),
+                            has_r ? blk(w.XL, cr) : nullptr, has_r ? blk(w.XU, cr) : nullptr};
+#pragma unroll
+    for (int m = 0; m < 6; ++m)
+      for (int e = threadIdx.x; e < BB; e += S::THREADS) sb[m * BB + e] = src[m] ? src[m][e] : 0.0;
+    for (int e = threadIdx.x; e < 2 * NU; e += S::THREADS)
+      sb[6 * BB + e] = e < NU ? y[(size_t)cl * NU + e] : (has_r ? y[(size_t)cr * NU + e - NU] : 0.0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < PR; e += S::THREADS) {
+      // product m of row o / NU, column o % NU; the last 2 NU are the vectors
+      const int m = e / BB, o = m < 4 ? e % BB : 0, v = e - 4 * BB;
+      const double* cf = sb + (m < 4 ? (m < 2 ? 0 : BB) + o / NU * NU : (v < NU ? 0 : BB) + v % NU * NU);
+      const double* xc = sb + (m < 4 ? (2 + m) * BB + o % NU : 6 * BB + v / NU * NU);
+      const int st = m < 4 ? NU : 1;
+      double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+      for (int h = 0; h < NU; h += 2) {
+        v0 = fma(cf[h], xc[h * st], v0);
+        v1 = fma(cf[h + 1], xc[(h + 1) * st], v1);
+      }
+      pr_s[e] = v0 + v1;
+    }
+    __syncthreads();
+  }
   double a[CPT];
 #pragma unroll
   for (int t = 0; t < CPT; ++t) {
-    const int j = q + t * TPR;
+    const int j = q + t * TPR, jb = j / NU, jc = j % NU;   // block 0 D, 1 L, 2 U, 3 r
     a[t] = 0.0;
-    if (live && j < W) {
-      if (FIRST)
-        a[t] = j < NU ? block_entry(P, n, newton, q_kt, ce, i, j) : j < 2 * NU ? (j - NU == i ? 1.0 : 0.0)
-                                                                              : r[(size_t)ce * NU + i];
-      else
-        a[t] = j < NU ? blk(w.D, ce)[i * NU + j]
-                      : j < 2 * NU ? blk(w.L, ce)[i * NU + j - NU]
-                                   : j < 3 * NU ? blk(w.U, ce)[i * NU + j - 2 * NU] : r[(size_t)ce * NU + i];
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < NU; ++p) {
-    const int bf = p & 1;
-    if (live) {
-      if (i == p)
-#pragma unroll
-        for (int t = 0; t < CPT; ++t)
-          if (q + t * TPR < W) rowb[bf][nb][q + t * TPR] = a[t];
-      if (q == p % TPR) {
-        colb[bf][nb][i] = a[p / TPR];
-        if (i == p) pinv[nb][p] = 1.0 / a[p / TPR];
+    if (!on || j >= S::W) continue;
+    if (FIRST) {
+      const double l = left_entry(P, c, i), u = has_r ? right_entry(P, c, i) : 0.0;
+      if (jb == 3) {
+        a[t] = r[(size_t)c * NU + i] - l * y[(size_t)cl * NU + i];
+        if (has_r) a[t] = fma(-u, y[(size_t)cr * NU + i], a[t]);
+        continue;
       }
-    }
-    __syncthreads();
-    if (live && i != p) {
-      const double f = colb[bf][nb][i] * pinv[nb][p];
-#pragma unroll
-      for (int t = 0; t < CPT; ++t)
-        if (p < (t + 1) * TPR - 1 && q + t * TPR < W)   // columns up to p are done with
-          a[t] = fma(-f, rowb[bf][nb][q + t * TPR], a[t]);
-    }
-  }
-  if (live) {
-    const bool store = nb == 0 || kk + 1 == K - 1;      // a shared neighbour is stored by the block on its right
-#pragma unroll
-    for (int t = 0; t < CPT; ++t) {
-      const int j = q + t * TPR - NU;
-      if (j < 0 || j >= WX) continue;
-      const double x = a[t] * pinv[nb][i];
-      X[nb][i][j] = x;
-      if (!store) continue;
-      if (j == WX - 1) y[(size_t)ce * NU + i] = x;
-      else if (FIRST) w.Dinv[((size_t)b * ((nx + 1) / 2) + ce / 2) * BB + i * NU + j] = x;
-      else (j < NU ? blk(w.XL, ce) : blk(w.XU, ce))[i * NU + j % NU] = x;
-    }
-  }
-  if (!kept) return;
-  __syncthreads();
-  if (FIRST) {
-    // couplings are diagonal: L' = -l Dinv_left diag(l_left), ...
-    for (int e = tid; e < BB; e += S::THREADS) {
-      const int ii = e / NU, j = e % NU;
-      const double l = left_entry(P, c, ii), u = right_entry(P, c, ii);
-      const double gl = -l * X[0][ii][j], gr = has_r ? -u * X[1][ii][j] : 0.0;
-      blk(w.D, c)[e] = block_entry(P, n, newton, q_kt, c, ii, j) + gl * right_entry(P, c - 1, j) +
-                       (has_r ? gr * left_entry(P, c + 1, j) : 0.0);
-      blk(w.L, c)[e] = gl * left_entry(P, c - 1, j);
-      blk(w.U, c)[e] = has_r ? gr * right_entry(P, c + 1, j) : 0.0;
-      if (j == 0)
-        r[(size_t)c * NU + ii] += -l * X[0][ii][WX - 1] + (has_r ? -u * X[1][ii][WX - 1] : 0.0);
-    }
-    return;
-  }
-  // products of this half's coupling block with [XL | XU | y] of its neighbour
-  constexpr int KX = (WX + TPR - 1) / TPR;
-  double acc[KX];
-#pragma unroll
-  for (int t = 0; t < KX; ++t) acc[t] = 0.0;
-  if (live) {
-    const double* C = (nb == 0 ? blk(w.L, c) : blk(w.U, c)) + i * NU;
+      const double* dl = w.Dinv + ((size_t)b * ((nx + 1) / 2) + cl / 2) * BB + i * NU + jc;
+      const double gl = jb < 2 ? -l * dl[0] : 0.0, gr = jb != 1 && has_r ? -u * dl[BB] : 0.0;
+      if (jb == 0) {
+        a[t] = fma(gl, right_entry(P, cl, jc), block_entry(P, n, newton, q_kt, c, i, jc));
+        if (has_r) a[t] = fma(gr, left_entry(P, cr, jc), a[t]);
+      } else if (jb == 1) {
+        a[t] = gl * left_entry(P, cl, jc);
+      } else if (has_r) {
+        a[t] = gr * right_entry(P, cr, jc);
+      }
+    } else if constexpr (STAGED) {
+      const int o = i * NU + jc;
+      if (jb == 0) a[t] = blk(w.D, c)[o] - (pr_s[BB + o] + pr_s[2 * BB + o]);
+      else if (jb == 1) a[t] = -pr_s[o];
+      else if (jb == 2) a[t] = -pr_s[3 * BB + o];
+      else a[t] = r[(size_t)c * NU + i] - (pr_s[4 * BB + i] + pr_s[4 * BB + NU + i]);
+    } else {
+      const double *Lc = blk(w.L, c) + i * NU, *Uc = blk(w.U, c) + i * NU;
+      // the factors of L and of U in this column (r: vectors)
+      const double *pl = jb == 3 ? y + (size_t)cl * NU : jb == 2 ? nullptr : blk(jb == 0 ? w.XU : w.XL, cl) + jc;
+      const double *pr = !has_r || jb == 1 ? nullptr
+                                           : jb == 3 ? y + (size_t)cr * NU : blk(jb == 0 ? w.XL : w.XU, cr) + jc;
+      const int st = jb == 3 ? 1 : NU;
+      double v = jb == 0 ? blk(w.D, c)[i * NU + jc] : jb == 3 ? r[(size_t)c * NU + i] : 0.0;
+      if (pl)
 #pragma unroll 4
-    for (int m = 0; m < NU; ++m) {
-      const double cm = C[m];
-#pragma unroll
-      for (int t = 0; t < KX; ++t)
-        if (q + t * TPR < WX) acc[t] = fma(cm, X[nb][m][q + t * TPR], acc[t]);
+        for (int m = 0; m < NU; ++m) v = fma(-Lc[m], pl[m * st], v);
+      if (pr)
+#pragma unroll 4
+        for (int m = 0; m < NU; ++m) v = fma(-Uc[m], pr[m * st], v);
+      a[t] = v;
     }
   }
-  __syncthreads();   // every thread has read its coupling row before L and U are overwritten
-  if (on && nb == 1)
+  const bool keep = k & 1;   // stays: the next level folds and eliminates it or keeps it on
+  if (keep) __syncthreads();   // the block's old L and U have been read
+  else eliminate<NU, 3>(a, i, q, on, rowb, colb, dg);   // 2.
+  if (!on) return;
 #pragma unroll
-    for (int t = 0; t < KX; ++t) {
-      const int j = q + t * TPR;
-      if (j < NU) E[i][j] = acc[t];
-      else if (j < 2 * NU) blk(w.U, c)[i * NU + j - NU] = -acc[t];
-      else if (j == 2 * NU) E[i][NU] = acc[t];
-    }
-  __syncthreads();
-  if (on && nb == 0)
-#pragma unroll
-    for (int t = 0; t < KX; ++t) {
-      const int j = q + t * TPR;
-      if (j < NU) blk(w.L, c)[i * NU + j] = -acc[t];
-      else if (j < 2 * NU) blk(w.D, c)[i * NU + j - NU] -= acc[t] + E[i][j - NU];
-      else if (j == 2 * NU) r[(size_t)c * NU + i] -= acc[t] + E[i][NU];
-    }
+  for (int t = 0; t < CPT; ++t) {
+    const int j = q + t * TPR, jb = j / NU, o = i * NU + j % NU;
+    if (jb == 0 && keep) blk(w.D, c)[o] = a[t];
+    else if (jb == 1) blk(keep ? w.L : w.XL, c)[o] = a[t];
+    else if (jb == 2) blk(keep ? w.U : w.XU, c)[o] = a[t];
+    else if (j == 3 * NU) (keep ? r : y)[(size_t)c * NU + i] = a[t];
+  }
 }
 
 // 3. Back substitution of levels hi .. lo (2^lo = s_lo): d_c = y_c - XL_c d_{c-s} - XU_c d_{c+s}.  With
-// gridDim.x == 1 the block takes every column of these levels; otherwise lo == 0 and block x takes the columns of
-// [8 x, 8 x + 8), whose ends above level 2 are known, in levels 2, 1, 0.  One thread per row of a column.
+// grouped == 0 the block takes every column of these levels; otherwise lo == 0 and block x takes the columns of
+// [8 x, 8 x + 8), whose ends above level 2 are known, in levels 2, 1, 0.  Eight threads per row of a column.
 template <int NU>
 __global__ void __launch_bounds__(kP2Threads) poisson2d_back_kernel(P2Dev P, P2Work w, int s_hi, int s_lo,
                                                                     int grouped) {
-  const int b = blockIdx.y, nx = P.nx, nh = nx / 2;
+  constexpr int LN = 8;
+  const int b = blockIdx.y, nx = P.nx, nh = nx / 2, sub = threadIdx.x % LN;
   const double* y = w.y + (size_t)b * nx * NU;
   double* d = w.d + (size_t)b * nx * NU;
   const int c0 = grouped ? 8 * blockIdx.x : 0, c1 = grouped ? min(nx, c0 + 8) : nx;
   for (int s = s_hi; s >= s_lo; s /= 2) {
     // columns eliminated at stride s: c = s - 1 + 2 s m
     const int cnt = c1 - c0 >= s ? (c1 - c0 - s) / (2 * s) + 1 : 0;
-    for (int e = threadIdx.x; e < cnt * NU; e += kP2Threads) {
-      const int c = c0 + s - 1 + 2 * s * (e / NU), i = e % NU;
+    for (int e0 = 0; e0 < cnt * NU; e0 += kP2Threads / LN) {
+      const int e = e0 + threadIdx.x / LN;
+      const bool on = e < cnt * NU;
+      const int c = c0 + s - 1 + 2 * s * ((on ? e : 0) / NU), i = (on ? e : 0) % NU;
       const bool hl = c - s >= 0, hr = c + s < nx;
       const double* dl = d + (size_t)(c - s) * NU;
       const double* dr = d + (size_t)(c + s) * NU;
-      double v0 = y[(size_t)c * NU + i], v1 = 0.0;
-      if (s == 1) {
-        const double* m = w.Dinv + (((size_t)b * ((nx + 1) / 2) + c / 2) * NU + i) * NU;
-#pragma unroll 4
-        for (int j = 0; j < NU; ++j) {
-          if (hl) v0 -= m[j] * (left_entry(P, c, j) * dl[j]);
-          if (hr) v1 -= m[j] * (right_entry(P, c, j) * dr[j]);
+      double v = 0.0;
+      if (on) {
+        if (s == 1) {
+          const double* m = w.Dinv + (((size_t)b * ((nx + 1) / 2) + c / 2) * NU + i) * NU;
+#pragma unroll
+          for (int j = sub; j < NU; j += LN) {
+            double t = 0.0;
+            if (hl) t = left_entry(P, c, j) * dl[j];
+            if (hr) t = fma(right_entry(P, c, j), dr[j], t);
+            v = fma(m[j], t, v);
+          }
+        } else {
+          const size_t o = (((size_t)b * nh + c / 2) * NU + i) * NU;
+#pragma unroll
+          for (int j = sub; j < NU; j += LN) {
+            if (hl) v = fma(w.XL[o + j], dl[j], v);
+            if (hr) v = fma(w.XU[o + j], dr[j], v);
+          }
         }
-      } else {
-        const size_t o = (((size_t)b * nh + c / 2) * NU + i) * NU;
-        if (hl)
-#pragma unroll 4
-          for (int j = 0; j < NU; ++j) v0 -= w.XL[o + j] * dl[j];
-        if (hr)
-#pragma unroll 4
-          for (int j = 0; j < NU; ++j) v1 -= w.XU[o + j] * dr[j];
       }
-      d[(size_t)c * NU + i] = v0 + v1;
+#pragma unroll
+      for (int o = LN / 2; o; o /= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (on && sub == 0) d[(size_t)c * NU + i] = y[(size_t)c * NU + i] - v;
     }
     __syncthreads();
   }
@@ -369,7 +441,7 @@ __global__ void __launch_bounds__(kP2Threads) poisson2d_finish_kernel(P2Dev P, P
                                                                       double* __restrict__ phi,
                                                                       double* __restrict__ density,
                                                                       wg_poisson2d_info* __restrict__ info) {
-  __shared__ double red[8];
+  __shared__ double red[8][8], all[kP2Part];
   __shared__ int last;
   const int b = blockIdx.y, nx = P.nx, nu = P.nu, nun = nu * nx;
   const size_t full = (size_t)nx * P.ny;
@@ -413,28 +485,26 @@ __global__ void __launch_bounds__(kP2Threads) poisson2d_finish_kernel(P2Dev P, P
       density[b * full + (size_t)nu * nx + ix] = n[k];
     }
   }
-  const double out[8] = {block_sum(e2, red),      block_sum(qnet, red),    block_sum(qabs_net, red),
-                         block_sum(qabs_n, red),  block_max(m_lin, red),   block_max(m_d, red),
-                         block_max(m_after, red), block_max(bad, red)};
   double* part = w.part + (size_t)b * kP2Part * gridDim.x;   // 0 .. 5 are the assembly's
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < 8; ++i) part[(6 + i) * gridDim.x + blockIdx.x] = out[i];
-    __threadfence();
-    last = atomicAdd(&w.count[b], 1) == (int)gridDim.x - 1;
-  }
+  const double v8[8] = {e2, qnet, qabs_net, qabs_n, m_lin, m_d, m_after, bad};
+  block_reduce<8, 4>(v8, red, part + 6 * gridDim.x + blockIdx.x, gridDim.x);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&w.count[b], 1) == (int)gridDim.x - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double all[kP2Part];
-  for (int i = 0; i < kP2Part; ++i) {
+  for (int i = threadIdx.x >> 5; i < kP2Part; i += kP2Threads / 32) {
     const bool sum = i < 2 || (i >= 6 && i < 10);
     double t = 0.0;
-    for (int q = threadIdx.x; q < (int)gridDim.x; q += kP2Threads) {
+    for (int q = threadIdx.x & 31; q < (int)gridDim.x; q += 32) {
       const double x = __ldcg(&part[i * gridDim.x + q]);
       t = sum ? t + x : fmax(t, x);
     }
-    all[i] = sum ? block_sum(t, red) : block_max(t, red);
+    t = sum ? warp_sum(t) : warp_max(t);
+    if ((threadIdx.x & 31) == 0) all[i] = t;
   }
+  __syncthreads();
   if (threadIdx.x == 0) {
     w.count[b] = 0;
     const double m_f = all[5], scale = fmax(fmax(all[2], all[3]), fmax(all[4], kQ));
@@ -535,15 +605,16 @@ cudaError_t launch_step(wg_poisson2d* h, const double* src, int is_dg, const dou
   poisson2d_assemble_kernel<<<nodes, kP2Threads, 0, st>>>(P, w, h->NU, src, is_dg, phi0, bc);
 #define WG_P2_CASE(NU_)                                                                                          \
   case NU_:                                                                                                      \
-    for (int s = 1; s <= top; s *= 2) {                                                                          \
-      const int K = P.nx / s;                                                                                    \
-      const dim3 grid((unsigned)std::max(1, K / 2), B);                                                          \
-      if (s == 1)                                                                                                \
+    poisson2d_invert_kernel<NU_><<<dim3((unsigned)((P.nx + 1) / 2), B), ReduceShape<NU_, 2>::THREADS, 0, st>>>(  \
+        P, w, newton, q_kt);                                                                                     \
+    for (int s = 2; s <= top; s *= 2) {                                                                          \
+      const dim3 grid((unsigned)(P.nx / s), B);                                                                  \
+      if (s == 2)                                                                                                \
         poisson2d_reduce_kernel<NU_, true>                                                                       \
-            <<<grid, ReduceShape<NU_, true>::THREADS, 0, st>>>(P, w, newton, q_kt, s, K);                        \
+            <<<grid, ReduceShape<NU_, 3>::THREADS, 0, st>>>(P, w, newton, q_kt, s);                                 \
       else                                                                                                       \
         poisson2d_reduce_kernel<NU_, false>                                                                      \
-            <<<grid, ReduceShape<NU_, false>::THREADS, 0, st>>>(P, w, newton, q_kt, s, K);                       \
+            <<<grid, ReduceShape<NU_, 3>::THREADS, 0, st>>>(P, w, newton, q_kt, s);                                 \
     }                                                                                                            \
     if (top >= 8) poisson2d_back_kernel<NU_><<<dim3(1, B), kP2Threads, 0, st>>>(P, w, top, 8, 0);               \
     poisson2d_back_kernel<NU_>                                                                                   \
