@@ -11,13 +11,13 @@
 // eigenvectors v = D w.  Per slice:
 //   subband_coarse_kernel   one warp per slice (problem, valley, x), all in FP32: Sturm counts (signs of the LDL^T
 //     pivots of T - x) around 0, then multisection of the eigenvalues with index in [n0 - nm, n0 + nm),
-//     n0 = #(< 0), to 1e-5 of the spectral radius (the candidates share the 32 lanes, g lanes count at g interior
+//     n0 = #(< 0), to 1e-6 of the spectral radius (the candidates share the 32 lanes, g lanes count at g interior
 //     points of a candidate's interval per step); the nm of smallest magnitude are a contiguous run around zero.
 //   subband_refine_kernel   one lane per (slice, mode), FP64: Rayleigh quotient steps of the twisted factorisation
 //     of T - lambda (Dhillon and Parlett, "Orthogonal eigenvectors and relative gaps", SIAM J. Matrix Anal.
 //     Appl. 25 (2004) 858-899): top-down pivots D+, bottom-up pivots D-, the twist index r of smallest |gamma_r|,
-//     z_r = 1 and the one-term recurrences out of r; lambda += gamma_r / |z|^2 converges cubically, so from 1e-5
-//     two steps reach rounding level and the third factorisation gives the vector.  The negative pivots
+//     z_r = 1 and the one-term recurrences out of r; lambda += gamma_r / |z|^2 squares the error over the gap, so from
+//     1e-6 two steps reach rounding level and the third factorisation gives the vector.  The negative pivots
 //     count the eigenvalues below lambda: it is eigenvalue k, or the slice goes to
 //   subband_bisect_kernel   one warp per listed slice: FP64 multisection to the end and the vectors from it.  It
 //     takes what the others cannot vouch for: two eigenvalues closer than the FP32 bracket, a tie of |lambda| at the
@@ -30,8 +30,8 @@
 // Bound by the FP64 pipe (a warp instruction takes a quarter's pipe for 64 cycles however many lanes are on):
 // the multisection needed ~20 FP64 sweeps with a division per row for each slice's own warp, the refinement takes
 // three factorisations with a 4-operation reciprocal for 32 modes (several slices) at once.
-// 25,664 slices of 71 rows, 8 modes: 34.0 -> 2.2 ms; one gate point of 234 slices, 67 rows, 4 modes (host call):
-// 0.93 -> 0.44 ms.
+// 25,664 slices of 71 rows, 8 modes: 34.0 -> 2.1 ms; one gate point of 234 slices, 67 rows, 4 modes (host call):
+// 0.93 -> 0.39 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -120,7 +120,7 @@ __device__ __forceinline__ int coarse_count(const float* a, const float* b2, int
 __host__ __device__ constexpr int coarse_floats(int ny) { return 2 * ny + 2 * kMaxModes + 2; }
 
 // Width of the FP32 brackets, and what two of them may be apart and still be confused, in units of the radius.
-constexpr float kCoarseTol = 1e-5f, kCoarseMargin = 2e-5f;
+constexpr float kCoarseTol = 1e-6f, kCoarseMargin = 2e-5f;
 
 // E[slice][k] <- the FP32 estimate of eigenvalue kfirst[slice] + k (kfirst = -1: left to the bisection).
 __global__ void __launch_bounds__(128) subband_coarse_kernel(const double* __restrict__ me_y,
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(32) subband_refine_kernel(const double* __rest
                                                             double* __restrict__ dplus, double* __restrict__ dminus,
                                                             const int* __restrict__ kfirst, FallbackList fb) {
   extern __shared__ double smem[];
-  __shared__ double r0s[32], r1s[32], gns[32], pvs[32];
+  __shared__ double r0s[32], r1s[32], gns[32];
   const int lane = threadIdx.x, s0 = blockIdx.x * sl;
   // T of every slice of the block; rows 0 and ny - 1 of Ht copy rows 1 and ny - 2
   for (int q = 0; q < sl && s0 + q < nslice; ++q) {
@@ -257,14 +257,13 @@ __global__ void __launch_bounds__(32) subband_refine_kernel(const double* __rest
     for (int i = lane; i < ny; i += 32) b[i] = i < ny - 1 ? hop(t0, m[i], m[i + 1]) : 0.0;
     __syncwarp();
     const double u0 = b[1], l0 = b[0], u1 = b[ny - 2], l1 = b[ny - 3];
-    float g = 0.f, bm = 0.f;
+    float g = 0.f;
     for (int i = lane; i < ny; i += 32) {
       const int r = i == 0 ? 1 : (i == ny - 1 ? ny - 2 : i);
       const double h = b[i];
       a[i] = -(b[r - 1] + b[r]) + V[r];
       b2[i] = i == 0 ? u0 * l0 : i == ny - 2 ? u1 * l1 : h * h;
       g = fmaxf(g, fabsf((float)a[i]) + 2.f * fmaxf(fabsf((float)b[r - 1]), fabsf((float)b[r])));
-      bm = fmaxf(bm, (float)b2[i]);
     }
     __syncwarp();
     if (lane == 0) {
@@ -275,14 +274,8 @@ __global__ void __launch_bounds__(32) subband_refine_kernel(const double* __rest
       b[ny - 2] = -sqrt(u1 * l1);
       r1s[q] = sqrt(l1 / u1);
     }
-    for (int o = 16; o; o >>= 1) {
-      g = fmaxf(g, __shfl_xor_sync(0xffffffffu, g, o));
-      bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
-    }
-    if (lane == 0) {
-      gns[q] = g;
-      pvs[q] = DBL_MIN * fmax(1.0, 2.0 * (double)bm);
-    }
+    for (int o = 16; o; o >>= 1) g = fmaxf(g, __shfl_xor_sync(0xffffffffu, g, o));
+    if (lane == 0) gns[q] = g;
     __syncwarp();
   }
   const int q = lane / nm, k = lane % nm, slice = s0 + q;
@@ -291,7 +284,9 @@ __global__ void __launch_bounds__(32) subband_refine_kernel(const double* __rest
   if (kf < 0) return;
   const double* a = smem + (size_t)q * refine_doubles(ny);
   const double *b2 = a + ny, *b = b2 + ny;
-  const double gnorm = gns[q], pivmin = pvs[q], atol = 4.0 * DBL_EPSILON * gnorm;
+  // pivots below 1e-30 of the radius (some are exactly zero at a converged lambda) are moved to -1e-30 of it: far
+  // below their rounding, and their reciprocals and the next pivots stay in range
+  const double gnorm = gns[q], pivmin = 1e-30 * gnorm, atol = 4.0 * DBL_EPSILON * gnorm;
   const unsigned long long pivbits = abs_bits(pivmin);
   const double lam0 = E[(size_t)slice * nm + k];
   double* dp = dplus + (size_t)slice * ny * nm + k;    // 1 / D+, then the vector [i][mode]
@@ -365,7 +360,8 @@ __global__ void __launch_bounds__(32) subband_refine_kernel(const double* __rest
     if (fabs(delta) > 16.0 * atol) sure = neg == kf + k + (delta < 0.0 ? 1 : 0);
     lam += delta;
     if (!(fabs(lam - lam0) < 2 * kCoarseMargin * gnorm)) break;
-    if (fabs(delta) <= atol + 2.0 * DBL_EPSILON * fabs(lam)) {
+    // a step at rounding level; a quarter of it while another factorisation is cheap
+    if (fabs(delta) <= (it < 4 ? 0.25 : 1.0) * atol + 2.0 * DBL_EPSILON * fabs(lam)) {
       ok = sure && (neg == kf + k || neg == kf + k + 1);
       break;
     }
