@@ -113,6 +113,8 @@ int set_kline_factors(Problem& P) {
   const int nK = s.nK, B = P.batch;
   const size_t per_d = (size_t)s.nk * nK * nK, per_h = (size_t)s.nk * nK;
   std::vector<double> dinv(per_d * B), hv(per_h * B);
+  P.kline_shift = P.shift;
+  P.kline_exact = true;
   double kmax = 0;
   for (double kk : s.k) kmax = std::max(kmax, std::fabs(kk));
   for (int b = 0; b < B; ++b) {
@@ -139,6 +141,7 @@ int set_kline_factors(Problem& P) {
           P.err = "singular shifted k-line block";
           return WG_ERR_NUMERIC;
         }
+        if (k != 0.0) P.kline_exact = false;   // k = 0 has no flux to invert
         for (int i = 0; i < nK * nK; ++i) Di[i] = 0;
         double nrm = 0;
         for (int i = 0; i < nK * nK; ++i) nrm = std::max(nrm, std::fabs(s.K1[i]) + std::fabs(s.K2[i]));

@@ -181,10 +181,10 @@ __device__ __forceinline__ bool last_block_of_problem(int* __restrict__ count, i
   return last;
 }
 
-// hcol[b][i] = sum_c partial[b][i][c] (FP64); H[b][k][i] = (first) or += hcol.  One block.
+// hcol[b][i] = sum_c partial[b][i][c] (FP64); H[b][k][i] = (first; diag added at i = k) or += hcol.  One block.
 __device__ void dot_reduce_block(const double2* __restrict__ partial, double2* __restrict__ hcol,
                                  float2* __restrict__ hcol32, double2* __restrict__ H, int b, int nv, int k,
-                                 int pstride, int m, int nchunk, int first) {
+                                 int pstride, int m, int nchunk, int first, double diag) {
   // warp w takes the coefficients w, w + nw, w + 2 nw, w + 3 nw together, so that the loads
   // of four partial rows are in flight at once (this tail runs after the grid's last block)
   constexpr int U = 4;
@@ -215,7 +215,7 @@ __device__ void dot_reduce_block(const double2* __restrict__ partial, double2* _
         hcol[b * pstride + i] = acc[u];
         if (hcol32) hcol32[b * pstride + i] = make_float2((float)acc[u].x, (float)acc[u].y);
         double2* h = H + (long long)b * pstride * m + (long long)k * pstride + i;
-        if (first) *h = acc[u];
+        if (first) *h = make_double2(acc[u].x + (i == k ? diag : 0.0), acc[u].y);
         else { h->x += acc[u].x; h->y += acc[u].y; }
       }
     }
@@ -317,6 +317,7 @@ struct KrylovTail {
   double* inv64;
   float* inv32;
   double eta2;         // DGKS threshold squared
+  double diag;         // added to H[k][k]: 1 when w is A M^-1 v_k - v_k (flux_is_inverted)
   int k, pstride, m, first;
 };
 
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(256, 3) multidot32_kernel(const VB* __restrict
     partial[((long long)b * pstride + i) * nchunk + c] = r;
   }
   if (!last_block_of_problem(tl.md_count, b)) return;
-  dot_reduce_block(partial, tl.hcol, tl.hcol32, tl.H, b, nv, tl.k, pstride, tl.m, nchunk, tl.first);
+  dot_reduce_block(partial, tl.hcol, tl.hcol32, tl.H, b, nv, tl.k, pstride, tl.m, nchunk, tl.first, tl.diag);
   if (threadIdx.x == 0) tl.md_count[b] = 0;
 }
 
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(256) multidot64_kernel(const double2* __restri
     partial[((long long)b * pstride + i0 + threadIdx.x) * nchunk + c] = t;
   }
   if (!last_block_of_problem(tl.md_count, b)) return;
-  dot_reduce_block(partial, tl.hcol, tl.hcol32, tl.H, b, nv, tl.k, pstride, tl.m, nchunk, tl.first);
+  dot_reduce_block(partial, tl.hcol, tl.hcol32, tl.H, b, nv, tl.k, pstride, tl.m, nchunk, tl.first, tl.diag);
   if (threadIdx.x == 0) tl.md_count[b] = 0;
 }
 
@@ -772,7 +773,7 @@ template <> float2* coef_col32<double2>(Problem&) { return nullptr; }
 template <> float2* coef_col32<float2>(Problem& P) { return P.mx.hcol; }
 
 template <typename T, typename VB = T, typename Prec, typename Apply>
-int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, Prec prec, Apply apply) {
+int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, bool pre, Prec prec, Apply apply) {
   const int B = P.batch, mp1 = m + 1, ps = P.restart_max + 1, mm = P.restart_max;
   const long long N = P.N;
   // V_k: step 0 reads the basis vector the cycle start wrote; later steps take the previous
@@ -789,7 +790,7 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, Prec prec, Apply apply) 
     else
       WG_CK(prec(wprev, N, P.inv64, V + (long long)k * N));
   }
-  WG_CK(apply());
+  WG_CK(apply(V + (long long)k * N));
   const int nv = k + 1;
   const double vec = (double)N * B * sizeof(T), vecb = (double)N * B * sizeof(VB);
   constexpr bool f32 = std::is_same<T, float2>::value;
@@ -804,7 +805,7 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, Prec prec, Apply apply) 
   const int passes = eta < 0 ? 1 : 2;
   KrylovTail tl{P.md_count, P.gs_count, P.partial, P.hcol, coef_col32<T>(P), P.H, P.cs, P.sn, P.g, P.active,
                 P.kused, P.reorth, P.target, P.nrm, sizeof(T) == sizeof(float2) ? nullptr : P.inv64,
-                sizeof(T) == sizeof(float2) ? P.mx.inv : nullptr, eta * eta, k, ps, mm, 1};
+                sizeof(T) == sizeof(float2) ? P.mx.inv : nullptr, eta * eta, pre ? 1.0 : 0.0, k, ps, mm, 1};
   // the DGKS flags are written only for problems that take part in the first pass
   if (passes == 2 && eta < 1) WG_CK(cudaMemsetAsync(P.reorth, 0, sizeof(int) * B, P.stream));
   for (int pass = 0; pass < passes; ++pass) {
@@ -1058,7 +1059,10 @@ int gmres_solve_fp64(Problem& P, const wg_solve_opts& o, bool warm, wg_solve_inf
   auto prec = [&](const double2* r, long long stride, const double* rscale, double2* rout) {
     return launch_precondition(P, r, stride, P.z, rscale, rout, (long long)mp1 * N);
   };
-  auto apply = [&]() { return launch_apply(P, P.z, P.w); };
+  const bool pre = flux_is_inverted(P) && !(P.fp64_tc && P.mx.ozaki);
+  auto apply = [&](const double2* v) {
+    return pre ? launch_apply_pre(P, P.z, v, (long long)mp1 * N, P.w) : launch_apply(P, P.z, P.w);
+  };
   for (int cyc = 0; cyc < maxit; ++cyc) {
     bool any = false;
     for (int b = 0; b < B; ++b) any |= (res[b] > tgt[b]) && std::isfinite(res[b]);
@@ -1071,7 +1075,7 @@ int gmres_solve_fp64(Problem& P, const wg_solve_opts& o, bool warm, wg_solve_inf
       const int k1 = chunk_end(k0, m);
       rc = run_arnoldi_chunk(P, P.graphs[0], m, k0, [&]() {
         for (int k = k0; k < k1; ++k) {
-          const int r = arnoldi_step<double2>(P, P.V, P.w, k, m, prec, apply);
+          const int r = arnoldi_step<double2>(P, P.V, P.w, k, m, pre, prec, apply);
           if (r) return r;
         }
         return (int)WG_OK;
@@ -1121,14 +1125,19 @@ int gmres_solve_mixed(Problem& P, const wg_solve_opts& o, bool warm, wg_solve_in
   if (rc) return rc;
   std::vector<int> iters(B, 0), cycles(B, 0), refs(B, 0);
   std::vector<double> res = initial, itgt(B), ones(B, 1.0);
+  // with the flux inverted by the preconditioner only z's BF16 copy is needed
+  const bool pre = flux_is_inverted(P) && !M.fused;
+  float2* zf = pre ? nullptr : M.z;
   // the inner Arnoldi steps skip problems that have converged in this cycle (P.active)
   auto prec = [&](const float2* r, long long stride, const float* rscale, float2* rout) {
-    return launch_precondition_mixed(P, r, stride, M.z, M.zb16, P.active, rscale, rout, (long long)mp1 * N);
+    return launch_precondition_mixed(P, r, stride, zf, M.zb16, P.active, rscale, rout, (long long)mp1 * N);
   };
   auto prec_h = [&](const float2* r, long long stride, const float* rscale, __half2* rout) {
-    return launch_precondition_mixed_h(P, r, stride, M.z, M.zb16, P.active, rscale, rout, (long long)mp1 * N);
+    return launch_precondition_mixed_h(P, r, stride, zf, M.zb16, P.active, rscale, rout, (long long)mp1 * N);
   };
-  auto apply = [&]() { return launch_apply_mixed(P, M.z, M.zb16, M.w, P.active); };
+  auto apply = [&](const auto*) {
+    return pre ? launch_apply_mixed_pre(P, M.w, P.active) : launch_apply_mixed(P, M.z, M.zb16, M.w, P.active);
+  };
   for (int ref = 0; ref < max_ref; ++ref) {
     bool any = false;
     for (int b = 0; b < B; ++b) any |= (res[b] > tgt[b]) && std::isfinite(res[b]);
@@ -1157,8 +1166,8 @@ int gmres_solve_mixed(Problem& P, const wg_solve_opts& o, bool warm, wg_solve_in
       const int k1 = chunk_end(k0, m);
       rc = run_arnoldi_chunk(P, P.graphs[1], m, k0, [&]() {
         for (int k = k0; k < k1; ++k) {
-          const int r = M.basis16 ? arnoldi_step<float2, __half2>(P, M.Vh, M.w, k, m, prec_h, apply)
-                                  : arnoldi_step<float2>(P, M.V, M.w, k, m, prec, apply);
+          const int r = M.basis16 ? arnoldi_step<float2, __half2>(P, M.Vh, M.w, k, m, pre, prec_h, apply)
+                                  : arnoldi_step<float2>(P, M.V, M.w, k, m, pre, prec, apply);
           if (r) return r;
         }
         return (int)WG_OK;

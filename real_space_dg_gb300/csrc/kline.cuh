@@ -16,7 +16,8 @@
 // Optional: r enters scaled by rscale[b] (the Arnoldi step's w / |w|), and the apply kernel
 // writes the scaled r to rout (the next basis vector), which replaces a separate scaling pass.
 // With an FP16 basis (rout of type __half2) both kernels round the scaled r to FP16 before
-// they use it, so z is the preconditioned image of exactly the stored basis vector.
+// they use it, so z is the preconditioned image of exactly the stored basis vector.  z may be null where the
+// BF16 copy zb alone is used.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(32 * kChunksPerBlock) kline_apply_kernel(
       zv.x = ux * inv_qd - h[a] * s.x;
       zv.y = uy * inv_qd - h[a] * s.y;
       const long long o = (long long)e * NK * nk + (long long)a * nk;
-      zbase[o] = zv;
+      if (z) zbase[o] = zv;
       if (zb) zb[(long long)b * N + j + o] = __floats2bfloat162_rn((float)zv.x, (float)zv.y);
       if (a == st) snew = zv;
     }

@@ -497,6 +497,31 @@ cudaError_t apply_mixed_nk(Problem& P, const float2* x, const bf162* xb, float2*
   return cudaGetLastError();
 }
 
+// y = G z (launch_apply_mixed_pre): GEMM 1 of zb16, the stencil, GEMM 2.
+template <int NK>
+cudaError_t apply_mixed_pre_nk(Problem& P, float2* y, const int* mask) {
+  MixedBuffers& M = P.mx;
+  const Shape& s = P.s;
+  const long long BN = P.N * P.batch;
+  const double ncols = (double)P.ncols, nxi = s.nxi, nkd = s.nk;
+  const double gemm_flops = 2.0 * (2 * nxi) * (2 * nkd) * ncols;
+  const int cpp = s.n_el * s.nK;
+  cudaEvent_t ev = prof_begin(P, PROF_GEMM_BF16, 1, 4.0 * BN + 8.0 * nxi * ncols, gemm_flops, mask);
+  cudaError_t e = launch_gemm<0>(M.tmA1, M.tmB1z, reinterpret_cast<float*>(M.xh), 2 * s.nxi, P.ncols, 2 * s.nk, M.err,
+                                 P.stream, mask, cpp);
+  prof_end(P, PROF_GEMM_BF16, ev);
+  if (e != cudaSuccess) return e;
+  ev = prof_begin(P, PROF_STENCIL, 1, 12.0 * nxi * ncols + 4.0 * P.batch * s.n_el * pair_count(NK) * M.ne4, 0, mask);
+  launch_stencil32<NK>(P, mask);
+  prof_end(P, PROF_STENCIL, ev);
+  ev = prof_begin(P, PROF_GEMM_BF16, 1, 4.0 * nxi * ncols + 8.0 * BN, gemm_flops, mask);
+  e = launch_gemm<0>(M.tmA2, M.tmB2, reinterpret_cast<float*>(y), 2 * s.nk, P.ncols, 2 * s.nxi, M.err, P.stream, mask,
+                     cpp);
+  prof_end(P, PROF_GEMM_BF16, ev);
+  if (e != cudaSuccess) return e;
+  return cudaGetLastError();
+}
+
 template <int NK, typename O>
 cudaError_t precond_mixed_nk(Problem& P, const float2* r, long long r_stride, float2* z, bf162* zb, const int* mask,
                              const float* rscale, O* rout, long long rout_stride) {
@@ -732,6 +757,14 @@ cudaError_t launch_apply_mixed(Problem& P, const float2* x, const __nv_bfloat162
     case 2: return apply_mixed_nk<2>(P, x, xb, y, mask);
     case 3: return apply_mixed_nk<3>(P, x, xb, y, mask);
     default: return apply_mixed_nk<4>(P, x, xb, y, mask);
+  }
+}
+
+cudaError_t launch_apply_mixed_pre(Problem& P, float2* y, const int* mask) {
+  switch (P.s.nK) {
+    case 2: return apply_mixed_pre_nk<2>(P, y, mask);
+    case 3: return apply_mixed_pre_nk<3>(P, y, mask);
+    default: return apply_mixed_pre_nk<4>(P, y, mask);
   }
 }
 

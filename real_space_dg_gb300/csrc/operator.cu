@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(kFluxThreads) flux_kernel(const double2* __res
 // of the complex product.  The adjoint i Phi^H is the same with the pair (A - i B, A + i B).
 //   MODE 0: Y  = Phi X          tab = phi_t[p][m] (p a wave number, m a xi row)
 //   MODE 1: Y += i Phi^H X      tab = phi [p][m]  (p a xi row, m a wave number)
+//   MODE 2: Y  = i Phi^H X, less `sub` in row m0 (launch_apply_pre; m0 = -1: nowhere)
 // Bound by the FP64 pipe (2 FMAs per clock and SM: a warp's FMA takes 64 cycles of its quarter, so
 // loads, address arithmetic and shared-memory reads hide behind it).  What matters is that
 // the 608 pipe quarters get equal shares: one warp takes TS rows x 32/TS columns, blocks of 4 warps, and TS
@@ -157,7 +158,8 @@ template <int MODE, int TS>
 __global__ void __launch_bounds__(kPairThreads) paired_kernel(const double2* __restrict__ tab, int ldt,
                                                               const double2* __restrict__ X,
                                                               double2* __restrict__ Y, int K, int M,
-                                                              long long ncol) {
+                                                              long long ncol, const double2* __restrict__ sub,
+                                                              long long sub_stride, int cols, int m0) {
   constexpr int CW = 32 / TS, CB = CW * (kPairThreads / 32), PC = kPairChunk, LD = CB * PC / kPairThreads;
   __shared__ double2 es[2][CB][PC + 1], os[2][CB][PC + 1];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -227,13 +229,18 @@ __global__ void __launch_bounds__(kPairThreads) paired_kernel(const double2* __r
   if (MODE == 0) {
     y[m] = make_double2(A.x - B.y, A.y + B.x);
     if (mr != m) y[mr] = make_double2(A.x + B.y, A.y - B.x);
-  } else {   // t = A -+ i B, y += i t
-    double2 o = y[m];
-    y[m] = make_double2(o.x - (A.y - B.x), o.y + (A.x + B.y));
-    if (mr != m) {
-      o = y[mr];
-      y[mr] = make_double2(o.x - (A.y + B.x), o.y + (A.x - B.y));
+  } else {   // t = A -+ i B, y (+)= i t
+    double2 o = make_double2(0.0, 0.0), or_ = o;
+    if (MODE == 1) {
+      o = y[m];
+      if (mr != m) or_ = y[mr];
+    } else if (m == m0) {   // the unpaired middle row
+      const int b = (int)c / cols;
+      const double2 v = sub[(long long)b * sub_stride + (c - (long long)b * cols) * M + m];
+      o = make_double2(-v.x, -v.y);
     }
+    y[m] = make_double2(o.x - (A.y - B.x), o.y + (A.x + B.y));
+    if (mr != m) y[mr] = make_double2(or_.x - (A.y + B.x), or_.y + (A.x - B.y));
   }
 }
 
@@ -248,12 +255,15 @@ int table_rows(int half) {
 
 template <int MODE>
 void paired_launch(const double2* tab, int ldt, const double2* X, double2* Y, int K, int M, long long ncol,
-                   cudaStream_t st) {
+                   cudaStream_t st, const double2* sub = nullptr, long long sub_stride = 0, int cols = 1, int m0 = -1) {
   const int half = (M + 1) / 2, ts = table_rows(half), cb = kPairThreads / ts;
   const dim3 grid((unsigned)((ncol + cb - 1) / cb), (unsigned)((half + ts - 1) / ts));
-  if (ts == 32) paired_kernel<MODE, 32><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol);
-  else if (ts == 16) paired_kernel<MODE, 16><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol);
-  else paired_kernel<MODE, 8><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol);
+  if (ts == 32) paired_kernel<MODE, 32><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol, sub, sub_stride,
+                                                                               cols, m0);
+  else if (ts == 16) paired_kernel<MODE, 16><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol, sub, sub_stride,
+                                                                               cols, m0);
+  else paired_kernel<MODE, 8><<<grid, kPairThreads, 0, st>>>(tab, ldt, X, Y, K, M, ncol, sub, sub_stride,
+                                                                               cols, m0);
 }
 
 // ---------------------------------------------------------------------------
@@ -460,13 +470,17 @@ void stencil_launch(const double2* xh, double2* yh, const double* beta, const do
   stencil_kernel<NK><<<grid, kFluxThreads, 0, st>>>(xh, yh, beta, betai, nxi, n_el, mask);
 }
 
+// v == nullptr: y = A x.  Otherwise x = M^-1 v and y = A x - v (launch_apply_pre).
 template <int NK>
-cudaError_t apply_nk(Problem& P, const double2* x, double2* y) {
+cudaError_t apply_nk(Problem& P, const double2* x, double2* y, const double2* v = nullptr, long long v_stride = 0) {
   const double BN = (double)P.N * P.batch, ncols = (double)P.ncols, nxi = P.s.nxi, nk = P.s.nk;
   const double gemm_flops = 2.0 * nxi * nk * ncols;   // paired rows and columns: a quarter of the complex product
-  cudaEvent_t ev = prof_begin(P, PROF_FLUX64, 1, 32.0 * BN, 8.0 * NK * BN);
-  flux_launch<NK>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream);
-  prof_end(P, PROF_FLUX64, ev);
+  cudaEvent_t ev;
+  if (!v) {
+    ev = prof_begin(P, PROF_FLUX64, 1, 32.0 * BN, 8.0 * NK * BN);
+    flux_launch<NK>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream);
+    prof_end(P, PROF_FLUX64, ev);
+  }
   ev = prof_begin(P, PROF_GEMM_F64, 1, 16.0 * (BN + nxi * ncols), gemm_flops);
   paired_launch<0>(P.phi_t, (P.s.nxi + 1) / 2, x, P.xh, P.s.nk, P.s.nxi, P.ncols, P.stream);
   prof_end(P, PROF_GEMM_F64, ev);
@@ -474,8 +488,11 @@ cudaError_t apply_nk(Problem& P, const double2* x, double2* y) {
                   16.0 * NK * nxi * ncols);
   stencil_launch<NK>(P.xh, P.yh, P.beta, P.betai, P.batch, P.s.n_el, P.s.nxi, P.stream);
   prof_end(P, PROF_STENCIL64, ev);
-  ev = prof_begin(P, PROF_GEMM_F64, 1, 16.0 * (2 * BN + nxi * ncols), gemm_flops);
-  paired_launch<1>(P.phi, P.s.nk, P.yh, y, P.s.nxi, P.s.nk, P.ncols, P.stream);
+  ev = prof_begin(P, PROF_GEMM_F64, 1, 16.0 * ((v ? 1 : 2) * BN + nxi * ncols), gemm_flops);
+  if (!v) paired_launch<1>(P.phi, P.s.nk, P.yh, y, P.s.nxi, P.s.nk, P.ncols, P.stream);
+  else  // the wave number 0 (odd Nk) has no flux, so nothing of v, unless the operator is shifted
+    paired_launch<2>(P.phi, P.s.nk, P.yh, y, P.s.nxi, P.s.nk, P.ncols, P.stream, v, v_stride, P.s.n_el * NK,
+                     P.s.nk % 2 && P.shift == 0 ? P.s.nk / 2 : -1);
   prof_end(P, PROF_GEMM_F64, ev);
   return cudaGetLastError();
 }
@@ -621,6 +638,16 @@ cudaError_t launch_apply(Problem& P, const double2* x, double2* y) {
     case 2: return apply_nk<2>(P, x, y);
     case 3: return apply_nk<3>(P, x, y);
     default: return apply_nk<4>(P, x, y);
+  }
+}
+
+bool flux_is_inverted(const Problem& P) { return P.kline_exact && P.shift == P.kline_shift; }
+
+cudaError_t launch_apply_pre(Problem& P, const double2* z, const double2* v, long long v_stride, double2* y) {
+  switch (P.s.nK) {
+    case 2: return apply_nk<2>(P, z, y, v, v_stride);
+    case 3: return apply_nk<3>(P, z, y, v, v_stride);
+    default: return apply_nk<4>(P, z, y, v, v_stride);
   }
 }
 

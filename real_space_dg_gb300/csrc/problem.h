@@ -214,6 +214,8 @@ struct Problem {
   double mem_budget = 0;
   FluxBlocks fb{};
   double shift = 0;         // sigma of the shifted operator A + sigma I (0: the stationary A)
+  double kline_shift = 0;   // sigma the k-line factors were built with
+  bool kline_exact = false; // every line block with a flux was inverted (set_kline_factors)
   bool fp64_tc = false;     // FP64 handle whose transforms run as FP64 emulated on the tensor cores
   bool inner_basis16 = true;  // mixed form: the inner Krylov basis stored in FP16
   std::string err;
@@ -314,6 +316,14 @@ void prof_release(Problem& P);
 
 // Kernel launchers (operator.cu)
 cudaError_t launch_apply(Problem& P, const double2* x, double2* y);
+// The k-line preconditioner is the exact inverse of the flux (and shift) part F of the operator A = F + G: each
+// line's block-bidiagonal system is solved, not approximated.  So A M^-1 v = v + G M^-1 v, and since v is a basis vector
+// the Arnoldi step orthogonalises G M^-1 v alone and adds 1 to the Hessenberg diagonal: no flux kernel, nothing
+// to accumulate into, and no identity part to cancel in the Gram-Schmidt pass.  True when the current shift is the one
+// the factors were built with.
+bool flux_is_inverted(const Problem& P);
+// y = A z - v for z = M^-1 v where flux_is_inverted (v: per-problem stride v_stride); not for fp64_tc handles.
+cudaError_t launch_apply_pre(Problem& P, const double2* z, const double2* v, long long v_stride, double2* y);
 // rscale (device, optional): r enters scaled by rscale[b]; rout (optional): the scaled r is written there
 // (per-problem stride rout_stride), the Arnoldi step's next basis vector.
 cudaError_t launch_precondition(Problem& P, const double2* r, long long r_stride, double2* z,
@@ -351,6 +361,8 @@ cudaError_t mixed_sync_weights(Problem& P);
 // mask (device, optional): problems b with mask[b] == 0 are skipped (their output is left as is).
 cudaError_t launch_apply_mixed(Problem& P, const float2* x, const __nv_bfloat162* xb, float2* y,
                                const int* mask = nullptr);
+// y = G z (A z - v for z = M^-1 v where flux_is_inverted), z given by its BF16 copy P.mx.zb16.
+cudaError_t launch_apply_mixed_pre(Problem& P, float2* y, const int* mask);
 cudaError_t launch_precondition_mixed(Problem& P, const float2* r, long long r_stride, float2* z,
                                       __nv_bfloat162* zb, const int* mask = nullptr, const float* rscale = nullptr,
                                       float2* rout = nullptr, long long rout_stride = 0);
