@@ -258,11 +258,14 @@ __global__ void __launch_bounds__(kFlux32Threads) flux32_kernel(const float2* __
 // ---------------------------------------------------------------------------
 // FP32 xi stencil, output as the BF16 B operand of GEMM 2:
 //   y_a(s) = sum_c beta_ac(s) (x_c(s) + x_c(s-1)) + beta_ac(s+1) (x_c(s) + x_c(s+1)),
-// beta = betar (symmetric in a, c: pairs a <= c stored) + i betai.  Each thread owns
-// CELLS (2 or 4, picked per shape by the autotuner) consecutive xi cells: vector loads
-// of x (16 bytes per two cells), of the weights (4 bytes per cell) and vector stores of
-// the BF16 output; the cells s0-1 and s0+CELLS come from the neighbouring lanes.  Grid
-// (batch * n_el, ceil(nxi / (64 CELLS))) of 64 threads; nxi % 4 == 0 (mixed form).
+// beta = betar (symmetric in a, c: pairs a <= c stored) + i capk_ac cap: the absorbing part is a product, so its
+// cells' factor u_c(s) = cap(s) (..) + cap(s+1) (..) is formed once per c and costs two FMAs per (a, c)
+// and one row of loads instead of nK^2.  Each thread owns CELLS (2 or 4, picked per shape by the autotuner)
+// consecutive xi cells: vector loads of x (16 bytes per two cells) and of the weights (4 bytes per cell), all
+// issued before the arithmetic, and vector stores of the BF16 output; the cells s0-1 and s0+CELLS and the next
+// weights come from the neighbouring lanes.  Grid (batch * n_el, ceil(nxi / (64 CELLS))) of 64 threads; nxi % 4 == 0
+// (mixed form).  Bound by HBM (x, the nK (nK + 1) / 2 weight rows, y).  16 problems of 240 elements, N_xi = 256,
+// nK = 4 (86 MB): 33.6 -> 18.4 us (4.6 TB/s) against one load per (a, c) of both weights, interleaved with the sums.
 // ---------------------------------------------------------------------------
 constexpr int kSt4Threads = 64;
 
@@ -270,27 +273,31 @@ __host__ __device__ constexpr int pair_count(int nk) { return nk * (nk + 1) / 2;
 // index of the pair (a, c), a <= c, in the order (0,0) (0,1) .. (0,nK-1) (1,1) ..
 __host__ __device__ constexpr int pair_index(int nk, int a, int c) { return a * nk - a * (a - 1) / 2 + (c - a); }
 
-__device__ __forceinline__ float2 f2add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-
 // CELLS consecutive floats (CELLS * 4 bytes aligned) into v[0..CELLS)
 template <int CELLS>
 __device__ __forceinline__ void ld_cells(const float* p, float* v) {
   if constexpr (CELLS == 4) {
-    const float4 t = *reinterpret_cast<const float4*>(p);
+    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
     v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
   } else {
-    const float2 t = *reinterpret_cast<const float2*>(p);
+    const float2 t = __ldg(reinterpret_cast<const float2*>(p));
     v[0] = t.x; v[1] = t.y;
   }
 }
+
+struct CapFactors {
+  float k[kMaxLocal * kMaxLocal];
+};
 
 template <int NK, int CELLS>
 __global__ void __launch_bounds__(kSt4Threads) stencil32_kernel(const float2* __restrict__ xh,
                                                                 bf162* __restrict__ yh,
                                                                 const float* __restrict__ betar,
-                                                                const float* __restrict__ betai, int nxi, int ne4,
-                                                                int n_el, const int* __restrict__ mask) {
+                                                                const float* __restrict__ cap, const CapFactors cf,
+                                                                int nxi, int ne4, int n_el,
+                                                                const int* __restrict__ mask) {
   static_assert(CELLS == 2 || CELLS == 4, "two or four cells per thread");
+  constexpr int NP = pair_count(NK);
   const int be = blockIdx.x;
   if (mask && !mask[be / n_el]) return;
   const int lane = threadIdx.x & 31;
@@ -298,75 +305,81 @@ __global__ void __launch_bounds__(kSt4Threads) stencil32_kernel(const float2* __
   const bool valid = s0 < nxi;                       // nxi % 4 == 0: then all CELLS cells are
   const bool edge = lane == 31 || s0 + CELLS >= nxi;  // s0 + CELLS not held by the next lane
   const float2* X = xh + (long long)be * NK * nxi;
+  const float* br = betar + (long long)be * NP * ne4;
   const float2 z2 = make_float2(0.f, 0.f);
-  float2 sm[NK][CELLS], sp[NK][CELLS];
+  float2 x[NK][CELLS], xm[NK], xp[NK];
+  float w[NP][CELLS + 1], cp[CELLS + 1];
 #pragma unroll
   for (int c = 0; c < NK; ++c) {
-    float2 x[CELLS];
 #pragma unroll
     for (int h = 0; h < CELLS / 2; ++h) {
       float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (valid) t = *reinterpret_cast<const float4*>(X + c * nxi + s0 + 2 * h);
-      x[2 * h] = make_float2(t.x, t.y);
-      x[2 * h + 1] = make_float2(t.z, t.w);
+      if (valid) t = __ldg(reinterpret_cast<const float4*>(X + c * nxi + s0 + 2 * h));
+      x[c][2 * h] = make_float2(t.x, t.y);
+      x[c][2 * h + 1] = make_float2(t.z, t.w);
     }
-    float2 xm, xp;
-    xm.x = __shfl_up_sync(0xffffffffu, x[CELLS - 1].x, 1);
-    xm.y = __shfl_up_sync(0xffffffffu, x[CELLS - 1].y, 1);
-    xp.x = __shfl_down_sync(0xffffffffu, x[0].x, 1);
-    xp.y = __shfl_down_sync(0xffffffffu, x[0].y, 1);
-    if (lane == 0) xm = (valid && s0 > 0) ? X[c * nxi + s0 - 1] : z2;
-    if (edge) xp = (valid && s0 + CELLS < nxi) ? X[c * nxi + s0 + CELLS] : z2;
-    if (s0 == 0) xm = z2;
+    xm[c] = lane == 0 && valid && s0 > 0 ? X[c * nxi + s0 - 1] : z2;
+    xp[c] = edge && valid && s0 + CELLS < nxi ? X[c * nxi + s0 + CELLS] : z2;
+  }
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+#pragma unroll
+    for (int j = 0; j < CELLS; ++j) w[p][j] = 0.f;
+    if (valid) ld_cells<CELLS>(br + p * ne4 + s0, w[p]);
+    w[p][CELLS] = edge && valid ? br[p * ne4 + s0 + CELLS] : 0.f;
+  }
+#pragma unroll
+  for (int j = 0; j < CELLS; ++j) cp[j] = 0.f;
+  if (valid) ld_cells<CELLS>(cap + s0, cp);
+  cp[CELLS] = valid ? cap[s0 + CELLS] : 0.f;
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    const float n = __shfl_down_sync(0xffffffffu, w[p][0], 1);
+    if (!edge) w[p][CELLS] = n;
+  }
+  float2 y[NK][CELLS];
+#pragma unroll
+  for (int a = 0; a < NK; ++a)
+#pragma unroll
+    for (int j = 0; j < CELLS; ++j) y[a][j] = z2;
+#pragma unroll
+  for (int c = 0; c < NK; ++c) {
+    float2 m, p;
+    m.x = __shfl_up_sync(0xffffffffu, x[c][CELLS - 1].x, 1);
+    m.y = __shfl_up_sync(0xffffffffu, x[c][CELLS - 1].y, 1);
+    p.x = __shfl_down_sync(0xffffffffu, x[c][0].x, 1);
+    p.y = __shfl_down_sync(0xffffffffu, x[c][0].y, 1);
+    if (lane == 0) m = xm[c];
+    if (edge) p = xp[c];
 #pragma unroll
     for (int j = 0; j < CELLS; ++j) {
-      sm[c][j] = f2add(x[j], j == 0 ? xm : x[j - 1]);
-      sp[c][j] = f2add(x[j], j == CELLS - 1 ? xp : x[j + 1]);
+      const float2 l = j == 0 ? m : x[c][j - 1], r = j == CELLS - 1 ? p : x[c][j + 1];
+      const float2 sm = make_float2(x[c][j].x + l.x, x[c][j].y + l.y);
+      const float2 sp = make_float2(x[c][j].x + r.x, x[c][j].y + r.y);
+      const float2 u = make_float2(fmaf(cp[j], sm.x, cp[j + 1] * sp.x), fmaf(cp[j], sm.y, cp[j + 1] * sp.y));
+#pragma unroll
+      for (int a = 0; a < NK; ++a) {
+        const int q = pair_index(NK, a < c ? a : c, a < c ? c : a);
+        const float k = cf.k[a * NK + c];
+        y[a][j].x = fmaf(w[q][j], sm.x, fmaf(w[q][j + 1], sp.x, fmaf(-k, u.y, y[a][j].x)));
+        y[a][j].y = fmaf(w[q][j], sm.y, fmaf(w[q][j + 1], sp.y, fmaf(k, u.x, y[a][j].y)));
+      }
     }
   }
-  const float* br = betar + (long long)be * pair_count(NK) * ne4;
+  if (!valid) return;
   bf162* Y = yh + (long long)be * NK * nxi;
 #pragma unroll
   for (int a = 0; a < NK; ++a) {
-    float vx[CELLS], vy[CELLS];
+    uint32_t o[CELLS];
 #pragma unroll
-    for (int j = 0; j < CELLS; ++j) vx[j] = vy[j] = 0.f;
-#pragma unroll
-    for (int c = 0; c < NK; ++c) {
-      const float* rr = br + pair_index(NK, a < c ? a : c, a < c ? c : a) * ne4;
-      const float* ri = betai + (a * NK + c) * ne4;
-      float r0[CELLS], i0[CELLS];
-#pragma unroll
-      for (int j = 0; j < CELLS; ++j) r0[j] = i0[j] = 0.f;
-      if (valid) {
-        ld_cells<CELLS>(rr + s0, r0);
-        ld_cells<CELLS>(ri + s0, i0);
-      }
-      // the weight of edge s0 + CELLS: the next lane's first, loaded at the warp's edge
-      float rn = __shfl_down_sync(0xffffffffu, r0[0], 1), in = __shfl_down_sync(0xffffffffu, i0[0], 1);
-      if (edge) {
-        rn = valid ? rr[s0 + CELLS] : 0.f;
-        in = valid ? ri[s0 + CELLS] : 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < CELLS; ++j) {
-        const float b1r = j == CELLS - 1 ? rn : r0[j + 1], b1i = j == CELLS - 1 ? in : i0[j + 1];
-        vx[j] += r0[j] * sm[c][j].x - i0[j] * sm[c][j].y + b1r * sp[c][j].x - b1i * sp[c][j].y;
-        vy[j] += r0[j] * sm[c][j].y + i0[j] * sm[c][j].x + b1r * sp[c][j].y + b1i * sp[c][j].x;
-      }
+    for (int j = 0; j < CELLS; ++j) {
+      bf162 t = __floats2bfloat162_rn(y[a][j].x, y[a][j].y);
+      o[j] = *reinterpret_cast<uint32_t*>(&t);
     }
-    if (valid) {
-      uint32_t o[CELLS];
-#pragma unroll
-      for (int j = 0; j < CELLS; ++j) {
-        bf162 t = __floats2bfloat162_rn(vx[j], vy[j]);
-        o[j] = *reinterpret_cast<uint32_t*>(&t);
-      }
-      if constexpr (CELLS == 4)
-        *reinterpret_cast<uint4*>(Y + a * nxi + s0) = make_uint4(o[0], o[1], o[2], o[3]);
-      else
-        *reinterpret_cast<uint2*>(Y + a * nxi + s0) = make_uint2(o[0], o[1]);
-    }
+    if constexpr (CELLS == 4)
+      *reinterpret_cast<uint4*>(Y + a * nxi + s0) = make_uint4(o[0], o[1], o[2], o[3]);
+    else
+      *reinterpret_cast<uint2*>(Y + a * nxi + s0) = make_uint2(o[0], o[1]);
   }
 }
 
@@ -376,12 +389,11 @@ void launch_stencil32(Problem& P, const int* mask) {
   MixedBuffers& M = P.mx;
   const int cells = P.st_cells == 2 ? 2 : 4;
   const dim3 grid((unsigned)(P.batch * s.n_el), (unsigned)((s.nxi + cells * kSt4Threads - 1) / (cells * kSt4Threads)));
-  if (cells == 2)
-    stencil32_kernel<NK, 2><<<grid, kSt4Threads, 0, P.stream>>>(reinterpret_cast<const float2*>(M.xh), M.yh16,
-                                                                M.beta, M.betai, s.nxi, M.ne4, s.n_el, mask);
-  else
-    stencil32_kernel<NK, 4><<<grid, kSt4Threads, 0, P.stream>>>(reinterpret_cast<const float2*>(M.xh), M.yh16,
-                                                                M.beta, M.betai, s.nxi, M.ne4, s.n_el, mask);
+  CapFactors cf;
+  for (int i = 0; i < NK * NK; ++i) cf.k[i] = M.capk[i];
+  auto kern = cells == 2 ? stencil32_kernel<NK, 2> : stencil32_kernel<NK, 4>;
+  kern<<<grid, kSt4Threads, 0, P.stream>>>(reinterpret_cast<const float2*>(M.xh), M.yh16, M.beta, M.cap, cf, s.nxi,
+                                           M.ne4, s.n_el, mask);
 }
 
 // FP32 packed copies of the potential weights: out[r][p][s] = beta[r][a*nK+c][s] for the
@@ -585,6 +597,7 @@ int mixed_alloc(Problem& P) {
   M.ne4 = (s.nxi + 1 + 3) & ~3;
   alloc((void**)&M.beta, sizeof(float) * (size_t)P.batch * s.n_el * pair_count(s.nK) * M.ne4);
   alloc((void**)&M.betai, sizeof(float) * (size_t)s.nK * s.nK * M.ne4);
+  alloc((void**)&M.cap, sizeof(float) * M.ne4);
   alloc((void**)&M.err, sizeof(int));
   alloc((void**)&M.kvec, sizeof(float) * s.nk);
   alloc((void**)&M.qd, sizeof(float) * P.batch);
@@ -610,6 +623,9 @@ int mixed_alloc(Problem& P) {
     M.fb.K3c[a] = (float)P.fb.K3c[a];
     M.fb.K5c[a] = (float)P.fb.K5c[a];
   }
+  std::vector<float> cap(M.ne4, 0.f);
+  for (int i = 0; i <= s.nxi; ++i) cap[i] = (float)s.cap[i];
+  for (int ac = 0; ac < s.nK * s.nK; ++ac) M.capk[ac] = (float)(-(s.delta_xi / 4 * s.mpc) * s.kap_sum[ac]);
   P.device_bytes += bytes;
   cudaMemsetAsync(M.err, 0, sizeof(int), P.stream);
   // BF16 real embeddings of Phi (GEMM 1) and i Phi^H (GEMM 2), interleaved (re, im) along both axes
@@ -631,7 +647,8 @@ int mixed_alloc(Problem& P) {
       a2[(2 * j + 1) * K2 + 2 * si + 0] = __float2bfloat16((float)pr);
       a2[(2 * j + 1) * K2 + 2 * si + 1] = __float2bfloat16((float)pi);
     }
-  e = cudaMemcpyAsync(M.phi1, a1.data(), sizeof(bf16) * a1.size(), cudaMemcpyHostToDevice, P.stream);
+  e = cudaMemcpyAsync(M.cap, cap.data(), sizeof(float) * cap.size(), cudaMemcpyHostToDevice, P.stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(M.phi1, a1.data(), sizeof(bf16) * a1.size(), cudaMemcpyHostToDevice, P.stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(M.phi2, a2.data(), sizeof(bf16) * a2.size(), cudaMemcpyHostToDevice, P.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(P.stream);
   if (e != cudaSuccess) {
@@ -726,7 +743,7 @@ int ozaki_alloc(Problem& P) {
 
 void mixed_free(Problem& P) {
   MixedBuffers& M = P.mx;
-  void* ptrs[] = {M.phi1, M.phi2, M.xin16, M.zb16, M.yh16, M.xh, M.V, M.Vh, M.w, M.z, M.r, M.d, M.beta, M.betai,
+  void* ptrs[] = {M.phi1, M.phi2, M.xin16, M.zb16, M.yh16, M.xh, M.V, M.Vh, M.w, M.z, M.r, M.d, M.beta, M.betai, M.cap,
                   M.err, M.kvec, M.qd, M.dinv, M.h, M.hcol, M.y, M.inv, M.oa1, M.oa2, M.ea1, M.ea2, M.ob, M.eb};
   for (void* p : ptrs)
     if (p) cudaFree(p);

@@ -89,6 +89,9 @@ struct MixedBuffers {
   // betai [nK*nK][ne4] the CAP part
   float* beta = nullptr;
   float* betai = nullptr;
+  // betai is a product: betai[a nK + c][s] = capk[a nK + c] cap[s] (the absorbing layers' profile over the xi edges)
+  float* cap = nullptr;              // [ne4]
+  float capk[kMaxLocal * kMaxLocal] = {};
   int ne4 = 0;
   float* kvec = nullptr;             // [nk]
   float* qd = nullptr;               // [B]

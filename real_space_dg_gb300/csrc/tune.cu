@@ -96,7 +96,8 @@ int autotune(Problem& P) {
     if (e != cudaSuccess) break;
     P.kline_L = L;
     const float ms = time_ms(P, a, b, [&]() {
-      return mixed ? launch_precondition_mixed(P, P.mx.d, N, P.mx.z, P.mx.zb16, nullptr)
+      return mixed ? launch_precondition_mixed(P, P.mx.d, N, flux_is_inverted(P) && !P.mx.fused ? nullptr : P.mx.z,
+                                               P.mx.zb16, nullptr)
                    : launch_precondition(P, P.w, N, P.z);
     }, reps, e);
     if (e == cudaSuccess && ms < best_ms) {
