@@ -111,15 +111,35 @@ unsigned slice_blocks(long long ncol) {
 
 template <int EPI>
 cudaError_t launch_ozaki(const CUtensorMap& a, const CUtensorMap& b, const int* ea, const int* eb, double* C, int M,
-                         long long Ncol, int K, int* err, cudaStream_t st, const int* mask = nullptr,
-                         int cols_per_problem = 1, int nd = oz::S, const int* nd_pp = nullptr) {
+                         long long Ncol, int K, int* err, cudaStream_t st, int nd = oz::S) {
   static const cudaError_t attr = cudaFuncSetAttribute(oz::gemm_ozaki_kernel<EPI>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, oz::SMEM_BYTES);
   if (attr != cudaSuccess) return attr;
   if (nd < 1 || nd > oz::S) return cudaErrorInvalidValue;
   dim3 grid((M + oz::BM - 1) / oz::BM, (unsigned)((Ncol + oz::BN - 1) / oz::BN));
-  oz::gemm_ozaki_kernel<EPI><<<grid, oz::THREADS, oz::SMEM_BYTES, st>>>(a, b, ea, eb, C, M, Ncol, K, err, mask,
-                                                                 cols_per_problem, nd, nd_pp);
+  oz::gemm_ozaki_kernel<EPI><<<grid, oz::THREADS, oz::SMEM_BYTES, st>>>(a, b, ea, eb, C, M, Ncol, K, err, nd);
+  return cudaGetLastError();
+}
+
+// Row length of the pair digits of K complex entries: K / 2 in whole 16-byte TMA rows, one k block at least.
+int pair_row(int K) { return std::max(oz::BK, (K / 2 + 7) & ~7); }
+
+// Y = Phi X (MODE 0) or Y += i Phi^H X (MODE 1) on the tensor cores: slicing and gemm_pairs_kernel.  X: K complex entries
+// per column, Y: M.
+template <int MODE>
+cudaError_t launch_pairs(Problem& P, const CUtensorMap& a, const CUtensorMap& b, const int* ea, const double2* X,
+                         double2* Y, int K, int M, const int* mask, int nd, const int* nd_pp) {
+  static const cudaError_t attr = cudaFuncSetAttribute(oz::gemm_pairs_kernel<MODE>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, oz::SMEM_BYTES);
+  if (attr != cudaSuccess) return attr;
+  if (nd < 1 || nd > oz::S) return cudaErrorInvalidValue;
+  const int npp = (int)(P.ncols / P.batch), Kp = pair_row(K);
+  auto slice = Kp <= 64 ? oz::slice_pairs_kernel<1> : Kp <= 128 ? oz::slice_pairs_kernel<2> : oz::slice_pairs_kernel<4>;
+  slice<<<slice_blocks(P.ncols), 32 * oz::kSliceColsPerBlock, 0, P.stream>>>(
+      X, K, P.ncols, P.mx.ob, P.mx.eb, mask, npp, Kp, nd, nd_pp);
+  const dim3 grid((M / 2 + oz::BM - 1) / oz::BM, (unsigned)((2 * P.ncols + oz::BN - 1) / oz::BN));
+  oz::gemm_pairs_kernel<MODE><<<grid, oz::PAIR_THREADS, oz::SMEM_BYTES, P.stream>>>(
+      a, b, ea, P.mx.eb, Y, M, 2 * P.ncols, Kp, P.mx.err, mask, 2 * npp, nd, nd_pp);
   return cudaGetLastError();
 }
 
@@ -691,36 +711,32 @@ int ozaki_alloc(Problem& P) {
   // exact grouped accumulation (K <= MAX_K) and 16-byte TMA rows of the digit slices
   M.ozaki = 2 * nk <= oz::MAX_K && 2 * nxi <= oz::MAX_K && nk % 4 == 0 && nxi % 4 == 0;
   if (M.ozaki) {
-    const int kmax = 2 * std::max(nk, nxi);
-    std::vector<double> A1((size_t)4 * nxi * nk), A2((size_t)4 * nxi * nk);
-    for (int si = 0; si < nxi; ++si)
-      for (int j = 0; j < nk; ++j) {
-        const double pr = s.phi[(size_t)si * nk + j].real(), pi = s.phi[(size_t)si * nk + j].imag();
-        const size_t K1 = 2 * (size_t)nk, K2 = 2 * (size_t)nxi;
-        A1[(2 * si + 0) * K1 + 2 * j + 0] = pr;
-        A1[(2 * si + 0) * K1 + 2 * j + 1] = -pi;
-        A1[(2 * si + 1) * K1 + 2 * j + 0] = pi;
-        A1[(2 * si + 1) * K1 + 2 * j + 1] = pr;
-        A2[(2 * j + 0) * K2 + 2 * si + 0] = pi;
-        A2[(2 * j + 0) * K2 + 2 * si + 1] = -pr;
-        A2[(2 * j + 1) * K2 + 2 * si + 0] = pr;
-        A2[(2 * j + 1) * K2 + 2 * si + 1] = pi;
+    // lower halves of the symmetric basis (gemm_pairs_kernel): real parts, then imaginary parts
+    const int hk = nk / 2, hs = nxi / 2, K1 = pair_row(nk), K2 = pair_row(nxi), kmax = std::max(K1, K2);
+    std::vector<double> A1((size_t)2 * hs * K1, 0.0), A2((size_t)2 * hk * K2, 0.0);
+    for (int si = 0; si < hs; ++si)
+      for (int j = 0; j < hk; ++j) {
+        const cplx v = s.phi[(size_t)si * nk + j];
+        A1[(size_t)si * K1 + j] = v.real();
+        A1[(size_t)(hs + si) * K1 + j] = v.imag();
+        A2[(size_t)j * K2 + si] = v.real();
+        A2[(size_t)(hk + j) * K2 + si] = v.imag();
       }
     std::vector<bf16> d1, d2;
     std::vector<int> e1, e2;
-    slice_rows_host(A1, 2 * nxi, 2 * nk, d1, e1);
-    slice_rows_host(A2, 2 * nk, 2 * nxi, d2, e2);
+    slice_rows_host(A1, 2 * hs, K1, d1, e1);
+    slice_rows_host(A2, 2 * hk, K2, d2, e2);
     cudaError_t ce = cudaSuccess;
     auto C2 = [&](cudaError_t r) { if (ce == cudaSuccess) ce = r; };
     C2(cudaMalloc(&M.oa1, sizeof(bf16) * d1.size()));
     C2(cudaMalloc(&M.oa2, sizeof(bf16) * d2.size()));
     C2(cudaMalloc(&M.ea1, sizeof(int) * e1.size()));
     C2(cudaMalloc(&M.ea2, sizeof(int) * e2.size()));
-    C2(cudaMalloc(&M.ob, sizeof(bf16) * (size_t)oz::S * P.ncols * kmax));
-    C2(cudaMalloc(&M.eb, sizeof(int) * (size_t)P.ncols));
+    C2(cudaMalloc(&M.ob, sizeof(bf16) * (size_t)oz::S * 4 * P.ncols * kmax));
+    C2(cudaMalloc(&M.eb, sizeof(int) * (size_t)4 * P.ncols));
     // columns of masked problems are not re-sliced: keep them finite from the start
-    C2(cudaMemset(M.ob, 0, sizeof(bf16) * (size_t)oz::S * P.ncols * kmax));
-    C2(cudaMemset(M.eb, 0, sizeof(int) * (size_t)P.ncols));
+    C2(cudaMemset(M.ob, 0, sizeof(bf16) * (size_t)oz::S * 4 * P.ncols * kmax));
+    C2(cudaMemset(M.eb, 0, sizeof(int) * (size_t)4 * P.ncols));
     C2(cudaMemcpy(M.oa1, d1.data(), sizeof(bf16) * d1.size(), cudaMemcpyHostToDevice));
     C2(cudaMemcpy(M.oa2, d2.data(), sizeof(bf16) * d2.size(), cudaMemcpyHostToDevice));
     C2(cudaMemcpy(M.ea1, e1.data(), sizeof(int) * e1.size(), cudaMemcpyHostToDevice));
@@ -730,9 +746,9 @@ int ozaki_alloc(Problem& P) {
       return ce == cudaErrorMemoryAllocation ? WG_ERR_OOM : WG_ERR_CUDA;
     }
     P.device_bytes += 2.0 * (d1.size() + d2.size()) + 4.0 * (e1.size() + e2.size()) +
-                      2.0 * oz::S * P.ncols * kmax + 4.0 * P.ncols;
-    ok = make_map3(&M.tmOA1, M.oa1, 2 * nxi, 2 * nk, oz::BM) && make_map3(&M.tmOA2, M.oa2, 2 * nk, 2 * nxi, oz::BM) &&
-         make_map3(&M.tmOB1, M.ob, P.ncols, 2 * nk, oz::BN) && make_map3(&M.tmOB2, M.ob, P.ncols, 2 * nxi, oz::BN);
+                      2.0 * oz::S * 4 * P.ncols * kmax + 16.0 * P.ncols;
+    ok = make_map3(&M.tmOA1, M.oa1, 2 * hs, K1, oz::BM) && make_map3(&M.tmOA2, M.oa2, 2 * hk, K2, oz::BM) &&
+         make_map3(&M.tmOB1, M.ob, 4 * P.ncols, K1, oz::BN) && make_map3(&M.tmOB2, M.ob, 4 * P.ncols, K2, oz::BN);
     if (!ok) {
       P.err = "cuTensorMapEncodeTiled failed for the FP64 tensor-core operands";
       return WG_ERR_CUDA;
@@ -929,29 +945,21 @@ cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const 
   MixedBuffers& M = P.mx;
   if (!M.ozaki) return launch_apply(P, x, y);
   const Shape& s = P.s;
-  const int K1 = 2 * s.nk, K2 = 2 * s.nxi;
   const double ncols = (double)P.ncols;
-  const int cpp = (int)(P.ncols / P.batch);   // columns (element, node) of one problem
   cudaError_t e = launch_flux_f64(P, x, y, mask);
   if (e != cudaSuccess) return e;
-  // work of one GEMM: read the FP64 operand (slicing), write the FP64 result; flops of
-  // ONE real-embedded BF16 digit-slice product, weighted by the products the digits need
-  const double prod_flops = 2.0 * (2.0 * s.nxi) * (2.0 * s.nk) * ncols;
+  // work of one transform: read the FP64 operand (slicing), write the FP64 result; flops of
+  // ONE BF16 digit-slice product of both planes, weighted by the products the digits need
+  const double prod_flops = 2.0 * (2.0 * s.nxi) * (2.0 * s.nk) * ncols / 4;
   cudaEvent_t ev = prof_begin(P, PROF_GEMM_F64TC, 2, 8.0 * P.N * P.batch + 16.0 * s.nxi * ncols, prod_flops, mask,
                               nd, nd_pp);
-  oz::slice_columns_kernel<<<slice_blocks(P.ncols), 32 * oz::kSliceColsPerBlock, 0, P.stream>>>(
-      reinterpret_cast<const double*>(x), K1, P.ncols, M.ob, M.eb, mask, cpp, 0, nd, nd_pp);
-  e = launch_ozaki<0>(M.tmOA1, M.tmOB1, M.ea1, M.eb, reinterpret_cast<double*>(P.xh), K2, P.ncols, K1, M.err,
-                      P.stream, mask, cpp, nd, nd_pp);
+  e = launch_pairs<0>(P, M.tmOA1, M.tmOB1, M.ea1, x, P.xh, s.nk, s.nxi, mask, nd, nd_pp);
   prof_end(P, PROF_GEMM_F64TC, ev);
   if (e != cudaSuccess) return e;
   e = launch_stencil_f64(P, P.xh, P.yh, mask);
   if (e != cudaSuccess) return e;
   ev = prof_begin(P, PROF_GEMM_F64TC, 2, 16.0 * s.nxi * ncols + 16.0 * P.N * P.batch, prod_flops, mask, nd, nd_pp);
-  oz::slice_columns_kernel<<<slice_blocks(P.ncols), 32 * oz::kSliceColsPerBlock, 0, P.stream>>>(
-      reinterpret_cast<const double*>(P.yh), K2, P.ncols, M.ob, M.eb, mask, cpp, 0, nd, nd_pp);
-  e = launch_ozaki<1>(M.tmOA2, M.tmOB2, M.ea2, M.eb, reinterpret_cast<double*>(y), K1, P.ncols, K2, M.err, P.stream,
-                      mask, cpp, nd, nd_pp);
+  e = launch_pairs<1>(P, M.tmOA2, M.tmOB2, M.ea2, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp);
   prof_end(P, PROF_GEMM_F64TC, ev);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
@@ -990,7 +998,7 @@ int debug_gemm_f64_tc(const double* A, const double* B, double* C, int M, int N,
       rc = WG_ERR_CUDA;
     } else {
       oz::slice_columns_kernel<<<slice_blocks(N), 32 * oz::kSliceColsPerBlock>>>(dB, K, N, db, deb);
-      e = launch_ozaki<0>(ma, mb, dea, deb, dC, M, N, K, derr, 0, nullptr, 1, nd);
+      e = launch_ozaki<0>(ma, mb, dea, deb, dC, M, N, K, derr, 0, nd);
       if (e == cudaSuccess) e = cudaDeviceSynchronize();
       int herr = 0;
       if (e == cudaSuccess) e = cudaMemcpy(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost);
@@ -1085,7 +1093,7 @@ cudaError_t ozaki_accumulate(const OzakiRowsDev& A, OzakiColsDev& B, const doubl
                              cudaStream_t st) {
   if (B.Kp != A.Kp) return cudaErrorInvalidValue;
   oz::slice_columns_kernel<<<slice_blocks(B.ncol), 32 * oz::kSliceColsPerBlock, 0, st>>>(X, A.K, B.ncol, B.dig, B.e,
-                                                                                        nullptr, 1, B.Kp);
+                                                                                        B.Kp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_ozaki<1>(A.map, B.map, A.e, B.e, C, A.M, B.ncol, A.Kp, err, st);
@@ -1095,7 +1103,7 @@ cudaError_t ozaki_multiply(const OzakiRowsDev& A, OzakiColsDev& B, const double*
                            cudaStream_t st) {
   if (B.Kp != A.Kp) return cudaErrorInvalidValue;
   oz::slice_columns_kernel<<<slice_blocks(B.ncol), 32 * oz::kSliceColsPerBlock, 0, st>>>(X, A.K, B.ncol, B.dig, B.e,
-                                                                                        nullptr, 1, B.Kp);
+                                                                                        B.Kp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_ozaki<0>(A.map, B.map, A.e, B.e, C, A.M, B.ncol, A.Kp, err, st);

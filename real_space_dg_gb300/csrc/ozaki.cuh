@@ -125,24 +125,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ozaki_kernel(const __grid_con
                                                             const __grid_constant__ CUtensorMap tmB,
                                                             const int* __restrict__ ea, const int* __restrict__ eb,
                                                             double* __restrict__ C, int M, long long Ncol, int K,
-                                                            int* __restrict__ err, const int* __restrict__ mask,
-                                                            int cols_per_problem, int nd,
-                                                            const int* __restrict__ nd_pp) {
+                                                            int* __restrict__ err, int nd) {
   // nd (1 .. S): leading digits used of each operand (products of weight < nd); the error grows
-  // to ~2^(-6 nd) of |A||B|.  nd_pp (optional): digits per problem, the tile takes the largest of
-  // its problems.  A column tile whose problems are all inactive has nothing to compute.
-  if (mask || nd_pp) {
-    const long long c0 = (long long)blockIdx.y * BN, c1 = min(Ncol, c0 + BN) - 1;
-    bool any = false;
-    int ndt = 1;
-    for (long long b = c0 / cols_per_problem; b <= c1 / cols_per_problem; ++b) {
-      const bool on = !mask || mask[b] != 0;
-      any |= on;
-      if (nd_pp && on) ndt = max(ndt, min(S, max(1, nd_pp[b])));
-    }
-    if (!any) return;
-    if (nd_pp) nd = ndt;
-  }
+  // to ~2^(-6 nd) of |A||B|
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // stage s: [nd][BM][BK] bf16 A slices, then [nd][BN][BK] bf16 B slices
@@ -278,23 +263,11 @@ __global__ void __launch_bounds__(32 * kSliceColsPerBlock) slice_columns_kernel(
                                                                                long long Ncol,
                                                                                __nv_bfloat16* __restrict__ slices,
                                                                                int* __restrict__ e_out,
-                                                                               const int* __restrict__ mask = nullptr,
-                                                                               int cols_per_problem = 1,
-                                                                               int Kout = 0, int nd = S,
-                                                                               const int* __restrict__ nd_pp = nullptr) {
+                                                                               int Kout = 0) {
   // Kout: row length of the slices (>= K, zero-padded; 0: K), for 16-byte TMA rows.
-  // nd, nd_pp: the digits gemm_ozaki_kernel reads for the column's 64-column tile (the same
-  // rule: nd_pp's largest over the tile's active problems, else nd); only those are written
   const int lane = threadIdx.x & 31;
   const long long c = (long long)blockIdx.x * kSliceColsPerBlock + (threadIdx.x >> 5);
-  if (c >= Ncol || (mask && !mask[c / cols_per_problem])) return;
-  int ndt = nd < 1 ? 1 : (nd > S ? S : nd);
-  if (nd_pp) {
-    const long long c0 = c / BN * BN, c1 = min(Ncol, c0 + BN) - 1;
-    ndt = 1;
-    for (long long b = c0 / cols_per_problem; b <= c1 / cols_per_problem; ++b)
-      if (!mask || mask[b] != 0) ndt = max(ndt, min(S, max(1, nd_pp[b])));
-  }
+  if (c >= Ncol) return;
   const int Ko = Kout > K ? Kout : K;
   const double2* x = reinterpret_cast<const double2*>(X + c * (long long)K);
   const int K2 = K / 2;
@@ -325,11 +298,252 @@ __global__ void __launch_bounds__(32 * kSliceColsPerBlock) slice_columns_kernel(
 #pragma unroll
     for (int p = S - 1; p > 0; --p) {
       const int d0 = (int)(((F0 + 32) & 63) - 32), d1 = (int)(((F1 + 32) & 63) - 32);
-      if (p < ndt) out[p * (slice_stride / 2) + k] = __floats2bfloat162_rn((float)d0, (float)d1);
+      out[p * (slice_stride / 2) + k] = __floats2bfloat162_rn((float)d0, (float)d1);
       F0 = (F0 - d0) >> BETA;
       F1 = (F1 - d1) >> BETA;
     }
     out[k] = __floats2bfloat162_rn((float)F0, (float)F1);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The plane-wave transforms of the 1D operator with the same digits.  Phi(m, p) = c + i d is symmetric under k -> -k and
+// xi -> -xi, so with E = x_p + x_p' and O = x_p - x_p' of the mirror pairs (p, p')
+//   A = sum_p c E, B = sum_p d O,   X^(m) = A + i B, X^(m') = A - i B
+// (the adjoint i Phi^H: A - i B and A + i B), two real matrices of half the rows and columns instead of
+// the 2 x 2 real embedding of a complex one: a quarter of the digit products, an eighth of the table.
+//   B operand: real columns 2 c + (0 re, 1 im) of node c, plane 0 = E, plane 1 = O: rows plane 2 ncols + 2 c + o
+//   A operand: rows plane hm + m, hm = M / 2 (plane 0 = c, plane 1 = d)
+// One CTA computes A, drains TMEM to FP64 registers, computes B into the same accumulators (its first loads are in
+// flight meanwhile), and writes both members of every output pair.  Warps 0 .. 15 drain, 16 loads, 17 issues.
+//   MODE 0: Y = Phi X.   MODE 1: Y += i Phi^H X.
+// The table's digits dominated the L2 traffic of the embedded product (1 MB per 64 nodes, a quarter of it per CTA;
+// now 0.5 MB per 32 nodes for both planes).  With slicing, per transform: 333 -> 219 us (16 problems of 960 nodes,
+// 256 x 256; slicing 55 of it), 240 -> 158 us (4 of 720 nodes, 512 x 512: 180 CTAs on 152 SMs).
+// ---------------------------------------------------------------------------------------------
+constexpr int PAIR_THREADS = THREADS + 64;
+
+template <int MODE>
+__global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pairs_kernel(
+    const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const int* __restrict__ ea,
+    const int* __restrict__ eb, double2* __restrict__ Y, int M, long long Ncol2, int K, int* __restrict__ err,
+    const int* __restrict__ mask, int cols_per_problem, int nd, const int* __restrict__ nd_pp) {
+  // Ncol2, cols_per_problem: real columns (two per node).  nd (1 .. S): leading digits used of each operand; nd_pp
+  // (optional): digits per problem, the tile takes the largest of its problems.  A column tile whose
+  // problems are all inactive has nothing to compute.
+  if (mask || nd_pp) {
+    const long long c0 = (long long)blockIdx.y * BN, c1 = min(Ncol2, c0 + BN) - 1;
+    bool any = false;
+    int ndt = 1;
+    for (long long b = c0 / cols_per_problem; b <= c1 / cols_per_problem; ++b) {
+      const bool on = !mask || mask[b] != 0;
+      any |= on;
+      if (nd_pp && on) ndt = max(ndt, min(S, max(1, nd_pp[b])));
+    }
+    if (!any) return;
+    if (nd_pp) nd = ndt;
+  }
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int ns = stages_for(nd);
+  const int stage = nd * (A_SLICE + B_SLICE);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + RING);
+  uint64_t* empty = full + MAX_STAGES;
+  uint64_t* done = empty + MAX_STAGES;   // [2] the accumulators of a plane are complete
+  uint64_t* drained = done + 2;          // plane 0 has been read out of TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int hm = M / 2, m0 = blockIdx.x * BM;
+  const long long n0 = (long long)blockIdx.y * BN;
+  const int nkb = (K + BK - 1) / BK;
+
+  if (threadIdx.x == 0) {
+    for (int st = 0; st < ns; ++st) {
+      tc::mbar_init(&full[st], 1);
+      tc::mbar_init(&empty[st], 1);
+    }
+    tc::mbar_init(&done[0], 1);
+    tc::mbar_init(&done[1], 1);
+    tc::mbar_init(drained, THREADS / 32);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) tc::tmem_alloc(tmem_slot, 512);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == THREADS / 32) {
+    if (lane == 0)
+      for (int it = 0; it < 2 * nkb; ++it) {
+        const int st = it % ns, ph = it / nkb, kb = it - ph * nkb;
+        if (it >= ns && !tc::mbar_wait(&empty[st], ((it / ns) + 1) & 1, err)) break;
+        uint8_t* sa = smem + st * stage;
+        uint8_t* sb = sa + nd * A_SLICE;
+        tc::mbar_expect_tx(&full[st], (uint32_t)(nd * (A_SLICE + B_SLICE)));
+        for (int p = 0; p < nd; ++p) {
+          tma_load_3d(sa + p * A_SLICE, &tmA, kb * BK, ph * hm + m0, p, &full[st]);
+          tma_load_3d(sb + p * B_SLICE, &tmB, kb * BK, (int)(ph * Ncol2 + n0), p, &full[st]);
+        }
+      }
+  } else if (warp == THREADS / 32 + 1) {
+    if (lane == 0) {
+      bool ok = true;
+      for (int ph = 0; ph < 2 && ok; ++ph) {
+        if (ph == 1) {
+          ok = tc::mbar_wait(drained, 0, err);
+          tc::fence_after();
+        }
+        for (int kb = 0; kb < nkb && ok; ++kb) {
+          const int it = ph * nkb + kb, st = it % ns;
+          if (!(ok = tc::mbar_wait(&full[st], (it / ns) & 1, err))) break;
+          tc::fence_after();
+          const uint8_t* sa = smem + st * stage;
+          const uint8_t* sb = sa + nd * A_SLICE;
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk)
+            for (int p = 0; p < nd; ++p)
+              for (int q0 = 0; q0 + p < nd; q0 += kSlicesPerMma) {   // as in gemm_ozaki_kernel
+                const int n = min(kSlicesPerMma, nd - p - q0);
+                tc::mma_bf16(tmem + (uint32_t)((p + q0) * BN), sdesc_sw64(sa + p * A_SLICE + kk * 32),
+                             sdesc_sw64(sb + q0 * B_SLICE + kk * 32), idesc_n(n * BN),
+                             (kb > 0 || kk > 0 || p > 0) ? 1u : 0u);
+              }
+          tc::mma_commit(&empty[st]);
+        }
+        if (ok) tc::mma_commit(&done[ph]);
+      }
+    }
+  } else {
+    // warp w reads TMEM lanes 32 (w % 4) .. +31 (rows) and the 16 real columns (8 nodes) of block w / 4
+    constexpr int EC = EPI_COLS;
+    const int wq = warp & 3, cb = warp >> 2;
+    const int row = m0 + wq * 32 + lane;
+    const long long c0 = n0 + cb * EC;
+    const int ncb = (int)max(0ll, min((long long)EC, Ncol2 - c0));
+    double va[EC], vb[EC];
+    bool ok = true;
+#pragma unroll
+    for (int ph = 0; ph < 2; ++ph) {
+      if (ok) ok = tc::mbar_wait(&done[ph], 0, err);
+      tc::fence_after();
+      if (ok) {
+        long long fx[EC];
+#pragma unroll
+        for (int i = 0; i < EC; ++i) fx[i] = 0;
+#pragma unroll 1
+        for (int g = 0; g < nd; ++g) {
+          float v[EC];
+          tmem_ld16(tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(g * BN + cb * EC), v);
+#pragma unroll
+          for (int i = 0; i < EC; ++i) fx[i] += group_fixed(v[i], g);
+        }
+        const int er = (row < hm ? ea[ph * hm + row] : 0) - kFixBits;
+        const int* ebp = eb + ph * Ncol2 + c0;
+#pragma unroll
+        for (int i = 0; i < EC; ++i)
+          (ph == 0 ? va : vb)[i] = fixed_to_double(fx[i], er + (i < ncb ? ebp[i] : 0));
+      }
+      if (ph == 0) {
+        tc::fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(drained);
+      }
+    }
+    if (ok && !*(volatile int*)err && row < hm) {
+      double2* y = Y + c0 / 2 * M;
+      const int mr = M - 1 - row;
+#pragma unroll
+      for (int i = 0; i < EC / 2; ++i) {
+        if (2 * i >= ncb) continue;
+        const double ar = va[2 * i], ai = va[2 * i + 1], br = vb[2 * i], bi = vb[2 * i + 1];
+        double2* p = y + (long long)i * M + row;
+        double2* q = y + (long long)i * M + mr;
+        if (MODE == 0) {
+          *p = make_double2(ar - bi, ai + br);
+          *q = make_double2(ar + bi, ai - br);
+        } else {
+          const double2 op = *p, oq = *q;
+          *p = make_double2(op.x - (ai - br), op.y + (ar + bi));
+          *q = make_double2(oq.x - (ai + br), oq.y + (ar - bi));
+        }
+      }
+    }
+  }
+  tc::fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc::fence_after();
+    tc::tmem_dealloc(tmem, 512);
+  }
+}
+
+// Digits of E and O of every node's complex column (K entries, K even and at most 512), one warp per node, two
+// consecutive pairs per lane and pass; the four real columns stay in registers between their maxima and their digits.
+// Rows of Kout entries (>= K / 2, zero-padded).  nd, nd_pp: the digits gemm_pairs_kernel reads for the node's tile.
+// PASSES of 64 entries cover Kout (1, 2 or 4).
+template <int PASSES>
+__global__ void __launch_bounds__(32 * kSliceColsPerBlock) slice_pairs_kernel(
+    const double2* __restrict__ X, int K, long long ncols, __nv_bfloat16* __restrict__ slices, int* __restrict__ e_out,
+    const int* __restrict__ mask, int nodes_per_problem, int Kout, int nd, const int* __restrict__ nd_pp) {
+  const int lane = threadIdx.x & 31;
+  const long long c = (long long)blockIdx.x * kSliceColsPerBlock + (threadIdx.x >> 5);
+  if (c >= ncols || (mask && !mask[c / nodes_per_problem])) return;
+  int ndt = nd < 1 ? 1 : (nd > S ? S : nd);
+  if (nd_pp) {
+    constexpr int NT = BN / 2;
+    const long long c0 = c / NT * NT, c1 = min(ncols, c0 + NT) - 1;
+    ndt = 1;
+    for (long long b = c0 / nodes_per_problem; b <= c1 / nodes_per_problem; ++b)
+      if (!mask || mask[b] != 0) ndt = max(ndt, min(S, max(1, nd_pp[b])));
+  }
+  const int h = K / 2;
+  const double2* x = X + c * K;
+  double v[4][PASSES][2];   // E re, E im, O re, O im
+  unsigned long long mx[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int t = 0; t < PASSES; ++t)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int p = 64 * t + 2 * lane + u;
+      const bool in = p < h;
+      const double2 a = in ? x[p] : make_double2(0.0, 0.0), b = in ? x[K - 1 - p] : make_double2(0.0, 0.0);
+      v[0][t][u] = in ? a.x + b.x : 0.0;
+      v[1][t][u] = in ? a.y + b.y : 0.0;
+      v[2][t][u] = in ? a.x - b.x : 0.0;
+      v[3][t][u] = in ? a.y - b.y : 0.0;
+#pragma unroll
+      for (int o = 0; o < 4; ++o) {
+        const unsigned long long w = (unsigned long long)__double_as_longlong(v[o][t][u]) & 0x7FFFFFFFFFFFFFFFull;
+        mx[o] = w > mx[o] ? w : mx[o];
+      }
+    }
+  const long long Ncol2 = 2 * ncols, slice_stride = 2 * Ncol2 * (long long)Kout;
+#pragma unroll
+  for (int o = 0; o < 4; ++o) {
+    for (int q = 16; q > 0; q >>= 1) {
+      const unsigned long long t = __shfl_xor_sync(0xffffffffu, mx[o], q);
+      mx[o] = t > mx[o] ? t : mx[o];
+    }
+    const int m = mx[o] == 0 ? 0 : (int)((mx[o] >> 52) & 0x7FF) - 1023 + 1;   // max|x| < 2^m
+    const long long r = (o >> 1) * Ncol2 + 2 * c + (o & 1);
+    if (lane == 0) e_out[r] = m + 1;
+    __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(slices + r * Kout);
+#pragma unroll
+    for (int t = 0; t < PASSES; ++t) {
+      const int k = 32 * t + lane;
+      if (2 * k >= Kout) continue;
+      long long F0 = round_scaled(__double_as_longlong(v[o][t][0]), m, mx[o] != 0);
+      long long F1 = round_scaled(__double_as_longlong(v[o][t][1]), m, mx[o] != 0);
+#pragma unroll
+      for (int p = S - 1; p > 0; --p) {
+        const int d0 = (int)(((F0 + 32) & 63) - 32), d1 = (int)(((F1 + 32) & 63) - 32);
+        if (p < ndt) out[p * (slice_stride / 2) + k] = __floats2bfloat162_rn((float)d0, (float)d1);
+        F0 = (F0 - d0) >> BETA;
+        F1 = (F1 - d1) >> BETA;
+      }
+      out[k] = __floats2bfloat162_rn((float)F0, (float)F1);
+    }
   }
 }
 

@@ -107,12 +107,12 @@ struct MixedBuffers {
   bool fused = false;                // the apply runs as GEMM 1 + stencil and GEMM 2 + flux (two launches)
   // FP64 outer residual on the tensor cores (digit slices, see ozaki.cuh)
   bool ozaki = false;
-  __nv_bfloat16* oa1 = nullptr;      // [S][2 N_xi][2 Nk] digits of Phi'
-  __nv_bfloat16* oa2 = nullptr;      // [S][2 Nk][2 N_xi] digits of (i Phi^H)'
-  int* ea1 = nullptr;                // [2 N_xi] row exponents
-  int* ea2 = nullptr;                // [2 Nk]
-  __nv_bfloat16* ob = nullptr;       // [S][ncols][max(2 Nk, 2 N_xi)] digits of the B operand
-  int* eb = nullptr;                 // [ncols] column exponents
+  __nv_bfloat16* oa1 = nullptr;      // [S][2 N_xi/2][pair row of Nk] digits of Re and Im Phi, lower halves
+  __nv_bfloat16* oa2 = nullptr;      // [S][2 Nk/2][pair row of N_xi] the same transposed
+  int* ea1 = nullptr;                // [N_xi] row exponents
+  int* ea2 = nullptr;                // [Nk]
+  __nv_bfloat16* ob = nullptr;       // [S][4 ncols][largest pair row] digits of the state's mirror sums and differences
+  int* eb = nullptr;                 // [4 ncols] column exponents
   CUtensorMap tmOA1, tmOA2, tmOB1, tmOB2;
 };
 

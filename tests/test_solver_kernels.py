@@ -66,3 +66,25 @@ def test_gram_schmidt_mixed(built_lib, n_el, nk, order, batch, inner_reorth, bas
         r = (P.rhs() - P.apply(rho)).reshape(batch, -1)
         assert st == 0
         assert np.all(np.linalg.norm(r, axis=1) <= 1.001e-10 * np.linalg.norm(P.rhs().reshape(batch, -1), axis=1))
+
+
+@pytest.mark.parametrize("n_el,nk,nxi,order,batch", [
+    (2, 16, 20, 1, 1), (3, 36, 40, 2, 2), (5, 64, 64, 3, 1), (2, 132, 140, 2, 3), (3, 256, 264, 1, 1),
+    (2, 260, 512, 1, 2), (4, 512, 512, 1, 1)])
+def test_paired_transforms_on_tensor_cores(built_lib, n_el, nk, nxi, order, batch):
+    """The digit-sliced transforms with rows below and above one tile of 128 pairs, padded rows, column tiles cut
+    by the end of a problem and of a plane: the operator against the native FP64 kernels.  48-bit digits of the
+    largest entry of each column: 2^-47 of |Phi| |x| per pair, sums of up to 512 of them, far below 1e-12 of |A x|."""
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order, n_xi=nxi)
+    rng = np.random.default_rng(nk)
+    out = []
+    for tc in (False, True):
+        with Problem1D(n_el=n_el, n_local=order + 1, nk=nk, n_xi=nxi, l_xi=spec.l_xi_m, batch=batch, fp64_tc=tc) as P:
+            for b in range(batch):
+                P.set_potential(b, mat["x"], E * (1 + 0.1 * b), m, spec.m_rel, spec.temp_k, efl, efr)
+            if not out:
+                x = rng.normal(size=P.N * batch) + 1j * rng.normal(size=P.N * batch)
+            out.append(P.apply(x).reshape(batch, -1))
+    want, got = out
+    assert np.all(np.linalg.norm(got - want, axis=1) <= 1e-12 * np.linalg.norm(want, axis=1))
