@@ -563,8 +563,17 @@ cudaError_t precond_mixed_nk(Problem& P, const float2* r, long long r_stride, fl
   const dim3 block(32, kline::kChunksPerBlock);
   float* ma = static_cast<float*>(P.kmap_a);
   float2* ms = static_cast<float2*>(P.kmap_s);
-  cudaEvent_t ev = prof_begin(P, PROF_PRECOND, 2,
-                              ((zb ? 28.0 : 24.0) + (rout ? (double)sizeof(O) : 0.0)) * P.N * P.batch, 0, mask);
+  const double written = (z ? 8.0 : 0.0) + (zb ? 4.0 : 0.0) + (rout ? (double)sizeof(O) : 0.0);
+  if (const int KL = kline::fused_lines<float, NK>(P.s.n_el, P.s.nk, P.batch, L)) {
+    const int th = (KL * nc + 31) / 32 * 32;
+    cudaEvent_t fe = prof_begin(P, PROF_PRECOND, 1, (8.0 + written) * P.N * P.batch, 0, mask);
+    kline::kline_fused_kernel<NK, float, O><<<dim3((P.s.nk + KL - 1) / KL, P.batch), th, 12 * KL * (th / 32), P.stream>>>(
+        r, z, zb, P.mx.kvec, P.mx.dinv, P.mx.h, P.mx.qd, P.s.n_el, P.s.nk, P.N, r_stride, L, nc, KL, mask, rscale, rout,
+        rout_stride);
+    prof_end(P, PROF_PRECOND, fe);
+    return cudaGetLastError();
+  }
+  cudaEvent_t ev = prof_begin(P, PROF_PRECOND, 2, (16.0 + written) * P.N * P.batch, 0, mask);
   kline::kline_maps_kernel<NK, float, RH><<<grid, block, 0, P.stream>>>(r, P.mx.kvec, P.mx.dinv, P.mx.h, P.mx.qd, ma,
                                                                         ms, P.s.n_el, P.s.nk, P.N, r_stride, L, nc,
                                                                         mask, rscale);

@@ -88,3 +88,44 @@ def test_paired_transforms_on_tensor_cores(built_lib, n_el, nk, nxi, order, batc
             out.append(P.apply(x).reshape(batch, -1))
     want, got = out
     assert np.all(np.linalg.norm(got - want, axis=1) <= 1e-12 * np.linalg.norm(want, axis=1))
+
+
+@pytest.mark.parametrize("n_el,nk,order,batch", [(64, 12, 1, 1), (64, 36, 1, 1), (63, 36, 3, 2), (33, 20, 2, 5),
+                                                 (33, 44, 2, 5), (8, 64, 2, 1), (2, 12, 1, 3), (2, 32, 1, 3),
+                                                 (257, 40, 1, 1)])
+def test_kline_sweep_in_one_launch(built_lib, n_el, nk, order, batch):
+    """Chunk lengths on both sides of the limit of the one-launch sweep, ragged last chunks, padded lines and
+    warps.  FP64 against the sequential sweep: sums of n_el contracting maps, 1e-12 as for the two-launch form.
+    Mixed (Nk of 32 and more): the chunk length changes FP32 rounding only, so the iterations stay within a quarter
+    (plus two; a wrong map doubles them) and the solution meets the tolerance by its own residual."""
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order, bias=0.05)
+    Ls = [L for L in (1, 2, 3, 5, 8, 10, 16, 17) if L <= n_el and -(-n_el // L) <= 64]
+    op = krylov.Operator1D(mat, dg1d.init_params(mat, efl, efr, E, m), E)
+    ref = krylov.KLinePreconditioner(op, use_drift_diag=False)
+    rng = np.random.default_rng(nk)
+    kw = dict(n_el=n_el, n_local=order + 1, nk=nk, l_xi=spec.l_xi_m, batch=batch)
+    with Problem1D(**kw) as P:
+        for b in range(batch):
+            P.set_potential(b, mat["x"], E, m, spec.m_rel, spec.temp_k, efl, efr)
+        x = rng.normal(size=(batch, P.N)) + 1j * rng.normal(size=(batch, P.N))
+        want = np.concatenate([ref.apply(v) for v in x])
+        for L in Ls:
+            P.set_launch_shapes(kline_chunk=L)
+            got = P.precondition(x)
+            assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want), L
+    if nk < 32:
+        return
+    its = []
+    with Problem1D(precision="mixed", **kw) as P:
+        for b in range(batch):
+            P.set_potential(b, mat["x"], E * (1 + 0.02 * b), m, spec.m_rel, spec.temp_k, efl, efr)
+        rhs = P.rhs().reshape(batch, -1)
+        for L in Ls:
+            P.set_launch_shapes(kline_chunk=L)
+            st, info = P.solve(tol=1e-10, maxit=60)
+            assert st == 0 and P.runtime_stats["kline_chunk"] == L
+            r = rhs - P.apply(np.concatenate([P.rho(b) for b in range(batch)])).reshape(batch, -1)
+            assert np.all(np.linalg.norm(r, axis=1) <= 1.001e-10 * np.linalg.norm(rhs, axis=1)), L
+            its.append(max(i["iterations"] for i in info))
+    assert max(its) - min(its) <= 2 + max(its) // 4, its
