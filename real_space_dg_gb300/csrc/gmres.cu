@@ -344,57 +344,74 @@ __device__ __forceinline__ R warp_sum8(R (&v)[8]) {
 // reduces the partials into the Hessenberg column.  The warps drop their sums of four vectors (real and
 // imaginary parts: 8 values) in shared memory and the block adds them at the end.
 //
-// FP32 vectors, basis of VB (FP16 or FP32): one block per (2,048 elements, problem); w stays in
-// registers, four basis vectors per pass with their loads in flight together (16 bytes each).  Bound by HBM.
-// 16 problems of 245,760 unknowns, 20 vectors (346 MB): 82 -> 75 us against 8-byte loads and 40 shuffles per sum.
+// FP32 vectors, basis of VB (FP16 or FP32): one block per (`quads` groups of four elements, problem), all blocks
+// resident at once (gs_quads); 2,048 elements of w at a time stay in registers, two basis vectors are loaded
+// (16 bytes per load) while two are summed.  Bound by HBM; with few vectors by the fixed latencies of a block (w, the
+// fence and the ticket), which every further wave of blocks paid again.
+// 16 problems of 245,760 unknowns: 25 -> 18 us with one vector, 82 -> 75 us with 20 (346 MB); 4 of 368,640, over a
+// solve: 21.1 -> 18.0 us.  (Tried and slower: the copies through a shared-memory ring, and this kernel and the update in
+// one launch by problem so that the basis stays in the L2: 150 us against 141 us for both.)
 constexpr int kMdChunk = 2048;
 template <typename VB>
 __global__ void __launch_bounds__(256, 3) multidot32_kernel(const VB* __restrict__ V, const float2* __restrict__ w,
                                                             double2* __restrict__ partial,
                                                             const int* __restrict__ active, long long N, int nv,
-                                                            int mp1, int pstride, int nchunk, KrylovTail tl) {
-  extern __shared__ float red32[];  // [nv rounded up to 4][2][8 warps]
+                                                            int mp1, int pstride, int nchunk, int quads,
+                                                            KrylovTail tl) {
+  extern __shared__ double red32[];  // [nv rounded up to 4][2][8 warps]
   const int b = blockIdx.y, c = blockIdx.x;
   if (!active[b]) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long N4 = N / 4, n0 = (long long)c * (kMdChunk / 4) + threadIdx.x, n1 = n0 + 256;
-  const bool in0 = n0 < N4, in1 = n1 < N4;
-  Quad<float2> w0, w1;
-  w0.zero();
-  w1.zero();
-  if (in0) w0.load(w + (long long)b * N, n0);
-  if (in1) w1.load(w + (long long)b * N, n1);
+  const long long lo = (long long)c * quads, hi = min(N / 4, lo + quads);
   const VB* v = V + (long long)b * mp1 * N;
-  for (int i = 0; i < nv; i += 4) {
+  for (long long base = lo; base < hi; base += 512) {
+    const long long n0 = base + threadIdx.x, n1 = n0 + 256;
+    const bool in0 = n0 < hi, in1 = n1 < hi;
+    Quad<float2> w0, w1;
+    w0.zero();
+    w1.zero();
+    if (in0) w0.load(w + (long long)b * N, n0);
+    if (in1) w1.load(w + (long long)b * N, n1);
+    // two vectors are in flight while two are summed
     Quad<VB> a0[4], a1[4];
+    auto load2 = [&](int i, int u0) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      a0[u].zero();
-      a1[u].zero();
-      if (i + u < nv && in0) a0[u].load(v + (long long)(i + u) * N, n0);
-      if (i + u < nv && in1) a1[u].load(v + (long long)(i + u) * N, n1);
+      for (int u = u0; u < u0 + 2; ++u) {
+        a0[u].zero();
+        a1[u].zero();
+        if (i + u < nv && in0) a0[u].load(v + (long long)(i + u) * N, n0);
+        if (i + u < nv && in1) a1[u].load(v + (long long)(i + u) * N, n1);
+      }
+    };
+    load2(0, 0);
+    for (int i = 0; i < nv; i += 4) {
+      float s[8];
+      load2(i, 2);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        AccF32 t;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) t.add_cdot(a0[u].get(q), w0.get(q));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) t.add_cdot(a1[u].get(q), w1.get(q));
+        s[2 * u] = t.re;
+        s[2 * u + 1] = t.im;
+        if (u == 1) load2(i + 4, 0);
+      }
+      const float r = warp_sum8(s);
+      if ((lane & 3) == 0) {   // always the same thread's slot
+        double* d = red32 + (2 * i + (lane >> 2)) * 8 + warp;
+        *d = base == lo ? (double)r : *d + (double)r;
+      }
     }
-    float s[8];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      AccF32 t;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) t.add_cdot(a0[u].get(q), w0.get(q));
-#pragma unroll
-      for (int q = 0; q < 4; ++q) t.add_cdot(a1[u].get(q), w1.get(q));
-      s[2 * u] = t.re;
-      s[2 * u + 1] = t.im;
-    }
-    const float r = warp_sum8(s);
-    if ((lane & 3) == 0) red32[(2 * i + (lane >> 2)) * 8 + warp] = r;
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nv; i += blockDim.x) {
     double2 r = make_double2(0.0, 0.0);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      r.x += (double)red32[16 * i + q];
-      r.y += (double)red32[16 * i + 8 + q];
+      r.x += red32[16 * i + q];
+      r.y += red32[16 * i + 8 + q];
     }
     partial[((long long)b * pstride + i) * nchunk + c] = r;
   }
@@ -503,11 +520,12 @@ __device__ void update_tail(Acc& a, const int b, double* __restrict__ nrm_partia
 }
 
 // w -= sum_i V_i hcol_i, FP32 vectors: 128 threads of four consecutive complex values, the loads of eight
-// basis vectors in flight per thread (16 bytes each of an FP16 basis).  Bound by HBM.  The problems are taken
-// in the reverse of the multi-dot's order: the basis vectors that one of the two reads last are the first of
-// the other, so the part that fits the L2 (129 MB) is not read from memory again.
-// 16 problems of 245,760 unknowns, 20 vectors: 105 -> 65 us (5.5 TB/s) against 8-byte loads in batches of four.
-constexpr int kUp32Threads = 128, kUp32Elems = 4 * kUp32Threads;
+// basis vectors in flight per thread (16 bytes each of an FP16 basis), the next four before the last four are used.
+// Bound by HBM.  One wave of blocks as in the multi-dot; the problems in the reverse of its order, so that the
+// basis vectors that one of the two reads last are the first of the other while they are in the L2.
+// 16 problems of 245,760 unknowns: 29 -> 21 us with one vector, 105 -> 64 us with 20; 4 of 368,640, over a solve:
+// 22.0 -> 18.8 us.
+constexpr int kUp32Threads = 128;
 template <int MODE, typename VB>
 __global__ void __launch_bounds__(kUp32Threads, 8) gs_update32_kernel(const VB* __restrict__ V,
                                                                       float2* __restrict__ w,
@@ -515,47 +533,52 @@ __global__ void __launch_bounds__(kUp32Threads, 8) gs_update32_kernel(const VB* 
                                                                       const int* __restrict__ mask,
                                                                       double* __restrict__ nrm_partial, long long N,
                                                                       int nv, int mp1, int pstride, int nblk,
-                                                                      KrylovTail tl) {
+                                                                      int quads, KrylovTail tl) {
   const int b = gridDim.y - 1 - blockIdx.y;
   if (!mask[b]) return;
   __shared__ float2 hs[kMaxRestart + 8];
   for (int i = threadIdx.x; i < ((nv + 7) & ~7); i += kUp32Threads)
     hs[i] = i < nv ? hcol[b * pstride + i] : make_float2(0.f, 0.f);
-  const long long N4 = N / 4, n4 = (long long)blockIdx.x * kUp32Threads + threadIdx.x;
-  const bool in = n4 < N4;
-  float4* wp = reinterpret_cast<float4*>(w + (long long)b * N) + 2 * n4;
-  float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
-  if (in) {
-    x0 = wp[0];
-    x1 = wp[1];
-  }
-  float2 acc[4] = {make_float2(x0.x, x0.y), make_float2(x0.z, x0.w), make_float2(x1.x, x1.y),
-                   make_float2(x1.z, x1.w)};
+  const long long lo = (long long)blockIdx.x * quads, hi = min(N / 4, lo + quads);
   const VB* v = V + (long long)b * mp1 * N;
   __syncthreads();
   constexpr int U = sizeof(VB) == 4 ? 8 : 4;
-  for (int i0 = 0; i0 < nv; i0 += U) {
+  double nrm2 = 0.0;   // sums of four values in FP32
+  for (long long n4 = lo + threadIdx.x; n4 < hi; n4 += kUp32Threads) {
+    float4* wp = reinterpret_cast<float4*>(w + (long long)b * N) + 2 * n4;
+    const float4 x0 = wp[0], x1 = wp[1];
+    float2 acc[4] = {make_float2(x0.x, x0.y), make_float2(x0.z, x0.w), make_float2(x1.x, x1.y),
+                     make_float2(x1.z, x1.w)};
     Quad<VB> q[U];
+    auto load = [&](int i0, int u0) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      q[u].zero();
-      if (in && i0 + u < nv) q[u].load(v + (long long)(i0 + u) * N, n4);
+      for (int u = u0; u < u0 + U / 2; ++u) {
+        q[u].zero();
+        if (i0 + u < nv) q[u].load(v + (long long)(i0 + u) * N, n4);
+      }
+    };
+    load(0, 0);
+    for (int i0 = 0; i0 < nv; i0 += U) {
+      load(i0, U / 2);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float2 h = hs[i0 + u];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) cms(acc[r], q[u].get(r), h);
+        if (u == U / 2 - 1) load(i0 + U, 0);
+      }
     }
+    wp[0] = make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
+    wp[1] = make_float4(acc[2].x, acc[2].y, acc[3].x, acc[3].y);
+    if (MODE) {
+      AccF32 f;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const float2 h = hs[i0 + u];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) cms(acc[r], q[u].get(r), h);
+      for (int r = 0; r < 4; ++r) f.add_norm(acc[r]);
+      nrm2 += (double)f.re;
     }
   }
   AccF32 a;
-  if (in) {
-    wp[0] = make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
-    wp[1] = make_float4(acc[2].x, acc[2].y, acc[3].x, acc[3].y);
-    if (MODE)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) a.add_norm(acc[r]);
-  }
+  a.re = (float)nrm2;
   if constexpr (MODE >= 1) update_tail<MODE>(a, b, nrm_partial, nv, pstride, nblk, tl);
 }
 
@@ -754,6 +777,13 @@ __global__ void __launch_bounds__(256) combine_kernel(const VB* __restrict__ V, 
   u[t] = acc;
 }
 
+// Groups of four elements per block of the FP32 Gram-Schmidt kernels: one wave of `per_sm` blocks on each SM
+// for the batch, at least `least` groups, whole warps.
+inline int gs_quads(long long N, int B, int per_sm, int least) {
+  const long long blocks = std::max(1, 152 * per_sm / B), q = (N / 4 + blocks - 1) / blocks;
+  return (int)std::max<long long>(least, (q + 31) / 32 * 32);
+}
+
 inline unsigned blocks_for(long long n) { return (unsigned)((n + 255) / 256); }
 
 #define WG_CK(expr)                                                        \
@@ -794,9 +824,11 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, bool pre, Prec prec, App
   const int nv = k + 1;
   const double vec = (double)N * B * sizeof(T), vecb = (double)N * B * sizeof(VB);
   constexpr bool f32 = std::is_same<T, float2>::value;
-  const long long per_blk = f32 ? kUp32Elems : 256;
-  const dim3 gu((unsigned)((N + per_blk - 1) / per_blk), B);
-  const int nblk = (int)gu.x;
+  // FP32: one wave of blocks
+  const int mq = gs_quads(N, B, 3, kMdChunk / 4), uq = gs_quads(N, B, 8, kUp32Threads);
+  const int mblk = (int)((N / 4 + mq - 1) / mq);
+  const int nblk = f32 ? (int)((N / 4 + uq - 1) / uq) : (int)((N + 255) / 256);
+  const dim3 gu(nblk, B);
   // classical Gram-Schmidt; the second pass runs for the problems that fail the DGKS
   // test (its kernels see P.reorth as their activity mask), for all with eta >= 1,
   // for none with eta < 0.  The reductions, the norm and the Givens step run in the
@@ -813,8 +845,8 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, bool pre, Prec prec, App
     tl.first = pass == 0;
     cudaEvent_t ev = prof_begin(P, PROF_MULTIDOT, 1, nv * vecb + vec, 8.0 * nv * N * B, mask);
     if constexpr (f32) {
-      multidot32_kernel<VB><<<dim3(P.nchunk, B), 256, sizeof(float) * 16 * ((nv + 3) & ~3), P.stream>>>(
-          V, w, P.partial, mask, N, nv, mp1, ps, P.nchunk, tl);
+      multidot32_kernel<VB><<<dim3(mblk, B), 256, sizeof(double) * 16 * ((nv + 3) & ~3), P.stream>>>(
+          V, w, P.partial, mask, N, nv, mp1, ps, mblk, mq, tl);
     } else {
       const dim3 gm(P.md_chunk, B, (nv + 3) / 4);
       auto md = P.md_e == 8 ? multidot64_kernel<8> : P.md_e == 4 ? multidot64_kernel<4>
@@ -827,7 +859,7 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, bool pre, Prec prec, App
     if constexpr (f32) {
       auto up = mode == 2 ? gs_update32_kernel<2, VB> : mode == 1 ? gs_update32_kernel<1, VB>
                                                                   : gs_update32_kernel<0, VB>;
-      up<<<gu, kUp32Threads, 0, P.stream>>>(V, w, P.mx.hcol, mask, P.nrm_partial, N, nv, mp1, ps, nblk, tl);
+      up<<<gu, kUp32Threads, 0, P.stream>>>(V, w, P.mx.hcol, mask, P.nrm_partial, N, nv, mp1, ps, nblk, uq, tl);
     } else {
       auto up = mode == 2 ? gs_update64_kernel<2> : mode == 1 ? gs_update64_kernel<1> : gs_update64_kernel<0>;
       up<<<gu, 256, 0, P.stream>>>(V, w, P.hcol, mask, P.nrm_partial, N, nv, mp1, ps, nblk, tl);

@@ -129,3 +129,21 @@ def test_kline_sweep_in_one_launch(built_lib, n_el, nk, order, batch):
             assert np.all(np.linalg.norm(r, axis=1) <= 1.001e-10 * np.linalg.norm(rhs, axis=1)), L
             its.append(max(i["iterations"] for i in info))
     assert max(its) - min(its) <= 2 + max(its) // 4, its
+
+
+@pytest.mark.parametrize("n_el,nk,order,batch", [(31, 68, 3, 152), (9, 64, 1, 500)])
+def test_gram_schmidt_many_problems(built_lib, n_el, nk, order, batch):
+    """More problems than resident blocks: a block of the inner Arnoldi's kernels takes several pieces of a problem,
+    the last one ragged.  Every problem meets the tolerance by its own FP64 residual."""
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order, bias=0.05)
+    with Problem1D(n_el=n_el, n_local=order + 1, nk=nk, l_xi=spec.l_xi_m, batch=batch, precision="mixed",
+                   inner_restart=21) as P:
+        for b in range(batch):
+            P.set_potential(b, mat["x"], E * (1 + 0.1 * b / batch), m, spec.m_rel, spec.temp_k, efl, efr)
+        st, info = P.solve(tol=1e-10, maxit=60)
+        rho = np.concatenate([P.rho(b) for b in range(batch)])
+        rhs = P.rhs().reshape(batch, -1)
+        r = rhs - P.apply(rho).reshape(batch, -1)
+        assert st == 0
+        assert np.all(np.linalg.norm(r, axis=1) <= 1.001e-10 * np.linalg.norm(rhs, axis=1))
