@@ -786,7 +786,7 @@ cudaError_t mixed_sync_weights(Problem& P) {
                                                                           ne, ne4);
   pack_weights_kernel<<<(unsigned)((ni + 255) / 256), 256, 0, P.stream>>>(P.betai, P.mx.betai, 1, s.nK,
                                                                           s.nK * s.nK, true, ne, ne4);
-  d2f_kernel<<<1, 256, 0, P.stream>>>(P.qd, P.mx.qd, P.batch);
+  d2f_kernel<<<(P.batch + 255) / 256, 256, 0, P.stream>>>(P.qd, P.mx.qd, P.batch);
   d2f_kernel<<<(unsigned)((s.nk + 255) / 256), 256, 0, P.stream>>>(P.kvec, P.mx.kvec, s.nk);
   const long long nd = (long long)P.batch * s.nk * s.nK * s.nK, nh = (long long)P.batch * s.nk * s.nK;
   d2f_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, P.stream>>>(P.pre_dinv, P.mx.dinv, nd);
