@@ -33,6 +33,7 @@
 #include <string>
 #include <vector>
 
+#include "krylov.cuh"
 #include "ozaki_api.h"
 #include "wigner_gb300.h"
 
@@ -99,7 +100,10 @@ struct wg2d_problem {
   double2* Zb = nullptr;          // [m][n] preconditioned basis (flexible GMRES)
   double2 *V = nullptr, *r = nullptr, *w = nullptr, *z = nullptr, *b = nullptr, *xs = nullptr;
   double2 *H = nullptr, *g = nullptr, *sn = nullptr, *hc = nullptr, *hp = nullptr, *yc = nullptr;
-  double *cs = nullptr, *partial = nullptr, *nrm = nullptr;
+  double2* cs = nullptr;
+  double *ktarget = nullptr;    // [1] zero
+  int* kctl = nullptr;          // [4] see F2dKrylov
+  double *partial = nullptr, *nrm = nullptr;
   double2 *bc_rt = nullptr, *bc_p = nullptr, *bc_ph = nullptr, *bc_sh = nullptr;   // BiCGSTAB vectors
   bool b_ready = false, xs_ready = false;   // resident right-hand side / solution of the last solve
   std::vector<double> resvec;               // residual norms of the last solve (initial, then per iteration)
@@ -801,60 +805,229 @@ __global__ void __launch_bounds__(256) f2d_d2f(const double* __restrict__ x, flo
   if (t < n) y[t] = (float)x[t];
 }
 
-__device__ __forceinline__ float2 f2d_ld(const float2& v) { return v; }
-__device__ __forceinline__ float2 f2d_ld(const __half2& v) { return __half22float2(v); }
-
-// FP32 inner products, summed per thread in FP32 and across threads and blocks in FP64; the basis
-// vectors V in FP32 or FP16 storage
-template <typename VB>
-__global__ void __launch_bounds__(256) f2d_dot_partial32(const VB* __restrict__ V, long long vstride,
-                                                         const float2* __restrict__ w, double* __restrict__ partial,
-                                                         long long n) {
-  __shared__ double sre[256], sim[256];
-  const int i = blockIdx.y;
-  const VB* v = V + (long long)i * vstride;
-  float re = 0.f, im = 0.f;
-  for (long long t = (long long)blockIdx.x * 256 + threadIdx.x; t < n; t += (long long)gridDim.x * 256) {
-    const float2 a = f2d_ld(v[t]), b = w[t];
-    re = fmaf(a.x, b.x, fmaf(a.y, b.y, re));
-    im = fmaf(a.x, b.y, fmaf(-a.y, b.x, im));
-  }
-  sre[threadIdx.x] = re;
-  sim[threadIdx.x] = im;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      sre[threadIdx.x] += sre[threadIdx.x + o];
-      sim[threadIdx.x] += sim[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    partial[((long long)i * gridDim.x + blockIdx.x) * 2] = sre[0];
-    partial[((long long)i * gridDim.x + blockIdx.x) * 2 + 1] = sim[0];
+// ---------------- Gram-Schmidt of the FP32 inner solve (basis VB: FP32 or FP16 storage)
+// Four consecutive complex values; VEC: n is a multiple of 4 (every row of the basis 16-byte aligned).
+template <bool VEC, typename VB>
+__device__ __forceinline__ void f2d_quad(wg::Quad<VB>& q, const VB* __restrict__ p, long long n4, long long n) {
+  if constexpr (VEC) {
+    q.load(p, n4);
+  } else {
+    q.zero();
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (4 * n4 + r < n) q.set(r, p[4 * n4 + r]);
   }
 }
 
-// w -= sum_i h_i V_i in FP32.  The coefficients are converted to FP32 once per block into shared memory:
-// converting them per element put every element x vector through the FP64 pipe (98% busy, DRAM at 35%).
-constexpr int kGsStage = 256;
-template <typename VB>
-__global__ void __launch_bounds__(256) f2d_gs_update32(const VB* __restrict__ V, long long vstride,
-                                                       float2* __restrict__ w, const double2* __restrict__ h, int nv,
-                                                       long long n) {
-  __shared__ float2 hs[kGsStage];
-  for (int i = threadIdx.x; i < min(nv, kGsStage); i += blockDim.x) hs[i] = make_float2((float)h[i].x, (float)h[i].y);
-  __syncthreads();
-  const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (t >= n) return;
-  float2 acc = w[t];
-  for (int i = 0; i < nv; ++i) {
-    const float2 v = f2d_ld(V[(long long)i * vstride + t]);
-    const float2 c = i < kGsStage ? hs[i] : make_float2((float)h[i].x, (float)h[i].y);
-    acc.x -= c.x * v.x - c.y * v.y;
-    acc.y -= c.x * v.y + c.y * v.x;
+// (s, e) += (b, be) with the rounding error of s + b kept in e
+__device__ __forceinline__ void f2d_two_sum(float& s, float& e, float b, float be) {
+  const float t = __fadd_rn(s, b), z = __fsub_rn(t, s);
+  e += be + __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(b, z));
+  s = t;
+}
+
+// Sums over a warp of 8 values per lane, lane l returns the sum of value l >> 2: each step exchanges half of the
+// values still held.  The rounding errors of the FP32 sums are carried along, so the result is a sum of the
+// lanes' values in more than FP32 without the FP64 pipe (64 cycles per warp instruction of a quarter).
+__device__ __forceinline__ double f2d_warp_sum8(float (&s)[8]) {
+  const int lane = threadIdx.x & 31;
+  float e[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) e[i] = 0.f;
+#pragma unroll
+  for (int h = 4; h >= 1; h /= 2) {
+    const bool up = lane & (4 * h);
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const float gs = up ? s[i] : s[i + h], ge = up ? e[i] : e[i + h];
+      s[i] = up ? s[i + h] : s[i];
+      e[i] = up ? e[i + h] : e[i];
+      const float os = __shfl_xor_sync(0xffffffffu, gs, 4 * h);
+      const float oe = h == 4 ? 0.f : __shfl_xor_sync(0xffffffffu, ge, 4 * h);
+      f2d_two_sum(s[i], e[i], os, oe);
+    }
   }
-  w[t] = acc;
+#pragma unroll
+  for (int o = 2; o >= 1; o /= 2) {
+    const float os = __shfl_xor_sync(0xffffffffu, s[0], o), oe = __shfl_xor_sync(0xffffffffu, e[0], o);
+    f2d_two_sum(s[0], e[0], os, oe);
+  }
+  return (double)s[0] + (double)e[0];
+}
+
+// partial[(i * blocks + blk) * 2 + {0,1}] = sum over the block's piece of conj(V_i) w for all i < nv: FP32 over the
+// four values of a thread's load, error-carrying across the warp, FP64 across warps, pieces and blocks.  run
+// (nullable): nothing to do when *run is 0.
+// All blocks resident at once, each on one contiguous piece; w stays in registers, half of the four vectors of a
+// step are loaded while the other half is summed.  Bound by HBM (the basis once; one launch row per
+// vector had read w nv times with 8-byte loads, 1.5 TB/s).  1,568,160 unknowns, 1 .. 40 FP32
+// vectors, mean of a cycle: 177 -> 49 us (5.2 TB/s).
+constexpr int kF2dUpThreads = 128;
+template <bool VEC, typename VB>
+__global__ void __launch_bounds__(256, 3) f2d_multidot32(const VB* __restrict__ V, const float2* __restrict__ w,
+                                                         double* __restrict__ partial, long long n, int nv, int quads,
+                                                         const int* __restrict__ run) {
+  extern __shared__ double f2d_red[];   // [nv rounded up to 4][2][8 warps]
+  if (run && !*run) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long lo = (long long)blockIdx.x * quads, hi = min((n + 3) / 4, lo + quads);
+  for (long long base = lo; base < hi; base += 256) {
+    const long long n0 = base + threadIdx.x;
+    const bool in = n0 < hi;
+    wg::Quad<float2> wq;
+    wq.zero();
+    if (in) f2d_quad<VEC>(wq, w, n0, n);
+    wg::Quad<VB> a[4];
+    auto load2 = [&](int i, int u0) {
+#pragma unroll
+      for (int u = u0; u < u0 + 2; ++u) {
+        a[u].zero();
+        if (i + u < nv && in) f2d_quad<VEC>(a[u], V + (long long)(i + u) * n, n0, n);
+      }
+    };
+    load2(0, 0);
+    for (int i = 0; i < nv; i += 4) {
+      float s[8];
+      load2(i, 2);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float re = 0.f, im = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 v = a[u].get(q), x = wq.get(q);
+          re = fmaf(v.x, x.x, fmaf(v.y, x.y, re));
+          im = fmaf(v.x, x.y, fmaf(-v.y, x.x, im));
+        }
+        s[2 * u] = re;
+        s[2 * u + 1] = im;
+        if (u == 1) load2(i + 4, 0);
+      }
+      const double r = f2d_warp_sum8(s);
+      if ((lane & 3) == 0) {   // always the same thread's slot
+        double* d = f2d_red + (2 * i + (lane >> 2)) * 8 + warp;
+        *d = base == lo ? r : *d + r;
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * nv; i += 256) {
+    double r = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) r += f2d_red[8 * i + q];
+    partial[((long long)(i / 2) * gridDim.x + blockIdx.x) * 2 + (i & 1)] = r;
+  }
+}
+
+// Device state of the inner solve's small work.
+struct F2dKrylov {
+  double2 *H, *hc, *cs, *sn, *g;
+  double* nrm;
+  double* target;   // 0: the Givens step never stops by itself, the host looks at g
+  int* ctl;         // active, kused, second pass, tickets of the update
+  int j, ldh;
+};
+
+// w -= sum_i h_i V_i in FP32, |w| and, when no second pass follows, the Givens step in the last block.  PASS 1 tests
+// |w'|^2 < (|w'|^2 + |h|^2) / 2 (Daniel-Gragg-Kaufman-Stewart) and leaves ctl[2]; PASS 2 runs when that is set.
+// 128 threads of four values, the loads of the next vectors ahead of the present ones; all blocks resident at once.
+// Bound by HBM.  1,568,160 unknowns, 1 .. 40 FP32 vectors, mean of a cycle: 53 us with the norm and the Givens step
+// (48 us, and 38 us in four launches for those, before).
+template <int PASS, bool VEC, typename VB>
+__global__ void __launch_bounds__(kF2dUpThreads, 8) f2d_gs_update32(const VB* __restrict__ V, float2* __restrict__ w,
+                                                                    const double2* __restrict__ h, int nv, long long n,
+                                                                    int quads, double* __restrict__ norms,
+                                                                    F2dKrylov k) {
+  if (PASS == 2 && !k.ctl[2]) return;
+  __shared__ float2 hs[wg::kMaxRestart + 8];
+  __shared__ double ws[kF2dUpThreads / 32];
+  __shared__ int last;
+  // the coefficients in FP32 once per block (per element the conversion kept the FP64 pipe 98% busy)
+  for (int i = threadIdx.x; i < ((nv + 7) & ~7); i += kF2dUpThreads)
+    hs[i] = i < nv ? make_float2((float)h[i].x, (float)h[i].y) : make_float2(0.f, 0.f);
+  __syncthreads();
+  constexpr int U = sizeof(VB) == 4 ? 8 : 4;
+  const long long lo = (long long)blockIdx.x * quads, hi = min((n + 3) / 4, lo + quads);
+  double nrm2 = 0.0;
+  for (long long n4 = lo + threadIdx.x; n4 < hi; n4 += kF2dUpThreads) {
+    wg::Quad<float2> wq;
+    if constexpr (VEC) {   // plain loads: w is written below
+      wq.u = reinterpret_cast<float4*>(w)[2 * n4];
+      wq.v = reinterpret_cast<float4*>(w)[2 * n4 + 1];
+    } else {
+      f2d_quad<false>(wq, (const float2*)w, n4, n);
+    }
+    float2 acc[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[r] = wq.get(r);
+    wg::Quad<VB> q[U];
+    auto load = [&](int i0, int u0) {
+#pragma unroll
+      for (int u = u0; u < u0 + U / 2; ++u) {
+        q[u].zero();
+        if (i0 + u < nv) f2d_quad<VEC>(q[u], V + (long long)(i0 + u) * n, n4, n);
+      }
+    };
+    load(0, 0);
+    for (int i0 = 0; i0 < nv; i0 += U) {
+      load(i0, U / 2);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float2 c = hs[i0 + u];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) wg::cms(acc[r], q[u].get(r), c);
+        if (u == U / 2 - 1) load(i0 + U, 0);
+      }
+    }
+    float f = 0.f;   // values past n are zero
+#pragma unroll
+    for (int r = 0; r < 4; ++r) f = fmaf(acc[r].x, acc[r].x, fmaf(acc[r].y, acc[r].y, f));
+    nrm2 += (double)f;
+    if constexpr (VEC) {
+      float4* wp = reinterpret_cast<float4*>(w) + 2 * n4;
+      wp[0] = make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
+      wp[1] = make_float4(acc[2].x, acc[2].y, acc[3].x, acc[3].y);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (4 * n4 + r < n) w[4 * n4 + r] = acc[r];
+    }
+  }
+  nrm2 = wg::warp_sum(nrm2);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = nrm2;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    norms[blockIdx.x] = (ws[0] + ws[1]) + (ws[2] + ws[3]);
+    __threadfence();
+    last = atomicAdd(&k.ctl[3], 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double w2p = 0.0;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < (int)gridDim.x; c += kF2dUpThreads) w2p += __ldcg(&norms[c]);
+  const double w2b = wg::block_sum1(w2p);
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const double w2 = __shfl_sync(0xffffffffu, w2b, 0);
+    int again = 0;
+    if (PASS == 1) {
+      double h2 = 0.0;
+      for (int i = lane; i < nv; i += 32) h2 += h[i].x * h[i].x + h[i].y * h[i].y;
+      h2 = wg::warp_sum(h2);
+      again = w2 < 0.5 * (w2 + h2);
+      if (lane == 0) k.ctl[2] = again;
+    }
+    if (!again) {
+      const double v = w2 > 0 ? sqrt(w2) : w2;   // NaN passes on
+      double2* col = k.H + (long long)k.j * k.ldh;
+      for (int i = lane; i <= k.j; i += 32) col[i] = k.hc[i];
+      if (lane == 0) k.nrm[0] = v;
+      __syncwarp();
+      wg::givens_warp(k.H, k.cs, k.sn, k.g, k.ctl, k.ctl + 1, k.target, 0, k.j, k.ldh, 0, v);
+    }
+  }
+  if (threadIdx.x == 0) k.ctl[3] = 0;
 }
 
 __global__ void __launch_bounds__(256) f2d_scale32(const float2* __restrict__ x, float2* __restrict__ out,
@@ -922,33 +1095,34 @@ __global__ void __launch_bounds__(256) f2d_dot_partial(const double2* __restrict
   }
 }
 
-// out[i] = sum of the partials of vector i; one block per vector
+// out[i] = sum of the partials of vector i, added to acc[i] as well (nullable); one block per vector.  run: as above.
 __global__ void __launch_bounds__(256) f2d_dot_reduce(const double* __restrict__ partial, double2* __restrict__ out,
-                                                      int nblk, int accumulate) {
-  __shared__ double sre[256], sim[256];
+                                                      double2* __restrict__ acc, int nblk,
+                                                      const int* __restrict__ run) {
+  __shared__ double2 ws[8];
+  if (run && !*run) return;
   const int i = blockIdx.x;
-  double re = 0.0, im = 0.0;
+  const double2* p = reinterpret_cast<const double2*>(partial) + (long long)i * nblk;
+  double2 r = make_double2(0.0, 0.0);
+#pragma unroll 4
   for (int b = threadIdx.x; b < nblk; b += 256) {
-    re += partial[((long long)i * nblk + b) * 2];
-    im += partial[((long long)i * nblk + b) * 2 + 1];
+    const double2 t = p[b];
+    r.x += t.x;
+    r.y += t.y;
   }
-  sre[threadIdx.x] = re;
-  sim[threadIdx.x] = im;
+  r.x = wg::warp_sum(r.x);
+  r.y = wg::warp_sum(r.y);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = r;
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      sre[threadIdx.x] += sre[threadIdx.x + o];
-      sim[threadIdx.x] += sim[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
-    if (accumulate) {
-      out[i].x += sre[0];
-      out[i].y += sim[0];
-    } else {
-      out[i] = make_double2(sre[0], sim[0]);
+    double2 t = ws[0];
+#pragma unroll
+    for (int q = 1; q < 8; ++q) {
+      t.x += ws[q].x;
+      t.y += ws[q].y;
     }
+    out[i] = t;
+    if (acc) acc[i] = make_double2(acc[i].x + t.x, acc[i].y + t.y);
   }
 }
 
@@ -1022,64 +1196,13 @@ __global__ void __launch_bounds__(256) f2d_rscale(double2* __restrict__ v, doubl
   v[t].y *= s;
 }
 
-// Hessenberg column j (hc[0..j] from Gram-Schmidt, nrm[0] = |w|): previous Givens rotations, the
-// new one, the rotated right-hand side; g[j+1] is the residual estimate.  One thread.
-__global__ void f2d_givens(double2* __restrict__ H, const double2* __restrict__ hc, const double* __restrict__ nrm,
-                           double* __restrict__ cs, double2* __restrict__ sn, double2* __restrict__ g, int j, int ldh) {
-  double2* col = H + (long long)j * ldh;
-  for (int i = 0; i <= j; ++i) col[i] = hc[i];
-  col[j + 1] = make_double2(nrm[0], 0.0);
-  for (int i = 0; i < j; ++i) {
-    const double c = cs[i];
-    const double2 s = sn[i], a = col[i], b = col[i + 1];
-    // [c s; -conj(s) c] [a; b]
-    col[i] = make_double2(c * a.x + s.x * b.x - s.y * b.y, c * a.y + s.x * b.y + s.y * b.x);
-    col[i + 1] = make_double2(-(s.x * a.x + s.y * a.y) + c * b.x, -(s.x * a.y - s.y * a.x) + c * b.y);
-  }
-  const double2 a = col[j];
-  const double bb = col[j + 1].x;
-  const double aa = hypot(a.x, a.y);
-  const double rho = hypot(aa, bb);
-  double c;
-  double2 s, top;
-  if (rho == 0.0) {
-    c = 1.0;
-    s = make_double2(0.0, 0.0);
-    top = a;
-  } else if (aa == 0.0) {
-    c = 0.0;
-    s = make_double2(1.0, 0.0);
-    top = make_double2(bb, 0.0);
-  } else {
-    c = aa / rho;
-    const double2 ph = make_double2(a.x / aa, a.y / aa);
-    s = make_double2(ph.x * bb / rho, ph.y * bb / rho);        // (a/|a|) conj(b) / rho, b real
-    top = make_double2(ph.x * rho, ph.y * rho);
-  }
-  cs[j] = c;
-  sn[j] = s;
-  col[j] = top;
-  col[j + 1] = make_double2(0.0, 0.0);
-  const double2 gj = g[j];
-  g[j] = make_double2(c * gj.x, c * gj.y);
-  g[j + 1] = make_double2(-(s.x * gj.x + s.y * gj.y), -(s.x * gj.y - s.y * gj.x));
-}
-
-// y = R^-1 g for the leading k x k upper triangle of H; one thread
-__global__ void f2d_backsolve(const double2* __restrict__ H, const double2* __restrict__ g, double2* __restrict__ y,
-                              int k, int ldh) {
-  for (int i = k - 1; i >= 0; --i) {
-    double2 s = g[i];
-    for (int j = i + 1; j < k; ++j) {
-      const double2 h = H[(long long)j * ldh + i], v = y[j];
-      s.x -= h.x * v.x - h.y * v.y;
-      s.y -= h.x * v.y + h.y * v.x;
-    }
-    const double2 d = H[(long long)i * ldh + i];
-    const double den = d.x * d.x + d.y * d.y;
-    y[i] = den > 0 ? make_double2((s.x * d.x + s.y * d.y) / den, (s.y * d.x - s.x * d.y) / den)
-                   : make_double2(0.0, 0.0);
-  }
+// Hessenberg column j (hc[0..j] from Gram-Schmidt, nrm[0] = |w|): previous Givens rotations, the new one, the
+// rotated right-hand side; g[j+1] is the residual estimate.  One warp.
+__global__ void f2d_givens(F2dKrylov k) {
+  double2* col = k.H + (long long)k.j * k.ldh;
+  for (int i = threadIdx.x; i <= k.j; i += 32) col[i] = k.hc[i];
+  __syncwarp();
+  wg::givens_warp(k.H, k.cs, k.sn, k.g, k.ctl, k.ctl + 1, k.target, 0, k.j, k.ldh, 0, k.nrm[0]);
 }
 
 // u = sum_i y_i V_i
@@ -1627,40 +1750,48 @@ static int precondition_device(wg2d_problem* h, const double2* r, double2* z) {
   return WG_OK;
 }
 
-// out[0..nv) = V_i^H w (accumulate: out += ...)
-static void dots(wg2d_problem* h, const double2* V, int nv, const double2* w, double2* out, int accumulate) {
+// out[0..nv) = V_i^H w (acc, nullable: added there too)
+static void dots(wg2d_problem* h, const double2* V, int nv, const double2* w, double2* out, double2* acc = nullptr) {
   f2d_dot_partial<<<dim3(kDotBlocks, nv), 256, 0, h->stream>>>(V, h->n, w, h->partial, h->n);
-  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, out, kDotBlocks, accumulate);
+  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, out, acc, kDotBlocks, nullptr);
 }
 
 static void vnorm(wg2d_problem* h, const double2* w) {
-  dots(h, w, 1, w, h->hp, 0);
+  dots(h, w, 1, w, h->hp);
   f2d_sqrt_real<<<1, 1, 0, h->stream>>>(h->hp, h->nrm);
 }
 
 }  // extern "C"
 
-template <typename VB>
-static void dots32(wg2d_problem* h, const VB* V, int nv, const float2* w, double2* out, int accumulate) {
-  f2d_dot_partial32<VB><<<dim3(kDotBlocks, nv), 256, 0, h->stream>>>(V, h->n, w, h->partial, h->n);
-  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, out, kDotBlocks, accumulate);
+// Gram-Schmidt of w against V_0 .. V_{k.j}, |w| and the Givens step: two launches of each kernel, the second ones idle
+// unless the first pass lost more than half of |w|^2 (decided on the device).
+template <bool VEC, typename VB>
+static void gram_schmidt32(wg2d_problem* h, const VB* V, float2* w, const F2dKrylov& k) {
+  const int nv = k.j + 1;
+  const long long n = h->n;
+  const int mq = wg::gs_quads(n + 3, 1, 3, 256), uq = wg::gs_quads(n + 3, 1, 8, kF2dUpThreads);
+  const unsigned mb = (unsigned)(((n + 3) / 4 + mq - 1) / mq), ub = (unsigned)(((n + 3) / 4 + uq - 1) / uq);
+  const size_t sm = sizeof(double) * 16 * ((nv + 3) & ~3);
+  f2d_multidot32<VEC, VB><<<mb, 256, sm, h->stream>>>(V, w, h->partial, n, nv, mq, nullptr);
+  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, h->hc, nullptr, mb, nullptr);
+  f2d_gs_update32<1, VEC, VB><<<ub, kF2dUpThreads, 0, h->stream>>>(V, w, h->hc, nv, n, uq, h->partial, k);
+  f2d_multidot32<VEC, VB><<<mb, 256, sm, h->stream>>>(V, w, h->partial, n, nv, mq, k.ctl + 2);
+  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, h->hp, h->hc, mb, k.ctl + 2);
+  f2d_gs_update32<2, VEC, VB><<<ub, kF2dUpThreads, 0, h->stream>>>(V, w, h->hp, nv, n, uq, h->partial, k);
 }
 
 extern "C" {
 
-static void vnorm32(wg2d_problem* h, const float2* w) {
-  dots32(h, w, 1, w, h->hp, 0);
-  f2d_sqrt_real<<<1, 1, 0, h->stream>>>(h->hp, h->nrm);
-}
-
 static void free_solver(wg2d_problem* h) {
   void* ptrs[] = {h->V, h->Zb, h->r, h->w, h->z, h->b, h->xs, h->H, h->g, h->sn, h->hc, h->hp, h->yc, h->cs,
-                  h->partial, h->nrm, h->bc_rt, h->bc_p, h->bc_ph, h->bc_sh};
+                  h->partial, h->nrm, h->ktarget, h->kctl, h->bc_rt, h->bc_p, h->bc_ph, h->bc_sh};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   h->bc_rt = h->bc_p = h->bc_ph = h->bc_sh = nullptr;
   h->V = h->Zb = h->r = h->w = h->z = h->b = h->xs = h->H = h->g = h->sn = h->hc = h->hp = h->yc = nullptr;
-  h->cs = h->partial = h->nrm = nullptr;
+  h->cs = nullptr;
+  h->partial = h->nrm = h->ktarget = nullptr;
+  h->kctl = nullptr;
   h->vm = 0;
 }
 
@@ -2047,6 +2178,10 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
     F2_CK(dalloc(&h->cs, m));
     F2_CK(dalloc(&h->partial, (size_t)2 * kDotBlocks * (m + 1)));
     F2_CK(dalloc(&h->nrm, 1));
+    F2_CK(dalloc(&h->ktarget, 1));
+    F2_CK(dalloc(&h->kctl, 4));
+    F2_CK(cudaMemsetAsync(h->ktarget, 0, sizeof(double), h->stream));
+    F2_CK(cudaMemsetAsync(h->kctl, 0, 4 * sizeof(int), h->stream));
     h->vm = m + 1;
   }
   std::memset(info, 0, sizeof(*info));
@@ -2118,41 +2253,19 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
       F2_CK(cudaMemsetAsync(h->g, 0, sizeof(double2) * (m + 1), h->stream));
       F2_CK(cudaMemcpyAsync(h->g, &one, sizeof(double2), cudaMemcpyHostToDevice, h->stream));
       const double itgt = std::max(inner_tol, 0.5 * target / beta);
-      int k = 0, j_cur = 0;
-      // the basis as the Gram-Schmidt kernels read it
-      auto gs_dots = [&](double2* out) {
-        if (b16) dots32(h, h->Vh32, j_cur + 1, h->w32, out, 0);
-        else dots32(h, h->V32, j_cur + 1, h->w32, out, 0);
-      };
-      auto gs_update = [&](const double2* coef) {
-        if (b16) f2d_gs_update32<<<blocks256(n), 256, 0, h->stream>>>(h->Vh32, n, h->w32, coef, j_cur + 1, n);
-        else f2d_gs_update32<<<blocks256(n), 256, 0, h->stream>>>(h->V32, n, h->w32, coef, j_cur + 1, n);
-      };
+      int k = 0;
       for (int j = 0; j < mi; ++j) {
-        j_cur = j;
         // the preconditioner works on the basis vector as stored (its FP32 copy with an FP16 basis)
         const float2* Vj = b16 ? h->vj32 : h->V32 + (long long)j * n;
         float2* Zj = h->Z32 + (long long)j * n;
         precond_stages<float2>(h, h->UH32, h->Us32, h->xinv32, h->xcpl32, h->tinv32, Vj, h->pa32, h->pb32, Zj);
         rc = apply32(h, Zj, h->w32);
         if (rc) return rc;
-        gs_dots(h->hc);
-        gs_update(h->hc);
-        vnorm32(h, h->w32);
-        std::vector<double2> hh(j + 1);
-        double w1 = 0;
-        F2_CK(cudaMemcpyAsync(hh.data(), h->hc, sizeof(double2) * (j + 1), cudaMemcpyDeviceToHost, h->stream));
-        F2_CK(cudaMemcpyAsync(&w1, h->nrm, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        F2_CK(cudaStreamSynchronize(h->stream));
-        double h2 = 0;
-        for (const double2& c : hh) h2 += c.x * c.x + c.y * c.y;
-        if (w1 * w1 < 0.5 * (w1 * w1 + h2)) {
-          gs_dots(h->hp);
-          f2d_dot_reduce<<<j + 1, 256, 0, h->stream>>>(h->partial, h->hc, kDotBlocks, 1);
-          gs_update(h->hp);
-          vnorm32(h, h->w32);
-        }
-        f2d_givens<<<1, 1, 0, h->stream>>>(h->H, h->hc, h->nrm, h->cs, h->sn, h->g, j, ldh);
+        const F2dKrylov kr{h->H, h->hc, h->cs, h->sn, h->g, h->nrm, h->ktarget, h->kctl, j, ldh};
+        if (b16 && n % 4 == 0) gram_schmidt32<true>(h, h->Vh32, h->w32, kr);
+        else if (b16) gram_schmidt32<false>(h, h->Vh32, h->w32, kr);
+        else if (n % 4 == 0) gram_schmidt32<true>(h, h->V32, h->w32, kr);
+        else gram_schmidt32<false>(h, h->V32, h->w32, kr);
         if (b16)
           f2d_scale16<<<blocks256(n), 256, 0, h->stream>>>(h->w32, h->Vh32 + (long long)(j + 1) * n, h->vj32,
                                                            h->nrm, n);
@@ -2166,7 +2279,7 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
         h->resvec.push_back(beta * std::hypot(gj.x, gj.y));
         if (!(std::hypot(gj.x, gj.y) > itgt)) break;
       }
-      f2d_backsolve<<<1, 1, 0, h->stream>>>(h->H, h->g, h->yc, k, ldh);
+      wg::backsolve_kernel<<<1, 32, 0, h->stream>>>(h->H, h->g, h->yc, nullptr, h->kctl + 1, ldh, k, 1);
       F2_CK(cudaMemcpyAsync(h->nrm, &beta, sizeof(double), cudaMemcpyHostToDevice, h->stream));
       f2d_correct32<<<blocks256(n), 256, 0, h->stream>>>(h->xs, h->Z32, n, h->yc, k, h->nrm, n);
       info->cycles += 1;
@@ -2189,7 +2302,7 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
       if (rc) return rc;
       // classical Gram-Schmidt; a second pass only when the first lost more than half of |w|^2
       // (Daniel-Gragg-Kaufman-Stewart: |w'|^2 < eta^2 (|w'|^2 + |h|^2), eta = 1/sqrt(2))
-      dots(h, h->V, j + 1, h->w, h->hc, 0);
+      dots(h, h->V, j + 1, h->w, h->hc);
       f2d_gs_update<<<blocks256(n), 256, 0, h->stream>>>(h->V, n, h->w, h->hc, j + 1, n);
       vnorm(h, h->w);
       std::vector<double2> hh(j + 1);
@@ -2200,13 +2313,12 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
       double h2 = 0;
       for (const double2& c : hh) h2 += c.x * c.x + c.y * c.y;
       if (w1 * w1 < 0.5 * (w1 * w1 + h2)) {
-        dots(h, h->V, j + 1, h->w, h->hp, 0);    // second pass
-        f2d_dot_reduce<<<j + 1, 256, 0, h->stream>>>(h->partial, h->hc, kDotBlocks, 1);   // hc += hp
+        dots(h, h->V, j + 1, h->w, h->hp, h->hc);    // second pass, hc += hp
         f2d_gs_update<<<blocks256(n), 256, 0, h->stream>>>(h->V, n, h->w, h->hp, j + 1, n);
         vnorm(h, h->w);
         info_reorth += 1;
       }
-      f2d_givens<<<1, 1, 0, h->stream>>>(h->H, h->hc, h->nrm, h->cs, h->sn, h->g, j, ldh);
+      f2d_givens<<<1, 32, 0, h->stream>>>({h->H, h->hc, h->cs, h->sn, h->g, h->nrm, h->ktarget, h->kctl, j, ldh});
       f2d_scale<<<blocks256(n), 256, 0, h->stream>>>(h->w, h->V + (long long)(j + 1) * n, h->nrm, n);
       double2 gj;
       F2_CK(cudaMemcpyAsync(&gj, h->g + j + 1, sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
@@ -2217,7 +2329,7 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
       h->resvec.push_back(est);
       if (!(est > target)) break;
     }
-    f2d_backsolve<<<1, 1, 0, h->stream>>>(h->H, h->g, h->yc, k, ldh);
+    wg::backsolve_kernel<<<1, 32, 0, h->stream>>>(h->H, h->g, h->yc, nullptr, h->kctl + 1, ldh, k, 1);
     f2d_combine<<<blocks256(n), 256, 0, h->stream>>>(h->Zb, n, h->yc, h->z, k, n);   // x += Z y
     f2d_axpy<<<blocks256(n), 256, 0, h->stream>>>(h->xs, h->z, n);
     info->cycles += 1;
@@ -2282,7 +2394,7 @@ int wg2d_solve_bicgstab(wg2d_problem* h, const double* rhs, double* x, const wg2
   }
   const unsigned nb = blocks256(n);
   auto read_dot = [&](const double2* a, const double2* b, double2* out) -> int {
-    dots(h, a, 1, b, h->hc, 0);
+    dots(h, a, 1, b, h->hc);
     F2_CK(cudaMemcpyAsync(out, h->hc, sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
     F2_CK(cudaStreamSynchronize(h->stream));
     return WG_OK;
