@@ -17,10 +17,9 @@
 //
 // Potential and CAP (applyFVConsistentDrift, get_Drift_full2D.m:331-364), per centre
 // element e and quadrature point q:
-//   f2d_interp_kernel    Uq[e][q][r] = sum_l W[q][l] U[r, id(e,l)]
-//   f2d_vertex_kernel    Rq[e][q][cell] = sum over the cell's 4 vertices v of dV[e][q][v] x
-//                        (sum of Uq over the <= 4 cells around v)   (P^T diag(dV) P)
-//   f2d_project_kernel   y[r, id(e,l)] = pot/16 sum_q Cp[q][l] Rq[e][q][r] + capc cap[r] U[r, id(e,l)]
+//   f2d_drift_kernel     y[r, id(e,l)] = pot/16 sum_q Cp[q][l] Rq[r] + capc cap[r] U[r, id(e,l)] with
+//                        Rq[r] = sum over the cell's 4 vertices v of dV[e][q][v] x (sum over the <= 4 cells
+//                        around v of sum_l W[q][l] U[., id(e,l)])   (P^T diag(dV) P)
 //   f2d_dv_kernel        dV from V on the material grid (bilinear, X clamped, Y clamped or wrapped).
 // All arithmetic FP64 (the plain form).
 #include <cuda_fp16.h>
@@ -66,7 +65,6 @@ struct wg2d_problem {
          *cap = nullptr, *dV = nullptr;
   double2 pot = {0, 0};
   double capc = 0;
-  double2 *Uq = nullptr, *Rq = nullptr;
   bool drift_ready = false, potential_ready = false;
   cudaEvent_t ev[4] = {};
   // line-transverse preconditioner (modes of -i D_rho_x, X lines, dense transverse inverses)
@@ -89,7 +87,7 @@ struct wg2d_problem {
   float *blocks32[2] = {nullptr, nullptr}, *coef32[2] = {nullptr, nullptr};
   float2* val32[2] = {nullptr, nullptr};
   float *interp32 = nullptr, *proj32 = nullptr, *cap32 = nullptr, *dV32 = nullptr;
-  float2 *Uq32 = nullptr, *Rq32 = nullptr, *G32 = nullptr;
+  float2* G32 = nullptr;
   int vm32 = 0;
   float2 *V32 = nullptr, *Z32 = nullptr, *w32 = nullptr;
   __half2* Vh32 = nullptr;    // the inner basis stored in FP16 (V32 unused then)
@@ -279,121 +277,114 @@ __global__ void __launch_bounds__(256) f2d_rely_kernel(const T* __restrict__ G, 
   y[i].y += acc.y;
 }
 
-// centre dof of local node l of element e (local order X fastest, elements X fastest)
-__device__ __forceinline__ long long center_id(int e, int l, int nex, int nkx, int nky, int nX) {
-  const int ex = e % nex, ey = e / nex;
-  const int lx = l % nkx, ly = l / nkx;
-  return (long long)(ex * nkx + lx) + (long long)nX * (ey * nky + ly);
-}
-
-// Uq[e][q][r] = sum_l W[q][l] F[r, id(e, l)]; grid (ceil(nrel/128), n_el)
+// Potential and CAP of one centre element: y[r, id(e,l)] = pot/16 sum_q Cp[q][l] sum_{vertices v of r} dV[e][q][v]
+// sum_{cells r' of v} sum_l' W[q][l'] F[r', id(e,l')] + capc cap[r] F[r, id(e,l)].  The quadrature sum is taken per
+// vertex, P_l(v) = sum_q Cp[q][l] dV_q(v) sum_l' W[q][l'] SF_l'(v) with SF the sums of F over the cells of v, so no
+// field at the quadrature points goes through memory.  A warp takes 32 vertices along rho_x (31 cells, P of the
+// next vertex by shuffle) and marches over `rows` rows of cells; the row below stays in registers.
+// Bound by the FMA chains per vertex (38 per point and vertex in FP32 at 9 local nodes; reads F and dV, writes y once).
+// 120 elements of 9 nodes, 25 points, 121 x 12 cells: 76 us in three launches -> 31 us in FP32, 641 -> 566 us in FP64
+// (64 cycles per warp instruction of a quarter: 480 us of sums with the repeated vertex rows).
 template <int NL, typename T, typename R>
-__global__ void __launch_bounds__(128) f2d_interp_kernel(const T* __restrict__ F, T* __restrict__ Uq,
-                                                         const R* __restrict__ W, int nq, int nrel, int nex,
-                                                         int nkx, int nky, int nX) {
-  const int r = blockIdx.x * 128 + threadIdx.x;
-  const int e = blockIdx.y;
-  if (r >= nrel) return;
-  T u[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) u[l] = F[center_id(e, l, nex, nkx, nky, nX) * nrel + r];
-  T* out = Uq + (long long)e * nq * nrel + r;
-  for (int q = 0; q < nq; ++q) {
-    T s = czero<T>();
+__global__ void __launch_bounds__(128) f2d_drift_kernel(const T* __restrict__ F, T* __restrict__ y,
+                                                        const R* __restrict__ W, const R* __restrict__ Cp,
+                                                        const R* __restrict__ dV, const R* __restrict__ cap, T pot16,
+                                                        R capc, int q0, int nqc, int nq, int nrx, int nry, int nvert,
+                                                        int nex, int nkx, int nX, int periodic, int xt, int bands,
+                                                        int rows, long long items) {
+  constexpr int NLP = (NL + 3) / 4 * 4;
+  extern __shared__ __align__(16) unsigned char drift_raw[];
+  R* sW = reinterpret_cast<R*>(drift_raw);   // [nqc][NLP]
+  R* sC = sW + nqc * NLP;
+  __shared__ long long off[NL];              // local node -> centre dof, times the cells
+  const long long nrel = (long long)nrx * nry;
+  for (int i = threadIdx.x; i < nqc * NLP; i += 128) {
+    const int q = i / NLP, l = i - q * NLP;
+    sW[i] = l < NL ? W[(q0 + q) * NL + l] : R(0);
+    sC[i] = l < NL ? Cp[(q0 + q) * NL + l] : R(0);
+  }
+  if (threadIdx.x < NL) off[threadIdx.x] = ((threadIdx.x % nkx) + (long long)nX * (threadIdx.x / nkx)) * nrel;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (item >= items) return;   // whole warps
+  const int xi = (int)(item % xt), band = (int)(item / xt % bands), e = (int)(item / xt / bands);
+  const int vi = xi * 31 + lane;                       // vertex; also the cell to its right
+  const bool left = vi >= 1 && vi - 1 < nrx, right = vi < nrx, on = vi <= nrx;
+  const int nky = NL / nkx;
+  const long long base = ((long long)(e % nex) * nkx + (long long)nX * (e / nex) * nky) * nrel;
+  const T* Fe = F + base + vi;
+  const R* De = dV + ((long long)e * nq + q0) * nvert + (on ? vi : 0);
+  const int j0 = band * rows, j1 = min(nry, j0 + rows);
+  T below[NL];
+  for (int vj = j0; vj <= j1; ++vj) {
+    int ja = vj - 1, jb = vj;                          // the rows of cells at this vertex row
+    if (periodic) {
+      ja = ja < 0 ? ja + nry : ja;
+      jb = jb >= nry ? jb - nry : jb;
+    }
+    const bool ra = ja >= 0, rb = jb < nry;
+    T SF[NL], P[NL];
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
-      const R w = W[q * NL + l];
-      s.x = fma(w, u[l].x, s.x);
-      s.y = fma(w, u[l].y, s.y);
+      const T* f = Fe + off[l];
+      T t0 = czero<T>(), t1 = t0, t2 = t0, t3 = t0;
+      if (ra && left) t0 = f[(long long)ja * nrx - 1];
+      if (ra && right) t1 = f[(long long)ja * nrx];
+      if (rb && left) t2 = f[(long long)jb * nrx - 1];
+      if (rb && right) t3 = f[(long long)jb * nrx];
+      SF[l].x = (t0.x + t1.x) + (t2.x + t3.x);
+      SF[l].y = (t0.y + t1.y) + (t2.y + t3.y);
+      P[l] = czero<T>();
     }
-    out[(long long)q * nrel] = s;
-  }
-}
-
-// sum of Uq over the cells around relative vertex (vi, vj) (cells vi-1..vi, vj-1..vj)
-template <typename T>
-__device__ __forceinline__ T vertex_sum(const T* __restrict__ U, int vi, int vj, int nrx, int nry,
-                                              bool periodic) {
-  T s = czero<T>();
+    const R* Dv = De + (long long)(periodic ? vj % nry : vj) * (nrx + 1);
+#pragma unroll 5
+    for (int q = 0; q < nqc; ++q) {
+      const R d = Dv[(long long)q * nvert];
+      T u = czero<T>();
 #pragma unroll
-  for (int dj = -1; dj <= 0; ++dj) {
-    int j = vj + dj;
-    if (periodic) j = (j + nry) % nry;
-    else if (j < 0 || j >= nry) continue;
+      for (int l = 0; l < NL; ++l) {
+        const R w = sW[q * NLP + l];
+        u.x = fma(w, SF[l].x, u.x);
+        u.y = fma(w, SF[l].y, u.y);
+      }
+      u.x *= d;
+      u.y *= d;
 #pragma unroll
-    for (int di = -1; di <= 0; ++di) {
-      const int i = vi + di;
-      if (i < 0 || i >= nrx) continue;
-      const T v = U[j * nrx + i];
-      s.x += v.x;
-      s.y += v.y;
+      for (int l = 0; l < NL; ++l) {
+        const R c = sC[q * NLP + l];
+        P[l].x = fma(c, u.x, P[l].x);
+        P[l].y = fma(c, u.y, P[l].y);
+      }
     }
-  }
-  return s;
-}
-
-// Rq[e][q][cell] = sum_{vertices v of cell} dV[e][q][v] vertex_sum(v); grid (ceil(nrel/128), nq, n_el)
-template <typename T, typename R>
-__global__ void __launch_bounds__(128) f2d_vertex_kernel(const T* __restrict__ Uq, T* __restrict__ Rq,
-                                                         const R* __restrict__ dV, int nrx, int nry, int nq,
-                                                         int nvert, int periodic) {
-  const int cell = blockIdx.x * 128 + threadIdx.x;
-  const int nrel = nrx * nry;
-  if (cell >= nrel) return;
-  const int q = blockIdx.y, e = blockIdx.z;
-  const long long slab = ((long long)e * nq + q);
-  const T* U = Uq + slab * nrel;
-  const R* D = dV + slab * nvert;
-  const int i = cell % nrx, j = cell / nrx;
-  const int nvx = nrx + 1;
-  T acc = czero<T>();
-#pragma unroll
-  for (int b = 0; b <= 1; ++b) {
-    int vj = j + b;
-    if (periodic) vj %= nry;
-#pragma unroll
-    for (int a = 0; a <= 1; ++a) {
-      const int vi = i + a;
-      const R d = D[vj * nvx + vi];
-      const T s = vertex_sum<T>(U, vi, vj, nrx, nry, periodic);
-      acc.x = fma(d, s.x, acc.x);
-      acc.y = fma(d, s.y, acc.y);
-    }
-  }
-  Rq[slab * nrel + cell] = acc;
-}
-
-// y[r, id(e,l)] = pot/16 sum_q Cp[q][l] Rq[e][q][r] + capc cap[r] F[r, id(e,l)]; grid (ceil(nrel/128), n_el)
-template <int NL, typename T, typename R>
-__global__ void __launch_bounds__(128) f2d_project_kernel(const T* __restrict__ Rq, const T* __restrict__ F,
-                                                          T* __restrict__ y, const R* __restrict__ Cp,
-                                                          const R* __restrict__ cap, T pot16, R capc,
-                                                          int nq, int nrel, int nex, int nkx, int nky, int nX) {
-  const int r = blockIdx.x * 128 + threadIdx.x;
-  const int e = blockIdx.y;
-  if (r >= nrel) return;
-  T s[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) s[l] = czero<T>();
-  const T* Rr = Rq + (long long)e * nq * nrel + r;
-  for (int q = 0; q < nq; ++q) {
-    const T v = Rr[(long long)q * nrel];
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
-      const R c = Cp[q * NL + l];
-      s[l].x = fma(c, v.x, s[l].x);
-      s[l].y = fma(c, v.y, s[l].y);
+      P[l].x += __shfl_down_sync(0xffffffffu, P[l].x, 1);
+      P[l].y += __shfl_down_sync(0xffffffffu, P[l].y, 1);
     }
-  }
-  const R cr = capc * cap[r];
+    if (vj > j0 && right && lane < 31) {
+      const long long cell = (long long)(vj - 1) * nrx;
+      const R cr = capc * cap[cell + vi];
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    const long long idx = center_id(e, l, nex, nkx, nky, nX) * nrel + r;
-    const T f = F[idx];
-    T o;
-    o.x = pot16.x * s[l].x - pot16.y * s[l].y + cr * f.x;
-    o.y = pot16.x * s[l].y + pot16.y * s[l].x + cr * f.y;
-    y[idx] = o;
+      for (int l = 0; l < NL; ++l) {
+        T* yo = y + base + off[l] + cell + vi;
+        T f = czero<T>();
+        if (q0 == 0) {
+          f = Fe[off[l] + cell];
+          f.x *= cr;
+          f.y *= cr;
+        } else {
+          f = *yo;
+        }
+        const T s = {below[l].x + P[l].x, below[l].y + P[l].y};
+        T o;
+        o.x = pot16.x * s.x - pot16.y * s.y + f.x;
+        o.y = pot16.x * s.y + pot16.y * s.x + f.y;
+        *yo = o;
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < NL; ++l) below[l] = P[l];
   }
 }
 
@@ -1251,7 +1242,7 @@ struct OpData {
   const T* val[2];
   const R* coef[2];
   const R *interp, *proj, *cap, *dV;
-  T *Uq, *Rq, *G;
+  T* G;
   T pot16;
   R capc;
 };
@@ -1301,8 +1292,6 @@ OpData<double2, double> op64(wg2d_problem* h) {
   d.proj = h->proj;
   d.cap = h->cap;
   d.dV = h->dV;
-  d.Uq = h->Uq;
-  d.Rq = h->Rq;
   d.G = h->G;
   d.pot16 = make_double2(h->pot.x / 16.0, h->pot.y / 16.0);
   d.capc = h->capc;
@@ -1325,13 +1314,20 @@ int apply_transport(wg2d_problem* h, int axis) {
 template <int NL, typename T, typename R>
 void launch_drift(wg2d_problem* h, const OpData<T, R>& d, const T* F, T* y) {
   const wg2d_shape& s = h->s;
-  const dim3 g1((unsigned)((h->nrel + 127) / 128), (unsigned)h->nel);
-  f2d_interp_kernel<NL, T, R><<<g1, 128, 0, h->stream>>>(F, d.Uq, d.interp, h->nq, h->nrel, s.n_el_x, s.nk_x, s.nk_y,
-                                                         h->nX);
-  const dim3 g2((unsigned)((h->nrel + 127) / 128), (unsigned)h->nq, (unsigned)h->nel);
-  f2d_vertex_kernel<T, R><<<g2, 128, 0, h->stream>>>(d.Uq, d.Rq, d.dV, h->nrx, h->nry, h->nq, h->nvert, s.periodic_y);
-  f2d_project_kernel<NL, T, R><<<g1, 128, 0, h->stream>>>(d.Rq, F, y, d.proj, d.cap, d.pot16, d.capc, h->nq, h->nrel,
-                                                          s.n_el_x, s.nk_x, s.nk_y, h->nX);
+  // rows of cells per warp: as many as still give 16 warps per SM, at least 3 (one more vertex row than cell rows)
+  const int xt = (h->nrx + 30) / 31;
+  const long long all = (long long)xt * h->nel * h->nry;
+  const int rows = (int)std::min<long long>(h->nry, std::max<long long>(3, all / (152 * 16)));
+  const int bands = (h->nry + rows - 1) / rows;
+  const long long items = (long long)xt * bands * h->nel;
+  // W and Cp of as many quadrature points as 40 KB hold, further points in further launches that add to y
+  constexpr int per_point = (int)sizeof(R) * 2 * ((NL + 3) / 4 * 4), most = 40 * 1024 / per_point;
+  for (int q0 = 0; q0 < h->nq; q0 += most) {
+    const int nqc = std::min(most, h->nq - q0);
+    f2d_drift_kernel<NL, T, R><<<(unsigned)((items + 3) / 4), 128, (size_t)per_point * nqc, h->stream>>>(
+        F, y, d.interp, d.proj, d.dV, d.cap, d.pot16, d.capc, q0, nqc, h->nq, h->nrx, h->nry, h->nvert, s.n_el_x, s.nk_x,
+        h->nX, s.periodic_y, xt, bands, rows, items);
+  }
 }
 
 template <typename T, typename R>
@@ -1449,8 +1445,6 @@ int wg2d_create(const wg2d_shape* s, wg2d_problem** out) {
   const size_t slab = (size_t)h->nel * h->nq;
   if (e == cudaSuccess) e = dalloc(&h->x, h->n);
   if (e == cudaSuccess) e = dalloc(&h->y, h->n);
-  if (e == cudaSuccess) e = dalloc(&h->Uq, slab * h->nrel);
-  if (e == cudaSuccess) e = dalloc(&h->Rq, slab * h->nrel);
   if (e == cudaSuccess) e = dalloc(&h->dV, slab * h->nvert);
   if (e == cudaSuccess) e = dalloc(&h->interp, (size_t)h->nq * h->nloc);
   if (e == cudaSuccess) e = dalloc(&h->proj, (size_t)h->nq * h->nloc);
@@ -1482,7 +1476,7 @@ int wg2d_destroy(wg2d_problem* h) {
   free_preconditioner(h);
   free32(h);
   wg::ozaki_free(h->cols);
-  void* ptrs[] = {h->x, h->y, h->G, h->Uq, h->Rq, h->dV, h->interp, h->proj, h->xq, h->yq, h->vx, h->vy, h->cap,
+  void* ptrs[] = {h->x, h->y, h->G, h->dV, h->interp, h->proj, h->xq, h->yq, h->vx, h->vy, h->cap,
                   h->tc_err, h->obs_W, h->obs_wj, h->obs_out, h->wall_act, h->wall_T, h->wall_T32, h->wall_u,
                   h->wall_u32};
   for (void* p : ptrs)
@@ -1916,13 +1910,13 @@ int wg2d_apply_repeat(wg2d_problem* h, int n, double* ms, double* parts_ms) {
 
 static void free32(wg2d_problem* h) {
   void* ptrs[] = {h->blocks32[0], h->blocks32[1], h->coef32[0], h->coef32[1], h->val32[0], h->val32[1], h->interp32,
-                  h->proj32, h->cap32, h->dV32, h->Uq32, h->Rq32, h->G32, h->V32, h->Z32, h->w32, h->Vh32, h->vj32};
+                  h->proj32, h->cap32, h->dV32, h->G32, h->V32, h->Z32, h->w32, h->Vh32, h->vj32};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   h->blocks32[0] = h->blocks32[1] = h->coef32[0] = h->coef32[1] = nullptr;
   h->val32[0] = h->val32[1] = nullptr;
   h->interp32 = h->proj32 = h->cap32 = h->dV32 = nullptr;
-  h->Uq32 = h->Rq32 = h->G32 = h->V32 = h->Z32 = h->w32 = h->vj32 = nullptr;
+  h->G32 = h->V32 = h->Z32 = h->w32 = h->vj32 = nullptr;
   h->Vh32 = nullptr;
   h->vm32 = 0;
   h->d32_ready = false;
@@ -1968,8 +1962,6 @@ static int ensure32(wg2d_problem* h) {
   if (!rc) rc = conv(&h->cap32, h->cap, h->nrel);
   if (!rc) rc = conv(&h->dV32, h->dV, slab * h->nvert);
   if (rc) return rc;
-  F2_CK(dalloc(&h->Uq32, slab * h->nrel));
-  F2_CK(dalloc(&h->Rq32, slab * h->nrel));
   F2_CK(dalloc(&h->G32, (size_t)std::max(1, std::max(h->ax[0].T, h->ax[1].T)) * h->n));
   if (h->nrx * kRelxCols * sizeof(float2) > 48 * 1024)
     F2_CK(cudaFuncSetAttribute(f2d_relx_kernel<float2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1992,8 +1984,6 @@ OpData<float2, float> op32(wg2d_problem* h) {
   d.proj = h->proj32;
   d.cap = h->cap32;
   d.dV = h->dV32;
-  d.Uq = h->Uq32;
-  d.Rq = h->Rq32;
   d.G = h->G32;
   d.pot16 = make_float2((float)(h->pot.x / 16.0), (float)(h->pot.y / 16.0));
   d.capc = (float)h->capc;
