@@ -643,11 +643,13 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, bool pre, Prec prec, App
   return WG_OK;
 }
 
+constexpr int kResidualDigits = 7;   // of the emulated FP64 transforms in the mixed form's residual (digits_for)
+
 // r = rhs - A x ; nrm[b] = |r_b|  (FP64)
 // r = b - A x and |r| (FP64; the mixed form's transforms on the tensor cores).  mask
 // (device, optional): only problems with mask[b] != 0 are evaluated, the others keep
 // their previous r and |r| (their x has not changed since).
-int true_residual(Problem& P, const int* mask = nullptr, int nd = 8, const int* nd_pp = nullptr) {
+int true_residual(Problem& P, const int* mask = nullptr, int nd = kResidualDigits, const int* nd_pp = nullptr) {
   const long long tot = P.N * P.batch;
   P.prof.launches[PROF_OTHER] += 3;
   if (P.precision == WG_PREC_MIXED) WG_CK(launch_apply_f64_tc(P, P.x, P.w, mask, nd, nd_pp));
@@ -662,13 +664,13 @@ int true_residual(Problem& P, const int* mask = nullptr, int nd = 8, const int* 
 }
 
 // Leading digits of the emulated FP64 transforms for the mixed form's true residual: enough
-// that the residual's error (~2^(-6 nd) |A||x|, with a margin of 2^21 for |A||x| / |b|) stays
-// below the loosest target among the problems it is evaluated for; 8 (the full split) for
-// tolerances of 1e-7 and below.  WG_RESIDUAL_DIGITS (1 .. 8) fixes it.
+// that the residual's error (~2^(-7 nd) |A||x|, with a margin of 2^21 for |A||x| / |b|) stays
+// below the loosest target among the problems it is evaluated for; 7 (49 bits) for
+// tolerances of 1e-6 and below.  WG_RESIDUAL_DIGITS (1 .. 8) fixes it.
 int digits_for(double t) {
-  if (!(t > 0) || !(t < 1e299)) return 8;
-  const int d = (int)std::ceil((std::log2(1.0 / t) + 21.0) / 6.0);
-  return std::max(4, std::min(8, d));
+  if (!(t > 0) || !(t < 1e299)) return kResidualDigits;
+  const int d = (int)std::ceil((std::log2(1.0 / t) + 21.0) / 7.0);
+  return std::max(4, std::min(kResidualDigits, d));
 }
 
 int residual_digits(const Problem& P, double tol, const std::vector<int>* hmask) {
@@ -690,7 +692,7 @@ int residual_digits(const Problem& P, double tol, const std::vector<int>* hmask)
 // uploads them and returns the device array, or nullptr when one count serves all.
 const int* residual_digits_pp(Problem& P, double tol) {
   if (P.tol_pp.empty() || std::getenv("WG_RESIDUAL_DIGITS")) return nullptr;
-  P.h_res_digits.assign(P.batch, 8);
+  P.h_res_digits.assign(P.batch, kResidualDigits);
   for (int b = 0; b < P.batch; ++b) P.h_res_digits[b] = digits_for(P.tol_pp[b]);
   if (cudaMemcpyAsync(P.res_digits, P.h_res_digits.data(), sizeof(int) * P.batch, cudaMemcpyHostToDevice,
                       P.stream) != cudaSuccess)
@@ -713,7 +715,7 @@ int solve_begin(Problem& P, double tol, bool warm, std::vector<double>& bnorm, s
   for (int b = 0; b < B; ++b) tgt[b] = (P.tol_pp.empty() ? tol : P.tol_pp[b]) * bnorm[b];
   // problems frozen by an unreachable tolerance keep their residual
   const int* mask = nullptr;
-  int nd = 8;
+  int nd = kResidualDigits;
   if (P.precision == WG_PREC_MIXED) {
     if (!P.tol_pp.empty()) {
       P.h_res_mask.assign(B, 1);

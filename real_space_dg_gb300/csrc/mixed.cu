@@ -77,10 +77,12 @@ bool make_map3(CUtensorMap* m, const void* base, long long rows, int K, int box_
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Digits of the rows of a row-major M x K FP64 matrix (host), the split of
-// slice_columns_kernel: row r with max|a| < 2^m has F = round(a 2^(6S-1-m)) written
-// in balanced base-64 digits, a = 2^e[r] sum_p t_p 2^(-6(p+1)), e[r] = m + 1.
-void slice_rows_host(const std::vector<double>& A, int M, int K, std::vector<bf16>& dig, std::vector<int>& e) {
+// Digits of the rows of a row-major M x K FP64 matrix (host), the split of slice_columns_kernel (bits = 6) and
+// slice_pairs_kernel (7): row r with max|a| < 2^m has F = round(a 2^(bits S-1-m)) written
+// in balanced digits, a = 2^e[r] sum_p t_p 2^(-bits(p+1)), e[r] = m + 1.
+void slice_rows_host(const std::vector<double>& A, int M, int K, std::vector<bf16>& dig, std::vector<int>& e,
+                     int bits = oz::BETA) {
+  const long long half = 1ll << (bits - 1), digit = (1ll << bits) - 1;
   dig.assign((size_t)oz::S * M * K, __float2bfloat16(0.f));
   e.assign(M, 0);
   for (int r = 0; r < M; ++r) {
@@ -92,13 +94,12 @@ void slice_rows_host(const std::vector<double>& A, int M, int K, std::vector<bf1
     e[r] = m + 1;
     for (int k = 0; k < K; ++k) {
       const double a = A[(size_t)r * K + k];
-      // |a| 2^(6S-1-m) < 2^47: adding one half is exact
-      long long F = (long long)std::floor(std::ldexp(std::fabs(a), oz::BETA * oz::S - 1 - m) + 0.5);
+      long long F = std::llrint(std::ldexp(std::fabs(a), bits * oz::S - 1 - m));
       if (a < 0) F = -F;
       for (int p = oz::S - 1; p > 0; --p) {
-        const long long d = ((F + 32) & 63) - 32;
+        const long long d = ((F + half) & digit) - half;
         dig[((size_t)p * M + r) * K + k] = __float2bfloat16((float)d);
-        F = (F - d) >> oz::BETA;
+        F = (F - d) >> bits;
       }
       dig[(size_t)r * K + k] = __float2bfloat16((float)F);
     }
@@ -135,7 +136,7 @@ cudaError_t launch_pairs(Problem& P, const CUtensorMap& a, const CUtensorMap& b,
   if (nd < 1 || nd > oz::S) return cudaErrorInvalidValue;
   const int npp = (int)(P.ncols / P.batch), Kp = pair_row(K);
   auto slice = Kp <= 64 ? oz::slice_pairs_kernel<1> : Kp <= 128 ? oz::slice_pairs_kernel<2> : oz::slice_pairs_kernel<4>;
-  slice<<<slice_blocks(P.ncols), 32 * oz::kSliceColsPerBlock, 0, P.stream>>>(
+  slice<<<(unsigned)((P.ncols + oz::kSlicePairNodes - 1) / oz::kSlicePairNodes), 128 * oz::kSlicePairNodes, 0, P.stream>>>(
       X, K, P.ncols, P.mx.ob, P.mx.eb, mask, npp, Kp, nd, nd_pp);
   const dim3 grid((M / 2 + oz::BM - 1) / oz::BM, (unsigned)((2 * P.ncols + oz::BN - 1) / oz::BN));
   oz::gemm_pairs_kernel<MODE><<<grid, oz::PAIR_THREADS, oz::SMEM_BYTES, P.stream>>>(
@@ -717,8 +718,8 @@ int ozaki_alloc(Problem& P) {
       return WG_ERR_CUDA;
     }
   }
-  // exact grouped accumulation (K <= MAX_K) and 16-byte TMA rows of the digit slices
-  M.ozaki = 2 * nk <= oz::MAX_K && 2 * nxi <= oz::MAX_K && nk % 4 == 0 && nxi % 4 == 0;
+  // exact grouped accumulation (K <= PAIR_MAX_K) and 16-byte TMA rows of the digit slices
+  M.ozaki = nk <= 2 * oz::PAIR_MAX_K && nxi <= 2 * oz::PAIR_MAX_K && nk % 4 == 0 && nxi % 4 == 0;
   if (M.ozaki) {
     // lower halves of the symmetric basis (gemm_pairs_kernel): real parts, then imaginary parts
     const int hk = nk / 2, hs = nxi / 2, K1 = pair_row(nk), K2 = pair_row(nxi), kmax = std::max(K1, K2);
@@ -733,8 +734,8 @@ int ozaki_alloc(Problem& P) {
       }
     std::vector<bf16> d1, d2;
     std::vector<int> e1, e2;
-    slice_rows_host(A1, 2 * hs, K1, d1, e1);
-    slice_rows_host(A2, 2 * hk, K2, d2, e2);
+    slice_rows_host(A1, 2 * hs, K1, d1, e1, oz::PAIR_BITS);
+    slice_rows_host(A2, 2 * hk, K2, d2, e2, oz::PAIR_BITS);
     cudaError_t ce = cudaSuccess;
     auto C2 = [&](cudaError_t r) { if (ce == cudaSuccess) ce = r; };
     C2(cudaMalloc(&M.oa1, sizeof(bf16) * d1.size()));

@@ -247,13 +247,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ozaki_kernel(const __grid_con
 // Integer arithmetic on the FP64 bit patterns only.
 constexpr int kSliceColsPerBlock = 8;   // one warp per column
 
+template <int BITS = BETA>
 __device__ __forceinline__ long long round_scaled(long long bits, int m, bool nonzero) {
   const int ex = (int)((bits >> 52) & 0x7FF);
-  long long F = 0;   // round(|x| 2^(6S-1-m)) <= 2^(6S-1)
+  long long F = 0;   // round(|x| 2^(BITS S-1-m)) <= 2^(BITS S-1)
   if (ex != 0 && nonzero) {
     const unsigned long long mant = ((unsigned long long)bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    const int rs = m - (ex - 1023 - 52) - (BETA * S - 1);   // >= 6 since |x| < 2^m
-    if (rs < 64) F = (long long)((mant + (1ull << (rs - 1))) >> rs);
+    const int rs = m - (ex - 1023 - 52) - (BITS * S - 1);   // >= 54 - BITS S since |x| < 2^m
+    if (rs <= 0) F = (long long)(mant << -rs);
+    else if (rs < 64) F = (long long)((mant + (1ull << (rs - 1))) >> rs);
   }
   return bits < 0 ? -F : F;
 }
@@ -318,11 +320,22 @@ __global__ void __launch_bounds__(32 * kSliceColsPerBlock) slice_columns_kernel(
 // flight meanwhile), and writes both members of every output pair.  Warps 0 .. 15 drain, 16 loads, 17 issues.
 //   MODE 0: Y = Phi X.   MODE 1: Y += i Phi^H X.
 // The table's digits dominated the L2 traffic of the embedded product (1 MB per 64 nodes, a quarter of it per CTA;
-// now 0.5 MB per 32 nodes for both planes).  With slicing, per transform: 333 -> 219 us (16 problems of 960 nodes,
-// 256 x 256; slicing 55 of it), 240 -> 158 us (4 of 720 nodes, 512 x 512: 180 CTAs on 152 SMs).
+// now 0.5 MB per 32 nodes for both planes).  Half the columns also leave room for 7 bits a digit: |t| <= 64, and 8
+// products of K <= 256 pairs stay at 8 * 64^2 * 256 = 2^23, exact in FP32.  Eight digits carry 56 bits of a column's
+// largest entry, more than FP64 keeps of a sum of K such terms; seven (28 products of digits instead of 36) carry 49, one more
+// than eight of 6 bits.  With slicing, per transform: 333 -> 210 us (16 problems of 960 nodes,
+// 256 x 256), 240 -> 133 us (4 of 720 nodes, 512 x 512: 180 CTAs on 152 SMs); with eight digits of 6 bits 219 and 158 us.
+// 36 products of digits take 10 us of a CTA's 40; the rest is the latency of its first loads, of two ring stages and
+// of reading the accumulators twice.
 // ---------------------------------------------------------------------------------------------
 constexpr int PAIR_THREADS = THREADS + 64;
-
+constexpr int PAIR_BITS = 7, PAIR_MAX_K = 256;   // bits per digit, pairs per row
+constexpr int kPairFixBits = 56;                 // unit 2^-56; |sum| <= K / 4 = 2^6 of it
+// Two neighbouring groups are one 32-bit integer (2^23 2^7 + 2^23); pair j (groups 2j, 2j + 1) has weight 2^(-21 - 14 j),
+// the last one is rounded by 7 bits.
+__device__ __forceinline__ long long pair_fixed(const int (&c)[4]) {
+  return ((long long)c[0] << 35) + ((long long)c[1] << 21) + ((long long)c[2] << 7) + ((c[3] + 64) >> 7);
+}
 template <int MODE>
 __global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pairs_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const int* __restrict__ ea,
@@ -428,21 +441,23 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pairs_kernel(
       if (ok) ok = tc::mbar_wait(&done[ph], 0, err);
       tc::fence_after();
       if (ok) {
-        long long fx[EC];
+        int c[EC][4];
 #pragma unroll
-        for (int i = 0; i < EC; ++i) fx[i] = 0;
-#pragma unroll 1
-        for (int g = 0; g < nd; ++g) {
-          float v[EC];
-          tmem_ld16(tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(g * BN + cb * EC), v);
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t t = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(2 * j * BN + cb * EC);
+          float v[EC], w[EC];
 #pragma unroll
-          for (int i = 0; i < EC; ++i) fx[i] += group_fixed(v[i], g);
+          for (int i = 0; i < EC; ++i) v[i] = w[i] = 0.f;
+          if (2 * j < nd) tmem_ld16(t, v);
+          if (2 * j + 1 < nd) tmem_ld16(t + BN, w);
+#pragma unroll
+          for (int i = 0; i < EC; ++i) c[i][j] = __float2int_rn(v[i]) * 128 + __float2int_rn(w[i]);
         }
-        const int er = (row < hm ? ea[ph * hm + row] : 0) - kFixBits;
+        const int er = (row < hm ? ea[ph * hm + row] : 0) - kPairFixBits;
         const int* ebp = eb + ph * Ncol2 + c0;
 #pragma unroll
         for (int i = 0; i < EC; ++i)
-          (ph == 0 ? va : vb)[i] = fixed_to_double(fx[i], er + (i < ncb ? ebp[i] : 0));
+          (ph == 0 ? va : vb)[i] = fixed_to_double(pair_fixed(c[i]), er + (i < ncb ? ebp[i] : 0));
       }
       if (ph == 0) {
         tc::fence_before();
@@ -478,16 +493,18 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pairs_kernel(
   }
 }
 
-// Digits of E and O of every node's complex column (K entries, K even and at most 512), one warp per node, two
-// consecutive pairs per lane and pass; the four real columns stay in registers between their maxima and their digits.
-// Rows of Kout entries (>= K / 2, zero-padded).  nd, nd_pp: the digits gemm_pairs_kernel reads for the node's tile.
-// PASSES of 64 entries cover Kout (1, 2 or 4).
+// Digits of E and O of every node's complex column (K entries, K even and at most 512), one warp per real column (E re,
+// E im, O re, O im of a node: four warps share its loads through the L1; one warp per node left a chain of 1,900
+// instructions, 14 us at 1,920 nodes of 256 entries against 11), two consecutive pairs per lane and pass; the column
+// stays in registers between its maximum and its digits.  Rows of Kout entries (>= K / 2, zero-padded).  nd, nd_pp:
+// the digits gemm_pairs_kernel reads for the node's tile.  PASSES of 64 entries cover Kout (1, 2 or 4).
+constexpr int kSlicePairNodes = 2;   // per block of eight warps
 template <int PASSES>
-__global__ void __launch_bounds__(32 * kSliceColsPerBlock) slice_pairs_kernel(
+__global__ void __launch_bounds__(128 * kSlicePairNodes) slice_pairs_kernel(
     const double2* __restrict__ X, int K, long long ncols, __nv_bfloat16* __restrict__ slices, int* __restrict__ e_out,
     const int* __restrict__ mask, int nodes_per_problem, int Kout, int nd, const int* __restrict__ nd_pp) {
-  const int lane = threadIdx.x & 31;
-  const long long c = (long long)blockIdx.x * kSliceColsPerBlock + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, o = (threadIdx.x >> 5) & 3;
+  const long long c = (long long)blockIdx.x * kSlicePairNodes + (threadIdx.x >> 7);
   if (c >= ncols || (mask && !mask[c / nodes_per_problem])) return;
   int ndt = nd < 1 ? 1 : (nd > S ? S : nd);
   if (nd_pp) {
@@ -498,52 +515,47 @@ __global__ void __launch_bounds__(32 * kSliceColsPerBlock) slice_pairs_kernel(
       if (!mask || mask[b] != 0) ndt = max(ndt, min(S, max(1, nd_pp[b])));
   }
   const int h = K / 2;
-  const double2* x = X + c * K;
-  double v[4][PASSES][2];   // E re, E im, O re, O im
-  unsigned long long mx[4] = {0, 0, 0, 0};
+  const double* x = reinterpret_cast<const double*>(X + c * K) + (o & 1);
+  const bool odd = o >> 1;
+  long long v[PASSES][2];
+  unsigned long long mx = 0;
 #pragma unroll
   for (int t = 0; t < PASSES; ++t)
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int p = 64 * t + 2 * lane + u;
-      const bool in = p < h;
-      const double2 a = in ? x[p] : make_double2(0.0, 0.0), b = in ? x[K - 1 - p] : make_double2(0.0, 0.0);
-      v[0][t][u] = in ? a.x + b.x : 0.0;
-      v[1][t][u] = in ? a.y + b.y : 0.0;
-      v[2][t][u] = in ? a.x - b.x : 0.0;
-      v[3][t][u] = in ? a.y - b.y : 0.0;
-#pragma unroll
-      for (int o = 0; o < 4; ++o) {
-        const unsigned long long w = (unsigned long long)__double_as_longlong(v[o][t][u]) & 0x7FFFFFFFFFFFFFFFull;
-        mx[o] = w > mx[o] ? w : mx[o];
+      double w = 0.0;
+      if (p < h) {
+        const double a = x[2 * p], b = x[2 * (K - 1 - p)];
+        w = odd ? a - b : a + b;
       }
+      v[t][u] = __double_as_longlong(w);
+      const unsigned long long m = (unsigned long long)v[t][u] & 0x7FFFFFFFFFFFFFFFull;
+      mx = m > mx ? m : mx;
     }
+  for (int q = 16; q > 0; q >>= 1) {
+    const unsigned long long t = __shfl_xor_sync(0xffffffffu, mx, q);
+    mx = t > mx ? t : mx;
+  }
+  const int m = mx == 0 ? 0 : (int)((mx >> 52) & 0x7FF) - 1023 + 1;   // max|x| < 2^m
   const long long Ncol2 = 2 * ncols, slice_stride = 2 * Ncol2 * (long long)Kout;
+  const long long r = (o >> 1) * Ncol2 + 2 * c + (o & 1);
+  if (lane == 0) e_out[r] = m + 1;
+  __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(slices + r * Kout);
 #pragma unroll
-  for (int o = 0; o < 4; ++o) {
-    for (int q = 16; q > 0; q >>= 1) {
-      const unsigned long long t = __shfl_xor_sync(0xffffffffu, mx[o], q);
-      mx[o] = t > mx[o] ? t : mx[o];
+  for (int t = 0; t < PASSES; ++t) {
+    const int k = 32 * t + lane;
+    if (2 * k >= Kout) continue;
+    long long F0 = round_scaled<PAIR_BITS>(v[t][0], m, mx != 0);
+    long long F1 = round_scaled<PAIR_BITS>(v[t][1], m, mx != 0);
+#pragma unroll
+    for (int p = S - 1; p > 0; --p) {
+      const int d0 = (int)(((F0 + 64) & 127) - 64), d1 = (int)(((F1 + 64) & 127) - 64);
+      if (p < ndt) out[p * (slice_stride / 2) + k] = __floats2bfloat162_rn((float)d0, (float)d1);
+      F0 = (F0 - d0) >> PAIR_BITS;
+      F1 = (F1 - d1) >> PAIR_BITS;
     }
-    const int m = mx[o] == 0 ? 0 : (int)((mx[o] >> 52) & 0x7FF) - 1023 + 1;   // max|x| < 2^m
-    const long long r = (o >> 1) * Ncol2 + 2 * c + (o & 1);
-    if (lane == 0) e_out[r] = m + 1;
-    __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(slices + r * Kout);
-#pragma unroll
-    for (int t = 0; t < PASSES; ++t) {
-      const int k = 32 * t + lane;
-      if (2 * k >= Kout) continue;
-      long long F0 = round_scaled(__double_as_longlong(v[o][t][0]), m, mx[o] != 0);
-      long long F1 = round_scaled(__double_as_longlong(v[o][t][1]), m, mx[o] != 0);
-#pragma unroll
-      for (int p = S - 1; p > 0; --p) {
-        const int d0 = (int)(((F0 + 32) & 63) - 32), d1 = (int)(((F1 + 32) & 63) - 32);
-        if (p < ndt) out[p * (slice_stride / 2) + k] = __floats2bfloat162_rn((float)d0, (float)d1);
-        F0 = (F0 - d0) >> BETA;
-        F1 = (F1 - d1) >> BETA;
-      }
-      out[k] = __floats2bfloat162_rn((float)F0, (float)F1);
-    }
+    out[k] = __floats2bfloat162_rn((float)F0, (float)F1);
   }
 }
 
