@@ -372,6 +372,21 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
       return fail(nullptr, mr, msg);
     }
   }
+  // FP64 transforms as digit products where they are faster: only within the admission budget, and while their
+  // buffers are a small part of the memory left (a later handle would have fitted before)
+  if (P.precision == WG_PREC_FP64 && !P.fp64_tc && wg::ozaki_pays(s)) {
+    const double extra = wg::ozaki_bytes(s, P.ncols);
+    size_t free_b = 0, total_b = 0;
+    if ((P.mem_budget <= 0 || est + extra <= P.mem_budget) && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+        16.0 * extra <= (double)free_b) {
+      P.fp64_tc = wg::ozaki_alloc(P) == WG_OK && P.mx.ozaki;
+      if (!P.fp64_tc) {
+        cudaGetLastError();
+        wg::mixed_free(P);
+        P.err.clear();
+      }
+    }
+  }
   P.hp.resize(batch);
   P.h_nrm.resize(batch);
   P.h_active.resize(batch);

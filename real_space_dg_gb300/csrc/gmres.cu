@@ -865,7 +865,7 @@ int gmres_solve_fp64(Problem& P, const wg_solve_opts& o, bool warm, wg_solve_inf
   auto prec = [&](const double2* r, long long stride, const double* rscale, double2* rout) {
     return launch_precondition(P, r, stride, P.z, rscale, rout, (long long)mp1 * N);
   };
-  const bool pre = flux_is_inverted(P) && !(P.fp64_tc && P.mx.ozaki);
+  const bool pre = flux_is_inverted(P);
   auto apply = [&](const double2* v) {
     return pre ? launch_apply_pre(P, P.z, v, (long long)mp1 * N, P.w) : launch_apply(P, P.z, P.w);
   };

@@ -125,7 +125,7 @@ cudaError_t launch_ozaki(const CUtensorMap& a, const CUtensorMap& b, const int* 
 // Row length of the pair digits of K complex entries: K / 2 in whole 16-byte TMA rows, one k block at least.
 int pair_row(int K) { return std::max(oz::BK, (K / 2 + 7) & ~7); }
 
-// Y = Phi X (MODE 0) or Y += i Phi^H X (MODE 1) on the tensor cores: slicing and gemm_pairs_kernel.  X: K complex entries
+// Y = Phi X (MODE 0), Y += i Phi^H X (MODE 1) or Y = i Phi^H X (MODE 2) on the tensor cores: slicing and gemm_pairs_kernel.  X: K complex entries
 // per column, Y: M.
 template <int MODE>
 cudaError_t launch_pairs(Problem& P, const CUtensorMap& a, const CUtensorMap& b, const int* ea, const double2* X,
@@ -707,6 +707,22 @@ int mixed_alloc(Problem& P) {
   return ozaki_alloc(P);
 }
 
+double ozaki_bytes(const Shape& s, long long ncols) {
+  const double kmax = std::max(pair_row(s.nk), pair_row(s.nxi));
+  return 2.0 * oz::S * 4 * (double)ncols * kmax + 16.0 * ncols + 2.0 * oz::S * 2 * kmax * std::max(s.nk, s.nxi);
+}
+
+// FP64 handles whose transforms are faster as products of digits: a CTA of gemm_pairs_kernel takes 40 us whatever
+// the number of nodes up to 32 an SM, the native kernel 2 us per 10^6 table entries and nodes of one problem.
+// 960 nodes of 256 x 256 (6.3e7): 125 -> 54 us, two problems 224 -> 58 us; 240 nodes (1.6e7): 42 us native, 54 us; 960 of
+// 128 x 128 (1.6e7): 41 us both.  A rule on one problem, so that its results do not depend on the batch it is in.  The
+// digits keep 56 bits of a column's largest entry: the rounding error of the operator on 116 to 240 elements, Nk = 200 to 512,
+// fell from 1.6e-16 .. 1.0e-15 (native sums) to 1.5e-16 .. 2.4e-16 of |A x|.
+bool ozaki_pays(const Shape& s) {
+  return s.nk % 4 == 0 && s.nxi % 4 == 0 && s.nk <= 2 * oz::PAIR_MAX_K && s.nxi <= 2 * oz::PAIR_MAX_K &&
+         (double)s.n_el * s.nK * s.nk * s.nxi >= 3e7;
+}
+
 int ozaki_alloc(Problem& P) {
   MixedBuffers& M = P.mx;
   const Shape& s = P.s;
@@ -951,12 +967,13 @@ int debug_gemm_bf16(const float* A, const float* B, float* C, int M, int N, int 
 // FP64 operator apply of the mixed form's outer residual: flux and xi stencil in
 // FP64, both transforms as digit-sliced FP64 GEMMs on the tensor cores.
 cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const int* mask, int nd,
-                                const int* nd_pp) {
+                                const int* nd_pp, bool potential_only) {
   MixedBuffers& M = P.mx;
   if (!M.ozaki) return launch_apply(P, x, y);
   const Shape& s = P.s;
   const double ncols = (double)P.ncols;
-  cudaError_t e = launch_flux_f64(P, x, y, mask);
+  cudaError_t e = cudaSuccess;
+  if (!potential_only) e = launch_flux_f64(P, x, y, mask);
   if (e != cudaSuccess) return e;
   // work of one transform: read the FP64 operand (slicing), write the FP64 result; flops of
   // ONE BF16 digit-slice product of both planes, weighted by the products the digits need
@@ -969,7 +986,8 @@ cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const 
   e = launch_stencil_f64(P, P.xh, P.yh, mask);
   if (e != cudaSuccess) return e;
   ev = prof_begin(P, PROF_GEMM_F64TC, 2, 16.0 * s.nxi * ncols + 16.0 * P.N * P.batch, prod_flops, mask, nd, nd_pp);
-  e = launch_pairs<1>(P, M.tmOA2, M.tmOB2, M.ea2, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp);
+  e = potential_only ? launch_pairs<2>(P, M.tmOA2, M.tmOB2, M.ea2, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp)
+                     : launch_pairs<1>(P, M.tmOA2, M.tmOB2, M.ea2, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp);
   prof_end(P, PROF_GEMM_F64TC, ev);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();

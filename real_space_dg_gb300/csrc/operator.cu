@@ -653,6 +653,7 @@ cudaError_t launch_apply(Problem& P, const double2* x, double2* y) {
 bool flux_is_inverted(const Problem& P) { return P.kline_exact && P.shift == P.kline_shift; }
 
 cudaError_t launch_apply_pre(Problem& P, const double2* z, const double2* v, long long v_stride, double2* y) {
+  if (P.fp64_tc && P.mx.ozaki) return launch_apply_f64_tc(P, z, y, nullptr, 8, nullptr, true);   // even Nk: no k = 0
   switch (P.s.nK) {
     case 2: return apply_nk<2>(P, z, y, v, v_stride);
     case 3: return apply_nk<3>(P, z, y, v, v_stride);

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(32 * kSliceColsPerBlock) slice_columns_kernel(
 //   A operand: rows plane hm + m, hm = M / 2 (plane 0 = c, plane 1 = d)
 // One CTA computes A, drains TMEM to FP64 registers, computes B into the same accumulators (its first loads are in
 // flight meanwhile), and writes both members of every output pair.  Warps 0 .. 15 drain, 16 loads, 17 issues.
-//   MODE 0: Y = Phi X.   MODE 1: Y += i Phi^H X.
+//   MODE 0: Y = Phi X.   MODE 1: Y += i Phi^H X.   MODE 2: Y = i Phi^H X.
 // The table's digits dominated the L2 traffic of the embedded product (1 MB per 64 nodes, a quarter of it per CTA;
 // now 0.5 MB per 32 nodes for both planes).  Half the columns also leave room for 7 bits a digit: |t| <= 64, and 8
 // products of K <= 256 pairs stay at 8 * 64^2 * 256 = 2^23, exact in FP32.  Eight digits carry 56 bits of a column's
@@ -477,6 +477,9 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pairs_kernel(
         if (MODE == 0) {
           *p = make_double2(ar - bi, ai + br);
           *q = make_double2(ar + bi, ai - br);
+        } else if (MODE == 2) {
+          *p = make_double2(br - ai, ar + bi);
+          *q = make_double2(-(ai + br), ar - bi);
         } else {
           const double2 op = *p, oq = *q;
           *p = make_double2(op.x - (ai - br), op.y + (ar + bi));

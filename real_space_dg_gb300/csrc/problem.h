@@ -325,7 +325,7 @@ cudaError_t launch_apply(Problem& P, const double2* x, double2* y);
 // to accumulate into, and no identity part to cancel in the Gram-Schmidt pass.  True when the current shift is the one
 // the factors were built with.
 bool flux_is_inverted(const Problem& P);
-// y = A z - v for z = M^-1 v where flux_is_inverted (v: per-problem stride v_stride); not for fp64_tc handles.
+// y = A z - v for z = M^-1 v where flux_is_inverted (v: per-problem stride v_stride).
 cudaError_t launch_apply_pre(Problem& P, const double2* z, const double2* v, long long v_stride, double2* y);
 // rscale (device, optional): r enters scaled by rscale[b]; rout (optional): the scaled r is written there
 // (per-problem stride rout_stride), the Arnoldi step's next basis vector.
@@ -338,11 +338,11 @@ double estimate_bytes(const Shape& s, int batch, int restart, int restart_inner,
                       bool basis16 = true);
 cudaError_t launch_flux_f64(Problem& P, const double2* x, double2* y, const int* mask = nullptr);
 cudaError_t launch_stencil_f64(Problem& P, const double2* xh, double2* yh, const int* mask = nullptr);
-// FP64 operator apply with the transforms emulated on the tensor cores (mixed form only).
-// nd: leading digits of the emulated FP64 transforms (8: ~1e-14 of |Phi||x|; fewer for a
-// residual that only has to resolve a loose tolerance, ~2^(-6 nd)).
+// FP64 operator apply with the transforms emulated on the tensor cores (mixed form and fp64_tc handles).
+// nd: leading digits of the emulated FP64 transforms (8: 56 bits of a column's largest entry; fewer for a
+// residual that only has to resolve a loose tolerance, ~2^(-7 nd)).  potential_only: y = G x (launch_apply_pre).
 cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const int* mask = nullptr, int nd = 8,
-                                const int* nd_pp = nullptr);
+                                const int* nd_pp = nullptr, bool potential_only = false);
 int debug_gemm_f64_tc(const double* A, const double* B, double* C, int M, int N, int K, std::string& err, int nd = 8);
 // Rebuild potential-dependent data (Vw weights, contact inflow rhs) of problems [b0, b1).
 // mask (device, optional): problems b with mask[b] == 0 are left untouched.
@@ -359,6 +359,8 @@ double mixed_bytes(const Shape& s, int batch, int restart, bool basis16);
 int mixed_alloc(Problem& P);
 // Digit slices of Phi, state slice buffer and tensor maps of the FP64 emulation (any precision).
 int ozaki_alloc(Problem& P);
+double ozaki_bytes(const Shape& s, long long ncols);
+bool ozaki_pays(const Shape& s);
 void mixed_free(Problem& P);
 cudaError_t mixed_sync_weights(Problem& P);
 // mask (device, optional): problems b with mask[b] == 0 are skipped (their output is left as is).

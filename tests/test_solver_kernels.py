@@ -147,3 +147,33 @@ def test_gram_schmidt_many_problems(built_lib, n_el, nk, order, batch):
         r = rhs - P.apply(rho).reshape(batch, -1)
         assert st == 0
         assert np.all(np.linalg.norm(r, axis=1) <= 1.001e-10 * np.linalg.norm(rhs, axis=1))
+
+
+@pytest.mark.parametrize("n_el,nk,nxi,order,batch,emulated", [
+    (116, 256, 256, 3, 1, True), (153, 256, 260, 2, 2, True), (58, 512, 512, 1, 1, True), (239, 252, 256, 1, 1, True),
+    (114, 256, 256, 3, 1, False), (400, 190, 190, 1, 1, False)])
+def test_large_fp64_transforms(built_lib, n_el, nk, nxi, order, batch, emulated):
+    """FP64 handles on both sides of 3e7 entries and nodes (and an Nk that is no multiple of 4): the operator
+    against the oracle's, 1e-13 of |A x| as two FP64 sums of up to 512 terms may differ, and an Arnoldi solve whose steps
+    use that the flux is inverted, by the oracle's residual."""
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order, n_xi=nxi, bias=0.05)
+    op = krylov.Operator1D(mat, dg1d.init_params(mat, efl, efr, E, m), E)
+    rng = np.random.default_rng(nk)
+    with Problem1D(n_el=n_el, n_local=order + 1, nk=nk, n_xi=nxi, l_xi=spec.l_xi_m, batch=batch) as P:
+        for b in range(batch):
+            P.set_potential(b, mat["x"], E, m, spec.m_rel, spec.temp_k, efl, efr)
+        x = rng.normal(size=(batch, P.N)) + 1j * rng.normal(size=(batch, P.N))
+        P.profile(on=True, reset=True)
+        y = P.apply(x).reshape(batch, -1)
+        prof = P.profile(on=False, reset=True)
+        assert (prof["gemm_f64_tc"][2] > 0) == emulated
+        for b in range(batch):
+            want = op.apply(x[b])
+            assert np.linalg.norm(y[b] - want) <= 1e-13 * np.linalg.norm(want)
+        st, info = P.solve(tol=1e-9, maxit=60)
+        rhs = P.rhs().reshape(batch, -1)
+        assert st == 0
+        for b in range(batch):
+            r = rhs[b] - op.apply(P.rho(b))
+            assert np.linalg.norm(r) <= 1.01e-9 * np.linalg.norm(rhs[b])
