@@ -6,7 +6,7 @@
 //  - an independent true-residual check that downgrades a converged flag (:314-320)
 // Arnoldi uses classical Gram-Schmidt applied twice (CGS2) with block reductions
 // and warp shuffles; Givens rotations and the Hessenberg back substitution run on
-// the device, one thread per problem.  Every problem of a batch has its own basis,
+// the device, one warp per problem.  Every problem of a batch has its own basis,
 // Hessenberg matrix and convergence state; a converged problem freezes.
 //
 // Two drivers share the Arnoldi step, templated on the basis vector type:

@@ -13,7 +13,7 @@
 //                       into its incoming s, then sweeps its chunk writing z.
 // Threads: x = 32 consecutive k (coalesced rows), y = 4 chunks; grid
 // (ceil(nk/32), ceil(n_chunks/4), batch) covers every SM even for one problem.
-// Chunks of up to fused_len elements take one launch instead (kline_fused_kernel): all chunks of a few lines in
+// Chunks of up to FusedLen elements take one launch instead (kline_fused_kernel): all chunks of a few lines in
 // one block, each thread's chunk of r in registers from its only read on, the maps in shared memory.
 // Optional: r enters scaled by rscale[b] (the Arnoldi step's w / |w|), and the apply kernel
 // writes the scaled r to rout (the next basis vector), which replaces a separate scaling pass.

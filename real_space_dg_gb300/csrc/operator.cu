@@ -7,7 +7,8 @@
 //   2. paired_kernel     X^ = Phi X over every DG node of the batch (one product),
 //      stencil_kernel    Y^_{e,a} = sum_b T(beta_{e,ab}) X^_{e,b} (xi-tridiagonal),
 //      paired_kernel     y += i Phi^H Y^ (second product, accumulating epilogue)
-//      (zgemm_kernel where the caller owns Phi: the allocation-free apply)
+//      (zgemm_kernel where the caller owns Phi: the allocation-free apply; digit
+//      products on the tensor cores on large shapes: ozaki_pays, mixed.cu)
 // plus the k-line preconditioner, the Vw(x,k) rebuild and the observables.
 #include <cuda_runtime.h>
 

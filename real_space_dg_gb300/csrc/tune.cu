@@ -1,7 +1,7 @@
 // Autotuner of the launch shapes that have more than one good value (sm_103a).
 //
 // On the first solve of a handle it times, on the handle's own stream and buffers,
-//   - the k-line preconditioner (maps + apply) for every candidate chunk length L
+//   - the k-line preconditioner (one launch or maps + apply) for every candidate chunk length L
 //     (kline::chunk_len_candidates: 2 .. 128 elements, at most 64 chunks), in the
 //     precision the handle iterates in;
 //   - the mixed form's FP32 xi stencil with 2 and 4 xi cells per thread;

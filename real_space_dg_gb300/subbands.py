@@ -9,8 +9,9 @@ entry, then valley 1's vectors sign-aligned with its first slice.  The results a
 the ``Esub`` [nv x Nx x nm] and ``Vsub`` [nv x Nx x nm x Ny] that
 ``solve_transport_DG_2D`` takes.
 
-All slices are solved at once by ``wg_subbands_*`` in libwigner_gb300.so (Sturm
-bisection and twisted-factorisation eigenvectors, one warp per slice).
+All slices are solved at once by ``wg_subbands_*`` in libwigner_gb300.so (eigenvalues
+located in FP32, refined by FP64 Rayleigh quotients on the twisted factorisation, checked
+by Sturm counts).
 """
 import ctypes as C
 
