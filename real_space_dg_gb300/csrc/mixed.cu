@@ -125,7 +125,7 @@ cudaError_t launch_ozaki(const CUtensorMap& a, const CUtensorMap& b, const int* 
 // Row length of the pair digits of K complex entries: K / 2 in whole 16-byte TMA rows, one k block at least.
 int pair_row(int K) { return std::max(oz::BK, (K / 2 + 7) & ~7); }
 
-// Y = Phi X (MODE 0), Y += i Phi^H X (MODE 1) or Y = i Phi^H X (MODE 2) on the tensor cores: slicing and gemm_pairs_kernel.  X: K complex entries
+// Y = Phi X (MODE 0) or Y = i Phi^H X (MODE 1) on the tensor cores: slicing and gemm_pairs_kernel.  X: K complex entries
 // per column, Y: M.
 template <int MODE>
 cudaError_t launch_pairs(Problem& P, const CUtensorMap& a, const CUtensorMap& b, const int* ea, const double2* X,
@@ -139,7 +139,7 @@ cudaError_t launch_pairs(Problem& P, const CUtensorMap& a, const CUtensorMap& b,
   slice<<<(unsigned)((P.ncols + oz::kSlicePairNodes - 1) / oz::kSlicePairNodes), 128 * oz::kSlicePairNodes, 0, P.stream>>>(
       X, K, P.ncols, P.mx.ob, P.mx.eb, mask, npp, Kp, nd, nd_pp);
   const dim3 grid((M / 2 + oz::BM - 1) / oz::BM, (unsigned)((2 * P.ncols + oz::BN - 1) / oz::BN));
-  oz::gemm_pairs_kernel<MODE><<<grid, oz::PAIR_THREADS, oz::SMEM_BYTES, P.stream>>>(
+  oz::gemm_pairs_kernel<MODE><<<grid, oz::THREADS, oz::SMEM_BYTES, P.stream>>>(
       a, b, ea, P.mx.eb, Y, M, 2 * P.ncols, Kp, P.mx.err, mask, 2 * npp, nd, nd_pp);
   return cudaGetLastError();
 }
@@ -712,12 +712,12 @@ double ozaki_bytes(const Shape& s, long long ncols) {
   return 2.0 * oz::S * 4 * (double)ncols * kmax + 16.0 * ncols + 2.0 * oz::S * 2 * kmax * std::max(s.nk, s.nxi);
 }
 
-// FP64 handles whose transforms are faster as products of digits: a CTA of gemm_pairs_kernel takes 40 us whatever
+// FP64 handles whose transforms are faster as products of digits: a CTA of gemm_pairs_kernel takes 36 us whatever
 // the number of nodes up to 32 an SM, the native kernel 2 us per 10^6 table entries and nodes of one problem.
-// 960 nodes of 256 x 256 (6.3e7): 125 -> 54 us, two problems 224 -> 58 us; 240 nodes (1.6e7): 42 us native, 54 us; 960 of
-// 128 x 128 (1.6e7): 41 us both.  A rule on one problem, so that its results do not depend on the batch it is in.  The
+// 960 nodes of 256 x 256 (6.3e7): 125 -> 47 us, two problems 224 -> 51 us; 240 nodes (1.6e7): 42 us native, 41 us; 960 of
+// 128 x 128 (1.6e7): 41 and 35 us.  A rule on one problem, so that its results do not depend on the batch it is in.  The
 // digits keep 56 bits of a column's largest entry: the rounding error of the operator on 116 to 240 elements, Nk = 200 to 512,
-// fell from 1.6e-16 .. 1.0e-15 (native sums) to 1.5e-16 .. 2.4e-16 of |A x|.
+// fell from 1.6e-16 .. 1.0e-15 (native sums) to 1.3e-16 .. 2.3e-16 of |A x|.
 bool ozaki_pays(const Shape& s) {
   return s.nk % 4 == 0 && s.nxi % 4 == 0 && s.nk <= 2 * oz::PAIR_MAX_K && s.nxi <= 2 * oz::PAIR_MAX_K &&
          (double)s.n_el * s.nK * s.nk * s.nxi >= 3e7;
@@ -752,6 +752,10 @@ int ozaki_alloc(Problem& P) {
     std::vector<int> e1, e2;
     slice_rows_host(A1, 2 * hs, K1, d1, e1, oz::PAIR_BITS);
     slice_rows_host(A2, 2 * hk, K2, d2, e2, oz::PAIR_BITS);
+    for (int r = 0; r < 2 * hs; ++r)
+      if (std::all_of(&A1[(size_t)r * K1], &A1[(size_t)r * K1] + K1, [](double a) { return a == 0; })) e1[r] = oz::kZeroExp;
+    for (int r = 0; r < 2 * hk; ++r)
+      if (std::all_of(&A2[(size_t)r * K2], &A2[(size_t)r * K2] + K2, [](double a) { return a == 0; })) e2[r] = oz::kZeroExp;
     cudaError_t ce = cudaSuccess;
     auto C2 = [&](cudaError_t r) { if (ce == cudaSuccess) ce = r; };
     C2(cudaMalloc(&M.oa1, sizeof(bf16) * d1.size()));
@@ -973,8 +977,6 @@ cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const 
   const Shape& s = P.s;
   const double ncols = (double)P.ncols;
   cudaError_t e = cudaSuccess;
-  if (!potential_only) e = launch_flux_f64(P, x, y, mask);
-  if (e != cudaSuccess) return e;
   // work of one transform: read the FP64 operand (slicing), write the FP64 result; flops of
   // ONE BF16 digit-slice product of both planes, weighted by the products the digits need
   const double prod_flops = 2.0 * (2.0 * s.nxi) * (2.0 * s.nk) * ncols / 4;
@@ -985,10 +987,11 @@ cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const 
   if (e != cudaSuccess) return e;
   e = launch_stencil_f64(P, P.xh, P.yh, mask);
   if (e != cudaSuccess) return e;
-  ev = prof_begin(P, PROF_GEMM_F64TC, 2, 16.0 * s.nxi * ncols + 16.0 * P.N * P.batch, prod_flops, mask, nd, nd_pp);
-  e = potential_only ? launch_pairs<2>(P, M.tmOA2, M.tmOB2, M.ea2, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp)
-                     : launch_pairs<1>(P, M.tmOA2, M.tmOB2, M.ea2, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp);
+  ev = prof_begin(P, PROF_GEMM_F64TC, 2, 8.0 * s.nxi * ncols + 16.0 * P.N * P.batch, prod_flops, mask, nd, nd_pp);
+  e = launch_pairs<1>(P, M.tmOA2, M.tmOB2, M.ea2, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp);
   prof_end(P, PROF_GEMM_F64TC, ev);
+  if (e != cudaSuccess) return e;
+  if (!potential_only) e = launch_flux_f64(P, x, y, mask, true);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }

@@ -36,7 +36,14 @@ __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_doub
 // ---------------------------------------------------------------------------
 constexpr int kFluxThreads = 128;
 
-template <int NK>
+template <bool ADD>
+__device__ __forceinline__ void flux_store(double2* y, double s, double2 f, double shift, double2 x) {
+  if constexpr (ADD) *y = make_double2(fma(s, f.x, fma(shift, x.x, y->x)), fma(s, f.y, fma(shift, x.y, y->y)));
+  else *y = make_double2(s * f.x + shift * x.x, s * f.y + shift * x.y);
+}
+
+// ADD: y += A_flux x (after the emulated transforms, whose epilogue then has no FP64 additions).
+template <int NK, bool ADD>
 __global__ void __launch_bounds__(kFluxThreads) flux_kernel(const double2* __restrict__ x, double2* __restrict__ y,
                                                             const double* __restrict__ kvec,
                                                             const double* __restrict__ qd, FluxBlocks fb, int n_el,
@@ -89,7 +96,7 @@ __global__ void __launch_bounds__(kFluxThreads) flux_kernel(const double2* __res
     double2* ye = y + (long long)be * NK * nk + j;
 #pragma unroll
     for (int a = 0; a < NK; ++a)
-      ye[(long long)a * nk] = make_double2(sk * acc[a].x + shift * xv[a].x, sk * acc[a].y + shift * xv[a].y);
+      flux_store<ADD>(ye + (long long)a * nk, sk, acc[a], shift, xv[a]);
     return;
   }
 #pragma unroll
@@ -133,7 +140,7 @@ __global__ void __launch_bounds__(kFluxThreads) flux_kernel(const double2* __res
   double2* ye = y + (long long)be * NK * nk + j;
 #pragma unroll
   for (int a = 0; a < NK; ++a)
-    ye[(long long)a * nk] = make_double2(s * acc[a].x + shift * xv[a].x, s * acc[a].y + shift * xv[a].y);
+    flux_store<ADD>(ye + (long long)a * nk, s, acc[a], shift, xv[a]);
 }
 
 // ---------------------------------------------------------------------------
@@ -459,9 +466,10 @@ __global__ void observables_kernel(const double2* __restrict__ rho, const double
 
 template <int NK>
 void flux_launch(const double2* x, double2* y, const double* kvec, const double* qd, const FluxBlocks& fb, int batch,
-                 int n_el, int nk, double shift, cudaStream_t st, const int* mask = nullptr) {
+                 int n_el, int nk, double shift, cudaStream_t st, const int* mask = nullptr, bool add = false) {
   const dim3 grid((unsigned)(batch * n_el), (unsigned)((nk + kFluxThreads - 1) / kFluxThreads));
-  flux_kernel<NK><<<grid, kFluxThreads, 0, st>>>(x, y, kvec, qd, fb, n_el, nk, shift, mask);
+  auto kernel = add ? flux_kernel<NK, true> : flux_kernel<NK, false>;
+  kernel<<<grid, kFluxThreads, 0, st>>>(x, y, kvec, qd, fb, n_el, nk, shift, mask);
 }
 
 template <int NK>
@@ -662,12 +670,12 @@ cudaError_t launch_apply_pre(Problem& P, const double2* z, const double2* v, lon
   }
 }
 
-cudaError_t launch_flux_f64(Problem& P, const double2* x, double2* y, const int* mask) {
+cudaError_t launch_flux_f64(Problem& P, const double2* x, double2* y, const int* mask, bool add) {
   cudaEvent_t ev = prof_begin(P, PROF_FLUX64, 1, 32.0 * P.N * P.batch, 8.0 * P.s.nK * P.N * P.batch, mask);
   switch (P.s.nK) {
-    case 2: flux_launch<2>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream, mask); break;
-    case 3: flux_launch<3>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream, mask); break;
-    default: flux_launch<4>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream, mask); break;
+    case 2: flux_launch<2>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream, mask, add); break;
+    case 3: flux_launch<3>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream, mask, add); break;
+    default: flux_launch<4>(x, y, P.kvec, P.qd, P.fb, P.batch, P.s.n_el, P.s.nk, P.shift, P.stream, mask, add); break;
   }
   prof_end(P, PROF_FLUX64, ev);
   return cudaGetLastError();

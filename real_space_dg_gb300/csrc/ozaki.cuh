@@ -93,30 +93,38 @@ __device__ __forceinline__ long long group_fixed(float v, int g) {
   return sh >= 0 ? (t << sh) : ((t + (1ll << (-sh - 1))) >> -sh);
 }
 
-// a * 2^e as the nearest double (ties to even), integer instructions only; results
-// below the normal range flush to zero.
-__device__ __forceinline__ double fixed_to_double(long long a, int e) {
-  if (a == 0) return 0.0;
-  const unsigned long long sign = a < 0 ? 1ull << 63 : 0ull;
-  unsigned long long u = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
-  int msb = 63 - __clzll((long long)u);
-  unsigned long long mant;
-  if (msb <= 52) {
-    mant = u << (52 - msb);
-  } else {
-    const int sh = msb - 52;
-    mant = u >> sh;
-    const unsigned long long rem = u & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-    if (rem > half || (rem == half && (mant & 1ull))) ++mant;
-    if (mant >> 53) {
-      mant >>= 1;
-      ++msb;
-    }
+// 32 lanes x 8 consecutive fp32 columns of TMEM at two places.
+__device__ __forceinline__ void tmem_ld8x2(uint32_t t0, uint32_t t1, float (&v)[8], float (&w)[8]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(t0), "r"(t1)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    v[i] = __uint_as_float(r[i]);
+    w[i] = __uint_as_float(r[8 + i]);
   }
-  const int ex = msb + e + 1023;
-  if (ex <= 0) return sign ? -0.0 : 0.0;
-  if (ex >= 0x7FF) return __longlong_as_double((long long)(sign | (0x7FFull << 52)));
-  return __longlong_as_double((long long)(sign | ((unsigned long long)ex << 52) | (mant & 0xFFFFFFFFFFFFFull)));
+}
+
+// a * 2^e as the nearest double (ties to even), integer instructions only, no branch (lanes take every side of one);
+// results below the normal range flush to zero.
+__device__ __forceinline__ double fixed_to_double(long long a, int e) {
+  const unsigned long long sign = (unsigned long long)a & (1ull << 63);
+  unsigned long long u = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
+  const int lz = __clzll((long long)u);
+  u <<= lz & 63;                                                     // the leading one at bit 63
+  const unsigned long long mant = (u >> 11) + (((u & 0x7FF) + ((u >> 11) & 1)) > 0x400 ? 1 : 0);
+  const int ex = 63 - lz + e + 1023;
+  // the leading one of mant adds to the exponent field, and so does the carry of a rounding to 2^53
+  unsigned long long bits = ((unsigned long long)(unsigned)(ex - 1) << 52) + mant;
+  bits = ex >= 0x7FF || bits >= (0x7FFull << 52) ? 0x7FFull << 52 : bits;
+  bits = ex <= 0 || a == 0 ? 0ull : bits;
+  return __longlong_as_double((long long)(sign | bits));
 }
 
 // EPI 0: C = A B.  EPI 1: C += A B.   ea[row], eb[col]: power-of-two exponents of A's rows and B's columns.
@@ -317,27 +325,61 @@ __global__ void __launch_bounds__(32 * kSliceColsPerBlock) slice_columns_kernel(
 //   B operand: real columns 2 c + (0 re, 1 im) of node c, plane 0 = E, plane 1 = O: rows plane 2 ncols + 2 c + o
 //   A operand: rows plane hm + m, hm = M / 2 (plane 0 = c, plane 1 = d)
 // One CTA computes A, drains TMEM to FP64 registers, computes B into the same accumulators (its first loads are in
-// flight meanwhile), and writes both members of every output pair.  Warps 0 .. 15 drain, 16 loads, 17 issues.
-//   MODE 0: Y = Phi X.   MODE 1: Y += i Phi^H X.   MODE 2: Y = i Phi^H X.
+// flight meanwhile), and writes both members of every output pair.  All 16 warps drain, warp 0 loads and warp 1 issues
+// between (two warps more had left 96 registers a thread and spilled the drain).
+//   MODE 0: Y = Phi X.   MODE 1: Y = i Phi^H X.
 // The table's digits dominated the L2 traffic of the embedded product (1 MB per 64 nodes, a quarter of it per CTA;
 // now 0.5 MB per 32 nodes for both planes).  Half the columns also leave room for 7 bits a digit: |t| <= 64, and 8
 // products of K <= 256 pairs stay at 8 * 64^2 * 256 = 2^23, exact in FP32.  Eight digits carry 56 bits of a column's
 // largest entry, more than FP64 keeps of a sum of K such terms; seven (28 products of digits instead of 36) carry 49, one more
-// than eight of 6 bits.  With slicing, per transform: 333 -> 210 us (16 problems of 960 nodes,
-// 256 x 256), 240 -> 133 us (4 of 720 nodes, 512 x 512: 180 CTAs on 152 SMs); with eight digits of 6 bits 219 and 158 us.
-// 36 products of digits take 10 us of a CTA's 40; the rest is the latency of its first loads, of two ring stages and
-// of reading the accumulators twice.
+// than eight of 6 bits.  With slicing, per transform: 333 -> 184 us (16 problems of 960 nodes,
+// 256 x 256), 240 -> 119 us (4 of 720 nodes, 512 x 512: 180 CTAs on 152 SMs); with eight digits of 6 bits, FP64 additions in the
+// epilogue and all of it inlined 219 and 158 us.  A CTA of 256 x 256 takes 36 us: 2 until its first stage, 8 of MMAs a
+// plane, 2 to read plane 0, the rest the conversions and stores of the results.
 // ---------------------------------------------------------------------------------------------
-constexpr int PAIR_THREADS = THREADS + 64;
 constexpr int PAIR_BITS = 7, PAIR_MAX_K = 256;   // bits per digit, pairs per row
-constexpr int kPairFixBits = 56;                 // unit 2^-56; |sum| <= K / 4 = 2^6 of it
+constexpr int kPairFixBits = 55;                 // unit 2^-55; |sum| <= K / 4 = 2^6, |A +- B| <= 2^7 of it
 // Two neighbouring groups are one 32-bit integer (2^23 2^7 + 2^23); pair j (groups 2j, 2j + 1) has weight 2^(-21 - 14 j),
-// the last one is rounded by 7 bits.
+// the last one is rounded by 8 bits.
 __device__ __forceinline__ long long pair_fixed(const int (&c)[4]) {
-  return ((long long)c[0] << 35) + ((long long)c[1] << 21) + ((long long)c[2] << 7) + ((c[3] + 64) >> 7);
+  return ((long long)c[0] << 34) + ((long long)c[1] << 20) + ((long long)c[2] << 6) + ((c[3] + 128) >> 8);
 }
+// The integer value of a group: up to 2^22 (K <= 128) by the rounding of an addition, which is two instructions of
+// the FP32 pipe; the conversion instruction runs at an eighth of their rate.
+template <bool SMALL>
+__device__ __forceinline__ int group_int(float v) {
+  if constexpr (SMALL) return __float_as_int(__fadd_rn(v, 12582912.f)) - 0x4B400000;   // 1.5 2^23
+  else return __float2int_rn(v);
+}
+// a and b of units 2^ea and 2^eb in the larger of the two, which ea becomes
+__device__ __forceinline__ void pair_align(long long& a, int& ea, long long& b, int eb) {
+  const int d = eb - ea, sa = min(max(d, 0), 62), sb = min(max(-d, 0), 62);
+  a = (a + ((1ll << sa) >> 1)) >> sa;
+  b = (b + ((1ll << sb) >> 1)) >> sb;
+  ea = max(ea, eb);
+}
+constexpr int kZeroExp = -4000;   // exponent of a row or column of zeros: it never sets the common unit
+
+// The pair of results of one node from A and B (units 2^(ea + xa), 2^(eb + xb)), as integers of a common unit with one
+// conversion per result: the FP64 additions of the pairs cost 64 cycles of an SM quarter each.  Not inlined: eight copies
+// of it are read from the instruction cache once per CTA (20,000 of its 75,000 cycles, 37,000 when it is cold).
 template <int MODE>
-__global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pairs_kernel(
+__device__ __noinline__ void pair_store(long long ar, long long ai, long long br, long long bi, int ea, int eb, int2 xa,
+                                        int2 xb, double2* p, double2* q) {
+  int e0 = ea + xa.x, e1 = ea + xa.y;
+  pair_align(ar, e0, bi, eb + xb.y);   // the results of Re A and Im B
+  pair_align(ai, e1, br, eb + xb.x);   // and of Im A and Re B
+  if (MODE == 0) {
+    *p = make_double2(fixed_to_double(ar - bi, e0), fixed_to_double(ai + br, e1));
+    *q = make_double2(fixed_to_double(ar + bi, e0), fixed_to_double(ai - br, e1));
+  } else {
+    *p = make_double2(fixed_to_double(br - ai, e1), fixed_to_double(ar + bi, e0));
+    *q = make_double2(fixed_to_double(-(ai + br), e1), fixed_to_double(ar - bi, e0));
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(THREADS, 1) gemm_pairs_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const int* __restrict__ ea,
     const int* __restrict__ eb, double2* __restrict__ Y, int M, long long Ncol2, int K, int* __restrict__ err,
     const int* __restrict__ mask, int cols_per_problem, int nd, const int* __restrict__ nd_pp) {
@@ -386,104 +428,110 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pairs_kernel(
   tc::fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == THREADS / 32) {
-    if (lane == 0)
-      for (int it = 0; it < 2 * nkb; ++it) {
-        const int st = it % ns, ph = it / nkb, kb = it - ph * nkb;
-        if (it >= ns && !tc::mbar_wait(&empty[st], ((it / ns) + 1) & 1, err)) break;
-        uint8_t* sa = smem + st * stage;
-        uint8_t* sb = sa + nd * A_SLICE;
-        tc::mbar_expect_tx(&full[st], (uint32_t)(nd * (A_SLICE + B_SLICE)));
-        for (int p = 0; p < nd; ++p) {
-          tma_load_3d(sa + p * A_SLICE, &tmA, kb * BK, ph * hm + m0, p, &full[st]);
-          tma_load_3d(sb + p * B_SLICE, &tmB, kb * BK, (int)(ph * Ncol2 + n0), p, &full[st]);
-        }
-      }
-  } else if (warp == THREADS / 32 + 1) {
-    if (lane == 0) {
-      bool ok = true;
-      for (int ph = 0; ph < 2 && ok; ++ph) {
-        if (ph == 1) {
-          ok = tc::mbar_wait(drained, 0, err);
-          tc::fence_after();
-        }
-        for (int kb = 0; kb < nkb && ok; ++kb) {
-          const int it = ph * nkb + kb, st = it % ns;
-          if (!(ok = tc::mbar_wait(&full[st], (it / ns) & 1, err))) break;
-          tc::fence_after();
-          const uint8_t* sa = smem + st * stage;
-          const uint8_t* sb = sa + nd * A_SLICE;
-#pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk)
-            for (int p = 0; p < nd; ++p)
-              for (int q0 = 0; q0 + p < nd; q0 += kSlicesPerMma) {   // as in gemm_ozaki_kernel
-                const int n = min(kSlicesPerMma, nd - p - q0);
-                tc::mma_bf16(tmem + (uint32_t)((p + q0) * BN), sdesc_sw64(sa + p * A_SLICE + kk * 32),
-                             sdesc_sw64(sb + q0 * B_SLICE + kk * 32), idesc_n(n * BN),
-                             (kb > 0 || kk > 0 || p > 0) ? 1u : 0u);
-              }
-          tc::mma_commit(&empty[st]);
-        }
-        if (ok) tc::mma_commit(&done[ph]);
+  auto load = [&](int it0, int it1) {
+    for (int it = it0; it < it1; ++it) {
+      const int st = it % ns, ph = it / nkb, kb = it - ph * nkb;
+      if (it >= ns && !tc::mbar_wait(&empty[st], ((it / ns) + 1) & 1, err)) break;
+      uint8_t* sa = smem + st * stage;
+      uint8_t* sb = sa + nd * A_SLICE;
+      tc::mbar_expect_tx(&full[st], (uint32_t)(nd * (A_SLICE + B_SLICE)));
+      for (int p = 0; p < nd; ++p) {
+        tma_load_3d(sa + p * A_SLICE, &tmA, kb * BK, ph * hm + m0, p, &full[st]);
+        tma_load_3d(sb + p * B_SLICE, &tmB, kb * BK, (int)(ph * Ncol2 + n0), p, &full[st]);
       }
     }
-  } else {
-    // warp w reads TMEM lanes 32 (w % 4) .. +31 (rows) and the 16 real columns (8 nodes) of block w / 4
+  };
+  auto multiply = [&](int ph) {
+    for (int kb = 0; kb < nkb; ++kb) {
+      const int it = ph * nkb + kb, st = it % ns;
+      if (!tc::mbar_wait(&full[st], (it / ns) & 1, err)) return;
+      tc::fence_after();
+      const uint8_t* sa = smem + st * stage;
+      const uint8_t* sb = sa + nd * A_SLICE;
+#pragma unroll
+      for (int kk = 0; kk < BK / 16; ++kk)
+        for (int p = 0; p < nd; ++p)
+          for (int q0 = 0; q0 + p < nd; q0 += kSlicesPerMma) {   // as in gemm_ozaki_kernel
+            const int n = min(kSlicesPerMma, nd - p - q0);
+            tc::mma_bf16(tmem + (uint32_t)((p + q0) * BN), sdesc_sw64(sa + p * A_SLICE + kk * 32),
+                         sdesc_sw64(sb + q0 * B_SLICE + kk * 32), idesc_n(n * BN),
+                         (kb > 0 || kk > 0 || p > 0) ? 1u : 0u);
+          }
+      tc::mma_commit(&empty[st]);
+    }
+    tc::mma_commit(&done[ph]);
+  };
+  {
+    // warp w reads TMEM lanes 32 (w % 4) .. +31 (rows) and the 16 real columns (8 nodes) of block w / 4, eight at a time
+    // (16 left no registers for plane 0's results)
     constexpr int EC = EPI_COLS;
     const int wq = warp & 3, cb = warp >> 2;
     const int row = m0 + wq * 32 + lane;
     const long long c0 = n0 + cb * EC;
     const int ncb = (int)max(0ll, min((long long)EC, Ncol2 - c0));
-    double va[EC], vb[EC];
-    bool ok = true;
+    const bool in = row < hm;
+    const uint32_t tbase = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(cb * EC);
+    const bool small = K <= PAIR_MAX_K / 2;
+    auto drain = [&](int half, long long* out) {
+      int c[8][4];
 #pragma unroll
-    for (int ph = 0; ph < 2; ++ph) {
-      if (ok) ok = tc::mbar_wait(&done[ph], 0, err);
-      tc::fence_after();
-      if (ok) {
-        int c[EC][4];
+      for (int j = 0; j < 4; ++j) {
+        float v[8], w[8];
+        const uint32_t t = tbase + (uint32_t)(2 * j * BN + 8 * half);
+        const bool two = 2 * j + 1 < nd;
+        if (2 * j < nd) tmem_ld8x2(t, two ? t + BN : t, v, w);
+        if (small) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t t = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(2 * j * BN + cb * EC);
-          float v[EC], w[EC];
+          for (int i = 0; i < 8; ++i)
+            c[i][j] = 2 * j < nd ? group_int<true>(v[i]) * 128 + (two ? group_int<true>(w[i]) : 0) : 0;
+        } else {
 #pragma unroll
-          for (int i = 0; i < EC; ++i) v[i] = w[i] = 0.f;
-          if (2 * j < nd) tmem_ld16(t, v);
-          if (2 * j + 1 < nd) tmem_ld16(t + BN, w);
-#pragma unroll
-          for (int i = 0; i < EC; ++i) c[i][j] = __float2int_rn(v[i]) * 128 + __float2int_rn(w[i]);
+          for (int i = 0; i < 8; ++i)
+            c[i][j] = 2 * j < nd ? group_int<false>(v[i]) * 128 + (two ? group_int<false>(w[i]) : 0) : 0;
         }
-        const int er = (row < hm ? ea[ph * hm + row] : 0) - kPairFixBits;
-        const int* ebp = eb + ph * Ncol2 + c0;
+      }
 #pragma unroll
-        for (int i = 0; i < EC; ++i)
-          (ph == 0 ? va : vb)[i] = fixed_to_double(pair_fixed(c[i]), er + (i < ncb ? ebp[i] : 0));
-      }
-      if (ph == 0) {
-        tc::fence_before();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(drained);
-      }
+      for (int i = 0; i < 8; ++i) out[i] = pair_fixed(c[i]);
+    };
+    // plane 0, and as many loads of plane 1 as the ring takes before the accumulators are read
+    const int ahead = min(nkb + ns, 2 * nkb);
+    if (warp == 0 && lane == 0) load(0, ahead);
+    if (warp == 1 && lane == 0) multiply(0);
+    __syncwarp();
+    long long va[EC];
+    bool ok = tc::mbar_wait(&done[0], 0, err);
+    tc::fence_after();
+    if (ok) {
+      drain(0, va);
+      drain(1, va + 8);
     }
-    if (ok && !*(volatile int*)err && row < hm) {
+    tc::fence_before();
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(drained);
+    if (warp == 0 && lane == 0) load(ahead, 2 * nkb);
+    if (warp == 1 && lane == 0 && tc::mbar_wait(drained, 0, err)) {
+      tc::fence_after();
+      multiply(1);
+    }
+    __syncwarp();
+    const int ea0 = in ? ea[row] - kPairFixBits : 0, ea1 = in ? ea[hm + row] - kPairFixBits : 0;
+    if (ok) ok = tc::mbar_wait(&done[1], 0, err);
+    tc::fence_after();
+    if (ok && !*(volatile int*)err) {
       double2* y = Y + c0 / 2 * M;
       const int mr = M - 1 - row;
 #pragma unroll
-      for (int i = 0; i < EC / 2; ++i) {
-        if (2 * i >= ncb) continue;
-        const double ar = va[2 * i], ai = va[2 * i + 1], br = vb[2 * i], bi = vb[2 * i + 1];
-        double2* p = y + (long long)i * M + row;
-        double2* q = y + (long long)i * M + mr;
-        if (MODE == 0) {
-          *p = make_double2(ar - bi, ai + br);
-          *q = make_double2(ar + bi, ai - br);
-        } else if (MODE == 2) {
-          *p = make_double2(br - ai, ar + bi);
-          *q = make_double2(-(ai + br), ar - bi);
-        } else {
-          const double2 op = *p, oq = *q;
-          *p = make_double2(op.x - (ai - br), op.y + (ar + bi));
-          *q = make_double2(oq.x - (ai + br), oq.y + (ar - bi));
+      for (int half = 0; half < 2; ++half) {
+        long long vb[8];
+        drain(half, vb);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int col = 8 * half + 2 * i;
+          if (!in || col >= ncb) continue;
+          const int2 xa = make_int2(eb[c0 + col], eb[c0 + col + 1]);
+          const int2 xb = make_int2(eb[Ncol2 + c0 + col], eb[Ncol2 + c0 + col + 1]);
+          double2* yn = y + (long long)(4 * half + i) * M;
+          pair_store<MODE>(va[col], va[col + 1], vb[2 * i], vb[2 * i + 1], ea0, ea1, xa, xb, yn + row, yn + mr);
         }
       }
     }
@@ -543,7 +591,7 @@ __global__ void __launch_bounds__(128 * kSlicePairNodes) slice_pairs_kernel(
   const int m = mx == 0 ? 0 : (int)((mx >> 52) & 0x7FF) - 1023 + 1;   // max|x| < 2^m
   const long long Ncol2 = 2 * ncols, slice_stride = 2 * Ncol2 * (long long)Kout;
   const long long r = (o >> 1) * Ncol2 + 2 * c + (o & 1);
-  if (lane == 0) e_out[r] = m + 1;
+  if (lane == 0) e_out[r] = mx == 0 ? kZeroExp : m + 1;
   __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(slices + r * Kout);
 #pragma unroll
   for (int t = 0; t < PASSES; ++t) {

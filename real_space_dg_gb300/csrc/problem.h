@@ -336,7 +336,7 @@ int set_kline_factors(Problem& P);
 // Device bytes of a handle before allocation (the admission estimate of wg_problem_create).
 double estimate_bytes(const Shape& s, int batch, int restart, int restart_inner, int precision, bool fp64_tc = false,
                       bool basis16 = true);
-cudaError_t launch_flux_f64(Problem& P, const double2* x, double2* y, const int* mask = nullptr);
+cudaError_t launch_flux_f64(Problem& P, const double2* x, double2* y, const int* mask = nullptr, bool add = false);
 cudaError_t launch_stencil_f64(Problem& P, const double2* xh, double2* yh, const int* mask = nullptr);
 // FP64 operator apply with the transforms emulated on the tensor cores (mixed form and fp64_tc handles).
 // nd: leading digits of the emulated FP64 transforms (8: 56 bits of a column's largest entry; fewer for a
