@@ -17,9 +17,10 @@
 //
 // Potential and CAP (applyFVConsistentDrift, get_Drift_full2D.m:331-364), per centre
 // element e and quadrature point q:
-//   f2d_drift_kernel     y[r, id(e,l)] = pot/16 sum_q Cp[q][l] Rq[r] + capc cap[r] U[r, id(e,l)] with
-//                        Rq[r] = sum over the cell's 4 vertices v of dV[e][q][v] x (sum over the <= 4 cells
-//                        around v of sum_l W[q][l] U[., id(e,l)])   (P^T diag(dV) P)
+//   f2d_interp_kernel    Uq[e][q][r] = sum_l W[q][l] U[r, id(e,l)]
+//   f2d_vertex_kernel    Rq[e][q][cell] = sum over the cell's 4 vertices v of dV[e][q][v] x
+//                        (sum of Uq over the <= 4 cells around v)   (P^T diag(dV) P)
+//   f2d_project_kernel   y[r, id(e,l)] = pot/16 sum_q Cp[q][l] Rq[e][q][r] + capc cap[r] U[r, id(e,l)]
 //   f2d_dv_kernel        dV from V on the material grid (bilinear, X clamped, Y clamped or wrapped).
 // All arithmetic FP64 (the plain form).
 #include <cuda_fp16.h>
@@ -32,22 +33,8 @@
 #include <string>
 #include <vector>
 
-#include "krylov.cuh"
 #include "ozaki_api.h"
 #include "wigner_gb300.h"
-
-constexpr int kMaxTerms = 6;
-// The relative factors c_t R_t of an axis with the k-th nonzeros of all rows together: entry (first[t] + k) rows + row
-// has its column in `col` and its value in re, im; rows with fewer entries repeat their last column with value
-// zero.  Bit t of `real`: no imaginary part, im is not read (the |A| factors; the FP32 copy drops what is
-// below 2^-40 of the row's largest entry, the rounding noise of |A|: half its entries and every imaginary part).
-template <typename R>
-struct EllTerms {
-  int* col = nullptr;
-  R *re = nullptr, *im = nullptr;
-  int first[kMaxTerms] = {}, len[kMaxTerms] = {};
-  unsigned real = 0;
-};
 
 struct wg2d_problem {
   wg2d_shape s{};
@@ -58,10 +45,13 @@ struct wg2d_problem {
   double2* y = nullptr;
   struct Axis {
     int T = 0;
+    std::vector<double> coef;
     double* blocks = nullptr;   // [T][n_el][3][nk][nk]
-    std::vector<int> rp, col;   // R_t as given: [T][n_rho + 1], columns over all terms
-    std::vector<double> val;    // c_t R_t, (re, im) over all terms
-    EllTerms<double> ell;
+    int* rp = nullptr;          // [T][n_rho + 1]
+    int* col = nullptr;         // concatenated over the terms
+    double2* val = nullptr;
+    int* offs = nullptr;        // [T] start of term t in col / val
+    double* dcoef = nullptr;    // [T]
     unsigned dense_mask = 0;    // terms applied by the emulated FP64 GEMM (rho_x axis)
     unsigned char* ymask = nullptr;   // rho_x axis: [T][nY] 1 where term t acts (closed X-face pieces); null: all
     std::vector<wg::OzakiRowsDev> dense;   // [T] digit slices of c_t R_t (real embedding) for those terms
@@ -75,6 +65,7 @@ struct wg2d_problem {
          *cap = nullptr, *dV = nullptr;
   double2 pot = {0, 0};
   double capc = 0;
+  double2 *Uq = nullptr, *Rq = nullptr;
   bool drift_ready = false, potential_ready = false;
   cudaEvent_t ev[4] = {};
   // line-transverse preconditioner (modes of -i D_rho_x, X lines, dense transverse inverses)
@@ -82,22 +73,22 @@ struct wg2d_problem {
   double sigma = 1.0;
   int nT = 0;
   wg::OzakiRowsDev UH, Us;        // real embeddings of U^H and U / sigma (tensor-core path)
-  double2 *UHd = nullptr, *Usd = nullptr;   // the same as complex [nrx][nrx] row-major transposed (FP64 path)
+  double2 *UHd = nullptr, *Usd = nullptr;   // the same as complex [nrx][nrx] row-major (FP64 path)
   double2 *xinv = nullptr, *xcpl = nullptr; // [nrx][n_el_x][nk][nk]
-  double2* xmaps = nullptr;                  // chunk maps of the X-line sweep [mode][chunk][nk][nk]
-  int x_chunk_len = 0, x_chunks = 1, x_lines = 32;
+  double2* xmaps = nullptr;                  // chunk maps of the X-line sweep [chunk][nk*nk+nk][line]
+  int x_chunk_len = 0, x_chunks = 1;
   int* fwd = nullptr;             // [nrx]
-  double2* tinv = nullptr;        // [nrx][nT][nT], each transposed
+  double2* tinv = nullptr;        // [nrx][nT][nT]
   double2 *pa = nullptr, *pb = nullptr;     // [n] scratch of the preconditioner
   bool pre32 = false;             // the preconditioner in FP32 (its factors and scratch below)
   float2 *UH32 = nullptr, *Us32 = nullptr, *xinv32 = nullptr, *xcpl32 = nullptr, *tinv32 = nullptr;
   float2 *pa32 = nullptr, *pb32 = nullptr;
   // FP32 copies of the operator for the mixed solve's inner iterations
   bool d32_ready = false;
-  float* blocks32[2] = {nullptr, nullptr};
-  EllTerms<float> ell32[2];
+  float *blocks32[2] = {nullptr, nullptr}, *coef32[2] = {nullptr, nullptr};
+  float2* val32[2] = {nullptr, nullptr};
   float *interp32 = nullptr, *proj32 = nullptr, *cap32 = nullptr, *dV32 = nullptr;
-  float2* G32 = nullptr;
+  float2 *Uq32 = nullptr, *Rq32 = nullptr, *G32 = nullptr;
   int vm32 = 0;
   float2 *V32 = nullptr, *Z32 = nullptr, *w32 = nullptr;
   __half2* Vh32 = nullptr;    // the inner basis stored in FP16 (V32 unused then)
@@ -108,10 +99,7 @@ struct wg2d_problem {
   double2* Zb = nullptr;          // [m][n] preconditioned basis (flexible GMRES)
   double2 *V = nullptr, *r = nullptr, *w = nullptr, *z = nullptr, *b = nullptr, *xs = nullptr;
   double2 *H = nullptr, *g = nullptr, *sn = nullptr, *hc = nullptr, *hp = nullptr, *yc = nullptr;
-  double2* cs = nullptr;
-  double *ktarget = nullptr;    // [1] zero
-  int* kctl = nullptr;          // [4] see F2dKrylov
-  double *partial = nullptr, *nrm = nullptr;
+  double *cs = nullptr, *partial = nullptr, *nrm = nullptr;
   double2 *bc_rt = nullptr, *bc_p = nullptr, *bc_ph = nullptr, *bc_sh = nullptr;   // BiCGSTAB vectors
   bool b_ready = false, xs_ready = false;   // resident right-hand side / solution of the last solve
   std::vector<double> resvec;               // residual norms of the last solve (initial, then per iteration)
@@ -137,6 +125,7 @@ struct wg2d_problem {
 namespace {
 
 constexpr int kMaxNK = 4;
+constexpr int kMaxTerms = 6;
 constexpr int kRelxCols = 8;
 
 __device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {   // c + a b
@@ -204,76 +193,25 @@ __global__ void __launch_bounds__(256) f2d_center_kernel(const T* __restrict__ F
   }
 }
 
-// Sums of complex products a b over a step index.  In FP32 two packed sums, (b.x, b.y) a.x and (b.x, b.y) a.y: one
-// packed multiply-add each, and only the factor shared by several sums (a) is spread over a pair.
-template <typename T> struct CSum;
-template <> struct CSum<double2> {
-  double2 v = make_double2(0.0, 0.0);
-  using Pair = double2;
-  __device__ __forceinline__ static Pair spread(double2 a) { return a; }
-  __device__ __forceinline__ void add(const Pair& a, const double2& b) { v = cfma(a, b, v); }
-  __device__ __forceinline__ void add_real(double a, const double2& b) {
-    v.x = fma(a, b.x, v.x);
-    v.y = fma(a, b.y, v.y);
-  }
-  __device__ __forceinline__ double2 get() const { return v; }
-};
-template <> struct CSum<float2> {
-  float2 p = make_float2(0.f, 0.f), q = make_float2(0.f, 0.f);
-  struct Pair {
-    float2 re, im;
-  };
-  __device__ __forceinline__ static Pair spread(float2 a) { return {make_float2(a.x, a.x), make_float2(a.y, a.y)}; }
-  __device__ __forceinline__ void add(const Pair& a, const float2& b) {
-    p = __ffma2_rn(a.re, b, p);
-    q = __ffma2_rn(a.im, b, q);
-  }
-  __device__ __forceinline__ void add_real(float a, const float2& b) { p = __ffma2_rn(make_float2(a, a), b, p); }
-  __device__ __forceinline__ float2 get() const { return make_float2(p.x - q.y, p.y + q.x); }
-};
-// N consecutive values from shared memory in 16-byte loads
-template <int N>
-__device__ __forceinline__ void lds_row(double2 (&o)[N], const double2* p) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) o[i] = p[i];
-}
-template <int N>
-__device__ __forceinline__ void lds_row(float2 (&o)[N], const float2* p) {
-#pragma unroll
-  for (int i = 0; i < N; i += 2) {
-    const float4 t = *reinterpret_cast<const float4*>(p + i);
-    o[i] = make_float2(t.x, t.y);
-    o[i + 1] = make_float2(t.z, t.w);
-  }
-}
-// One value to shared memory without a register in between (zero when !on); async_wait before the barrier.
-template <typename T>
-__device__ __forceinline__ void async_put(T* dst, const T* src, bool on) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = on ? (int)sizeof(T) : 0;
-  if constexpr (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-template <typename T> constexpr int kColPitch = sizeof(T) == 8 ? kRelxCols + 2 : kRelxCols + 1;   // 16-byte rows
-
-// y[rx, col] += sum_t sum_k val_t[k] G_t[col_t[k], col] for kRelxCols columns per block; the G_t columns are staged in
-// shared memory, thread rx owns row rx (blockDim = nrx rounded up to a warp multiple, at most 512).  The k-th entries
-// of a warp's rows are read together and their columns are neighbours, so the staged rows come as broadcasts.
-// Bound by the reads and writes of G_t and y.  121 rows (2 and 61 entries, the latter real), 12,960 columns, FP32:
-// 100 us (all 121 + 121 complex entries, read row by row) -> 42 us.
+// y[rx, col] += sum_t c_t sum_k val_t[k] G_t[col_t[k], col] for kRelxCols columns per block;
+// the G_t columns are staged in shared memory, thread rx owns row rx (blockDim = nrx rounded
+// up to a warp multiple, at most 512).
 template <typename T, typename R>
-__global__ void __launch_bounds__(512) f2d_relx_kernel(const T* __restrict__ G, T* __restrict__ y, EllTerms<R> E,
-                                                       int nterm, int nrx, long long ncols, long long n,
-                                                       unsigned skip_mask,
+__global__ void __launch_bounds__(512) f2d_relx_kernel(const T* __restrict__ G, T* __restrict__ y,
+                                                       const int* __restrict__ rp, const int* __restrict__ col,
+                                                       const T* __restrict__ val, const int* __restrict__ nnz_off,
+                                                       const R* __restrict__ coef, int nterm, int nrx,
+                                                       long long ncols, long long n, unsigned skip_mask,
                                                        const unsigned char* __restrict__ ymask = nullptr,
                                                        long long cols_per_y = 1, int nY = 1) {
   extern __shared__ __align__(16) unsigned char sgr_raw[];
-  T* sg = reinterpret_cast<T*>(sgr_raw);   // [nrx][kColPitch]
+  T* sg = reinterpret_cast<T*>(sgr_raw);   // [kRelxCols][nrx]
   const long long c0 = (long long)blockIdx.x * kRelxCols;
   const int nc = (int)min((long long)kRelxCols, ncols - c0);
-  const int rx = min((int)threadIdx.x, nrx - 1);
-  CSum<T> acc[kRelxCols];
+  const int rx = threadIdx.x;
+  T acc[kRelxCols];
+#pragma unroll
+  for (int j = 0; j < kRelxCols; ++j) acc[j] = czero<T>();
   for (int t = 0; t < nterm; ++t) {
     if ((skip_mask >> t) & 1u) continue;          // applied on the tensor cores
     __syncthreads();
@@ -281,202 +219,177 @@ __global__ void __launch_bounds__(512) f2d_relx_kernel(const T* __restrict__ G, 
       const int j = i / nrx, k = i - j * nrx;
       // a masked term (a closed X-face piece) acts only on its own Y dofs
       const bool on = j < nc && (!ymask || ymask[(long long)t * nY + (c0 + j) / cols_per_y]);
-      async_put(sg + k * kColPitch<T> + j, G + (long long)t * n + (on ? (c0 + j) * nrx + k : 0), on);
+      sg[i] = on ? G[(long long)t * n + (c0 + j) * nrx + k] : czero<T>();
     }
-    async_wait();
     __syncthreads();
-    const int* col = E.col + (long long)E.first[t] * nrx + rx;
-    const R *re = E.re + (long long)E.first[t] * nrx + rx, *im = E.im + (long long)E.first[t] * nrx + rx;
-    if ((E.real >> t) & 1u) {
-#pragma unroll 4
-      for (int k = 0; k < E.len[t]; ++k) {
-        T v[kRelxCols];
-        lds_row(v, sg + col[k * nrx] * kColPitch<T>);
-        const R a = re[k * nrx];
+    if (rx < nrx) {
+      const R ct = coef[t];
+      const int* rpt = rp + t * (nrx + 1);
+      const int off = nnz_off[t];
+      for (int k = rpt[rx]; k < rpt[rx + 1]; ++k) {
+        const int cidx = col[off + k];
+        T v = val[off + k];
+        v.x *= ct;
+        v.y *= ct;
 #pragma unroll
-        for (int j = 0; j < kRelxCols; ++j) acc[j].add_real(a, v[j]);
-      }
-    } else {
-#pragma unroll 4
-      for (int k = 0; k < E.len[t]; ++k) {
-        T v[kRelxCols], a;
-        lds_row(v, sg + col[k * nrx] * kColPitch<T>);
-        a.x = re[k * nrx];
-        a.y = im[k * nrx];
-        const typename CSum<T>::Pair p = CSum<T>::spread(a);
-#pragma unroll
-        for (int j = 0; j < kRelxCols; ++j) acc[j].add(p, v[j]);
+        for (int j = 0; j < kRelxCols; ++j) acc[j] = cfma(v, sg[j * nrx + cidx], acc[j]);
       }
     }
   }
-  if (threadIdx.x >= nrx) return;
+  if (rx >= nrx) return;
 #pragma unroll
   for (int j = 0; j < kRelxCols; ++j) {
     if (j < nc) {
       T* o = y + (c0 + j) * nrx + rx;
-      const T a = acc[j].get();
-      o->x += a.x;
-      o->y += a.y;
+      o->x += acc[j].x;
+      o->y += acc[j].y;
     }
   }
 }
 
-// y[rx, ry, c] += sum_t sum_k val_t[k] G_t[rx, col_t[k], c]: one thread per entry, grid (centre dofs, ceil(nrel / 256)).
-// STAGED: the terms' entries of all rows in shared memory, so that the loads of G_t wait for no other load.
-// Bound by the reads and writes of G_t and y.  12 rows (2 and 6 entries), 1.57 M unknowns, FP32:
-// 43 us (12 complex entries) -> 36 us, 23 us with the staged table.
-template <bool STAGED, typename T, typename R>
-__global__ void __launch_bounds__(256) f2d_rely_kernel(const T* __restrict__ G, T* __restrict__ y, EllTerms<R> E,
-                                                       int nterm, int nrx, int nry, long long n, int entries) {
-  extern __shared__ __align__(16) unsigned char rely_raw[];
-  R* sre = reinterpret_cast<R*>(rely_raw);   // [entries]
-  R* sim = sre + entries;
-  int* scol = reinterpret_cast<int*>(sim + entries);
-  if constexpr (STAGED) {
-    for (int i = threadIdx.x; i < entries; i += 256) {
-      sre[i] = E.re[i];
-      sim[i] = E.im[i];
-      scol[i] = E.col[i] * nrx;
-    }
-    __syncthreads();
-  }
-  const int i = blockIdx.y * 256 + threadIdx.x;
-  if (i >= nrx * nry) return;
-  const int ry = i / nrx, rx = i - ry * nrx;
-  const long long cbase = (long long)blockIdx.x * nrx * nry;
-  T* o = y + cbase + i;
-  const T old = *o;
-  CSum<T> acc;
+// y[rx, ry, c] += sum_t c_t sum_k val_t[k] G_t[rx, col_t[k], c]   (one thread per entry)
+template <typename T, typename R>
+__global__ void __launch_bounds__(256) f2d_rely_kernel(const T* __restrict__ G, T* __restrict__ y,
+                                                       const int* __restrict__ rp, const int* __restrict__ col,
+                                                       const T* __restrict__ val, const int* __restrict__ nnz_off,
+                                                       const R* __restrict__ coef, int nterm, int nrx, int nry,
+                                                       long long n) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const int rx = (int)(i % nrx);
+  const long long q = i / nrx;
+  const int ry = (int)(q % nry);
+  const long long c = q / nry;
+  const long long cbase = c * (long long)nrx * nry + rx;
+  T acc = czero<T>();
   for (int t = 0; t < nterm; ++t) {
-    const T* g = G + (long long)t * n + cbase + rx;
-    const int f = E.first[t] * nry + ry, len = E.len[t];
-    if ((E.real >> t) & 1u) {
-#pragma unroll 6
-      for (int k = 0; k < len; ++k)
-        acc.add_real(STAGED ? sre[f + k * nry] : E.re[f + k * nry],
-                     g[STAGED ? scol[f + k * nry] : E.col[f + k * nry] * nrx]);
-    } else {
-#pragma unroll 6
-      for (int k = 0; k < len; ++k) {
-        T a;
-        a.x = STAGED ? sre[f + k * nry] : E.re[f + k * nry];
-        a.y = STAGED ? sim[f + k * nry] : E.im[f + k * nry];
-        acc.add(CSum<T>::spread(a), g[STAGED ? scol[f + k * nry] : E.col[f + k * nry] * nrx]);
-      }
-    }
+    const int* rpt = rp + t * (nry + 1);
+    const int off = nnz_off[t];
+    T s = czero<T>();
+    for (int k = rpt[ry]; k < rpt[ry + 1]; ++k)
+      s = cfma(val[off + k], G[(long long)t * n + cbase + (long long)col[off + k] * nrx], s);
+    acc.x = fma(coef[t], s.x, acc.x);
+    acc.y = fma(coef[t], s.y, acc.y);
   }
-  const T a = acc.get();
-  *o = {old.x + a.x, old.y + a.y};
+  y[i].x += acc.x;
+  y[i].y += acc.y;
 }
 
-// Potential and CAP of one centre element: y[r, id(e,l)] = pot/16 sum_q Cp[q][l] sum_{vertices v of r} dV[e][q][v]
-// sum_{cells r' of v} sum_l' W[q][l'] F[r', id(e,l')] + capc cap[r] F[r, id(e,l)].  The quadrature sum is taken per
-// vertex, P_l(v) = sum_q Cp[q][l] dV_q(v) sum_l' W[q][l'] SF_l'(v) with SF the sums of F over the cells of v, so no
-// field at the quadrature points goes through memory.  A warp takes 32 vertices along rho_x (31 cells, P of the
-// next vertex by shuffle) and marches over `rows` rows of cells; the row below stays in registers.
-// Bound by the FMA chains per vertex (38 per point and vertex in FP32 at 9 local nodes; reads F and dV, writes y once).
-// 120 elements of 9 nodes, 25 points, 121 x 12 cells: 76 us in three launches -> 31 us in FP32, 641 -> 566 us in FP64
-// (64 cycles per warp instruction of a quarter: 480 us of sums with the repeated vertex rows).
+// centre dof of local node l of element e (local order X fastest, elements X fastest)
+__device__ __forceinline__ long long center_id(int e, int l, int nex, int nkx, int nky, int nX) {
+  const int ex = e % nex, ey = e / nex;
+  const int lx = l % nkx, ly = l / nkx;
+  return (long long)(ex * nkx + lx) + (long long)nX * (ey * nky + ly);
+}
+
+// Uq[e][q][r] = sum_l W[q][l] F[r, id(e, l)]; grid (ceil(nrel/128), n_el)
 template <int NL, typename T, typename R>
-__global__ void __launch_bounds__(128) f2d_drift_kernel(const T* __restrict__ F, T* __restrict__ y,
-                                                        const R* __restrict__ W, const R* __restrict__ Cp,
-                                                        const R* __restrict__ dV, const R* __restrict__ cap, T pot16,
-                                                        R capc, int q0, int nqc, int nq, int nrx, int nry, int nvert,
-                                                        int nex, int nkx, int nX, int periodic, int xt, int bands,
-                                                        int rows, long long items) {
-  constexpr int NLP = (NL + 3) / 4 * 4;
-  extern __shared__ __align__(16) unsigned char drift_raw[];
-  R* sW = reinterpret_cast<R*>(drift_raw);   // [nqc][NLP]
-  R* sC = sW + nqc * NLP;
-  __shared__ long long off[NL];              // local node -> centre dof, times the cells
-  const long long nrel = (long long)nrx * nry;
-  for (int i = threadIdx.x; i < nqc * NLP; i += 128) {
-    const int q = i / NLP, l = i - q * NLP;
-    sW[i] = l < NL ? W[(q0 + q) * NL + l] : R(0);
-    sC[i] = l < NL ? Cp[(q0 + q) * NL + l] : R(0);
+__global__ void __launch_bounds__(128) f2d_interp_kernel(const T* __restrict__ F, T* __restrict__ Uq,
+                                                         const R* __restrict__ W, int nq, int nrel, int nex,
+                                                         int nkx, int nky, int nX) {
+  const int r = blockIdx.x * 128 + threadIdx.x;
+  const int e = blockIdx.y;
+  if (r >= nrel) return;
+  T u[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) u[l] = F[center_id(e, l, nex, nkx, nky, nX) * nrel + r];
+  T* out = Uq + (long long)e * nq * nrel + r;
+  for (int q = 0; q < nq; ++q) {
+    T s = czero<T>();
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      const R w = W[q * NL + l];
+      s.x = fma(w, u[l].x, s.x);
+      s.y = fma(w, u[l].y, s.y);
+    }
+    out[(long long)q * nrel] = s;
   }
-  if (threadIdx.x < NL) off[threadIdx.x] = ((threadIdx.x % nkx) + (long long)nX * (threadIdx.x / nkx)) * nrel;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (item >= items) return;   // whole warps
-  const int xi = (int)(item % xt), band = (int)(item / xt % bands), e = (int)(item / xt / bands);
-  const int vi = xi * 31 + lane;                       // vertex; also the cell to its right
-  const bool left = vi >= 1 && vi - 1 < nrx, right = vi < nrx, on = vi <= nrx;
-  const int nky = NL / nkx;
-  const long long base = ((long long)(e % nex) * nkx + (long long)nX * (e / nex) * nky) * nrel;
-  const T* Fe = F + base + vi;
-  const R* De = dV + ((long long)e * nq + q0) * nvert + (on ? vi : 0);
-  const int j0 = band * rows, j1 = min(nry, j0 + rows);
-  T below[NL];
-  for (int vj = j0; vj <= j1; ++vj) {
-    int ja = vj - 1, jb = vj;                          // the rows of cells at this vertex row
-    if (periodic) {
-      ja = ja < 0 ? ja + nry : ja;
-      jb = jb >= nry ? jb - nry : jb;
+}
+
+// sum of Uq over the cells around relative vertex (vi, vj) (cells vi-1..vi, vj-1..vj)
+template <typename T>
+__device__ __forceinline__ T vertex_sum(const T* __restrict__ U, int vi, int vj, int nrx, int nry,
+                                              bool periodic) {
+  T s = czero<T>();
+#pragma unroll
+  for (int dj = -1; dj <= 0; ++dj) {
+    int j = vj + dj;
+    if (periodic) j = (j + nry) % nry;
+    else if (j < 0 || j >= nry) continue;
+#pragma unroll
+    for (int di = -1; di <= 0; ++di) {
+      const int i = vi + di;
+      if (i < 0 || i >= nrx) continue;
+      const T v = U[j * nrx + i];
+      s.x += v.x;
+      s.y += v.y;
     }
-    const bool ra = ja >= 0, rb = jb < nry;
-    T SF[NL], P[NL];
+  }
+  return s;
+}
+
+// Rq[e][q][cell] = sum_{vertices v of cell} dV[e][q][v] vertex_sum(v); grid (ceil(nrel/128), nq, n_el)
+template <typename T, typename R>
+__global__ void __launch_bounds__(128) f2d_vertex_kernel(const T* __restrict__ Uq, T* __restrict__ Rq,
+                                                         const R* __restrict__ dV, int nrx, int nry, int nq,
+                                                         int nvert, int periodic) {
+  const int cell = blockIdx.x * 128 + threadIdx.x;
+  const int nrel = nrx * nry;
+  if (cell >= nrel) return;
+  const int q = blockIdx.y, e = blockIdx.z;
+  const long long slab = ((long long)e * nq + q);
+  const T* U = Uq + slab * nrel;
+  const R* D = dV + slab * nvert;
+  const int i = cell % nrx, j = cell / nrx;
+  const int nvx = nrx + 1;
+  T acc = czero<T>();
+#pragma unroll
+  for (int b = 0; b <= 1; ++b) {
+    int vj = j + b;
+    if (periodic) vj %= nry;
+#pragma unroll
+    for (int a = 0; a <= 1; ++a) {
+      const int vi = i + a;
+      const R d = D[vj * nvx + vi];
+      const T s = vertex_sum<T>(U, vi, vj, nrx, nry, periodic);
+      acc.x = fma(d, s.x, acc.x);
+      acc.y = fma(d, s.y, acc.y);
+    }
+  }
+  Rq[slab * nrel + cell] = acc;
+}
+
+// y[r, id(e,l)] = pot/16 sum_q Cp[q][l] Rq[e][q][r] + capc cap[r] F[r, id(e,l)]; grid (ceil(nrel/128), n_el)
+template <int NL, typename T, typename R>
+__global__ void __launch_bounds__(128) f2d_project_kernel(const T* __restrict__ Rq, const T* __restrict__ F,
+                                                          T* __restrict__ y, const R* __restrict__ Cp,
+                                                          const R* __restrict__ cap, T pot16, R capc,
+                                                          int nq, int nrel, int nex, int nkx, int nky, int nX) {
+  const int r = blockIdx.x * 128 + threadIdx.x;
+  const int e = blockIdx.y;
+  if (r >= nrel) return;
+  T s[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) s[l] = czero<T>();
+  const T* Rr = Rq + (long long)e * nq * nrel + r;
+  for (int q = 0; q < nq; ++q) {
+    const T v = Rr[(long long)q * nrel];
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
-      const T* f = Fe + off[l];
-      T t0 = czero<T>(), t1 = t0, t2 = t0, t3 = t0;
-      if (ra && left) t0 = f[(long long)ja * nrx - 1];
-      if (ra && right) t1 = f[(long long)ja * nrx];
-      if (rb && left) t2 = f[(long long)jb * nrx - 1];
-      if (rb && right) t3 = f[(long long)jb * nrx];
-      SF[l].x = (t0.x + t1.x) + (t2.x + t3.x);
-      SF[l].y = (t0.y + t1.y) + (t2.y + t3.y);
-      P[l] = czero<T>();
+      const R c = Cp[q * NL + l];
+      s[l].x = fma(c, v.x, s[l].x);
+      s[l].y = fma(c, v.y, s[l].y);
     }
-    const R* Dv = De + (long long)(periodic ? vj % nry : vj) * (nrx + 1);
-#pragma unroll 5
-    for (int q = 0; q < nqc; ++q) {
-      const R d = Dv[(long long)q * nvert];
-      T u = czero<T>();
+  }
+  const R cr = capc * cap[r];
 #pragma unroll
-      for (int l = 0; l < NL; ++l) {
-        const R w = sW[q * NLP + l];
-        u.x = fma(w, SF[l].x, u.x);
-        u.y = fma(w, SF[l].y, u.y);
-      }
-      u.x *= d;
-      u.y *= d;
-#pragma unroll
-      for (int l = 0; l < NL; ++l) {
-        const R c = sC[q * NLP + l];
-        P[l].x = fma(c, u.x, P[l].x);
-        P[l].y = fma(c, u.y, P[l].y);
-      }
-    }
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      P[l].x += __shfl_down_sync(0xffffffffu, P[l].x, 1);
-      P[l].y += __shfl_down_sync(0xffffffffu, P[l].y, 1);
-    }
-    if (vj > j0 && right && lane < 31) {
-      const long long cell = (long long)(vj - 1) * nrx;
-      const R cr = capc * cap[cell + vi];
-#pragma unroll
-      for (int l = 0; l < NL; ++l) {
-        T* yo = y + base + off[l] + cell + vi;
-        T f = czero<T>();
-        if (q0 == 0) {
-          f = Fe[off[l] + cell];
-          f.x *= cr;
-          f.y *= cr;
-        } else {
-          f = *yo;
-        }
-        const T s = {below[l].x + P[l].x, below[l].y + P[l].y};
-        T o;
-        o.x = pot16.x * s.x - pot16.y * s.y + f.x;
-        o.y = pot16.x * s.y + pot16.y * s.x + f.y;
-        *yo = o;
-      }
-    }
-#pragma unroll
-    for (int l = 0; l < NL; ++l) below[l] = P[l];
+  for (int l = 0; l < NL; ++l) {
+    const long long idx = center_id(e, l, nex, nkx, nky, nX) * nrel + r;
+    const T f = F[idx];
+    T o;
+    o.x = pot16.x * s[l].x - pot16.y * s[l].y + cr * f.x;
+    o.y = pot16.x * s[l].y + pot16.y * s[l].x + cr * f.y;
+    y[idx] = o;
   }
 }
 
@@ -524,275 +437,255 @@ __global__ void __launch_bounds__(128) f2d_dv_kernel(double* __restrict__ dV, co
                                             v_bilinear(gx, gy, V, nx, ny, X - hx, Y - hy, periodic);
 }
 
-// out = A in over rho_x (dense complex nrx x nrx, given transposed: At[k][row]) for kRelxCols columns (rho_y, X, Y) a
-// block.  The states keep rho_x fastest; the modal fields of the preconditioner keep the column fastest (each mode's
-// lines together), so TO writes out[row][col] and !TO reads in[k][col].  Thread `row` reads At coalesced; the columns'
-// values are broadcast from shared memory.  Bound by the FP32 pipe (21 us of
-// sums) and the latency of At from the L1 and L2.  121 x 121 on 12,960 columns: 58 -> 42 us; two rows a thread: 67 us
-// (half the warps).
-inline __host__ __device__ int modal_rows(int nrx) { return (nrx + 3) / 4 * 4; }
-template <typename T, bool TO>
-__global__ void __launch_bounds__(512) f2d_modal_kernel(const T* __restrict__ At, const T* __restrict__ in,
-                                                        T* __restrict__ out, int nrx, long long ncols) {
+// out[rx, col] = scale sum_j A[rx][j] G[j, col]  (dense complex A [nrx][nrx] row-major; FP64 modal transforms)
+template <typename T>
+__global__ void __launch_bounds__(512) f2d_dense_rx_kernel(const T* __restrict__ A, const T* __restrict__ G,
+                                                           T* __restrict__ out, int nrx, long long ncols) {
   extern __shared__ __align__(16) unsigned char sg_raw[];
-  T* sg = reinterpret_cast<T*>(sg_raw);   // [modal_rows][kColPitch]
+  T* sg = reinterpret_cast<T*>(sg_raw);   // [kRelxCols][nrx]
   const long long c0 = (long long)blockIdx.x * kRelxCols;
   const int nc = (int)min((long long)kRelxCols, ncols - c0);
-  const int kpad = modal_rows(nrx);
   for (int i = threadIdx.x; i < kRelxCols * nrx; i += blockDim.x) {
-    const int j = TO ? i / nrx : i % kRelxCols, k = TO ? i - j * nrx : i / kRelxCols;
-    const bool on = j < nc;
-    async_put(sg + k * kColPitch<T> + j, TO ? in + (on ? (c0 + j) * nrx + k : 0) : in + (on ? k * ncols + c0 + j : 0), on);
+    const int j = i / nrx, k = i - j * nrx;
+    sg[i] = j < nc ? G[(c0 + j) * nrx + k] : czero<T>();
   }
-  for (int i = nrx * kColPitch<T> + threadIdx.x; i < kpad * kColPitch<T>; i += blockDim.x) sg[i] = czero<T>();
-  const int row = min((int)threadIdx.x, nrx - 1);
-  // four rows of At ahead of the sums (zero rows past nrx)
-  const T* Ak = At + row;
-  T a[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) a[i] = Ak[(long long)i * nrx];
-  async_wait();
   __syncthreads();
-  CSum<T> acc[kRelxCols];
-  for (int k = 0; k < kpad; k += 4) {
-    T n[4];
-    Ak += 4ll * nrx;
+  const int rx = threadIdx.x;
+  if (rx >= nrx) return;
+  T acc[kRelxCols];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) n[i] = Ak[(long long)i * nrx];
+  for (int j = 0; j < kRelxCols; ++j) acc[j] = czero<T>();
+  const T* Ar = A + (long long)rx * nrx;
+  for (int k = 0; k < nrx; ++k) {
+    const T a = Ar[k];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const typename CSum<T>::Pair p = CSum<T>::spread(a[i]);
-      T v[kRelxCols];
-      lds_row(v, sg + (k + i) * kColPitch<T>);
-#pragma unroll
-      for (int j = 0; j < kRelxCols; ++j) acc[j].add(p, v[j]);
-      a[i] = n[i];
-    }
+    for (int j = 0; j < kRelxCols; ++j) acc[j] = cfma(a, sg[j * nrx + k], acc[j]);
   }
-  if (threadIdx.x >= nrx) return;
-  if constexpr (TO) {
-    T* o = out + (long long)row * ncols + c0;
-    if (sizeof(T) == 8 && nc == kRelxCols && ncols % 2 == 0) {
 #pragma unroll
-      for (int j = 0; j < kRelxCols; j += 2) {
-        const T u = acc[j].get(), w = acc[j + 1].get();
-        *reinterpret_cast<float4*>(o + j) = make_float4((float)u.x, (float)u.y, (float)w.x, (float)w.y);
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < kRelxCols; ++j)
-        if (j < nc) o[j] = acc[j].get();
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < kRelxCols; ++j)
-      if (j < nc) out[(c0 + j) * nrx + row] = acc[j].get();
-  }
+  for (int j = 0; j < kRelxCols; ++j)
+    if (j < nc) out[(c0 + j) * nrx + rx] = acc[j];
 }
 
 // X lines per mode (xFactors / applyInverse of get_LineTransversePreconditioner_full2D.m:177-222):
 // for mode k, transverse (ry, Y): sweep the X elements upwind (forward[k]: e = 0 .. ne-1), each
-// element's nk values: prev = inv[k][e] (w_e - cpl[k][e] prev).  The recurrence is affine in the incoming state, so
-// the elements are cut into chunks of L (sweep order), a chunk being prev_out = M prev_in + b with M a matter of the
-// mode alone (f2d_xline_maps_kernel, once per preconditioner).
-// f2d_xline_kernel: a block holds all chunks of LB lines; a thread (line, chunk) forms b, folds the maps of
-// the chunks upwind and sweeps its elements.  BYMODE: the fields are [mode][col] and the lines of a mode neighbours, so
-// the coefficients are one load a warp; otherwise rho_x (the mode) is fastest.
-// 60 elements of 3 on 8,712 lines, FP32: 79 us in two launches (maps per line, coefficients per thread) -> 20 us.
+// element's nk values: prev = inv[k][e] (w_e - cpl[k][e] prev).  Thread per (k, ry, Y), k fastest.
 template <int NK, typename T>
-__global__ void __launch_bounds__(128) f2d_xline_maps_kernel(T* __restrict__ maps, const T* __restrict__ inv,
-                                                             const T* __restrict__ cpl, const int* __restrict__ fwd,
-                                                             int nrx, int ne, int L, int nchunk) {
-  const int t = blockIdx.x * 128 + threadIdx.x;   // (mode, chunk, column of M)
-  if (t >= nrx * nchunk * NK) return;
-  const int j = t % NK, c = t / NK % nchunk, k = t / NK / nchunk;
-  T m[NK];
-#pragma unroll
-  for (int a = 0; a < NK; ++a) m[a] = a == j ? cone<T>() : czero<T>();
-  for (int i = c * L; i < min(ne, (c + 1) * L); ++i) {
-    const int e = fwd[k] ? i : ne - 1 - i;
-    const T* Ci = cpl + ((long long)k * ne + e) * NK * NK;
-    const T* Ii = inv + ((long long)k * ne + e) * NK * NK;
-    T v[NK];
-#pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T s = czero<T>();
-#pragma unroll
-      for (int b = 0; b < NK; ++b) s = cfma(Ci[a * NK + b], m[b], s);
-      v[a] = s;
-    }
-#pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T s = czero<T>();
-#pragma unroll
-      for (int b = 0; b < NK; ++b) s = cfma(Ii[a * NK + b], v[b], s);
-      m[a] = cneg(s);
-    }
-  }
-#pragma unroll
-  for (int a = 0; a < NK; ++a) maps[(((long long)k * nchunk + c) * NK + a) * NK + j] = m[a];
-}
-
-// one element: prev <- inv (w - cpl prev)
-template <int NK, typename T>
-__device__ __forceinline__ void f2d_xline_step(T (&prev)[NK], const T (&w)[NK], const T* __restrict__ Ci,
-                                               const T* __restrict__ Ii) {
-  T v[NK];
-#pragma unroll
-  for (int a = 0; a < NK; ++a) {
-    v[a] = w[a];
-#pragma unroll
-    for (int b = 0; b < NK; ++b) v[a] = cfma(cneg(Ci[a * NK + b]), prev[b], v[a]);
-  }
-#pragma unroll
-  for (int a = 0; a < NK; ++a) {
-    T s = czero<T>();
-#pragma unroll
-    for (int b = 0; b < NK; ++b) s = cfma(Ii[a * NK + b], v[b], s);
-    prev[a] = s;
-  }
-}
-
-constexpr int kXlineThreads = 512;
-template <int NK, typename T, bool BYMODE>
-__global__ void __launch_bounds__(kXlineThreads) f2d_xline_kernel(const T* __restrict__ W, T* __restrict__ out,
-                                                                  const T* __restrict__ maps,
-                                                                  const T* __restrict__ inv, const T* __restrict__ cpl,
-                                                                  const int* __restrict__ fwd, int nrx, int nry,
-                                                                  int nX, int nY, int ne, int L, int nchunk, int LB) {
-  extern __shared__ __align__(16) unsigned char xl_raw[];
-  T* bs = reinterpret_cast<T*>(xl_raw);   // [nchunk][NK][LB]
-  const int jl = threadIdx.x % LB, c = threadIdx.x / LB;
-  const long long line = (long long)blockIdx.x * LB + jl, lines = (long long)nrx * nry * nY;
-  const bool on = line < lines;
-  int k = 0;
-  long long base = 0, step = 0;
-  if (on) {
-    if (BYMODE) {
-      const int ry = (int)(line % nry);
-      const long long q = line / nry;
-      k = (int)(q / nY);
-      base = (long long)k * nry * nX * nY + ry + (long long)nry * nX * (q % nY);
-      step = nry;
-    } else {
-      k = (int)(line % nrx);
-      const long long q = line / nrx, nrel = (long long)nrx * nry;
-      base = k + nrx * (q % nry) + nrel * (long long)nX * (q / nry);
-      step = nrel;
-    }
-  }
+__global__ void __launch_bounds__(128) f2d_xline_kernel(const T* __restrict__ W, T* __restrict__ out,
+                                                        const T* __restrict__ inv, const T* __restrict__ cpl,
+                                                        const int* __restrict__ fwd, int nrx, int nry, int nX, int nY,
+                                                        int ne) {
+  const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
+  const long long lines = (long long)nrx * nry * nY;
+  if (t >= lines) return;
+  const int k = (int)(t % nrx);
+  const long long q = t / nrx;
+  const int ry = (int)(q % nry);
+  const int Y = (int)(q / nry);
+  const long long nrel = (long long)nrx * nry;
+  const long long base = k + (long long)nrx * ry + nrel * (long long)nX * Y;
   const bool f = fwd[k] != 0;
-  const int i0 = c * L, i1 = on ? min(ne, i0 + L) : i0;
   T prev[NK];
 #pragma unroll
   for (int a = 0; a < NK; ++a) prev[a] = czero<T>();
-  if (nchunk > 1) {
-    if (c < nchunk - 1) {
-#pragma unroll 2
-      for (int i = i0; i < i1; ++i) {
-        const int e = f ? i : ne - 1 - i;
-        T w[NK];
-#pragma unroll
-        for (int a = 0; a < NK; ++a) w[a] = W[base + step * (e * NK + a)];
-        f2d_xline_step<NK, T>(prev, w, cpl + ((long long)k * ne + e) * NK * NK, inv + ((long long)k * ne + e) * NK * NK);
-      }
-#pragma unroll
-      for (int a = 0; a < NK; ++a) bs[(c * NK + a) * LB + jl] = prev[a];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < NK; ++a) prev[a] = czero<T>();
-    for (int cc = 0; cc < c; ++cc) {
-      const T* M = maps + ((long long)k * nchunk + cc) * NK * NK;
-      T nxt[NK];
-#pragma unroll
-      for (int a = 0; a < NK; ++a) {
-        T s = bs[(cc * NK + a) * LB + jl];
-#pragma unroll
-        for (int j = 0; j < NK; ++j) s = cfma(M[a * NK + j], prev[j], s);
-        nxt[a] = s;
-      }
-#pragma unroll
-      for (int a = 0; a < NK; ++a) prev[a] = nxt[a];
-    }
-  }
-#pragma unroll 2
-  for (int i = i0; i < i1; ++i) {
+  for (int i = 0; i < ne; ++i) {
     const int e = f ? i : ne - 1 - i;
-    T w[NK];
+    const T* Ci = cpl + ((long long)k * ne + e) * NK * NK;
+    const T* Ii = inv + ((long long)k * ne + e) * NK * NK;
+    T blk[NK];
 #pragma unroll
-    for (int a = 0; a < NK; ++a) w[a] = W[base + step * (e * NK + a)];
-    f2d_xline_step<NK, T>(prev, w, cpl + ((long long)k * ne + e) * NK * NK, inv + ((long long)k * ne + e) * NK * NK);
+    for (int a = 0; a < NK; ++a) {
+      T v = W[base + nrel * (e * NK + a)];
 #pragma unroll
-    for (int a = 0; a < NK; ++a) out[base + step * (e * NK + a)] = prev[a];
+      for (int b = 0; b < NK; ++b) {
+        const T c = Ci[a * NK + b];
+        v.x -= c.x * prev[b].x - c.y * prev[b].y;
+        v.y -= c.x * prev[b].y + c.y * prev[b].x;
+      }
+      blk[a] = v;
+    }
+#pragma unroll
+    for (int a = 0; a < NK; ++a) {
+      T v = czero<T>();
+#pragma unroll
+      for (int b = 0; b < NK; ++b) v = cfma(Ii[a * NK + b], blk[b], v);
+      prev[a] = v;
+      out[base + nrel * (e * NK + a)] = v;
+    }
   }
 }
 
+// The same sweep cut into chunks of L elements (sweep order).  The element recurrence is affine in
+// the incoming state, prev_e = -Inv_e Cpl_e prev_{e-1} + Inv_e w_e, so a chunk composes to
+// prev_out = M prev_in + b:
+//   f2d_xline_maps_kernel   (line, chunk): M and b of the chunk from M = I, b = 0;
+//   f2d_xline_apply_kernel  (line, chunk): the incoming state folded from the maps of the chunks
+//                           upwind, then the chunk's elements swept as above, writing out.
+// Threads (line, chunk) with the line fastest; maps stored [chunk][entry][line].
+template <int NK, typename T>
+__global__ void __launch_bounds__(128) f2d_xline_maps_kernel(const T* __restrict__ W, T* __restrict__ maps,
+                                                             const T* __restrict__ inv, const T* __restrict__ cpl,
+                                                             const int* __restrict__ fwd, int nrx, int nry, int nX,
+                                                             int nY, int ne, int L, int nchunk) {
+  const long long lines = (long long)nrx * nry * nY;
+  const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
+  if (t >= lines * nchunk) return;
+  const long long line = t % lines;
+  const int c = (int)(t / lines);
+  const int k = (int)(line % nrx);
+  const long long q = line / nrx;
+  const int ry = (int)(q % nry);
+  const int Y = (int)(q / nry);
+  const long long nrel = (long long)nrx * nry;
+  const long long base = k + (long long)nrx * ry + nrel * (long long)nX * Y;
+  const bool f = fwd[k] != 0;
+  T M[NK][NK], b[NK];
+#pragma unroll
+  for (int a = 0; a < NK; ++a) {
+    b[a] = czero<T>();
+#pragma unroll
+    for (int j = 0; j < NK; ++j) M[a][j] = a == j ? cone<T>() : czero<T>();
+  }
+  const int i1 = min(ne, (c + 1) * L);
+  for (int i = c * L; i < i1; ++i) {
+    const int e = f ? i : ne - 1 - i;
+    const T* Ci = cpl + ((long long)k * ne + e) * NK * NK;
+    const T* Ii = inv + ((long long)k * ne + e) * NK * NK;
+    T CM[NK][NK], r[NK];
+#pragma unroll
+    for (int a = 0; a < NK; ++a) {
+      T v = W[base + nrel * (e * NK + a)];
+#pragma unroll
+      for (int j = 0; j < NK; ++j) {
+        T s = czero<T>();
+#pragma unroll
+        for (int m = 0; m < NK; ++m) s = cfma(Ci[a * NK + m], M[m][j], s);
+        CM[a][j] = s;
+      }
+#pragma unroll
+      for (int m = 0; m < NK; ++m) {
+        const T cc = Ci[a * NK + m];
+        v.x -= cc.x * b[m].x - cc.y * b[m].y;
+        v.y -= cc.x * b[m].y + cc.y * b[m].x;
+      }
+      r[a] = v;
+    }
+#pragma unroll
+    for (int a = 0; a < NK; ++a) {
+      T bb = czero<T>();
+#pragma unroll
+      for (int m = 0; m < NK; ++m) bb = cfma(Ii[a * NK + m], r[m], bb);
+      b[a] = bb;
+#pragma unroll
+      for (int j = 0; j < NK; ++j) {
+        T s = czero<T>();
+#pragma unroll
+        for (int m = 0; m < NK; ++m) s = cfma(Ii[a * NK + m], CM[m][j], s);
+        M[a][j] = cneg(s);
+      }
+    }
+  }
+  T* o = maps + (long long)c * (NK * NK + NK) * lines + line;
+#pragma unroll
+  for (int a = 0; a < NK; ++a) {
+#pragma unroll
+    for (int j = 0; j < NK; ++j) o[(long long)(a * NK + j) * lines] = M[a][j];
+    o[(long long)(NK * NK + a) * lines] = b[a];
+  }
+}
+
+template <int NK, typename T>
+__global__ void __launch_bounds__(128) f2d_xline_apply_kernel(const T* __restrict__ W, T* __restrict__ out,
+                                                              const T* __restrict__ maps, const T* __restrict__ inv,
+                                                              const T* __restrict__ cpl, const int* __restrict__ fwd,
+                                                              int nrx, int nry, int nX, int nY, int ne, int L,
+                                                              int nchunk) {
+  const long long lines = (long long)nrx * nry * nY;
+  const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
+  if (t >= lines * nchunk) return;
+  const long long line = t % lines;
+  const int c = (int)(t / lines);
+  const int k = (int)(line % nrx);
+  const long long q = line / nrx;
+  const int ry = (int)(q % nry);
+  const int Y = (int)(q / nry);
+  const long long nrel = (long long)nrx * nry;
+  const long long base = k + (long long)nrx * ry + nrel * (long long)nX * Y;
+  const bool f = fwd[k] != 0;
+  T prev[NK];
+#pragma unroll
+  for (int a = 0; a < NK; ++a) prev[a] = czero<T>();
+  for (int cc = 0; cc < c; ++cc) {
+    const T* o = maps + (long long)cc * (NK * NK + NK) * lines + line;
+    T nxt[NK];
+#pragma unroll
+    for (int a = 0; a < NK; ++a) {
+      T s = o[(long long)(NK * NK + a) * lines];
+#pragma unroll
+      for (int j = 0; j < NK; ++j) s = cfma(o[(long long)(a * NK + j) * lines], prev[j], s);
+      nxt[a] = s;
+    }
+#pragma unroll
+    for (int a = 0; a < NK; ++a) prev[a] = nxt[a];
+  }
+  const int i1 = min(ne, (c + 1) * L);
+  for (int i = c * L; i < i1; ++i) {
+    const int e = f ? i : ne - 1 - i;
+    const T* Ci = cpl + ((long long)k * ne + e) * NK * NK;
+    const T* Ii = inv + ((long long)k * ne + e) * NK * NK;
+    T blk[NK];
+#pragma unroll
+    for (int a = 0; a < NK; ++a) {
+      T v = W[base + nrel * (e * NK + a)];
+#pragma unroll
+      for (int m = 0; m < NK; ++m) {
+        const T cc2 = Ci[a * NK + m];
+        v.x -= cc2.x * prev[m].x - cc2.y * prev[m].y;
+        v.y -= cc2.x * prev[m].y + cc2.y * prev[m].x;
+      }
+      blk[a] = v;
+    }
+#pragma unroll
+    for (int a = 0; a < NK; ++a) {
+      T v = czero<T>();
+#pragma unroll
+      for (int m = 0; m < NK; ++m) v = cfma(Ii[a * NK + m], blk[m], v);
+      prev[a] = v;
+      out[base + nrel * (e * NK + a)] = v;
+    }
+  }
+}
+
+constexpr int kTxTile = 32;
 // transverse solve per mode k and X dof: v[k, t, X] <- Binv[k] v[k, :, X] over t = ry + nry Y.
-// Block (tile of kTxTile X dofs, k; at most 152 rows t fit the shared memory); Binv[k] (given transposed: Bt[k][s][t]) and the tile staged in shared memory.  A
-// warp takes kTxRows rows t of the tile: per s one value of the tile and the rows' coefficients as broadcasts.
-// 72 x 72 for 121 modes on 180 dofs, FP32: 69 us (8 bytes of each 968 of the field, two shared loads per sum) -> 37 us;
-// 64 X dofs a block: 70 us (half the warps).
-constexpr int kTxTile = 32, kTxRows = 8, kTxPitch = kTxTile + 1;
-inline int tx_pitch(int nT) { return std::max(kTxRows, nT + (nT & 1)); }
-inline size_t tx_smem(int nT, size_t elem) { return elem * ((size_t)nT * tx_pitch(nT) + (size_t)nT * kTxPitch); }
-template <typename T, bool BYMODE>
-__global__ void __launch_bounds__(640) f2d_transverse_kernel(const T* __restrict__ Vin, T* __restrict__ Vout,
-                                                              const T* __restrict__ Bt, int nrx, int nry,
-                                                              int nX, int nY, int nT, int pitch) {
+// Block (k, tile of kTxTile X dofs); Binv[k] and the tile staged in shared memory.
+template <typename T>
+__global__ void __launch_bounds__(256) f2d_transverse_kernel(const T* __restrict__ Vin, T* __restrict__ Vout,
+                                                             const T* __restrict__ Binv, int nrx, int nry,
+                                                             int nX, int nY, int nT) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  T* Bs = reinterpret_cast<T*>(sm_raw);   // [nT][pitch] then [nT][kTxPitch]
-  T* Ts = Bs + (long long)nT * pitch;
+  T* Bs = reinterpret_cast<T*>(sm_raw);   // [nT][nT] then [nT][kTxTile]
+  T* Ts = Bs + (long long)nT * nT;
   const int k = blockIdx.y;
   const int X0 = blockIdx.x * kTxTile;
   const int nx = min(kTxTile, nX - X0);
-  const T* Bk = Bt + (long long)k * nT * nT;
-  for (int i = threadIdx.x; i < nT * pitch; i += blockDim.x) {
-    const int s = i / pitch, t = i - s * pitch;
-    async_put(Bs + i, Bk + (t < nT ? s * nT + t : 0), t < nT);
-  }
-  // field index of (t, xx) of the tile; i runs over the tile with the field's fastest index first
-  auto at = [&](int i, int& t, int& xx) -> long long {
-    if (BYMODE) {
-      const int ry = i % nry, q = i / nry, Y = q / nx;
-      xx = q - Y * nx;
-      t = ry + nry * Y;
-      return (long long)k * nry * nX * nY + ry + (long long)nry * (X0 + xx + (long long)nX * Y);
-    }
-    t = i / nx;
-    xx = i - t * nx;
-    const long long nrel = (long long)nrx * nry;
-    return k + (long long)nrx * (t % nry) + nrel * ((long long)(X0 + xx) + (long long)nX * (t / nry));
-  };
-  for (int i = threadIdx.x; i < nT * nx; i += blockDim.x) {
-    int t, xx;
-    const long long o = at(i, t, xx);
-    async_put(Ts + t * kTxPitch + xx, Vin + o, true);
-  }
-  async_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31, t0 = min((int)(threadIdx.x >> 5) * kTxRows, pitch - kTxRows);
-  CSum<T> acc[kTxRows];
-  if (lane < nx) {
-#pragma unroll 4
-    for (int s = 0; s < nT; ++s) {
-      const typename CSum<T>::Pair v = CSum<T>::spread(Ts[s * kTxPitch + lane]);
-      T b[kTxRows];
-      lds_row(b, Bs + (long long)s * pitch + t0);
-#pragma unroll
-      for (int r = 0; r < kTxRows; ++r) acc[r].add(v, b[r]);
-    }
+  const long long nrel = (long long)nrx * nry;
+  const T* Bk = Binv + (long long)k * nT * nT;
+  for (int i = threadIdx.x; i < nT * nT; i += blockDim.x) Bs[i] = Bk[i];
+  for (int i = threadIdx.x; i < nT * kTxTile; i += blockDim.x) {
+    const int s = i / kTxTile, xx = i - s * kTxTile;
+    const int ry = s % nry, Y = s / nry;
+    Ts[i] = xx < nx ? Vin[k + (long long)nrx * ry + nrel * ((long long)(X0 + xx) + (long long)nX * Y)]
+                    : czero<T>();
   }
   __syncthreads();
-  if (lane < nx)
-#pragma unroll
-    for (int r = 0; r < kTxRows; ++r)
-      if (t0 + r < nT) Ts[(t0 + r) * kTxPitch + lane] = acc[r].get();   // rows of two warps: the same values
-  __syncthreads();
-  for (int i = threadIdx.x; i < nT * nx; i += blockDim.x) {
-    int t, xx;
-    const long long o = at(i, t, xx);
-    Vout[o] = Ts[t * kTxPitch + xx];
+  for (int i = threadIdx.x; i < nT * kTxTile; i += blockDim.x) {
+    const int tt = i / kTxTile, xx = i - tt * kTxTile;
+    if (xx >= nx) continue;
+    T acc = czero<T>();
+    const T* Br = Bs + (long long)tt * nT;
+    for (int s2 = 0; s2 < nT; ++s2) acc = cfma(Br[s2], Ts[s2 * kTxTile + xx], acc);
+    const int ry = tt % nry, Y = tt / nry;
+    Vout[k + (long long)nrx * ry + nrel * ((long long)(X0 + xx) + (long long)nX * Y)] = acc;
   }
 }
 
@@ -908,229 +801,60 @@ __global__ void __launch_bounds__(256) f2d_d2f(const double* __restrict__ x, flo
   if (t < n) y[t] = (float)x[t];
 }
 
-// ---------------- Gram-Schmidt of the FP32 inner solve (basis VB: FP32 or FP16 storage)
-// Four consecutive complex values; VEC: n is a multiple of 4 (every row of the basis 16-byte aligned).
-template <bool VEC, typename VB>
-__device__ __forceinline__ void f2d_quad(wg::Quad<VB>& q, const VB* __restrict__ p, long long n4, long long n) {
-  if constexpr (VEC) {
-    q.load(p, n4);
-  } else {
-    q.zero();
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-      if (4 * n4 + r < n) q.set(r, p[4 * n4 + r]);
-  }
-}
+__device__ __forceinline__ float2 f2d_ld(const float2& v) { return v; }
+__device__ __forceinline__ float2 f2d_ld(const __half2& v) { return __half22float2(v); }
 
-// (s, e) += (b, be) with the rounding error of s + b kept in e
-__device__ __forceinline__ void f2d_two_sum(float& s, float& e, float b, float be) {
-  const float t = __fadd_rn(s, b), z = __fsub_rn(t, s);
-  e += be + __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(b, z));
-  s = t;
-}
-
-// Sums over a warp of 8 values per lane, lane l returns the sum of value l >> 2: each step exchanges half of the
-// values still held.  The rounding errors of the FP32 sums are carried along, so the result is a sum of the
-// lanes' values in more than FP32 without the FP64 pipe (64 cycles per warp instruction of a quarter).
-__device__ __forceinline__ double f2d_warp_sum8(float (&s)[8]) {
-  const int lane = threadIdx.x & 31;
-  float e[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) e[i] = 0.f;
-#pragma unroll
-  for (int h = 4; h >= 1; h /= 2) {
-    const bool up = lane & (4 * h);
-#pragma unroll
-    for (int i = 0; i < h; ++i) {
-      const float gs = up ? s[i] : s[i + h], ge = up ? e[i] : e[i + h];
-      s[i] = up ? s[i + h] : s[i];
-      e[i] = up ? e[i + h] : e[i];
-      const float os = __shfl_xor_sync(0xffffffffu, gs, 4 * h);
-      const float oe = h == 4 ? 0.f : __shfl_xor_sync(0xffffffffu, ge, 4 * h);
-      f2d_two_sum(s[i], e[i], os, oe);
-    }
+// FP32 inner products, summed per thread in FP32 and across threads and blocks in FP64; the basis
+// vectors V in FP32 or FP16 storage
+template <typename VB>
+__global__ void __launch_bounds__(256) f2d_dot_partial32(const VB* __restrict__ V, long long vstride,
+                                                         const float2* __restrict__ w, double* __restrict__ partial,
+                                                         long long n) {
+  __shared__ double sre[256], sim[256];
+  const int i = blockIdx.y;
+  const VB* v = V + (long long)i * vstride;
+  float re = 0.f, im = 0.f;
+  for (long long t = (long long)blockIdx.x * 256 + threadIdx.x; t < n; t += (long long)gridDim.x * 256) {
+    const float2 a = f2d_ld(v[t]), b = w[t];
+    re = fmaf(a.x, b.x, fmaf(a.y, b.y, re));
+    im = fmaf(a.x, b.y, fmaf(-a.y, b.x, im));
   }
-#pragma unroll
-  for (int o = 2; o >= 1; o /= 2) {
-    const float os = __shfl_xor_sync(0xffffffffu, s[0], o), oe = __shfl_xor_sync(0xffffffffu, e[0], o);
-    f2d_two_sum(s[0], e[0], os, oe);
-  }
-  return (double)s[0] + (double)e[0];
-}
-
-// partial[(i * blocks + blk) * 2 + {0,1}] = sum over the block's piece of conj(V_i) w for all i < nv: FP32 over the
-// four values of a thread's load, error-carrying across the warp, FP64 across warps, pieces and blocks.  run
-// (nullable): nothing to do when *run is 0.
-// All blocks resident at once, each on one contiguous piece; w stays in registers, half of the four vectors of a
-// step are loaded while the other half is summed.  Bound by HBM (the basis once; one launch row per
-// vector had read w nv times with 8-byte loads, 1.5 TB/s).  1,568,160 unknowns, 1 .. 40 FP32
-// vectors, mean of a cycle: 177 -> 49 us (5.2 TB/s).
-constexpr int kF2dUpThreads = 128;
-template <bool VEC, typename VB>
-__global__ void __launch_bounds__(256, 3) f2d_multidot32(const VB* __restrict__ V, const float2* __restrict__ w,
-                                                         double* __restrict__ partial, long long n, int nv, int quads,
-                                                         const int* __restrict__ run) {
-  extern __shared__ double f2d_red[];   // [nv rounded up to 4][2][8 warps]
-  if (run && !*run) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long lo = (long long)blockIdx.x * quads, hi = min((n + 3) / 4, lo + quads);
-  for (long long base = lo; base < hi; base += 256) {
-    const long long n0 = base + threadIdx.x;
-    const bool in = n0 < hi;
-    wg::Quad<float2> wq;
-    wq.zero();
-    if (in) f2d_quad<VEC>(wq, w, n0, n);
-    wg::Quad<VB> a[4];
-    auto load2 = [&](int i, int u0) {
-#pragma unroll
-      for (int u = u0; u < u0 + 2; ++u) {
-        a[u].zero();
-        if (i + u < nv && in) f2d_quad<VEC>(a[u], V + (long long)(i + u) * n, n0, n);
-      }
-    };
-    load2(0, 0);
-    for (int i = 0; i < nv; i += 4) {
-      float s[8];
-      load2(i, 2);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float re = 0.f, im = 0.f;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float2 v = a[u].get(q), x = wq.get(q);
-          re = fmaf(v.x, x.x, fmaf(v.y, x.y, re));
-          im = fmaf(v.x, x.y, fmaf(-v.y, x.x, im));
-        }
-        s[2 * u] = re;
-        s[2 * u + 1] = im;
-        if (u == 1) load2(i + 4, 0);
-      }
-      const double r = f2d_warp_sum8(s);
-      if ((lane & 3) == 0) {   // always the same thread's slot
-        double* d = f2d_red + (2 * i + (lane >> 2)) * 8 + warp;
-        *d = base == lo ? r : *d + r;
-      }
-    }
-  }
+  sre[threadIdx.x] = re;
+  sim[threadIdx.x] = im;
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * nv; i += 256) {
-    double r = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) r += f2d_red[8 * i + q];
-    partial[((long long)(i / 2) * gridDim.x + blockIdx.x) * 2 + (i & 1)] = r;
+  for (int o = 128; o > 0; o >>= 1) {
+    if (threadIdx.x < o) {
+      sre[threadIdx.x] += sre[threadIdx.x + o];
+      sim[threadIdx.x] += sim[threadIdx.x + o];
+    }
+    __syncthreads();
   }
-}
-
-// Device state of the inner solve's small work.
-struct F2dKrylov {
-  double2 *H, *hc, *cs, *sn, *g;
-  double* nrm;
-  double* target;   // 0: the Givens step never stops by itself, the host looks at g
-  int* ctl;         // active, kused, second pass, tickets of the update
-  int j, ldh;
-};
-
-// w -= sum_i h_i V_i in FP32, |w| and, when no second pass follows, the Givens step in the last block.  PASS 1 tests
-// |w'|^2 < (|w'|^2 + |h|^2) / 2 (Daniel-Gragg-Kaufman-Stewart) and leaves ctl[2]; PASS 2 runs when that is set.
-// 128 threads of four values, the loads of the next vectors ahead of the present ones; all blocks resident at once.
-// Bound by HBM.  1,568,160 unknowns, 1 .. 40 FP32 vectors, mean of a cycle: 53 us with the norm and the Givens step
-// (48 us, and 38 us in four launches for those, before).
-template <int PASS, bool VEC, typename VB>
-__global__ void __launch_bounds__(kF2dUpThreads, 8) f2d_gs_update32(const VB* __restrict__ V, float2* __restrict__ w,
-                                                                    const double2* __restrict__ h, int nv, long long n,
-                                                                    int quads, double* __restrict__ norms,
-                                                                    F2dKrylov k) {
-  if (PASS == 2 && !k.ctl[2]) return;
-  __shared__ float2 hs[wg::kMaxRestart + 8];
-  __shared__ double ws[kF2dUpThreads / 32];
-  __shared__ int last;
-  // the coefficients in FP32 once per block (per element the conversion kept the FP64 pipe 98% busy)
-  for (int i = threadIdx.x; i < ((nv + 7) & ~7); i += kF2dUpThreads)
-    hs[i] = i < nv ? make_float2((float)h[i].x, (float)h[i].y) : make_float2(0.f, 0.f);
-  __syncthreads();
-  constexpr int U = sizeof(VB) == 4 ? 8 : 4;
-  const long long lo = (long long)blockIdx.x * quads, hi = min((n + 3) / 4, lo + quads);
-  double nrm2 = 0.0;
-  for (long long n4 = lo + threadIdx.x; n4 < hi; n4 += kF2dUpThreads) {
-    wg::Quad<float2> wq;
-    if constexpr (VEC) {   // plain loads: w is written below
-      wq.u = reinterpret_cast<float4*>(w)[2 * n4];
-      wq.v = reinterpret_cast<float4*>(w)[2 * n4 + 1];
-    } else {
-      f2d_quad<false>(wq, (const float2*)w, n4, n);
-    }
-    float2 acc[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) acc[r] = wq.get(r);
-    wg::Quad<VB> q[U];
-    auto load = [&](int i0, int u0) {
-#pragma unroll
-      for (int u = u0; u < u0 + U / 2; ++u) {
-        q[u].zero();
-        if (i0 + u < nv) f2d_quad<VEC>(q[u], V + (long long)(i0 + u) * n, n4, n);
-      }
-    };
-    load(0, 0);
-    for (int i0 = 0; i0 < nv; i0 += U) {
-      load(i0, U / 2);
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float2 c = hs[i0 + u];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) wg::cms(acc[r], q[u].get(r), c);
-        if (u == U / 2 - 1) load(i0 + U, 0);
-      }
-    }
-    float f = 0.f;   // values past n are zero
-#pragma unroll
-    for (int r = 0; r < 4; ++r) f = fmaf(acc[r].x, acc[r].x, fmaf(acc[r].y, acc[r].y, f));
-    nrm2 += (double)f;
-    if constexpr (VEC) {
-      float4* wp = reinterpret_cast<float4*>(w) + 2 * n4;
-      wp[0] = make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
-      wp[1] = make_float4(acc[2].x, acc[2].y, acc[3].x, acc[3].y);
-    } else {
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (4 * n4 + r < n) w[4 * n4 + r] = acc[r];
-    }
-  }
-  nrm2 = wg::warp_sum(nrm2);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = nrm2;
-  __syncthreads();
   if (threadIdx.x == 0) {
-    norms[blockIdx.x] = (ws[0] + ws[1]) + (ws[2] + ws[3]);
-    __threadfence();
-    last = atomicAdd(&k.ctl[3], 1) == (int)gridDim.x - 1;
+    partial[((long long)i * gridDim.x + blockIdx.x) * 2] = sre[0];
+    partial[((long long)i * gridDim.x + blockIdx.x) * 2 + 1] = sim[0];
   }
+}
+
+// w -= sum_i h_i V_i in FP32.  The coefficients are converted to FP32 once per block into shared memory:
+// converting them per element put every element x vector through the FP64 pipe (98% busy, DRAM at 35%).
+constexpr int kGsStage = 256;
+template <typename VB>
+__global__ void __launch_bounds__(256) f2d_gs_update32(const VB* __restrict__ V, long long vstride,
+                                                       float2* __restrict__ w, const double2* __restrict__ h, int nv,
+                                                       long long n) {
+  __shared__ float2 hs[kGsStage];
+  for (int i = threadIdx.x; i < min(nv, kGsStage); i += blockDim.x) hs[i] = make_float2((float)h[i].x, (float)h[i].y);
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double w2p = 0.0;
-#pragma unroll 4
-  for (int c = threadIdx.x; c < (int)gridDim.x; c += kF2dUpThreads) w2p += __ldcg(&norms[c]);
-  const double w2b = wg::block_sum1(w2p);
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    const double w2 = __shfl_sync(0xffffffffu, w2b, 0);
-    int again = 0;
-    if (PASS == 1) {
-      double h2 = 0.0;
-      for (int i = lane; i < nv; i += 32) h2 += h[i].x * h[i].x + h[i].y * h[i].y;
-      h2 = wg::warp_sum(h2);
-      again = w2 < 0.5 * (w2 + h2);
-      if (lane == 0) k.ctl[2] = again;
-    }
-    if (!again) {
-      const double v = w2 > 0 ? sqrt(w2) : w2;   // NaN passes on
-      double2* col = k.H + (long long)k.j * k.ldh;
-      for (int i = lane; i <= k.j; i += 32) col[i] = k.hc[i];
-      if (lane == 0) k.nrm[0] = v;
-      __syncwarp();
-      wg::givens_warp(k.H, k.cs, k.sn, k.g, k.ctl, k.ctl + 1, k.target, 0, k.j, k.ldh, 0, v);
-    }
+  const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (t >= n) return;
+  float2 acc = w[t];
+  for (int i = 0; i < nv; ++i) {
+    const float2 v = f2d_ld(V[(long long)i * vstride + t]);
+    const float2 c = i < kGsStage ? hs[i] : make_float2((float)h[i].x, (float)h[i].y);
+    acc.x -= c.x * v.x - c.y * v.y;
+    acc.y -= c.x * v.y + c.y * v.x;
   }
-  if (threadIdx.x == 0) k.ctl[3] = 0;
+  w[t] = acc;
 }
 
 __global__ void __launch_bounds__(256) f2d_scale32(const float2* __restrict__ x, float2* __restrict__ out,
@@ -1198,34 +922,33 @@ __global__ void __launch_bounds__(256) f2d_dot_partial(const double2* __restrict
   }
 }
 
-// out[i] = sum of the partials of vector i, added to acc[i] as well (nullable); one block per vector.  run: as above.
+// out[i] = sum of the partials of vector i; one block per vector
 __global__ void __launch_bounds__(256) f2d_dot_reduce(const double* __restrict__ partial, double2* __restrict__ out,
-                                                      double2* __restrict__ acc, int nblk,
-                                                      const int* __restrict__ run) {
-  __shared__ double2 ws[8];
-  if (run && !*run) return;
+                                                      int nblk, int accumulate) {
+  __shared__ double sre[256], sim[256];
   const int i = blockIdx.x;
-  const double2* p = reinterpret_cast<const double2*>(partial) + (long long)i * nblk;
-  double2 r = make_double2(0.0, 0.0);
-#pragma unroll 4
+  double re = 0.0, im = 0.0;
   for (int b = threadIdx.x; b < nblk; b += 256) {
-    const double2 t = p[b];
-    r.x += t.x;
-    r.y += t.y;
+    re += partial[((long long)i * nblk + b) * 2];
+    im += partial[((long long)i * nblk + b) * 2 + 1];
   }
-  r.x = wg::warp_sum(r.x);
-  r.y = wg::warp_sum(r.y);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = r;
+  sre[threadIdx.x] = re;
+  sim[threadIdx.x] = im;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double2 t = ws[0];
-#pragma unroll
-    for (int q = 1; q < 8; ++q) {
-      t.x += ws[q].x;
-      t.y += ws[q].y;
+  for (int o = 128; o > 0; o >>= 1) {
+    if (threadIdx.x < o) {
+      sre[threadIdx.x] += sre[threadIdx.x + o];
+      sim[threadIdx.x] += sim[threadIdx.x + o];
     }
-    out[i] = t;
-    if (acc) acc[i] = make_double2(acc[i].x + t.x, acc[i].y + t.y);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    if (accumulate) {
+      out[i].x += sre[0];
+      out[i].y += sim[0];
+    } else {
+      out[i] = make_double2(sre[0], sim[0]);
+    }
   }
 }
 
@@ -1299,13 +1022,64 @@ __global__ void __launch_bounds__(256) f2d_rscale(double2* __restrict__ v, doubl
   v[t].y *= s;
 }
 
-// Hessenberg column j (hc[0..j] from Gram-Schmidt, nrm[0] = |w|): previous Givens rotations, the new one, the
-// rotated right-hand side; g[j+1] is the residual estimate.  One warp.
-__global__ void f2d_givens(F2dKrylov k) {
-  double2* col = k.H + (long long)k.j * k.ldh;
-  for (int i = threadIdx.x; i <= k.j; i += 32) col[i] = k.hc[i];
-  __syncwarp();
-  wg::givens_warp(k.H, k.cs, k.sn, k.g, k.ctl, k.ctl + 1, k.target, 0, k.j, k.ldh, 0, k.nrm[0]);
+// Hessenberg column j (hc[0..j] from Gram-Schmidt, nrm[0] = |w|): previous Givens rotations, the
+// new one, the rotated right-hand side; g[j+1] is the residual estimate.  One thread.
+__global__ void f2d_givens(double2* __restrict__ H, const double2* __restrict__ hc, const double* __restrict__ nrm,
+                           double* __restrict__ cs, double2* __restrict__ sn, double2* __restrict__ g, int j, int ldh) {
+  double2* col = H + (long long)j * ldh;
+  for (int i = 0; i <= j; ++i) col[i] = hc[i];
+  col[j + 1] = make_double2(nrm[0], 0.0);
+  for (int i = 0; i < j; ++i) {
+    const double c = cs[i];
+    const double2 s = sn[i], a = col[i], b = col[i + 1];
+    // [c s; -conj(s) c] [a; b]
+    col[i] = make_double2(c * a.x + s.x * b.x - s.y * b.y, c * a.y + s.x * b.y + s.y * b.x);
+    col[i + 1] = make_double2(-(s.x * a.x + s.y * a.y) + c * b.x, -(s.x * a.y - s.y * a.x) + c * b.y);
+  }
+  const double2 a = col[j];
+  const double bb = col[j + 1].x;
+  const double aa = hypot(a.x, a.y);
+  const double rho = hypot(aa, bb);
+  double c;
+  double2 s, top;
+  if (rho == 0.0) {
+    c = 1.0;
+    s = make_double2(0.0, 0.0);
+    top = a;
+  } else if (aa == 0.0) {
+    c = 0.0;
+    s = make_double2(1.0, 0.0);
+    top = make_double2(bb, 0.0);
+  } else {
+    c = aa / rho;
+    const double2 ph = make_double2(a.x / aa, a.y / aa);
+    s = make_double2(ph.x * bb / rho, ph.y * bb / rho);        // (a/|a|) conj(b) / rho, b real
+    top = make_double2(ph.x * rho, ph.y * rho);
+  }
+  cs[j] = c;
+  sn[j] = s;
+  col[j] = top;
+  col[j + 1] = make_double2(0.0, 0.0);
+  const double2 gj = g[j];
+  g[j] = make_double2(c * gj.x, c * gj.y);
+  g[j + 1] = make_double2(-(s.x * gj.x + s.y * gj.y), -(s.x * gj.y - s.y * gj.x));
+}
+
+// y = R^-1 g for the leading k x k upper triangle of H; one thread
+__global__ void f2d_backsolve(const double2* __restrict__ H, const double2* __restrict__ g, double2* __restrict__ y,
+                              int k, int ldh) {
+  for (int i = k - 1; i >= 0; --i) {
+    double2 s = g[i];
+    for (int j = i + 1; j < k; ++j) {
+      const double2 h = H[(long long)j * ldh + i], v = y[j];
+      s.x -= h.x * v.x - h.y * v.y;
+      s.y -= h.x * v.y + h.y * v.x;
+    }
+    const double2 d = H[(long long)i * ldh + i];
+    const double den = d.x * d.x + d.y * d.y;
+    y[i] = den > 0 ? make_double2((s.x * d.x + s.y * d.y) / den, (s.y * d.x - s.x * d.y) / den)
+                   : make_double2(0.0, 0.0);
+  }
 }
 
 // u = sum_i y_i V_i
@@ -1335,65 +1109,14 @@ cudaError_t dalloc(T** p, size_t n) {
   return cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * (n ? n : 1));
 }
 
-template <typename R>
-void free_ell(EllTerms<R>& e) {
-  cudaFree(e.col);
-  cudaFree(e.re);
-  cudaFree(e.im);
-  e = EllTerms<R>{};
-}
-
-// The terms of an axis of nr rows for the device; parts of entries at or below drop times the row's largest entry
-// count as zero (drop = 0: everything stored is kept).
-template <typename R>
-cudaError_t ell_upload(const wg2d_problem::Axis& a, int nr, double drop, EllTerms<R>& out) {
-  free_ell(out);
-  std::vector<int> col;
-  std::vector<R> re, im;
-  int off = 0, first = 0;
-  for (int t = 0; t < a.T; ++t) {
-    const int* rp = a.rp.data() + (size_t)t * (nr + 1);
-    std::vector<std::vector<int>> keep(nr);
-    std::vector<double> cut(nr, 0.0);
-    int len = 0;
-    for (int i = 0; i < nr; ++i) {
-      for (int k = off + rp[i]; k < off + rp[i + 1]; ++k)
-        cut[i] = std::max(cut[i], drop * std::hypot(a.val[2 * k], a.val[2 * k + 1]));
-      for (int k = off + rp[i]; k < off + rp[i + 1]; ++k)
-        if (drop == 0 || !(std::fabs(a.val[2 * k]) <= cut[i] && std::fabs(a.val[2 * k + 1]) <= cut[i]))
-          keep[i].push_back(k);
-      len = std::max(len, (int)keep[i].size());
-    }
-    bool real = true;
-    for (int k = 0; k < len; ++k)
-      for (int i = 0; i < nr; ++i) {
-        const bool in = k < (int)keep[i].size();
-        const int e = in ? keep[i][k] : 0;
-        auto part = [&](double v) { return drop > 0 && std::fabs(v) <= cut[i] ? R(0) : (R)v; };
-        col.push_back(in ? a.col[e] : keep[i].empty() ? i : a.col[keep[i].back()]);
-        re.push_back(in ? part(a.val[2 * e]) : R(0));
-        im.push_back(in ? part(a.val[2 * e + 1]) : R(0));
-        real = real && im.back() == R(0);
-      }
-    out.first[t] = first;
-    out.len[t] = len;
-    if (real) out.real |= 1u << t;
-    first += len;
-    off += rp[nr];
-  }
-  cudaError_t e = dalloc(&out.col, col.size());
-  if (e == cudaSuccess) e = dalloc(&out.re, re.size());
-  if (e == cudaSuccess) e = dalloc(&out.im, im.size());
-  if (e == cudaSuccess) e = cudaMemcpy(out.col, col.data(), sizeof(int) * col.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(out.re, re.data(), sizeof(R) * re.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(out.im, im.data(), sizeof(R) * im.size(), cudaMemcpyHostToDevice);
-  return e;
-}
-
 void free_axis(wg2d_problem::Axis& a) {
   for (wg::OzakiRowsDev& d : a.dense) wg::ozaki_free(d);
   cudaFree(a.blocks);
-  free_ell(a.ell);
+  cudaFree(a.rp);
+  cudaFree(a.col);
+  cudaFree(a.val);
+  cudaFree(a.offs);
+  cudaFree(a.dcoef);
   cudaFree(a.ymask);
   a = wg2d_problem::Axis{};
 }
@@ -1402,9 +1125,10 @@ void free_axis(wg2d_problem::Axis& a) {
 template <typename T, typename R>
 struct OpData {
   const R* blocks[2];
-  EllTerms<R> ell[2];
+  const T* val[2];
+  const R* coef[2];
   const R *interp, *proj, *cap, *dV;
-  T* G;
+  T *Uq, *Rq, *G;
   T pot16;
   R capc;
 };
@@ -1431,20 +1155,15 @@ void transport_terms(wg2d_problem* h, int axis, const OpData<T, R>& d, const T* 
   }
   if (axis == 0) {
     const long long ncols = h->n / h->nrx;
-    const size_t smem = sizeof(T) * kColPitch<T> * h->nrx;
+    const size_t smem = sizeof(T) * kRelxCols * h->nrx;
     const int threads = (h->nrx + 31) / 32 * 32;
     if (skip_mask != (1u << a.T) - 1u)
       f2d_relx_kernel<T, R><<<(unsigned)((ncols + kRelxCols - 1) / kRelxCols), threads, smem, h->stream>>>(
-          d.G, y, d.ell[0], a.T, h->nrx, ncols, h->n, skip_mask, a.ymask,
+          d.G, y, a.rp, a.col, d.val[0], a.offs, d.coef[0], a.T, h->nrx, ncols, h->n, skip_mask, a.ymask,
           (long long)h->nry * h->nX, h->nY);
   } else {
-    const int entries = (d.ell[1].first[a.T - 1] + d.ell[1].len[a.T - 1]) * h->nry;
-    const size_t smem = entries * (2 * sizeof(R) + sizeof(int));
-    const dim3 grid((unsigned)h->ncen, (unsigned)((h->nrel + 255) / 256));
-    if (smem <= 12 * 1024)   // eight blocks' tables on an SM
-      f2d_rely_kernel<true, T, R><<<grid, 256, smem, h->stream>>>(d.G, y, d.ell[1], a.T, h->nrx, h->nry, h->n, entries);
-    else
-      f2d_rely_kernel<false, T, R><<<grid, 256, 0, h->stream>>>(d.G, y, d.ell[1], a.T, h->nrx, h->nry, h->n, 0);
+    f2d_rely_kernel<T, R><<<(unsigned)((h->n + 255) / 256), 256, 0, h->stream>>>(d.G, y, a.rp, a.col, d.val[1], a.offs,
+                                                                                d.coef[1], a.T, h->nrx, h->nry, h->n);
   }
 }
 
@@ -1452,12 +1171,15 @@ OpData<double2, double> op64(wg2d_problem* h) {
   OpData<double2, double> d;
   for (int a = 0; a < 2; ++a) {
     d.blocks[a] = h->ax[a].blocks;
-    d.ell[a] = h->ax[a].ell;
+    d.val[a] = h->ax[a].val;
+    d.coef[a] = h->ax[a].dcoef;
   }
   d.interp = h->interp;
   d.proj = h->proj;
   d.cap = h->cap;
   d.dV = h->dV;
+  d.Uq = h->Uq;
+  d.Rq = h->Rq;
   d.G = h->G;
   d.pot16 = make_double2(h->pot.x / 16.0, h->pot.y / 16.0);
   d.capc = h->capc;
@@ -1480,20 +1202,13 @@ int apply_transport(wg2d_problem* h, int axis) {
 template <int NL, typename T, typename R>
 void launch_drift(wg2d_problem* h, const OpData<T, R>& d, const T* F, T* y) {
   const wg2d_shape& s = h->s;
-  // rows of cells per warp: as many as still give 16 warps per SM, at least 3 (one more vertex row than cell rows)
-  const int xt = (h->nrx + 30) / 31;
-  const long long all = (long long)xt * h->nel * h->nry;
-  const int rows = (int)std::min<long long>(h->nry, std::max<long long>(3, all / (152 * 16)));
-  const int bands = (h->nry + rows - 1) / rows;
-  const long long items = (long long)xt * bands * h->nel;
-  // W and Cp of as many quadrature points as 40 KB hold, further points in further launches that add to y
-  constexpr int per_point = (int)sizeof(R) * 2 * ((NL + 3) / 4 * 4), most = 40 * 1024 / per_point;
-  for (int q0 = 0; q0 < h->nq; q0 += most) {
-    const int nqc = std::min(most, h->nq - q0);
-    f2d_drift_kernel<NL, T, R><<<(unsigned)((items + 3) / 4), 128, (size_t)per_point * nqc, h->stream>>>(
-        F, y, d.interp, d.proj, d.dV, d.cap, d.pot16, d.capc, q0, nqc, h->nq, h->nrx, h->nry, h->nvert, s.n_el_x, s.nk_x,
-        h->nX, s.periodic_y, xt, bands, rows, items);
-  }
+  const dim3 g1((unsigned)((h->nrel + 127) / 128), (unsigned)h->nel);
+  f2d_interp_kernel<NL, T, R><<<g1, 128, 0, h->stream>>>(F, d.Uq, d.interp, h->nq, h->nrel, s.n_el_x, s.nk_x, s.nk_y,
+                                                         h->nX);
+  const dim3 g2((unsigned)((h->nrel + 127) / 128), (unsigned)h->nq, (unsigned)h->nel);
+  f2d_vertex_kernel<T, R><<<g2, 128, 0, h->stream>>>(d.Uq, d.Rq, d.dV, h->nrx, h->nry, h->nq, h->nvert, s.periodic_y);
+  f2d_project_kernel<NL, T, R><<<g1, 128, 0, h->stream>>>(d.Rq, F, y, d.proj, d.cap, d.pot16, d.capc, h->nq, h->nrel,
+                                                          s.n_el_x, s.nk_x, s.nk_y, h->nX);
 }
 
 template <typename T, typename R>
@@ -1611,6 +1326,8 @@ int wg2d_create(const wg2d_shape* s, wg2d_problem** out) {
   const size_t slab = (size_t)h->nel * h->nq;
   if (e == cudaSuccess) e = dalloc(&h->x, h->n);
   if (e == cudaSuccess) e = dalloc(&h->y, h->n);
+  if (e == cudaSuccess) e = dalloc(&h->Uq, slab * h->nrel);
+  if (e == cudaSuccess) e = dalloc(&h->Rq, slab * h->nrel);
   if (e == cudaSuccess) e = dalloc(&h->dV, slab * h->nvert);
   if (e == cudaSuccess) e = dalloc(&h->interp, (size_t)h->nq * h->nloc);
   if (e == cudaSuccess) e = dalloc(&h->proj, (size_t)h->nq * h->nloc);
@@ -1623,9 +1340,9 @@ int wg2d_create(const wg2d_shape* s, wg2d_problem** out) {
   if (e == cudaSuccess) e = cudaMemset(h->tc_err, 0, sizeof(int));
   for (cudaEvent_t& ev : h->ev)
     if (e == cudaSuccess) e = cudaEventCreate(&ev);
-  if (e == cudaSuccess && h->nrx * kColPitch<double2> * sizeof(double2) > 48 * 1024)
+  if (e == cudaSuccess && h->nrx * kRelxCols * sizeof(double2) > 48 * 1024)
     e = cudaFuncSetAttribute(f2d_relx_kernel<double2, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(h->nrx * kColPitch<double2> * sizeof(double2)));
+                             (int)(h->nrx * kRelxCols * sizeof(double2)));
   if (e != cudaSuccess) {
     wg2d_destroy(h);
     return e == cudaErrorMemoryAllocation ? WG_ERR_OOM : WG_ERR_CUDA;
@@ -1642,7 +1359,7 @@ int wg2d_destroy(wg2d_problem* h) {
   free_preconditioner(h);
   free32(h);
   wg::ozaki_free(h->cols);
-  void* ptrs[] = {h->x, h->y, h->G, h->dV, h->interp, h->proj, h->xq, h->yq, h->vx, h->vy, h->cap,
+  void* ptrs[] = {h->x, h->y, h->G, h->Uq, h->Rq, h->dV, h->interp, h->proj, h->xq, h->yq, h->vx, h->vy, h->cap,
                   h->tc_err, h->obs_W, h->obs_wj, h->obs_out, h->wall_act, h->wall_T, h->wall_T32, h->wall_u,
                   h->wall_u32};
   for (void* p : ptrs)
@@ -1679,16 +1396,22 @@ int wg2d_set_transport(wg2d_problem* h, int axis, int n_terms, const double* coe
   free_axis(a);
   h->d32_ready = false;
   a.T = n_terms;
+  a.coef.assign(coef, coef + n_terms);
   if (n_terms == 0) return WG_OK;
+  const int nrp = n_terms * (nr + 1);
   const size_t nb = (size_t)n_terms * n_el * 3 * nk * nk;
   F2_CK(dalloc(&a.blocks, nb));
+  F2_CK(dalloc(&a.rp, nrp));
+  F2_CK(dalloc(&a.col, off[n_terms]));
+  F2_CK(dalloc(&a.val, off[n_terms]));
+  F2_CK(dalloc(&a.offs, n_terms));
+  F2_CK(dalloc(&a.dcoef, n_terms));
   F2_CK(cudaMemcpy(a.blocks, center_blocks, sizeof(double) * nb, cudaMemcpyHostToDevice));
-  a.rp.assign(row_ptr, row_ptr + (size_t)n_terms * (nr + 1));
-  a.col.assign(col, col + off[n_terms]);
-  a.val.resize(2 * (size_t)off[n_terms]);
-  for (int t = 0; t < n_terms; ++t)
-    for (int k = 2 * off[t]; k < 2 * off[t + 1]; ++k) a.val[k] = coef[t] * val[k];
-  F2_CK(ell_upload(a, nr, 0.0, a.ell));
+  F2_CK(cudaMemcpy(a.rp, row_ptr, sizeof(int) * nrp, cudaMemcpyHostToDevice));
+  F2_CK(cudaMemcpy(a.offs, off.data(), sizeof(int) * n_terms, cudaMemcpyHostToDevice));
+  F2_CK(cudaMemcpy(a.dcoef, coef, sizeof(double) * n_terms, cudaMemcpyHostToDevice));
+  F2_CK(cudaMemcpy(a.col, col, sizeof(int) * std::max(1, off[n_terms]), cudaMemcpyHostToDevice));
+  F2_CK(cudaMemcpy(a.val, val, sizeof(double2) * std::max(1, off[n_terms]), cudaMemcpyHostToDevice));
   // dense rho_x factors on the tensor cores: the real embedding of c_t R_t, digit-sliced once
   a.dense.assign(n_terms, wg::OzakiRowsDev{});
   a.dense_mask = 0;
@@ -1836,72 +1559,48 @@ static unsigned blocks256(long long n) { return (unsigned)((n + 255) / 256); }
 // FP64 with the mode transforms on the tensor cores.
 }  // extern "C"
 
-template <int NK, typename T, bool BYMODE>
-static void xline_launch(wg2d_problem* h, const T* xinv, const T* xcpl, const T* in, T* out) {
-  const int C = h->x_chunks, LB = h->x_lines;
-  const long long lines = (long long)h->nrx * h->nry * h->nY;
-  f2d_xline_kernel<NK, T, BYMODE><<<(unsigned)((lines + LB - 1) / LB), LB * C, sizeof(T) * NK * LB * C, h->stream>>>(
-      in, out, reinterpret_cast<const T*>(h->xmaps), xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX, h->nY, h->s.n_el_x,
-      h->x_chunk_len, C, LB);
-}
-
-// z = M^-1 r.  With UH and Us (transposed) the modal fields lie by mode; without, the caller has transformed r into pa
-// and transforms pa back, rho_x fastest.
-template <typename T, bool BYMODE>
-static void precond_lines(wg2d_problem* h, const T* xinv, const T* xcpl, const T* tinv, T* pa, T* pb) {
-  switch (h->s.nk_x) {
-    case 2: xline_launch<2, T, BYMODE>(h, xinv, xcpl, pa, pb); break;
-    case 3: xline_launch<3, T, BYMODE>(h, xinv, xcpl, pa, pb); break;
-    default: xline_launch<4, T, BYMODE>(h, xinv, xcpl, pa, pb); break;
-  }
-  const dim3 tg((unsigned)((h->nX + kTxTile - 1) / kTxTile), (unsigned)h->nrx);
-  f2d_transverse_kernel<T, BYMODE><<<tg, 32 * ((h->nT + kTxRows - 1) / kTxRows), tx_smem(h->nT, sizeof(T)), h->stream>>>(
-      pb, pa, tinv, h->nrx, h->nry, h->nX, h->nY, h->nT, tx_pitch(h->nT));
-}
-
 template <typename T>
 static void precond_stages(wg2d_problem* h, const T* UH, const T* Us, const T* xinv, const T* xcpl, const T* tinv,
                            const T* r, T* pa, T* pb, T* z) {
-  if (!UH) {
-    precond_lines<T, false>(h, xinv, xcpl, tinv, pa, pb);
-    return;
-  }
   const long long ncols = h->n / h->nrx;
   const int threads = (h->nrx + 31) / 32 * 32;
-  const unsigned blocks = (unsigned)((ncols + kRelxCols - 1) / kRelxCols);
-  const size_t smem = sizeof(T) * kColPitch<T> * modal_rows(h->nrx);
-  f2d_modal_kernel<T, true><<<blocks, threads, smem, h->stream>>>(UH, r, pa, h->nrx, ncols);
-  precond_lines<T, true>(h, xinv, xcpl, tinv, pa, pb);
-  f2d_modal_kernel<T, false><<<blocks, threads, smem, h->stream>>>(Us, pa, z, h->nrx, ncols);
-}
-
-// Chunk maps of the X-line sweep for the factors just uploaded.
-template <typename T>
-static cudaError_t xline_maps(wg2d_problem* h, const T* xinv, const T* xcpl) {
-  if (h->x_chunks < 2) return cudaSuccess;
-  T* maps = reinterpret_cast<T*>(h->xmaps);
-  const int C = h->x_chunks, ne = h->s.n_el_x, nk = h->s.nk_x, L = h->x_chunk_len;
-  const unsigned blocks = (unsigned)(((size_t)h->nrx * C * nk + 127) / 128);
-  switch (nk) {
-    case 2: f2d_xline_maps_kernel<2, T><<<blocks, 128, 0, h->stream>>>(maps, xinv, xcpl, h->fwd, h->nrx, ne, L, C); break;
-    case 3: f2d_xline_maps_kernel<3, T><<<blocks, 128, 0, h->stream>>>(maps, xinv, xcpl, h->fwd, h->nrx, ne, L, C); break;
-    default: f2d_xline_maps_kernel<4, T><<<blocks, 128, 0, h->stream>>>(maps, xinv, xcpl, h->fwd, h->nrx, ne, L, C); break;
+  const size_t smem = sizeof(T) * kRelxCols * h->nrx;
+  if (UH)
+    f2d_dense_rx_kernel<T><<<(unsigned)((ncols + kRelxCols - 1) / kRelxCols), threads, smem, h->stream>>>(
+        UH, r, pa, h->nrx, ncols);
+  const long long lines = (long long)h->nrx * h->nry * h->nY;
+  if (h->x_chunks > 1 && h->xmaps) {
+    T* maps = reinterpret_cast<T*>(h->xmaps);
+    const int L = h->x_chunk_len, C = h->x_chunks, ne = h->s.n_el_x;
+    const unsigned cb = (unsigned)((lines * C + 127) / 128);
+#define WG_XLINE_CHUNKED(NK_)                                                                                \
+  f2d_xline_maps_kernel<NK_, T><<<cb, 128, 0, h->stream>>>(pa, maps, xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX, \
+                                                          h->nY, ne, L, C);                                   \
+  f2d_xline_apply_kernel<NK_, T><<<cb, 128, 0, h->stream>>>(pa, pb, maps, xinv, xcpl, h->fwd, h->nrx, h->nry,  \
+                                                           h->nX, h->nY, ne, L, C);
+    switch (h->s.nk_x) {
+      case 2: WG_XLINE_CHUNKED(2) break;
+      case 3: WG_XLINE_CHUNKED(3) break;
+      default: WG_XLINE_CHUNKED(4) break;
+    }
+#undef WG_XLINE_CHUNKED
+  } else {
+    const unsigned lb = (unsigned)((lines + 127) / 128);
+    switch (h->s.nk_x) {
+      case 2: f2d_xline_kernel<2, T><<<lb, 128, 0, h->stream>>>(pa, pb, xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX,
+                                                               h->nY, h->s.n_el_x); break;
+      case 3: f2d_xline_kernel<3, T><<<lb, 128, 0, h->stream>>>(pa, pb, xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX,
+                                                               h->nY, h->s.n_el_x); break;
+      default: f2d_xline_kernel<4, T><<<lb, 128, 0, h->stream>>>(pa, pb, xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX,
+                                                                h->nY, h->s.n_el_x); break;
+    }
   }
-  return cudaGetLastError();
-}
-
-// Shared memory of the preconditioner's kernels of one precision beyond the default limit.
-template <typename T>
-static cudaError_t precond_attributes(wg2d_problem* h) {
-  const int tsm = (int)tx_smem(h->nT, sizeof(T)), msm = (int)(sizeof(T) * kColPitch<T> * modal_rows(h->nrx));
-  cudaError_t e = cudaFuncSetAttribute(f2d_transverse_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(f2d_transverse_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
-  if (e == cudaSuccess && msm > 48 * 1024)
-    e = cudaFuncSetAttribute(f2d_modal_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, msm);
-  if (e == cudaSuccess && msm > 48 * 1024)
-    e = cudaFuncSetAttribute(f2d_modal_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, msm);
-  return e;
+  const size_t tsm = sizeof(T) * ((size_t)h->nT * h->nT + (size_t)h->nT * kTxTile);
+  const dim3 tg((unsigned)((h->nX + kTxTile - 1) / kTxTile), (unsigned)h->nrx);
+  f2d_transverse_kernel<T><<<tg, 256, tsm, h->stream>>>(pb, pa, tinv, h->nrx, h->nry, h->nX, h->nY, h->nT);
+  if (Us)
+    f2d_dense_rx_kernel<T><<<(unsigned)((ncols + kRelxCols - 1) / kRelxCols), threads, smem, h->stream>>>(
+        Us, pa, z, h->nrx, ncols);
 }
 
 extern "C" {
@@ -1928,48 +1627,40 @@ static int precondition_device(wg2d_problem* h, const double2* r, double2* z) {
   return WG_OK;
 }
 
-// out[0..nv) = V_i^H w (acc, nullable: added there too)
-static void dots(wg2d_problem* h, const double2* V, int nv, const double2* w, double2* out, double2* acc = nullptr) {
+// out[0..nv) = V_i^H w (accumulate: out += ...)
+static void dots(wg2d_problem* h, const double2* V, int nv, const double2* w, double2* out, int accumulate) {
   f2d_dot_partial<<<dim3(kDotBlocks, nv), 256, 0, h->stream>>>(V, h->n, w, h->partial, h->n);
-  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, out, acc, kDotBlocks, nullptr);
+  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, out, kDotBlocks, accumulate);
 }
 
 static void vnorm(wg2d_problem* h, const double2* w) {
-  dots(h, w, 1, w, h->hp);
+  dots(h, w, 1, w, h->hp, 0);
   f2d_sqrt_real<<<1, 1, 0, h->stream>>>(h->hp, h->nrm);
 }
 
 }  // extern "C"
 
-// Gram-Schmidt of w against V_0 .. V_{k.j}, |w| and the Givens step: two launches of each kernel, the second ones idle
-// unless the first pass lost more than half of |w|^2 (decided on the device).
-template <bool VEC, typename VB>
-static void gram_schmidt32(wg2d_problem* h, const VB* V, float2* w, const F2dKrylov& k) {
-  const int nv = k.j + 1;
-  const long long n = h->n;
-  const int mq = wg::gs_quads(n + 3, 1, 3, 256), uq = wg::gs_quads(n + 3, 1, 8, kF2dUpThreads);
-  const unsigned mb = (unsigned)(((n + 3) / 4 + mq - 1) / mq), ub = (unsigned)(((n + 3) / 4 + uq - 1) / uq);
-  const size_t sm = sizeof(double) * 16 * ((nv + 3) & ~3);
-  f2d_multidot32<VEC, VB><<<mb, 256, sm, h->stream>>>(V, w, h->partial, n, nv, mq, nullptr);
-  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, h->hc, nullptr, mb, nullptr);
-  f2d_gs_update32<1, VEC, VB><<<ub, kF2dUpThreads, 0, h->stream>>>(V, w, h->hc, nv, n, uq, h->partial, k);
-  f2d_multidot32<VEC, VB><<<mb, 256, sm, h->stream>>>(V, w, h->partial, n, nv, mq, k.ctl + 2);
-  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, h->hp, h->hc, mb, k.ctl + 2);
-  f2d_gs_update32<2, VEC, VB><<<ub, kF2dUpThreads, 0, h->stream>>>(V, w, h->hp, nv, n, uq, h->partial, k);
+template <typename VB>
+static void dots32(wg2d_problem* h, const VB* V, int nv, const float2* w, double2* out, int accumulate) {
+  f2d_dot_partial32<VB><<<dim3(kDotBlocks, nv), 256, 0, h->stream>>>(V, h->n, w, h->partial, h->n);
+  f2d_dot_reduce<<<nv, 256, 0, h->stream>>>(h->partial, out, kDotBlocks, accumulate);
 }
 
 extern "C" {
 
+static void vnorm32(wg2d_problem* h, const float2* w) {
+  dots32(h, w, 1, w, h->hp, 0);
+  f2d_sqrt_real<<<1, 1, 0, h->stream>>>(h->hp, h->nrm);
+}
+
 static void free_solver(wg2d_problem* h) {
   void* ptrs[] = {h->V, h->Zb, h->r, h->w, h->z, h->b, h->xs, h->H, h->g, h->sn, h->hc, h->hp, h->yc, h->cs,
-                  h->partial, h->nrm, h->ktarget, h->kctl, h->bc_rt, h->bc_p, h->bc_ph, h->bc_sh};
+                  h->partial, h->nrm, h->bc_rt, h->bc_p, h->bc_ph, h->bc_sh};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   h->bc_rt = h->bc_p = h->bc_ph = h->bc_sh = nullptr;
   h->V = h->Zb = h->r = h->w = h->z = h->b = h->xs = h->H = h->g = h->sn = h->hc = h->hp = h->yc = nullptr;
-  h->cs = nullptr;
-  h->partial = h->nrm = h->ktarget = nullptr;
-  h->kctl = nullptr;
+  h->cs = h->partial = h->nrm = nullptr;
   h->vm = 0;
 }
 
@@ -2093,14 +1784,14 @@ int wg2d_apply_repeat(wg2d_problem* h, int n, double* ms, double* parts_ms) {
 
 
 static void free32(wg2d_problem* h) {
-  for (EllTerms<float>& e : h->ell32) free_ell(e);
-  void* ptrs[] = {h->blocks32[0], h->blocks32[1], h->interp32,
-                  h->proj32, h->cap32, h->dV32, h->G32, h->V32, h->Z32, h->w32, h->Vh32, h->vj32};
+  void* ptrs[] = {h->blocks32[0], h->blocks32[1], h->coef32[0], h->coef32[1], h->val32[0], h->val32[1], h->interp32,
+                  h->proj32, h->cap32, h->dV32, h->Uq32, h->Rq32, h->G32, h->V32, h->Z32, h->w32, h->Vh32, h->vj32};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  h->blocks32[0] = h->blocks32[1] = nullptr;
+  h->blocks32[0] = h->blocks32[1] = h->coef32[0] = h->coef32[1] = nullptr;
+  h->val32[0] = h->val32[1] = nullptr;
   h->interp32 = h->proj32 = h->cap32 = h->dV32 = nullptr;
-  h->G32 = h->V32 = h->Z32 = h->w32 = h->vj32 = nullptr;
+  h->Uq32 = h->Rq32 = h->G32 = h->V32 = h->Z32 = h->w32 = h->vj32 = nullptr;
   h->Vh32 = nullptr;
   h->vm32 = 0;
   h->d32_ready = false;
@@ -2131,9 +1822,14 @@ static int ensure32(wg2d_problem* h) {
     if (!ax.T) continue;
     const int nk = a == 0 ? h->s.nk_x : h->s.nk_y, ne = a == 0 ? h->s.n_el_x : h->s.n_el_y;
     const int nr = a == 0 ? h->nrx : h->nry;
+    int nnz = 0;
+    std::vector<int> rp((size_t)ax.T * (nr + 1));
+    F2_CK(cudaMemcpy(rp.data(), ax.rp, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost));
+    for (int t = 0; t < ax.T; ++t) nnz += rp[(size_t)t * (nr + 1) + nr];
     int rc = conv(&h->blocks32[a], ax.blocks, (long long)ax.T * ne * 3 * nk * nk);
+    if (!rc) rc = conv(&h->coef32[a], ax.dcoef, ax.T);
+    if (!rc) rc = conv(reinterpret_cast<float**>(&h->val32[a]), reinterpret_cast<const double*>(ax.val), 2LL * nnz);
     if (rc) return rc;
-    F2_CK(ell_upload(ax, nr, std::ldexp(1.0, -40), h->ell32[a]));
   }
   const long long slab = (long long)h->nel * h->nq;
   int rc = conv(&h->interp32, h->interp, (long long)h->nq * h->nloc);
@@ -2141,10 +1837,12 @@ static int ensure32(wg2d_problem* h) {
   if (!rc) rc = conv(&h->cap32, h->cap, h->nrel);
   if (!rc) rc = conv(&h->dV32, h->dV, slab * h->nvert);
   if (rc) return rc;
+  F2_CK(dalloc(&h->Uq32, slab * h->nrel));
+  F2_CK(dalloc(&h->Rq32, slab * h->nrel));
   F2_CK(dalloc(&h->G32, (size_t)std::max(1, std::max(h->ax[0].T, h->ax[1].T)) * h->n));
-  if (h->nrx * kColPitch<float2> * sizeof(float2) > 48 * 1024)
+  if (h->nrx * kRelxCols * sizeof(float2) > 48 * 1024)
     F2_CK(cudaFuncSetAttribute(f2d_relx_kernel<float2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(h->nrx * kColPitch<float2> * sizeof(float2))));
+                               (int)(h->nrx * kRelxCols * sizeof(float2))));
   F2_CK(cudaStreamSynchronize(h->stream));
   h->d32_ready = true;
   return WG_OK;
@@ -2156,12 +1854,15 @@ OpData<float2, float> op32(wg2d_problem* h) {
   OpData<float2, float> d;
   for (int a = 0; a < 2; ++a) {
     d.blocks[a] = h->blocks32[a];
-    d.ell[a] = h->ell32[a];
+    d.val[a] = h->val32[a];
+    d.coef[a] = h->coef32[a];
   }
   d.interp = h->interp32;
   d.proj = h->proj32;
   d.cap = h->cap32;
   d.dV = h->dV32;
+  d.Uq = h->Uq32;
+  d.Rq = h->Rq32;
   d.G = h->G32;
   d.pot16 = make_float2((float)(h->pot.x / 16.0), (float)(h->pot.y / 16.0));
   d.capc = (float)h->capc;
@@ -2223,32 +1924,24 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
   // WG_XLINE_CHUNKS=<n> sets the chunk count, 0 or 1 keeps one sequential sweep per line
   {
     int C = ne >= 8 ? std::min(16, ne / 4) : 1;
-    if (const char* env = getenv("WG_XLINE_CHUNKS")) C = std::max(1, std::min({atoi(env), ne, kXlineThreads / 4}));
+    if (const char* env = getenv("WG_XLINE_CHUNKS")) C = std::max(1, std::min(atoi(env), ne));
     const int L = (ne + C - 1) / std::max(1, C);
     h->x_chunk_len = L;
     h->x_chunks = C > 1 ? (ne + L - 1) / L : 1;
-    // lines per block: 32 (one mode's coefficients a warp), fewer when the chunks fill the block
-    for (h->x_lines = 32; h->x_lines > 4 && h->x_lines * h->x_chunks > kXlineThreads;) h->x_lines /= 2;
-    if (h->x_chunks > 1) F2_CK(dalloc(&h->xmaps, (size_t)nr * h->x_chunks * nk * nk));
+    if (h->x_chunks > 1)
+      F2_CK(dalloc(&h->xmaps, (size_t)h->x_chunks * (nk * nk + nk) * ((size_t)nr * h->nry * h->nY)));
   }
   F2_CK(dalloc(&h->fwd, nr));
   F2_CK(cudaMemcpy(h->fwd, forward, sizeof(int) * nr, cudaMemcpyHostToDevice));
-  // U^H and U / sigma as complex [nr][nr], transposed; the transverse inverses transposed per mode
-  const size_t nu = (size_t)nr * (modal_rows(nr) + 4);   // zero rows past nr
-  std::vector<double> uh(2 * nu, 0.0), us(2 * nu, 0.0), ti(2 * nt);
+  // U^H and U / sigma as complex [nr][nr] row-major
+  std::vector<double> uh((size_t)2 * nr * nr), us((size_t)2 * nr * nr);
   for (int i = 0; i < nr; ++i)
     for (int j = 0; j < nr; ++j) {
-      const size_t src = 2 * ((size_t)j * nr + i), dst = 2 * ((size_t)j * nr + i), tr = 2 * ((size_t)i * nr + j);
-      uh[dst] = U[src];          // (U^H)_ij = conj(U_ji), stored at [j][i]
-      uh[dst + 1] = -U[src + 1];
-      us[dst] = U[tr] / sigma;   // U_ij / sigma, stored at [j][i]
-      us[dst + 1] = U[tr + 1] / sigma;
+      uh[2 * ((size_t)i * nr + j)] = U[2 * ((size_t)j * nr + i)];
+      uh[2 * ((size_t)i * nr + j) + 1] = -U[2 * ((size_t)j * nr + i) + 1];
+      us[2 * ((size_t)i * nr + j)] = U[2 * ((size_t)i * nr + j)] / sigma;
+      us[2 * ((size_t)i * nr + j) + 1] = U[2 * ((size_t)i * nr + j) + 1] / sigma;
     }
-  for (int k = 0; k < nr; ++k)
-    for (int t = 0; t < nT; ++t)
-      for (int q = 0; q < nT; ++q)
-        for (int c = 0; c < 2; ++c)
-          ti[2 * (((size_t)k * nT + q) * nT + t) + c] = t_inverse[2 * (((size_t)k * nT + t) * nT + q) + c];
   if (fp32) {
     auto up32 = [&](float2** dst, const double* src, size_t count) -> int {
       std::vector<float> f(2 * count);
@@ -2259,14 +1952,16 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
     };
     int rc = up32(&h->xinv32, x_inverse, nx);
     if (!rc) rc = up32(&h->xcpl32, x_coupling, nx);
-    if (!rc) rc = up32(&h->tinv32, ti.data(), nt);
-    if (!rc) rc = up32(&h->UH32, uh.data(), nu);
-    if (!rc) rc = up32(&h->Us32, us.data(), nu);
+    if (!rc) rc = up32(&h->tinv32, t_inverse, nt);
+    if (!rc) rc = up32(&h->UH32, uh.data(), (size_t)nr * nr);
+    if (!rc) rc = up32(&h->Us32, us.data(), (size_t)nr * nr);
     if (rc) return rc;
     F2_CK(dalloc(&h->pa32, h->n));
     F2_CK(dalloc(&h->pb32, h->n));
-    F2_CK(precond_attributes<float2>(h));
-    F2_CK(xline_maps(h, h->xinv32, h->xcpl32));
+    F2_CK(cudaFuncSetAttribute(f2d_transverse_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
+    if (h->nrx * kRelxCols * sizeof(float2) > 48 * 1024)
+      F2_CK(cudaFuncSetAttribute(f2d_dense_rx_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(h->nrx * kRelxCols * sizeof(float2))));
     h->pre32 = true;
     h->pre_ready = true;
     return WG_OK;
@@ -2278,17 +1973,19 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
   F2_CK(dalloc(&h->pb, h->n));
   F2_CK(cudaMemcpy(h->xinv, x_inverse, sizeof(double2) * nx, cudaMemcpyHostToDevice));
   F2_CK(cudaMemcpy(h->xcpl, x_coupling, sizeof(double2) * nx, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(h->tinv, ti.data(), sizeof(double2) * nt, cudaMemcpyHostToDevice));
-  F2_CK(precond_attributes<double2>(h));
-  F2_CK(xline_maps(h, h->xinv, h->xcpl));
+  F2_CK(cudaMemcpy(h->tinv, t_inverse, sizeof(double2) * nt, cudaMemcpyHostToDevice));
+  F2_CK(cudaFuncSetAttribute(f2d_transverse_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
+  if (h->nrx * kRelxCols * sizeof(double2) > 48 * 1024)
+    F2_CK(cudaFuncSetAttribute(f2d_dense_rx_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(h->nrx * kRelxCols * sizeof(double2))));
   if (h->s.tensor_cores) {
     int rc = wg::ozaki_rows_upload(embed(U, nr, 1.0, true), 2 * nr, 2 * nr, h->UH, h->err);
     if (!rc) rc = wg::ozaki_rows_upload(embed(U, nr, 1.0 / sigma, false), 2 * nr, 2 * nr, h->Us, h->err);
     if (!rc && !h->cols.dig) rc = wg::ozaki_cols_alloc(h->n / nr, 2 * nr, h->cols, h->err);
     if (rc) return rc;
   } else {
-    F2_CK(dalloc(&h->UHd, nu));
-    F2_CK(dalloc(&h->Usd, nu));
+    F2_CK(dalloc(&h->UHd, (size_t)nr * nr));
+    F2_CK(dalloc(&h->Usd, (size_t)nr * nr));
     F2_CK(cudaMemcpy(h->UHd, uh.data(), sizeof(double) * uh.size(), cudaMemcpyHostToDevice));
     F2_CK(cudaMemcpy(h->Usd, us.data(), sizeof(double) * us.size(), cudaMemcpyHostToDevice));
   }
@@ -2350,10 +2047,6 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
     F2_CK(dalloc(&h->cs, m));
     F2_CK(dalloc(&h->partial, (size_t)2 * kDotBlocks * (m + 1)));
     F2_CK(dalloc(&h->nrm, 1));
-    F2_CK(dalloc(&h->ktarget, 1));
-    F2_CK(dalloc(&h->kctl, 4));
-    F2_CK(cudaMemsetAsync(h->ktarget, 0, sizeof(double), h->stream));
-    F2_CK(cudaMemsetAsync(h->kctl, 0, 4 * sizeof(int), h->stream));
     h->vm = m + 1;
   }
   std::memset(info, 0, sizeof(*info));
@@ -2425,19 +2118,41 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
       F2_CK(cudaMemsetAsync(h->g, 0, sizeof(double2) * (m + 1), h->stream));
       F2_CK(cudaMemcpyAsync(h->g, &one, sizeof(double2), cudaMemcpyHostToDevice, h->stream));
       const double itgt = std::max(inner_tol, 0.5 * target / beta);
-      int k = 0;
+      int k = 0, j_cur = 0;
+      // the basis as the Gram-Schmidt kernels read it
+      auto gs_dots = [&](double2* out) {
+        if (b16) dots32(h, h->Vh32, j_cur + 1, h->w32, out, 0);
+        else dots32(h, h->V32, j_cur + 1, h->w32, out, 0);
+      };
+      auto gs_update = [&](const double2* coef) {
+        if (b16) f2d_gs_update32<<<blocks256(n), 256, 0, h->stream>>>(h->Vh32, n, h->w32, coef, j_cur + 1, n);
+        else f2d_gs_update32<<<blocks256(n), 256, 0, h->stream>>>(h->V32, n, h->w32, coef, j_cur + 1, n);
+      };
       for (int j = 0; j < mi; ++j) {
+        j_cur = j;
         // the preconditioner works on the basis vector as stored (its FP32 copy with an FP16 basis)
         const float2* Vj = b16 ? h->vj32 : h->V32 + (long long)j * n;
         float2* Zj = h->Z32 + (long long)j * n;
         precond_stages<float2>(h, h->UH32, h->Us32, h->xinv32, h->xcpl32, h->tinv32, Vj, h->pa32, h->pb32, Zj);
         rc = apply32(h, Zj, h->w32);
         if (rc) return rc;
-        const F2dKrylov kr{h->H, h->hc, h->cs, h->sn, h->g, h->nrm, h->ktarget, h->kctl, j, ldh};
-        if (b16 && n % 4 == 0) gram_schmidt32<true>(h, h->Vh32, h->w32, kr);
-        else if (b16) gram_schmidt32<false>(h, h->Vh32, h->w32, kr);
-        else if (n % 4 == 0) gram_schmidt32<true>(h, h->V32, h->w32, kr);
-        else gram_schmidt32<false>(h, h->V32, h->w32, kr);
+        gs_dots(h->hc);
+        gs_update(h->hc);
+        vnorm32(h, h->w32);
+        std::vector<double2> hh(j + 1);
+        double w1 = 0;
+        F2_CK(cudaMemcpyAsync(hh.data(), h->hc, sizeof(double2) * (j + 1), cudaMemcpyDeviceToHost, h->stream));
+        F2_CK(cudaMemcpyAsync(&w1, h->nrm, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        F2_CK(cudaStreamSynchronize(h->stream));
+        double h2 = 0;
+        for (const double2& c : hh) h2 += c.x * c.x + c.y * c.y;
+        if (w1 * w1 < 0.5 * (w1 * w1 + h2)) {
+          gs_dots(h->hp);
+          f2d_dot_reduce<<<j + 1, 256, 0, h->stream>>>(h->partial, h->hc, kDotBlocks, 1);
+          gs_update(h->hp);
+          vnorm32(h, h->w32);
+        }
+        f2d_givens<<<1, 1, 0, h->stream>>>(h->H, h->hc, h->nrm, h->cs, h->sn, h->g, j, ldh);
         if (b16)
           f2d_scale16<<<blocks256(n), 256, 0, h->stream>>>(h->w32, h->Vh32 + (long long)(j + 1) * n, h->vj32,
                                                            h->nrm, n);
@@ -2451,7 +2166,7 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
         h->resvec.push_back(beta * std::hypot(gj.x, gj.y));
         if (!(std::hypot(gj.x, gj.y) > itgt)) break;
       }
-      wg::backsolve_kernel<<<1, 32, 0, h->stream>>>(h->H, h->g, h->yc, nullptr, h->kctl + 1, ldh, k, 1);
+      f2d_backsolve<<<1, 1, 0, h->stream>>>(h->H, h->g, h->yc, k, ldh);
       F2_CK(cudaMemcpyAsync(h->nrm, &beta, sizeof(double), cudaMemcpyHostToDevice, h->stream));
       f2d_correct32<<<blocks256(n), 256, 0, h->stream>>>(h->xs, h->Z32, n, h->yc, k, h->nrm, n);
       info->cycles += 1;
@@ -2474,7 +2189,7 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
       if (rc) return rc;
       // classical Gram-Schmidt; a second pass only when the first lost more than half of |w|^2
       // (Daniel-Gragg-Kaufman-Stewart: |w'|^2 < eta^2 (|w'|^2 + |h|^2), eta = 1/sqrt(2))
-      dots(h, h->V, j + 1, h->w, h->hc);
+      dots(h, h->V, j + 1, h->w, h->hc, 0);
       f2d_gs_update<<<blocks256(n), 256, 0, h->stream>>>(h->V, n, h->w, h->hc, j + 1, n);
       vnorm(h, h->w);
       std::vector<double2> hh(j + 1);
@@ -2485,12 +2200,13 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
       double h2 = 0;
       for (const double2& c : hh) h2 += c.x * c.x + c.y * c.y;
       if (w1 * w1 < 0.5 * (w1 * w1 + h2)) {
-        dots(h, h->V, j + 1, h->w, h->hp, h->hc);    // second pass, hc += hp
+        dots(h, h->V, j + 1, h->w, h->hp, 0);    // second pass
+        f2d_dot_reduce<<<j + 1, 256, 0, h->stream>>>(h->partial, h->hc, kDotBlocks, 1);   // hc += hp
         f2d_gs_update<<<blocks256(n), 256, 0, h->stream>>>(h->V, n, h->w, h->hp, j + 1, n);
         vnorm(h, h->w);
         info_reorth += 1;
       }
-      f2d_givens<<<1, 32, 0, h->stream>>>({h->H, h->hc, h->cs, h->sn, h->g, h->nrm, h->ktarget, h->kctl, j, ldh});
+      f2d_givens<<<1, 1, 0, h->stream>>>(h->H, h->hc, h->nrm, h->cs, h->sn, h->g, j, ldh);
       f2d_scale<<<blocks256(n), 256, 0, h->stream>>>(h->w, h->V + (long long)(j + 1) * n, h->nrm, n);
       double2 gj;
       F2_CK(cudaMemcpyAsync(&gj, h->g + j + 1, sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
@@ -2501,7 +2217,7 @@ int wg2d_solve(wg2d_problem* h, const double* rhs, double* x, const wg2d_solve_o
       h->resvec.push_back(est);
       if (!(est > target)) break;
     }
-    wg::backsolve_kernel<<<1, 32, 0, h->stream>>>(h->H, h->g, h->yc, nullptr, h->kctl + 1, ldh, k, 1);
+    f2d_backsolve<<<1, 1, 0, h->stream>>>(h->H, h->g, h->yc, k, ldh);
     f2d_combine<<<blocks256(n), 256, 0, h->stream>>>(h->Zb, n, h->yc, h->z, k, n);   // x += Z y
     f2d_axpy<<<blocks256(n), 256, 0, h->stream>>>(h->xs, h->z, n);
     info->cycles += 1;
@@ -2566,7 +2282,7 @@ int wg2d_solve_bicgstab(wg2d_problem* h, const double* rhs, double* x, const wg2
   }
   const unsigned nb = blocks256(n);
   auto read_dot = [&](const double2* a, const double2* b, double2* out) -> int {
-    dots(h, a, 1, b, h->hc);
+    dots(h, a, 1, b, h->hc, 0);
     F2_CK(cudaMemcpyAsync(out, h->hc, sizeof(double2), cudaMemcpyDeviceToHost, h->stream));
     F2_CK(cudaStreamSynchronize(h->stream));
     return WG_OK;

@@ -1,5 +1,4 @@
-// Pieces of the Krylov solvers of the 1D (gmres.cu) and the Full-2D form (full2d.cu): basis loads, block
-// reductions, the Givens step and the back substitution.
+// Pieces of the Krylov solver (gmres.cu): basis loads, block reductions, the Givens step and the back substitution.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -21,10 +20,6 @@ template <> struct Quad<float2> {
     v = __ldg(reinterpret_cast<const float4*>(p) + 2 * n4 + 1);
   }
   __device__ __forceinline__ void zero() { u = v = make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ __forceinline__ void set(int i, float2 x) {
-    (i < 2 ? (i ? u.z : u.x) : (i == 3 ? v.z : v.x)) = x.x;
-    (i < 2 ? (i ? u.w : u.y) : (i == 3 ? v.w : v.y)) = x.y;
-  }
   __device__ __forceinline__ float2 get(int i) const {
     return i == 0 ? make_float2(u.x, u.y) : i == 1 ? make_float2(u.z, u.w)
                                                    : i == 2 ? make_float2(v.x, v.y) : make_float2(v.z, v.w);
@@ -36,9 +31,6 @@ template <> struct Quad<__half2> {
     u = __ldg(reinterpret_cast<const uint4*>(p) + n4);
   }
   __device__ __forceinline__ void zero() { u = make_uint4(0u, 0u, 0u, 0u); }
-  __device__ __forceinline__ void set(int i, __half2 x) {
-    (i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w) = *reinterpret_cast<const unsigned*>(&x);
-  }
   __device__ __forceinline__ float2 get(int i) const {
     const unsigned w = i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w;
     return __half22float2(*reinterpret_cast<const __half2*>(&w));

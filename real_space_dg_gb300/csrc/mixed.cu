@@ -94,7 +94,9 @@ void slice_rows_host(const std::vector<double>& A, int M, int K, std::vector<bf1
     e[r] = m + 1;
     for (int k = 0; k < K; ++k) {
       const double a = A[(size_t)r * K + k];
-      long long F = std::llrint(std::ldexp(std::fabs(a), bits * oz::S - 1 - m));
+      // 6 bits: |a| 2^(6S-1-m) < 2^47, adding one half is exact; 7 bits: up to 2^55, an integer from 2^52 on
+      const double scaled = std::ldexp(std::fabs(a), bits * oz::S - 1 - m);
+      long long F = bits == oz::BETA ? (long long)std::floor(scaled + 0.5) : std::llrint(scaled);
       if (a < 0) F = -F;
       for (int p = oz::S - 1; p > 0; --p) {
         const long long d = ((F + half) & digit) - half;
