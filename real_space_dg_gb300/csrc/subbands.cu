@@ -116,6 +116,48 @@ __device__ __forceinline__ int coarse_count(const float* a, const float* b2, int
   return c;
 }
 
+// 1 / x to rounding level: the hardware's approximation (rcp.approx.ftz.f64, about 20 bits) and one third-order
+// Newton step r (1 + e + e^2), e = 1 - x r (error e^3).
+__device__ __forceinline__ double fast_rcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+
+// Of eigenvalue kp > 0 and eigenvalue kn < 0 of T, whose magnitudes lie in (lo, hi): is |lambda_kn| the smaller?  FP64
+// counts at 16 magnitudes of either sign by the lanes of a warp, four rounds (the interval shrinks 17-fold in each); -1: not
+// settled.  a, b2: the slice's T in global memory.  A slice left to the bisection costs a chain of 500 us however
+// few there are; one round costs 15 us.
+__device__ int tie_smaller(const double* a, const double* b2, int n, int kp, int kn, double lo, double hi,
+                           double pivmin) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long pivbits = abs_bits(pivmin);
+  for (int round = 0; round < 4; ++round) {
+    const double step = (hi - lo) * (1.0 / 17.0), s = lo + ((lane >> 1) + 1) * step, x = lane & 1 ? -s : s;
+    double q = a[0] - x;
+    if (abs_bits(q) < pivbits) q = -pivmin;
+    int c = q < 0.0;
+    for (int i = 1; i < n; ++i) {
+      q = fma(-b2[i - 1], fast_rcp(q), a[i] - x);
+      if (abs_bits(q) < pivbits) q = -pivmin;
+      c += q < 0.0;
+    }
+    // inside: the eigenvalue's magnitude is below s
+    const unsigned in = __ballot_sync(0xffffffffu, lane & 1 ? c <= kn : c > kp);
+    const unsigned pos = in & 0x55555555u, neg = (in >> 1) & 0x55555555u;
+    const int fp = pos ? (__ffs(pos) - 1) / 2 : 16, fn = neg ? (__ffs(neg) - 1) / 2 : 16;
+    if (fp != fn) return fn < fp;
+    const double l = lo + fp * step;
+    hi = fp == 16 ? hi : l + step;
+    lo = l;
+  }
+  return -1;
+}
+
 // Shared memory of the coarse stage per warp: a, b^2 [ny] and up to 2 nm + 1 candidates.
 __host__ __device__ constexpr int coarse_floats(int ny) { return 2 * ny + 2 * kMaxModes + 2; }
 
@@ -126,7 +168,9 @@ constexpr float kCoarseTol = 1e-6f, kCoarseMargin = 2e-5f;
 __global__ void __launch_bounds__(128) subband_coarse_kernel(const double* __restrict__ me_y,
                                                              const double* __restrict__ pot, float t0, int nslice,
                                                              int nv, int nx, int ny, int nm, double* __restrict__ E,
-                                                             int* __restrict__ kfirst, FallbackList fb) {
+                                                             int* __restrict__ kfirst, double t0d, double* dplus,
+                                                             double* dminus, FallbackList fb) {
+  // dplus, dminus: the refinement's scratch, here T of a slice with a tie
   extern __shared__ float smf[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slice = blockIdx.x * (blockDim.x >> 5) + warp;   // slice = (problem * nv + v) * nx + x
@@ -203,12 +247,36 @@ __global__ void __launch_bounds__(128) subband_coarse_kernel(const double* __res
       if (hi < nc && (lo < 0 || fabsf(lam[hi]) <= fabsf(lam[lo]))) ++hi;
       else --lo;
     }
-    // the last one taken and the first one left out on the other side must not be a tie
+    // the last one taken and the first one left out on the other side: a tie in FP32 is settled by FP64 counts
     if (!bad) {
-      if (lo >= 0 && hi - 1 > lo && fabsf(lam[lo]) - fabsf(lam[hi - 1]) < 2 * kCoarseMargin * gnorm) bad = true;
-      if (hi < nc && lo + 1 < hi && fabsf(lam[hi]) - fabsf(lam[lo + 1]) < 2 * kCoarseMargin * gnorm &&
-          lam[lo + 1] < 0.f)
-        bad = true;
+      const float margin = 2 * kCoarseMargin * gnorm;
+      const bool low = lo >= 0 && hi - 1 > lo && lam[hi - 1] > 0.f && fabsf(lam[lo]) - lam[hi - 1] < margin;
+      const bool high = hi < nc && lo + 1 < hi && lam[lo + 1] < 0.f && fabsf(lam[hi]) - fabsf(lam[lo + 1]) < margin;
+      bad = low && high;
+      if (low != high) {
+        const int p = low ? hi - 1 : hi, n = low ? lo : lo + 1;   // the positive and the negative candidate
+        double* ta = dplus + (size_t)slice * ny * nm;
+        double* tb = dminus + (size_t)slice * ny * nm;
+        for (int i = lane; i < ny; i += 32) {
+          const int r = i == 0 ? 1 : (i == ny - 1 ? ny - 2 : i);
+          ta[i] = -(hop(t0d, m[r - 1], m[r]) + hop(t0d, m[r], m[r + 1])) + V[r];
+          tb[i] = i == ny - 1 ? 0.0
+                              : (i == 0 ? hop(t0d, m[1], m[2]) : hop(t0d, m[i], m[i + 1])) *
+                                    (i + 1 == ny - 1 ? hop(t0d, m[ny - 3], m[ny - 2]) : hop(t0d, m[i], m[i + 1]));
+        }
+        __syncwarp();
+        const float x = fminf(lam[p], -lam[n]), y = fmaxf(lam[p], -lam[n]);
+        const int neg = tie_smaller(ta, tb, ny, c0 + p, c0 + n, (double)fmaxf(x - margin, 0.f), (double)(y + margin),
+                                    1e-30 * (double)gnorm);
+        bad = neg < 0;
+        const int shift = low ? (neg == 1 ? -1 : 0) : (neg == 0 ? 1 : 0);
+        lo += shift;
+        hi += shift;
+        // the window moved past another candidate that close: left to the bisection
+        if (shift < 0 && lo >= 0 && hi - 1 > lo && lam[hi - 1] > 0.f && fabsf(lam[lo]) - lam[hi - 1] < margin) bad = true;
+        if (shift > 0 && hi < nc && lo + 1 < hi && lam[lo + 1] < 0.f && fabsf(lam[hi]) - fabsf(lam[lo + 1]) < margin)
+          bad = true;
+      }
       first = c0 + lo + 1;
       for (int k = lane; k < nm; k += 32) E[(size_t)slice * nm + k] = lam[lo + 1 + k];
     }
@@ -217,18 +285,6 @@ __global__ void __launch_bounds__(128) subband_coarse_kernel(const double* __res
     kfirst[slice] = bad ? -1 : first;
     if (bad) fb.add(slice);
   }
-}
-
-// 1 / x to rounding level: the hardware's approximation (rcp.approx.ftz.f64, about 20 bits) and one third-order
-// Newton step r (1 + e + e^2), e = 1 - x r (error e^3).
-__device__ __forceinline__ double fast_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-__device__ __forceinline__ unsigned long long abs_bits(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
 }
 
 // Shared memory of the refinement: per slice a, b^2, b [ny], and the slices a block of one warp takes (32 / nm
@@ -696,7 +752,7 @@ int wg_subbands_solve_device(wg_subbands* h, double dy_nm, const double* me_y, c
   const FallbackList fb{h->fallback, h->fallback + 1, h->fallback + 1 + slices};
   cudaMemsetAsync(h->fallback, 0, (1 + (size_t)slices) * sizeof(int), st);
   subband_coarse_kernel<<<(slices + 3) / 4, 128, 4 * coarse_floats(h->ny) * sizeof(float), st>>>(
-      me_y, V, (float)t0, slices, h->nv, h->nx, h->ny, h->nm, E, h->kfirst, fb);
+      me_y, V, (float)t0, slices, h->nv, h->nx, h->ny, h->nm, E, h->kfirst, t0, h->dp, h->dm, fb);
   const int sl = refine_slices(h->ny, h->nm);
   subband_refine_kernel<<<(slices + sl - 1) / sl, 32, sl * refine_doubles(h->ny) * sizeof(double), st>>>(
       me_y, V, t0, slices, h->nv, h->nx, h->ny, h->nm, sl, E, Vsub, h->dp, h->dm, h->kfirst, fb);

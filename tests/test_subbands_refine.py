@@ -91,3 +91,32 @@ def test_beyond_fp32(built_lib):
         w = np.linalg.eigvalsh(S.transversal_hamiltonian(me[0, ix], V[ix], 0.1))
         assert np.abs(E[0, ix] - w[:4]).max() <= 16 * 2.3e-16 * w[-1]
     assert np.all(np.isfinite(E))
+
+
+@pytest.mark.parametrize("nm,ny", [(1, 70), (2, 71), (5, 40), (8, 133)])
+def test_near_ties(built_lib, nm, ny):
+    """Magnitudes of opposite sign from 1e-3 to 1e-13 of the radius apart, either one the smaller: above the rounding
+    of the counts the kept set is that of the dense solve."""
+    dy = 0.1
+    base = _well(ny, 1, dy)[0] + 0.02 * np.random.default_rng(ny).normal(size=ny)
+    me1 = np.full(ny, 0.25)
+    w = np.linalg.eigvalsh(S.transversal_hamiltonian(me1, base, dy))
+    rad = w[-1] - w[0]
+    V, gaps = [], []
+    for g in (1e-3, 3e-5, 1e-5, 1e-6, 1e-7, 1e-8, 1e-9, 1e-10, 1e-11, 1e-13):
+        for s in (-1, 1):
+            for j in (2, 7):
+                # eigenvalues j and j + nm at -x and x + s g: the last of nm kept is one of the two
+                V.append(base - 0.5 * (w[j] + w[j + nm]) + 0.5 * s * g * rad)
+                gaps.append(g)
+    V = np.stack(V)
+    E, _ = _solve(np.tile(me1, (1, len(V), 1)), V, dy, nm)
+    for ix in range(len(V)):
+        u = np.linalg.eigvalsh(S.transversal_hamiltonian(me1, V[ix], dy))
+        r = np.abs(u).max()
+        keep = np.sort(u[np.argsort(np.abs(u))[:nm]])
+        tol = 64 * 2.3e-16 * r       # numpy's eigenvalues and the device's
+        if gaps[ix] * rad > 4 * tol:
+            assert np.abs(np.sort(E[0, ix]) - keep).max() <= tol, (ix, gaps[ix])
+        else:
+            assert np.abs(np.sort(np.abs(E[0, ix])) - np.sort(np.abs(keep))).max() <= tol + gaps[ix] * rad
