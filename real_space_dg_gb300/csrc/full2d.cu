@@ -73,12 +73,12 @@ struct wg2d_problem {
   double sigma = 1.0;
   int nT = 0;
   wg::OzakiRowsDev UH, Us;        // real embeddings of U^H and U / sigma (tensor-core path)
-  double2 *UHd = nullptr, *Usd = nullptr;   // the same as complex [nrx][nrx] row-major (FP64 path)
+  double2 *UHd = nullptr, *Usd = nullptr;   // the same as complex [nrx][nrx] row-major transposed (FP64 path)
   double2 *xinv = nullptr, *xcpl = nullptr; // [nrx][n_el_x][nk][nk]
-  double2* xmaps = nullptr;                  // chunk maps of the X-line sweep [chunk][nk*nk+nk][line]
-  int x_chunk_len = 0, x_chunks = 1;
+  double2* xmaps = nullptr;                  // chunk maps of the X-line sweep [mode][chunk][nk][nk]
+  int x_chunk_len = 0, x_chunks = 1, x_lines = 32;
   int* fwd = nullptr;             // [nrx]
-  double2* tinv = nullptr;        // [nrx][nT][nT]
+  double2* tinv = nullptr;        // [nrx][nT][nT], each transposed
   double2 *pa = nullptr, *pb = nullptr;     // [n] scratch of the preconditioner
   bool pre32 = false;             // the preconditioner in FP32 (its factors and scratch below)
   float2 *UH32 = nullptr, *Us32 = nullptr, *xinv32 = nullptr, *xcpl32 = nullptr, *tinv32 = nullptr;
@@ -437,255 +437,309 @@ __global__ void __launch_bounds__(128) f2d_dv_kernel(double* __restrict__ dV, co
                                             v_bilinear(gx, gy, V, nx, ny, X - hx, Y - hy, periodic);
 }
 
-// out[rx, col] = scale sum_j A[rx][j] G[j, col]  (dense complex A [nrx][nrx] row-major; FP64 modal transforms)
+// N consecutive values from shared memory in 16-byte loads
+template <int N>
+__device__ __forceinline__ void lds_row(double2 (&o)[N], const double2* p) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) o[i] = p[i];
+}
+template <int N>
+__device__ __forceinline__ void lds_row(float2 (&o)[N], const float2* p) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const float4 t = *reinterpret_cast<const float4*>(p + i);
+    o[i] = make_float2(t.x, t.y);
+    o[i + 1] = make_float2(t.z, t.w);
+  }
+}
+// One value to shared memory without a register in between (zero when !on); async_wait before the barrier.
 template <typename T>
-__global__ void __launch_bounds__(512) f2d_dense_rx_kernel(const T* __restrict__ A, const T* __restrict__ G,
-                                                           T* __restrict__ out, int nrx, long long ncols) {
+__device__ __forceinline__ void async_put(T* dst, const T* src, bool on) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = on ? (int)sizeof(T) : 0;
+  if constexpr (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+template <typename T> constexpr int kColPitch = sizeof(T) == 8 ? kRelxCols + 2 : kRelxCols + 1;   // 16-byte rows
+
+// out = A in over rho_x (dense complex nrx x nrx, given transposed: At[k][row]) for kRelxCols columns (rho_y, X, Y) a
+// block.  The states keep rho_x fastest; the modal fields of the preconditioner keep the column fastest (each mode's
+// lines together), so TO writes out[row][col] and !TO reads in[k][col].  Thread `row` reads At coalesced; the columns'
+// values are broadcast from shared memory.  Bound by the FP32 pipe (21 us of
+// sums) and the latency of At from the L1 and L2.  121 x 121 on 12,960 columns: 58 -> 45 us; two rows a thread: 67 us
+// (half the warps).  The sums run over k in order, as before.
+inline __host__ __device__ int modal_rows(int nrx) { return (nrx + 3) / 4 * 4; }
+template <typename T, bool TO>
+__global__ void __launch_bounds__(512) f2d_modal_kernel(const T* __restrict__ At, const T* __restrict__ in,
+                                                        T* __restrict__ out, int nrx, long long ncols) {
   extern __shared__ __align__(16) unsigned char sg_raw[];
-  T* sg = reinterpret_cast<T*>(sg_raw);   // [kRelxCols][nrx]
+  T* sg = reinterpret_cast<T*>(sg_raw);   // [modal_rows][kColPitch]
   const long long c0 = (long long)blockIdx.x * kRelxCols;
   const int nc = (int)min((long long)kRelxCols, ncols - c0);
+  const int kpad = modal_rows(nrx);
   for (int i = threadIdx.x; i < kRelxCols * nrx; i += blockDim.x) {
-    const int j = i / nrx, k = i - j * nrx;
-    sg[i] = j < nc ? G[(c0 + j) * nrx + k] : czero<T>();
+    const int j = TO ? i / nrx : i % kRelxCols, k = TO ? i - j * nrx : i / kRelxCols;
+    const bool on = j < nc;
+    async_put(sg + k * kColPitch<T> + j, TO ? in + (on ? (c0 + j) * nrx + k : 0) : in + (on ? k * ncols + c0 + j : 0), on);
   }
+  for (int i = nrx * kColPitch<T> + threadIdx.x; i < kpad * kColPitch<T>; i += blockDim.x) sg[i] = czero<T>();
+  const int row = min((int)threadIdx.x, nrx - 1);
+  // four rows of At ahead of the sums (zero rows past nrx)
+  const T* Ak = At + row;
+  T a[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) a[i] = Ak[(long long)i * nrx];
+  async_wait();
   __syncthreads();
-  const int rx = threadIdx.x;
-  if (rx >= nrx) return;
   T acc[kRelxCols];
 #pragma unroll
   for (int j = 0; j < kRelxCols; ++j) acc[j] = czero<T>();
-  const T* Ar = A + (long long)rx * nrx;
-  for (int k = 0; k < nrx; ++k) {
-    const T a = Ar[k];
+  for (int k = 0; k < kpad; k += 4) {
+    T n[4];
+    Ak += 4ll * nrx;
 #pragma unroll
-    for (int j = 0; j < kRelxCols; ++j) acc[j] = cfma(a, sg[j * nrx + k], acc[j]);
+    for (int i = 0; i < 4; ++i) n[i] = Ak[(long long)i * nrx];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      T v[kRelxCols];
+      lds_row(v, sg + (k + i) * kColPitch<T>);
+#pragma unroll
+      for (int j = 0; j < kRelxCols; ++j) acc[j] = cfma(a[i], v[j], acc[j]);
+      a[i] = n[i];
+    }
   }
+  if (threadIdx.x >= nrx) return;
+  if constexpr (TO) {
+    T* o = out + (long long)row * ncols + c0;
+    if (sizeof(T) == 8 && nc == kRelxCols && ncols % 2 == 0) {
 #pragma unroll
-  for (int j = 0; j < kRelxCols; ++j)
-    if (j < nc) out[(c0 + j) * nrx + rx] = acc[j];
+      for (int j = 0; j < kRelxCols; j += 2) {
+        const T u = acc[j], w = acc[j + 1];
+        *reinterpret_cast<float4*>(o + j) = make_float4((float)u.x, (float)u.y, (float)w.x, (float)w.y);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < kRelxCols; ++j)
+        if (j < nc) o[j] = acc[j];
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kRelxCols; ++j)
+      if (j < nc) out[(c0 + j) * nrx + row] = acc[j];
+  }
 }
 
 // X lines per mode (xFactors / applyInverse of get_LineTransversePreconditioner_full2D.m:177-222):
 // for mode k, transverse (ry, Y): sweep the X elements upwind (forward[k]: e = 0 .. ne-1), each
-// element's nk values: prev = inv[k][e] (w_e - cpl[k][e] prev).  Thread per (k, ry, Y), k fastest.
+// element's nk values: prev = inv[k][e] (w_e - cpl[k][e] prev).  The recurrence is affine in the incoming state, so
+// the elements are cut into chunks of L (sweep order), a chunk being prev_out = M prev_in + b with M a matter of the
+// mode alone (f2d_xline_maps_kernel, once per preconditioner).
+// f2d_xline_kernel: a block holds all chunks of LB lines; a thread (line, chunk) forms b, folds the maps of
+// the chunks upwind and sweeps its elements.  BYMODE: the fields are [mode][col] and the lines of a mode neighbours, so
+// the coefficients are one load a warp; otherwise rho_x (the mode) is fastest.
+// 60 elements of 3 on 8,712 lines, FP32: 80 us in two launches (maps per line, coefficients per thread) -> 22 us.
+// The same operations per element in the same order, so the same bits.
 template <int NK, typename T>
-__global__ void __launch_bounds__(128) f2d_xline_kernel(const T* __restrict__ W, T* __restrict__ out,
-                                                        const T* __restrict__ inv, const T* __restrict__ cpl,
-                                                        const int* __restrict__ fwd, int nrx, int nry, int nX, int nY,
-                                                        int ne) {
-  const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
-  const long long lines = (long long)nrx * nry * nY;
-  if (t >= lines) return;
-  const int k = (int)(t % nrx);
-  const long long q = t / nrx;
-  const int ry = (int)(q % nry);
-  const int Y = (int)(q / nry);
-  const long long nrel = (long long)nrx * nry;
-  const long long base = k + (long long)nrx * ry + nrel * (long long)nX * Y;
+__global__ void __launch_bounds__(128) f2d_xline_maps_kernel(T* __restrict__ maps, const T* __restrict__ inv,
+                                                             const T* __restrict__ cpl, const int* __restrict__ fwd,
+                                                             int nrx, int ne, int L, int nchunk) {
+  const int t = blockIdx.x * 128 + threadIdx.x;   // (mode, chunk, column of M)
+  if (t >= nrx * nchunk * NK) return;
+  const int j = t % NK, c = t / NK % nchunk, k = t / NK / nchunk;
+  T m[NK];
+#pragma unroll
+  for (int a = 0; a < NK; ++a) m[a] = a == j ? cone<T>() : czero<T>();
+  for (int i = c * L; i < min(ne, (c + 1) * L); ++i) {
+    const int e = fwd[k] ? i : ne - 1 - i;
+    const T* Ci = cpl + ((long long)k * ne + e) * NK * NK;
+    const T* Ii = inv + ((long long)k * ne + e) * NK * NK;
+    T v[NK];
+#pragma unroll
+    for (int a = 0; a < NK; ++a) {
+      T s = czero<T>();
+#pragma unroll
+      for (int b = 0; b < NK; ++b) s = cfma(Ci[a * NK + b], m[b], s);
+      v[a] = s;
+    }
+#pragma unroll
+    for (int a = 0; a < NK; ++a) {
+      T s = czero<T>();
+#pragma unroll
+      for (int b = 0; b < NK; ++b) s = cfma(Ii[a * NK + b], v[b], s);
+      m[a] = cneg(s);
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < NK; ++a) maps[(((long long)k * nchunk + c) * NK + a) * NK + j] = m[a];
+}
+
+// one element: prev <- inv (w - cpl prev)
+template <int NK, typename T>
+__device__ __forceinline__ void f2d_xline_step(T (&prev)[NK], const T (&w)[NK], const T* __restrict__ Ci,
+                                               const T* __restrict__ Ii) {
+  T v[NK];
+#pragma unroll
+  for (int a = 0; a < NK; ++a) {
+    v[a] = w[a];
+#pragma unroll
+    for (int b = 0; b < NK; ++b) {
+      const T c = Ci[a * NK + b];
+      v[a].x -= c.x * prev[b].x - c.y * prev[b].y;
+      v[a].y -= c.x * prev[b].y + c.y * prev[b].x;
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < NK; ++a) {
+    T s = czero<T>();
+#pragma unroll
+    for (int b = 0; b < NK; ++b) s = cfma(Ii[a * NK + b], v[b], s);
+    prev[a] = s;
+  }
+}
+
+constexpr int kXlineThreads = 512;
+template <int NK, typename T, bool BYMODE>
+__global__ void __launch_bounds__(kXlineThreads) f2d_xline_kernel(const T* __restrict__ W, T* __restrict__ out,
+                                                                  const T* __restrict__ maps,
+                                                                  const T* __restrict__ inv, const T* __restrict__ cpl,
+                                                                  const int* __restrict__ fwd, int nrx, int nry,
+                                                                  int nX, int nY, int ne, int L, int nchunk, int LB) {
+  extern __shared__ __align__(16) unsigned char xl_raw[];
+  T* bs = reinterpret_cast<T*>(xl_raw);   // [nchunk][NK][LB]
+  const int jl = threadIdx.x % LB, c = threadIdx.x / LB;
+  const long long line = (long long)blockIdx.x * LB + jl, lines = (long long)nrx * nry * nY;
+  const bool on = line < lines;
+  int k = 0;
+  long long base = 0, step = 0;
+  if (on) {
+    if (BYMODE) {
+      const int ry = (int)(line % nry);
+      const long long q = line / nry;
+      k = (int)(q / nY);
+      base = (long long)k * nry * nX * nY + ry + (long long)nry * nX * (q % nY);
+      step = nry;
+    } else {
+      k = (int)(line % nrx);
+      const long long q = line / nrx, nrel = (long long)nrx * nry;
+      base = k + nrx * (q % nry) + nrel * (long long)nX * (q / nry);
+      step = nrel;
+    }
+  }
   const bool f = fwd[k] != 0;
+  const int i0 = c * L, i1 = on ? min(ne, i0 + L) : i0;
   T prev[NK];
 #pragma unroll
   for (int a = 0; a < NK; ++a) prev[a] = czero<T>();
-  for (int i = 0; i < ne; ++i) {
-    const int e = f ? i : ne - 1 - i;
-    const T* Ci = cpl + ((long long)k * ne + e) * NK * NK;
-    const T* Ii = inv + ((long long)k * ne + e) * NK * NK;
-    T blk[NK];
+  if (nchunk > 1) {
+    if (c < nchunk - 1) {
+#pragma unroll 2
+      for (int i = i0; i < i1; ++i) {
+        const int e = f ? i : ne - 1 - i;
+        T w[NK];
 #pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T v = W[base + nrel * (e * NK + a)];
-#pragma unroll
-      for (int b = 0; b < NK; ++b) {
-        const T c = Ci[a * NK + b];
-        v.x -= c.x * prev[b].x - c.y * prev[b].y;
-        v.y -= c.x * prev[b].y + c.y * prev[b].x;
+        for (int a = 0; a < NK; ++a) w[a] = W[base + step * (e * NK + a)];
+        f2d_xline_step<NK, T>(prev, w, cpl + ((long long)k * ne + e) * NK * NK, inv + ((long long)k * ne + e) * NK * NK);
       }
-      blk[a] = v;
-    }
 #pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T v = czero<T>();
-#pragma unroll
-      for (int b = 0; b < NK; ++b) v = cfma(Ii[a * NK + b], blk[b], v);
-      prev[a] = v;
-      out[base + nrel * (e * NK + a)] = v;
+      for (int a = 0; a < NK; ++a) bs[(c * NK + a) * LB + jl] = prev[a];
     }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < NK; ++a) prev[a] = czero<T>();
+    for (int cc = 0; cc < c; ++cc) {
+      const T* M = maps + ((long long)k * nchunk + cc) * NK * NK;
+      T nxt[NK];
+#pragma unroll
+      for (int a = 0; a < NK; ++a) {
+        T s = bs[(cc * NK + a) * LB + jl];
+#pragma unroll
+        for (int j = 0; j < NK; ++j) s = cfma(M[a * NK + j], prev[j], s);
+        nxt[a] = s;
+      }
+#pragma unroll
+      for (int a = 0; a < NK; ++a) prev[a] = nxt[a];
+    }
+  }
+#pragma unroll 2
+  for (int i = i0; i < i1; ++i) {
+    const int e = f ? i : ne - 1 - i;
+    T w[NK];
+#pragma unroll
+    for (int a = 0; a < NK; ++a) w[a] = W[base + step * (e * NK + a)];
+    f2d_xline_step<NK, T>(prev, w, cpl + ((long long)k * ne + e) * NK * NK, inv + ((long long)k * ne + e) * NK * NK);
+#pragma unroll
+    for (int a = 0; a < NK; ++a) out[base + step * (e * NK + a)] = prev[a];
   }
 }
 
-// The same sweep cut into chunks of L elements (sweep order).  The element recurrence is affine in
-// the incoming state, prev_e = -Inv_e Cpl_e prev_{e-1} + Inv_e w_e, so a chunk composes to
-// prev_out = M prev_in + b:
-//   f2d_xline_maps_kernel   (line, chunk): M and b of the chunk from M = I, b = 0;
-//   f2d_xline_apply_kernel  (line, chunk): the incoming state folded from the maps of the chunks
-//                           upwind, then the chunk's elements swept as above, writing out.
-// Threads (line, chunk) with the line fastest; maps stored [chunk][entry][line].
-template <int NK, typename T>
-__global__ void __launch_bounds__(128) f2d_xline_maps_kernel(const T* __restrict__ W, T* __restrict__ maps,
-                                                             const T* __restrict__ inv, const T* __restrict__ cpl,
-                                                             const int* __restrict__ fwd, int nrx, int nry, int nX,
-                                                             int nY, int ne, int L, int nchunk) {
-  const long long lines = (long long)nrx * nry * nY;
-  const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
-  if (t >= lines * nchunk) return;
-  const long long line = t % lines;
-  const int c = (int)(t / lines);
-  const int k = (int)(line % nrx);
-  const long long q = line / nrx;
-  const int ry = (int)(q % nry);
-  const int Y = (int)(q / nry);
-  const long long nrel = (long long)nrx * nry;
-  const long long base = k + (long long)nrx * ry + nrel * (long long)nX * Y;
-  const bool f = fwd[k] != 0;
-  T M[NK][NK], b[NK];
-#pragma unroll
-  for (int a = 0; a < NK; ++a) {
-    b[a] = czero<T>();
-#pragma unroll
-    for (int j = 0; j < NK; ++j) M[a][j] = a == j ? cone<T>() : czero<T>();
-  }
-  const int i1 = min(ne, (c + 1) * L);
-  for (int i = c * L; i < i1; ++i) {
-    const int e = f ? i : ne - 1 - i;
-    const T* Ci = cpl + ((long long)k * ne + e) * NK * NK;
-    const T* Ii = inv + ((long long)k * ne + e) * NK * NK;
-    T CM[NK][NK], r[NK];
-#pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T v = W[base + nrel * (e * NK + a)];
-#pragma unroll
-      for (int j = 0; j < NK; ++j) {
-        T s = czero<T>();
-#pragma unroll
-        for (int m = 0; m < NK; ++m) s = cfma(Ci[a * NK + m], M[m][j], s);
-        CM[a][j] = s;
-      }
-#pragma unroll
-      for (int m = 0; m < NK; ++m) {
-        const T cc = Ci[a * NK + m];
-        v.x -= cc.x * b[m].x - cc.y * b[m].y;
-        v.y -= cc.x * b[m].y + cc.y * b[m].x;
-      }
-      r[a] = v;
-    }
-#pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T bb = czero<T>();
-#pragma unroll
-      for (int m = 0; m < NK; ++m) bb = cfma(Ii[a * NK + m], r[m], bb);
-      b[a] = bb;
-#pragma unroll
-      for (int j = 0; j < NK; ++j) {
-        T s = czero<T>();
-#pragma unroll
-        for (int m = 0; m < NK; ++m) s = cfma(Ii[a * NK + m], CM[m][j], s);
-        M[a][j] = cneg(s);
-      }
-    }
-  }
-  T* o = maps + (long long)c * (NK * NK + NK) * lines + line;
-#pragma unroll
-  for (int a = 0; a < NK; ++a) {
-#pragma unroll
-    for (int j = 0; j < NK; ++j) o[(long long)(a * NK + j) * lines] = M[a][j];
-    o[(long long)(NK * NK + a) * lines] = b[a];
-  }
-}
-
-template <int NK, typename T>
-__global__ void __launch_bounds__(128) f2d_xline_apply_kernel(const T* __restrict__ W, T* __restrict__ out,
-                                                              const T* __restrict__ maps, const T* __restrict__ inv,
-                                                              const T* __restrict__ cpl, const int* __restrict__ fwd,
-                                                              int nrx, int nry, int nX, int nY, int ne, int L,
-                                                              int nchunk) {
-  const long long lines = (long long)nrx * nry * nY;
-  const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
-  if (t >= lines * nchunk) return;
-  const long long line = t % lines;
-  const int c = (int)(t / lines);
-  const int k = (int)(line % nrx);
-  const long long q = line / nrx;
-  const int ry = (int)(q % nry);
-  const int Y = (int)(q / nry);
-  const long long nrel = (long long)nrx * nry;
-  const long long base = k + (long long)nrx * ry + nrel * (long long)nX * Y;
-  const bool f = fwd[k] != 0;
-  T prev[NK];
-#pragma unroll
-  for (int a = 0; a < NK; ++a) prev[a] = czero<T>();
-  for (int cc = 0; cc < c; ++cc) {
-    const T* o = maps + (long long)cc * (NK * NK + NK) * lines + line;
-    T nxt[NK];
-#pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T s = o[(long long)(NK * NK + a) * lines];
-#pragma unroll
-      for (int j = 0; j < NK; ++j) s = cfma(o[(long long)(a * NK + j) * lines], prev[j], s);
-      nxt[a] = s;
-    }
-#pragma unroll
-    for (int a = 0; a < NK; ++a) prev[a] = nxt[a];
-  }
-  const int i1 = min(ne, (c + 1) * L);
-  for (int i = c * L; i < i1; ++i) {
-    const int e = f ? i : ne - 1 - i;
-    const T* Ci = cpl + ((long long)k * ne + e) * NK * NK;
-    const T* Ii = inv + ((long long)k * ne + e) * NK * NK;
-    T blk[NK];
-#pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T v = W[base + nrel * (e * NK + a)];
-#pragma unroll
-      for (int m = 0; m < NK; ++m) {
-        const T cc2 = Ci[a * NK + m];
-        v.x -= cc2.x * prev[m].x - cc2.y * prev[m].y;
-        v.y -= cc2.x * prev[m].y + cc2.y * prev[m].x;
-      }
-      blk[a] = v;
-    }
-#pragma unroll
-    for (int a = 0; a < NK; ++a) {
-      T v = czero<T>();
-#pragma unroll
-      for (int m = 0; m < NK; ++m) v = cfma(Ii[a * NK + m], blk[m], v);
-      prev[a] = v;
-      out[base + nrel * (e * NK + a)] = v;
-    }
-  }
-}
-
-constexpr int kTxTile = 32;
 // transverse solve per mode k and X dof: v[k, t, X] <- Binv[k] v[k, :, X] over t = ry + nry Y.
-// Block (k, tile of kTxTile X dofs); Binv[k] and the tile staged in shared memory.
-template <typename T>
-__global__ void __launch_bounds__(256) f2d_transverse_kernel(const T* __restrict__ Vin, T* __restrict__ Vout,
-                                                             const T* __restrict__ Binv, int nrx, int nry,
-                                                             int nX, int nY, int nT) {
+// Block (tile of kTxTile X dofs, k; at most 152 rows t fit the shared memory); Binv[k] (given transposed: Bt[k][s][t]) and the tile staged in shared memory.  A
+// warp takes kTxRows rows t of the tile: per s one value of the tile and the rows' coefficients as broadcasts.
+// 72 x 72 for 121 modes on 180 dofs, FP32: 69 us (8 bytes of each 968 of the field, two shared loads per sum) -> 45 us;
+// 64 X dofs a block: 70 us (half the warps).
+constexpr int kTxTile = 32, kTxRows = 8, kTxPitch = kTxTile + 1;
+inline int tx_pitch(int nT) { return std::max(kTxRows, nT + (nT & 1)); }
+inline size_t tx_smem(int nT, size_t elem) { return elem * ((size_t)nT * tx_pitch(nT) + (size_t)nT * kTxPitch); }
+template <typename T, bool BYMODE>
+__global__ void __launch_bounds__(640) f2d_transverse_kernel(const T* __restrict__ Vin, T* __restrict__ Vout,
+                                                              const T* __restrict__ Bt, int nrx, int nry,
+                                                              int nX, int nY, int nT, int pitch) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  T* Bs = reinterpret_cast<T*>(sm_raw);   // [nT][nT] then [nT][kTxTile]
-  T* Ts = Bs + (long long)nT * nT;
+  T* Bs = reinterpret_cast<T*>(sm_raw);   // [nT][pitch] then [nT][kTxPitch]
+  T* Ts = Bs + (long long)nT * pitch;
   const int k = blockIdx.y;
   const int X0 = blockIdx.x * kTxTile;
   const int nx = min(kTxTile, nX - X0);
-  const long long nrel = (long long)nrx * nry;
-  const T* Bk = Binv + (long long)k * nT * nT;
-  for (int i = threadIdx.x; i < nT * nT; i += blockDim.x) Bs[i] = Bk[i];
-  for (int i = threadIdx.x; i < nT * kTxTile; i += blockDim.x) {
-    const int s = i / kTxTile, xx = i - s * kTxTile;
-    const int ry = s % nry, Y = s / nry;
-    Ts[i] = xx < nx ? Vin[k + (long long)nrx * ry + nrel * ((long long)(X0 + xx) + (long long)nX * Y)]
-                    : czero<T>();
+  const T* Bk = Bt + (long long)k * nT * nT;
+  for (int i = threadIdx.x; i < nT * pitch; i += blockDim.x) {
+    const int s = i / pitch, t = i - s * pitch;
+    async_put(Bs + i, Bk + (t < nT ? s * nT + t : 0), t < nT);
+  }
+  // field index of (t, xx) of the tile; i runs over the tile with the field's fastest index first
+  auto at = [&](int i, int& t, int& xx) -> long long {
+    if (BYMODE) {
+      const int ry = i % nry, q = i / nry, Y = q / nx;
+      xx = q - Y * nx;
+      t = ry + nry * Y;
+      return (long long)k * nry * nX * nY + ry + (long long)nry * (X0 + xx + (long long)nX * Y);
+    }
+    t = i / nx;
+    xx = i - t * nx;
+    const long long nrel = (long long)nrx * nry;
+    return k + (long long)nrx * (t % nry) + nrel * ((long long)(X0 + xx) + (long long)nX * (t / nry));
+  };
+  for (int i = threadIdx.x; i < nT * nx; i += blockDim.x) {
+    int t, xx;
+    const long long o = at(i, t, xx);
+    async_put(Ts + t * kTxPitch + xx, Vin + o, true);
+  }
+  async_wait();
+  __syncthreads();
+  const int lane = threadIdx.x & 31, t0 = min((int)(threadIdx.x >> 5) * kTxRows, pitch - kTxRows);
+  T acc[kTxRows];
+#pragma unroll
+  for (int r = 0; r < kTxRows; ++r) acc[r] = czero<T>();
+  if (lane < nx) {
+#pragma unroll 4
+    for (int s = 0; s < nT; ++s) {
+      const T v = Ts[s * kTxPitch + lane];
+      T b[kTxRows];
+      lds_row(b, Bs + (long long)s * pitch + t0);
+#pragma unroll
+      for (int r = 0; r < kTxRows; ++r) acc[r] = cfma(b[r], v, acc[r]);
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nT * kTxTile; i += blockDim.x) {
-    const int tt = i / kTxTile, xx = i - tt * kTxTile;
-    if (xx >= nx) continue;
-    T acc = czero<T>();
-    const T* Br = Bs + (long long)tt * nT;
-    for (int s2 = 0; s2 < nT; ++s2) acc = cfma(Br[s2], Ts[s2 * kTxTile + xx], acc);
-    const int ry = tt % nry, Y = tt / nry;
-    Vout[k + (long long)nrx * ry + nrel * ((long long)(X0 + xx) + (long long)nX * Y)] = acc;
+  if (lane < nx)
+#pragma unroll
+    for (int r = 0; r < kTxRows; ++r)
+      if (t0 + r < nT) Ts[(t0 + r) * kTxPitch + lane] = acc[r];   // rows of two warps: the same values
+  __syncthreads();
+  for (int i = threadIdx.x; i < nT * nx; i += blockDim.x) {
+    int t, xx;
+    const long long o = at(i, t, xx);
+    Vout[o] = Ts[t * kTxPitch + xx];
   }
 }
 
@@ -1590,48 +1644,72 @@ static unsigned blocks256(long long n) { return (unsigned)((n + 255) / 256); }
 // FP64 with the mode transforms on the tensor cores.
 }  // extern "C"
 
+template <int NK, typename T, bool BYMODE>
+static void xline_launch(wg2d_problem* h, const T* xinv, const T* xcpl, const T* in, T* out) {
+  const int C = h->x_chunks, LB = h->x_lines;
+  const long long lines = (long long)h->nrx * h->nry * h->nY;
+  f2d_xline_kernel<NK, T, BYMODE><<<(unsigned)((lines + LB - 1) / LB), LB * C, sizeof(T) * NK * LB * C, h->stream>>>(
+      in, out, reinterpret_cast<const T*>(h->xmaps), xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX, h->nY, h->s.n_el_x,
+      h->x_chunk_len, C, LB);
+}
+
+// z = M^-1 r.  With UH and Us (transposed) the modal fields lie by mode; without, the caller has transformed r into pa
+// and transforms pa back, rho_x fastest.
+template <typename T, bool BYMODE>
+static void precond_lines(wg2d_problem* h, const T* xinv, const T* xcpl, const T* tinv, T* pa, T* pb) {
+  switch (h->s.nk_x) {
+    case 2: xline_launch<2, T, BYMODE>(h, xinv, xcpl, pa, pb); break;
+    case 3: xline_launch<3, T, BYMODE>(h, xinv, xcpl, pa, pb); break;
+    default: xline_launch<4, T, BYMODE>(h, xinv, xcpl, pa, pb); break;
+  }
+  const dim3 tg((unsigned)((h->nX + kTxTile - 1) / kTxTile), (unsigned)h->nrx);
+  f2d_transverse_kernel<T, BYMODE><<<tg, 32 * ((h->nT + kTxRows - 1) / kTxRows), tx_smem(h->nT, sizeof(T)), h->stream>>>(
+      pb, pa, tinv, h->nrx, h->nry, h->nX, h->nY, h->nT, tx_pitch(h->nT));
+}
+
 template <typename T>
 static void precond_stages(wg2d_problem* h, const T* UH, const T* Us, const T* xinv, const T* xcpl, const T* tinv,
                            const T* r, T* pa, T* pb, T* z) {
+  if (!UH) {
+    precond_lines<T, false>(h, xinv, xcpl, tinv, pa, pb);
+    return;
+  }
   const long long ncols = h->n / h->nrx;
   const int threads = (h->nrx + 31) / 32 * 32;
-  const size_t smem = sizeof(T) * kRelxCols * h->nrx;
-  if (UH)
-    f2d_dense_rx_kernel<T><<<(unsigned)((ncols + kRelxCols - 1) / kRelxCols), threads, smem, h->stream>>>(
-        UH, r, pa, h->nrx, ncols);
-  const long long lines = (long long)h->nrx * h->nry * h->nY;
-  if (h->x_chunks > 1 && h->xmaps) {
-    T* maps = reinterpret_cast<T*>(h->xmaps);
-    const int L = h->x_chunk_len, C = h->x_chunks, ne = h->s.n_el_x;
-    const unsigned cb = (unsigned)((lines * C + 127) / 128);
-#define WG_XLINE_CHUNKED(NK_)                                                                                \
-  f2d_xline_maps_kernel<NK_, T><<<cb, 128, 0, h->stream>>>(pa, maps, xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX, \
-                                                          h->nY, ne, L, C);                                   \
-  f2d_xline_apply_kernel<NK_, T><<<cb, 128, 0, h->stream>>>(pa, pb, maps, xinv, xcpl, h->fwd, h->nrx, h->nry,  \
-                                                           h->nX, h->nY, ne, L, C);
-    switch (h->s.nk_x) {
-      case 2: WG_XLINE_CHUNKED(2) break;
-      case 3: WG_XLINE_CHUNKED(3) break;
-      default: WG_XLINE_CHUNKED(4) break;
-    }
-#undef WG_XLINE_CHUNKED
-  } else {
-    const unsigned lb = (unsigned)((lines + 127) / 128);
-    switch (h->s.nk_x) {
-      case 2: f2d_xline_kernel<2, T><<<lb, 128, 0, h->stream>>>(pa, pb, xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX,
-                                                               h->nY, h->s.n_el_x); break;
-      case 3: f2d_xline_kernel<3, T><<<lb, 128, 0, h->stream>>>(pa, pb, xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX,
-                                                               h->nY, h->s.n_el_x); break;
-      default: f2d_xline_kernel<4, T><<<lb, 128, 0, h->stream>>>(pa, pb, xinv, xcpl, h->fwd, h->nrx, h->nry, h->nX,
-                                                                h->nY, h->s.n_el_x); break;
-    }
+  const unsigned blocks = (unsigned)((ncols + kRelxCols - 1) / kRelxCols);
+  const size_t smem = sizeof(T) * kColPitch<T> * modal_rows(h->nrx);
+  f2d_modal_kernel<T, true><<<blocks, threads, smem, h->stream>>>(UH, r, pa, h->nrx, ncols);
+  precond_lines<T, true>(h, xinv, xcpl, tinv, pa, pb);
+  f2d_modal_kernel<T, false><<<blocks, threads, smem, h->stream>>>(Us, pa, z, h->nrx, ncols);
+}
+
+// Chunk maps of the X-line sweep for the factors just uploaded.
+template <typename T>
+static cudaError_t xline_maps(wg2d_problem* h, const T* xinv, const T* xcpl) {
+  if (h->x_chunks < 2) return cudaSuccess;
+  T* maps = reinterpret_cast<T*>(h->xmaps);
+  const int C = h->x_chunks, ne = h->s.n_el_x, nk = h->s.nk_x, L = h->x_chunk_len;
+  const unsigned blocks = (unsigned)(((size_t)h->nrx * C * nk + 127) / 128);
+  switch (nk) {
+    case 2: f2d_xline_maps_kernel<2, T><<<blocks, 128, 0, h->stream>>>(maps, xinv, xcpl, h->fwd, h->nrx, ne, L, C); break;
+    case 3: f2d_xline_maps_kernel<3, T><<<blocks, 128, 0, h->stream>>>(maps, xinv, xcpl, h->fwd, h->nrx, ne, L, C); break;
+    default: f2d_xline_maps_kernel<4, T><<<blocks, 128, 0, h->stream>>>(maps, xinv, xcpl, h->fwd, h->nrx, ne, L, C); break;
   }
-  const size_t tsm = sizeof(T) * ((size_t)h->nT * h->nT + (size_t)h->nT * kTxTile);
-  const dim3 tg((unsigned)((h->nX + kTxTile - 1) / kTxTile), (unsigned)h->nrx);
-  f2d_transverse_kernel<T><<<tg, 256, tsm, h->stream>>>(pb, pa, tinv, h->nrx, h->nry, h->nX, h->nY, h->nT);
-  if (Us)
-    f2d_dense_rx_kernel<T><<<(unsigned)((ncols + kRelxCols - 1) / kRelxCols), threads, smem, h->stream>>>(
-        Us, pa, z, h->nrx, ncols);
+  return cudaGetLastError();
+}
+
+// Shared memory of the preconditioner's kernels of one precision beyond the default limit.
+template <typename T>
+static cudaError_t precond_attributes(wg2d_problem* h) {
+  const int tsm = (int)tx_smem(h->nT, sizeof(T)), msm = (int)(sizeof(T) * kColPitch<T> * modal_rows(h->nrx));
+  cudaError_t e = cudaFuncSetAttribute(f2d_transverse_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(f2d_transverse_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
+  if (e == cudaSuccess && msm > 48 * 1024)
+    e = cudaFuncSetAttribute(f2d_modal_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, msm);
+  if (e == cudaSuccess && msm > 48 * 1024)
+    e = cudaFuncSetAttribute(f2d_modal_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, msm);
+  return e;
 }
 
 extern "C" {
@@ -1956,24 +2034,32 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
   // WG_XLINE_CHUNKS=<n> sets the chunk count, 0 or 1 keeps one sequential sweep per line
   {
     int C = ne >= 8 ? std::min(16, ne / 4) : 1;
-    if (const char* env = getenv("WG_XLINE_CHUNKS")) C = std::max(1, std::min(atoi(env), ne));
+    if (const char* env = getenv("WG_XLINE_CHUNKS")) C = std::max(1, std::min({atoi(env), ne, kXlineThreads / 4}));
     const int L = (ne + C - 1) / std::max(1, C);
     h->x_chunk_len = L;
     h->x_chunks = C > 1 ? (ne + L - 1) / L : 1;
-    if (h->x_chunks > 1)
-      F2_CK(dalloc(&h->xmaps, (size_t)h->x_chunks * (nk * nk + nk) * ((size_t)nr * h->nry * h->nY)));
+    // lines per block: 32 (one mode's coefficients a warp), fewer when the chunks fill the block
+    for (h->x_lines = 32; h->x_lines > 4 && h->x_lines * h->x_chunks > kXlineThreads;) h->x_lines /= 2;
+    if (h->x_chunks > 1) F2_CK(dalloc(&h->xmaps, (size_t)nr * h->x_chunks * nk * nk));
   }
   F2_CK(dalloc(&h->fwd, nr));
   F2_CK(cudaMemcpy(h->fwd, forward, sizeof(int) * nr, cudaMemcpyHostToDevice));
-  // U^H and U / sigma as complex [nr][nr] row-major
-  std::vector<double> uh((size_t)2 * nr * nr), us((size_t)2 * nr * nr);
+  // U^H and U / sigma as complex [nr][nr], transposed; the transverse inverses transposed per mode
+  const size_t nu = (size_t)nr * (modal_rows(nr) + 4);   // zero rows past nr
+  std::vector<double> uh(2 * nu, 0.0), us(2 * nu, 0.0), ti(2 * nt);
   for (int i = 0; i < nr; ++i)
     for (int j = 0; j < nr; ++j) {
-      uh[2 * ((size_t)i * nr + j)] = U[2 * ((size_t)j * nr + i)];
-      uh[2 * ((size_t)i * nr + j) + 1] = -U[2 * ((size_t)j * nr + i) + 1];
-      us[2 * ((size_t)i * nr + j)] = U[2 * ((size_t)i * nr + j)] / sigma;
-      us[2 * ((size_t)i * nr + j) + 1] = U[2 * ((size_t)i * nr + j) + 1] / sigma;
+      const size_t src = 2 * ((size_t)j * nr + i), dst = 2 * ((size_t)j * nr + i), tr = 2 * ((size_t)i * nr + j);
+      uh[dst] = U[src];          // (U^H)_ij = conj(U_ji), stored at [j][i]
+      uh[dst + 1] = -U[src + 1];
+      us[dst] = U[tr] / sigma;   // U_ij / sigma, stored at [j][i]
+      us[dst + 1] = U[tr + 1] / sigma;
     }
+  for (int k = 0; k < nr; ++k)
+    for (int t = 0; t < nT; ++t)
+      for (int q = 0; q < nT; ++q)
+        for (int c = 0; c < 2; ++c)
+          ti[2 * (((size_t)k * nT + q) * nT + t) + c] = t_inverse[2 * (((size_t)k * nT + t) * nT + q) + c];
   if (fp32) {
     auto up32 = [&](float2** dst, const double* src, size_t count) -> int {
       std::vector<float> f(2 * count);
@@ -1984,16 +2070,14 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
     };
     int rc = up32(&h->xinv32, x_inverse, nx);
     if (!rc) rc = up32(&h->xcpl32, x_coupling, nx);
-    if (!rc) rc = up32(&h->tinv32, t_inverse, nt);
-    if (!rc) rc = up32(&h->UH32, uh.data(), (size_t)nr * nr);
-    if (!rc) rc = up32(&h->Us32, us.data(), (size_t)nr * nr);
+    if (!rc) rc = up32(&h->tinv32, ti.data(), nt);
+    if (!rc) rc = up32(&h->UH32, uh.data(), nu);
+    if (!rc) rc = up32(&h->Us32, us.data(), nu);
     if (rc) return rc;
     F2_CK(dalloc(&h->pa32, h->n));
     F2_CK(dalloc(&h->pb32, h->n));
-    F2_CK(cudaFuncSetAttribute(f2d_transverse_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-    if (h->nrx * kRelxCols * sizeof(float2) > 48 * 1024)
-      F2_CK(cudaFuncSetAttribute(f2d_dense_rx_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(h->nrx * kRelxCols * sizeof(float2))));
+    F2_CK(precond_attributes<float2>(h));
+    F2_CK(xline_maps(h, h->xinv32, h->xcpl32));
     h->pre32 = true;
     h->pre_ready = true;
     return WG_OK;
@@ -2005,19 +2089,17 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
   F2_CK(dalloc(&h->pb, h->n));
   F2_CK(cudaMemcpy(h->xinv, x_inverse, sizeof(double2) * nx, cudaMemcpyHostToDevice));
   F2_CK(cudaMemcpy(h->xcpl, x_coupling, sizeof(double2) * nx, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(h->tinv, t_inverse, sizeof(double2) * nt, cudaMemcpyHostToDevice));
-  F2_CK(cudaFuncSetAttribute(f2d_transverse_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
-  if (h->nrx * kRelxCols * sizeof(double2) > 48 * 1024)
-    F2_CK(cudaFuncSetAttribute(f2d_dense_rx_kernel<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(h->nrx * kRelxCols * sizeof(double2))));
+  F2_CK(cudaMemcpy(h->tinv, ti.data(), sizeof(double2) * nt, cudaMemcpyHostToDevice));
+  F2_CK(precond_attributes<double2>(h));
+  F2_CK(xline_maps(h, h->xinv, h->xcpl));
   if (h->s.tensor_cores) {
     int rc = wg::ozaki_rows_upload(embed(U, nr, 1.0, true), 2 * nr, 2 * nr, h->UH, h->err);
     if (!rc) rc = wg::ozaki_rows_upload(embed(U, nr, 1.0 / sigma, false), 2 * nr, 2 * nr, h->Us, h->err);
     if (!rc && !h->cols.dig) rc = wg::ozaki_cols_alloc(h->n / nr, 2 * nr, h->cols, h->err);
     if (rc) return rc;
   } else {
-    F2_CK(dalloc(&h->UHd, (size_t)nr * nr));
-    F2_CK(dalloc(&h->Usd, (size_t)nr * nr));
+    F2_CK(dalloc(&h->UHd, nu));
+    F2_CK(dalloc(&h->Usd, nu));
     F2_CK(cudaMemcpy(h->UHd, uh.data(), sizeof(double) * uh.size(), cudaMemcpyHostToDevice));
     F2_CK(cudaMemcpy(h->Usd, us.data(), sizeof(double) * us.size(), cudaMemcpyHostToDevice));
   }
