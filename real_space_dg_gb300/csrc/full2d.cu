@@ -36,6 +36,18 @@
 #include "ozaki_api.h"
 #include "wigner_gb300.h"
 
+constexpr int kMaxTerms = 6;
+// The relative factors R_t of an axis with the k-th nonzeros of all rows together: entry (first[t] + k) rows + row,
+// k < count[t rows + row]; rows with fewer entries are padded and not read past their count.
+template <typename T>
+struct EllTerms {
+  int* col = nullptr;
+  T* val = nullptr;
+  int* count = nullptr;
+  int first[kMaxTerms] = {};
+  int total = 0;   // entries per row over all terms
+};
+
 struct wg2d_problem {
   wg2d_shape s{};
   int nX = 0, nY = 0, nrx = 0, nry = 0, nrel = 0, ncen = 0, nel = 0, nloc = 0, nq = 0, nvert = 0;
@@ -47,10 +59,9 @@ struct wg2d_problem {
     int T = 0;
     std::vector<double> coef;
     double* blocks = nullptr;   // [T][n_el][3][nk][nk]
-    int* rp = nullptr;          // [T][n_rho + 1]
-    int* col = nullptr;         // concatenated over the terms
-    double2* val = nullptr;
-    int* offs = nullptr;        // [T] start of term t in col / val
+    std::vector<int> rp, col;   // R_t as given: [T][n_rho + 1], columns over all terms
+    std::vector<double> val;    // (re, im) over all terms
+    EllTerms<double2> ell;
     double* dcoef = nullptr;    // [T]
     unsigned dense_mask = 0;    // terms applied by the emulated FP64 GEMM (rho_x axis)
     unsigned char* ymask = nullptr;   // rho_x axis: [T][nY] 1 where term t acts (closed X-face pieces); null: all
@@ -86,7 +97,7 @@ struct wg2d_problem {
   // FP32 copies of the operator for the mixed solve's inner iterations
   bool d32_ready = false;
   float *blocks32[2] = {nullptr, nullptr}, *coef32[2] = {nullptr, nullptr};
-  float2* val32[2] = {nullptr, nullptr};
+  EllTerms<float2> ell32[2];
   float *interp32 = nullptr, *proj32 = nullptr, *cap32 = nullptr, *dV32 = nullptr;
   float2 *Uq32 = nullptr, *Rq32 = nullptr, *G32 = nullptr;
   int vm32 = 0;
@@ -125,7 +136,6 @@ struct wg2d_problem {
 namespace {
 
 constexpr int kMaxNK = 4;
-constexpr int kMaxTerms = 6;
 constexpr int kRelxCols = 8;
 
 __device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {   // c + a b
@@ -193,22 +203,48 @@ __global__ void __launch_bounds__(256) f2d_center_kernel(const T* __restrict__ F
   }
 }
 
-// y[rx, col] += sum_t c_t sum_k val_t[k] G_t[col_t[k], col] for kRelxCols columns per block;
-// the G_t columns are staged in shared memory, thread rx owns row rx (blockDim = nrx rounded
-// up to a warp multiple, at most 512).
+// N consecutive values from shared memory in 16-byte loads
+template <int N>
+__device__ __forceinline__ void lds_row(double2 (&o)[N], const double2* p) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) o[i] = p[i];
+}
+template <int N>
+__device__ __forceinline__ void lds_row(float2 (&o)[N], const float2* p) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const float4 t = *reinterpret_cast<const float4*>(p + i);
+    o[i] = make_float2(t.x, t.y);
+    o[i + 1] = make_float2(t.z, t.w);
+  }
+}
+// One value to shared memory without a register in between (zero when !on); async_wait before the barrier.
+template <typename T>
+__device__ __forceinline__ void async_put(T* dst, const T* src, bool on) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = on ? (int)sizeof(T) : 0;
+  if constexpr (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+template <typename T> constexpr int kColPitch = sizeof(T) == 8 ? kRelxCols + 2 : kRelxCols + 1;   // 16-byte rows
+
+// y[rx, col] += sum_t c_t sum_k val_t[k] G_t[col_t[k], col] for kRelxCols columns per block; the G_t columns are staged in
+// shared memory, thread rx owns row rx (blockDim = nrx rounded up to a warp multiple, at most 512).  The k-th
+// nonzeros of all rows lie together (EllTerms), so a warp reads them coalesced and its staged rows, neighbours, as
+// broadcasts; the sums run over a row's nonzeros in order.  121 rows (2 and 121 entries), 12,960 columns, FP32: 100 -> 73 us
+// (96 us with the loads of an entry before its sums; 42 us would need the rounding-level half of |A| dropped).
 template <typename T, typename R>
-__global__ void __launch_bounds__(512) f2d_relx_kernel(const T* __restrict__ G, T* __restrict__ y,
-                                                       const int* __restrict__ rp, const int* __restrict__ col,
-                                                       const T* __restrict__ val, const int* __restrict__ nnz_off,
-                                                       const R* __restrict__ coef, int nterm, int nrx,
-                                                       long long ncols, long long n, unsigned skip_mask,
+__global__ void __launch_bounds__(512) f2d_relx_kernel(const T* __restrict__ G, T* __restrict__ y, EllTerms<T> E,
+                                                       const R* __restrict__ coef, int nterm, int nrx, long long ncols,
+                                                       long long n, unsigned skip_mask,
                                                        const unsigned char* __restrict__ ymask = nullptr,
                                                        long long cols_per_y = 1, int nY = 1) {
   extern __shared__ __align__(16) unsigned char sgr_raw[];
-  T* sg = reinterpret_cast<T*>(sgr_raw);   // [kRelxCols][nrx]
+  T* sg = reinterpret_cast<T*>(sgr_raw);   // [nrx][kColPitch]
   const long long c0 = (long long)blockIdx.x * kRelxCols;
   const int nc = (int)min((long long)kRelxCols, ncols - c0);
-  const int rx = threadIdx.x;
+  const int rx = min((int)threadIdx.x, nrx - 1);
   T acc[kRelxCols];
 #pragma unroll
   for (int j = 0; j < kRelxCols; ++j) acc[j] = czero<T>();
@@ -219,24 +255,47 @@ __global__ void __launch_bounds__(512) f2d_relx_kernel(const T* __restrict__ G, 
       const int j = i / nrx, k = i - j * nrx;
       // a masked term (a closed X-face piece) acts only on its own Y dofs
       const bool on = j < nc && (!ymask || ymask[(long long)t * nY + (c0 + j) / cols_per_y]);
-      sg[i] = on ? G[(long long)t * n + (c0 + j) * nrx + k] : czero<T>();
+      async_put(sg + k * kColPitch<T> + j, G + (long long)t * n + (on ? (c0 + j) * nrx + k : 0), on);
     }
+    async_wait();
     __syncthreads();
-    if (rx < nrx) {
-      const R ct = coef[t];
-      const int* rpt = rp + t * (nrx + 1);
-      const int off = nnz_off[t];
-      for (int k = rpt[rx]; k < rpt[rx + 1]; ++k) {
-        const int cidx = col[off + k];
-        T v = val[off + k];
-        v.x *= ct;
-        v.y *= ct;
+    const long long first = (long long)E.first[t] * nrx + rx;
+    const R ct = coef[t];
+    const int len = E.count[t * nrx + rx];
+    // four entries ahead of the sums
+    T vn[4];
+    int cn[4];
+    auto fetch = [&](int k) {
 #pragma unroll
-        for (int j = 0; j < kRelxCols; ++j) acc[j] = cfma(v, sg[j * nrx + cidx], acc[j]);
+      for (int i = 0; i < 4; ++i) {
+        const long long e = first + (long long)max(0, min(k + i, len - 1)) * nrx;
+        vn[i] = E.val[e];
+        cn[i] = E.col[e];
+      }
+    };
+    if (len > 0) fetch(0);
+    for (int k = 0; k < len; k += 4) {
+      T v[4];
+      int c[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[i] = vn[i];
+        c[i] = cn[i];
+      }
+      fetch(k + 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (k + i >= len) break;
+        T g[kRelxCols];
+        v[i].x *= ct;
+        v[i].y *= ct;
+        lds_row(g, sg + c[i] * kColPitch<T>);
+#pragma unroll
+        for (int j = 0; j < kRelxCols; ++j) acc[j] = cfma(v[i], g[j], acc[j]);
       }
     }
   }
-  if (rx >= nrx) return;
+  if (threadIdx.x >= nrx) return;
 #pragma unroll
   for (int j = 0; j < kRelxCols; ++j) {
     if (j < nc) {
@@ -247,32 +306,42 @@ __global__ void __launch_bounds__(512) f2d_relx_kernel(const T* __restrict__ G, 
   }
 }
 
-// y[rx, ry, c] += sum_t c_t sum_k val_t[k] G_t[rx, col_t[k], c]   (one thread per entry)
-template <typename T, typename R>
-__global__ void __launch_bounds__(256) f2d_rely_kernel(const T* __restrict__ G, T* __restrict__ y,
-                                                       const int* __restrict__ rp, const int* __restrict__ col,
-                                                       const T* __restrict__ val, const int* __restrict__ nnz_off,
+// y[rx, ry, c] += sum_t c_t sum_k val_t[k] G_t[rx, col_t[k], c]: one thread per entry, grid (centre dofs, ceil(nrel / 256)).
+// STAGED: the terms' entries of all rows in shared memory, so that the loads of G_t wait for no other load (and no
+// 64-bit division per thread).  12 rows (2 and 12 entries), 1.57 M unknowns, FP32: 43 -> 29 us.
+template <bool STAGED, typename T, typename R>
+__global__ void __launch_bounds__(256) f2d_rely_kernel(const T* __restrict__ G, T* __restrict__ y, EllTerms<T> E,
                                                        const R* __restrict__ coef, int nterm, int nrx, int nry,
-                                                       long long n) {
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n) return;
-  const int rx = (int)(i % nrx);
-  const long long q = i / nrx;
-  const int ry = (int)(q % nry);
-  const long long c = q / nry;
-  const long long cbase = c * (long long)nrx * nry + rx;
+                                                       long long n, int entries) {
+  extern __shared__ __align__(16) unsigned char rely_raw[];
+  T* sval = reinterpret_cast<T*>(rely_raw);   // [entries]
+  int* scol = reinterpret_cast<int*>(sval + entries);
+  if constexpr (STAGED) {
+    for (int i = threadIdx.x; i < entries; i += 256) {
+      sval[i] = E.val[i];
+      scol[i] = E.col[i] * nrx;
+    }
+    __syncthreads();
+  }
+  const int i = blockIdx.y * 256 + threadIdx.x;
+  if (i >= nrx * nry) return;
+  const int ry = i / nrx, rx = i - ry * nrx;
+  const long long cbase = (long long)blockIdx.x * nrx * nry;
   T acc = czero<T>();
   for (int t = 0; t < nterm; ++t) {
-    const int* rpt = rp + t * (nry + 1);
-    const int off = nnz_off[t];
+    const T* g = G + (long long)t * n + cbase + rx;
+    const int f = E.first[t] * nry + ry, len = E.count[t * nry + ry];
     T s = czero<T>();
-    for (int k = rpt[ry]; k < rpt[ry + 1]; ++k)
-      s = cfma(val[off + k], G[(long long)t * n + cbase + (long long)col[off + k] * nrx], s);
+#pragma unroll 6
+    for (int k = 0; k < len; ++k)
+      s = cfma(STAGED ? sval[f + k * nry] : E.val[f + k * nry],
+               g[STAGED ? (long long)scol[f + k * nry] : (long long)E.col[f + k * nry] * nrx], s);
     acc.x = fma(coef[t], s.x, acc.x);
     acc.y = fma(coef[t], s.y, acc.y);
   }
-  y[i].x += acc.x;
-  y[i].y += acc.y;
+  T* o = y + cbase + i;
+  o->x += acc.x;
+  o->y += acc.y;
 }
 
 // centre dof of local node l of element e (local order X fastest, elements X fastest)
@@ -436,32 +505,6 @@ __global__ void __launch_bounds__(128) f2d_dv_kernel(double* __restrict__ dV, co
   dV[((long long)e * nq + q) * nvert + v] = v_bilinear(gx, gy, V, nx, ny, X + hx, Y + hy, periodic) -
                                             v_bilinear(gx, gy, V, nx, ny, X - hx, Y - hy, periodic);
 }
-
-// N consecutive values from shared memory in 16-byte loads
-template <int N>
-__device__ __forceinline__ void lds_row(double2 (&o)[N], const double2* p) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) o[i] = p[i];
-}
-template <int N>
-__device__ __forceinline__ void lds_row(float2 (&o)[N], const float2* p) {
-#pragma unroll
-  for (int i = 0; i < N; i += 2) {
-    const float4 t = *reinterpret_cast<const float4*>(p + i);
-    o[i] = make_float2(t.x, t.y);
-    o[i + 1] = make_float2(t.z, t.w);
-  }
-}
-// One value to shared memory without a register in between (zero when !on); async_wait before the barrier.
-template <typename T>
-__device__ __forceinline__ void async_put(T* dst, const T* src, bool on) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = on ? (int)sizeof(T) : 0;
-  if constexpr (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-template <typename T> constexpr int kColPitch = sizeof(T) == 8 ? kRelxCols + 2 : kRelxCols + 1;   // 16-byte rows
 
 // out = A in over rho_x (dense complex nrx x nrx, given transposed: At[k][row]) for kRelxCols columns (rho_y, X, Y) a
 // block.  The states keep rho_x fastest; the modal fields of the preconditioner keep the column fastest (each mode's
@@ -1194,13 +1237,52 @@ cudaError_t dalloc(T** p, size_t n) {
   return cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * (n ? n : 1));
 }
 
+template <typename T>
+void free_ell(EllTerms<T>& e) {
+  cudaFree(e.col);
+  cudaFree(e.val);
+  cudaFree(e.count);
+  e = EllTerms<T>{};
+}
+
+// The terms of an axis of nr rows for the device.
+template <typename T, typename R>
+cudaError_t ell_upload(const wg2d_problem::Axis& a, int nr, EllTerms<T>& out) {
+  free_ell(out);
+  std::vector<int> col, count((size_t)a.T * nr);
+  std::vector<T> val;
+  int off = 0;
+  for (int t = 0; t < a.T; ++t) {
+    const int* rp = a.rp.data() + (size_t)t * (nr + 1);
+    int len = 0;
+    for (int i = 0; i < nr; ++i) len = std::max(len, count[(size_t)t * nr + i] = rp[i + 1] - rp[i]);
+    out.first[t] = out.total;
+    out.total += len;
+    for (int k = 0; k < len; ++k)
+      for (int i = 0; i < nr; ++i) {
+        const bool in = k < rp[i + 1] - rp[i];
+        const int e = in ? off + rp[i] + k : 0;
+        T v;
+        v.x = in ? (R)a.val[2 * e] : R(0);
+        v.y = in ? (R)a.val[2 * e + 1] : R(0);
+        col.push_back(in ? a.col[e] : 0);
+        val.push_back(v);
+      }
+    off += rp[nr];
+  }
+  cudaError_t e = dalloc(&out.col, col.size());
+  if (e == cudaSuccess) e = dalloc(&out.val, val.size());
+  if (e == cudaSuccess) e = dalloc(&out.count, count.size());
+  if (e == cudaSuccess) e = cudaMemcpy(out.col, col.data(), sizeof(int) * col.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(out.val, val.data(), sizeof(T) * val.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(out.count, count.data(), sizeof(int) * count.size(), cudaMemcpyHostToDevice);
+  return e;
+}
+
 void free_axis(wg2d_problem::Axis& a) {
   for (wg::OzakiRowsDev& d : a.dense) wg::ozaki_free(d);
   cudaFree(a.blocks);
-  cudaFree(a.rp);
-  cudaFree(a.col);
-  cudaFree(a.val);
-  cudaFree(a.offs);
+  free_ell(a.ell);
   cudaFree(a.dcoef);
   cudaFree(a.ymask);
   a = wg2d_problem::Axis{};
@@ -1210,7 +1292,7 @@ void free_axis(wg2d_problem::Axis& a) {
 template <typename T, typename R>
 struct OpData {
   const R* blocks[2];
-  const T* val[2];
+  EllTerms<T> ell[2];
   const R* coef[2];
   const R *interp, *proj, *cap, *dV;
   T *Uq, *Rq, *G;
@@ -1240,15 +1322,21 @@ void transport_terms(wg2d_problem* h, int axis, const OpData<T, R>& d, const T* 
   }
   if (axis == 0) {
     const long long ncols = h->n / h->nrx;
-    const size_t smem = sizeof(T) * kRelxCols * h->nrx;
+    const size_t smem = sizeof(T) * kColPitch<T> * h->nrx;
     const int threads = (h->nrx + 31) / 32 * 32;
     if (skip_mask != (1u << a.T) - 1u)
       f2d_relx_kernel<T, R><<<(unsigned)((ncols + kRelxCols - 1) / kRelxCols), threads, smem, h->stream>>>(
-          d.G, y, a.rp, a.col, d.val[0], a.offs, d.coef[0], a.T, h->nrx, ncols, h->n, skip_mask, a.ymask,
+          d.G, y, d.ell[0], d.coef[0], a.T, h->nrx, ncols, h->n, skip_mask, a.ymask,
           (long long)h->nry * h->nX, h->nY);
   } else {
-    f2d_rely_kernel<T, R><<<(unsigned)((h->n + 255) / 256), 256, 0, h->stream>>>(d.G, y, a.rp, a.col, d.val[1], a.offs,
-                                                                                d.coef[1], a.T, h->nrx, h->nry, h->n);
+    const int entries = d.ell[1].total * h->nry;
+    const size_t smem = entries * (sizeof(T) + sizeof(int));
+    const dim3 grid((unsigned)h->ncen, (unsigned)((h->nrel + 255) / 256));
+    if (smem <= 12 * 1024)   // eight blocks' tables on an SM
+      f2d_rely_kernel<true, T, R><<<grid, 256, smem, h->stream>>>(d.G, y, d.ell[1], d.coef[1], a.T, h->nrx, h->nry, h->n,
+                                                                  entries);
+    else
+      f2d_rely_kernel<false, T, R><<<grid, 256, 0, h->stream>>>(d.G, y, d.ell[1], d.coef[1], a.T, h->nrx, h->nry, h->n, 0);
   }
 }
 
@@ -1256,7 +1344,7 @@ OpData<double2, double> op64(wg2d_problem* h) {
   OpData<double2, double> d;
   for (int a = 0; a < 2; ++a) {
     d.blocks[a] = h->ax[a].blocks;
-    d.val[a] = h->ax[a].val;
+    d.ell[a] = h->ax[a].ell;
     d.coef[a] = h->ax[a].dcoef;
   }
   d.interp = h->interp;
@@ -1425,9 +1513,9 @@ int wg2d_create(const wg2d_shape* s, wg2d_problem** out) {
   if (e == cudaSuccess) e = cudaMemset(h->tc_err, 0, sizeof(int));
   for (cudaEvent_t& ev : h->ev)
     if (e == cudaSuccess) e = cudaEventCreate(&ev);
-  if (e == cudaSuccess && h->nrx * kRelxCols * sizeof(double2) > 48 * 1024)
+  if (e == cudaSuccess && h->nrx * kColPitch<double2> * sizeof(double2) > 48 * 1024)
     e = cudaFuncSetAttribute(f2d_relx_kernel<double2, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(h->nrx * kRelxCols * sizeof(double2)));
+                             (int)(h->nrx * kColPitch<double2> * sizeof(double2)));
   if (e != cudaSuccess) {
     wg2d_destroy(h);
     return e == cudaErrorMemoryAllocation ? WG_ERR_OOM : WG_ERR_CUDA;
@@ -1483,20 +1571,15 @@ int wg2d_set_transport(wg2d_problem* h, int axis, int n_terms, const double* coe
   a.T = n_terms;
   a.coef.assign(coef, coef + n_terms);
   if (n_terms == 0) return WG_OK;
-  const int nrp = n_terms * (nr + 1);
   const size_t nb = (size_t)n_terms * n_el * 3 * nk * nk;
   F2_CK(dalloc(&a.blocks, nb));
-  F2_CK(dalloc(&a.rp, nrp));
-  F2_CK(dalloc(&a.col, off[n_terms]));
-  F2_CK(dalloc(&a.val, off[n_terms]));
-  F2_CK(dalloc(&a.offs, n_terms));
   F2_CK(dalloc(&a.dcoef, n_terms));
   F2_CK(cudaMemcpy(a.blocks, center_blocks, sizeof(double) * nb, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(a.rp, row_ptr, sizeof(int) * nrp, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(a.offs, off.data(), sizeof(int) * n_terms, cudaMemcpyHostToDevice));
   F2_CK(cudaMemcpy(a.dcoef, coef, sizeof(double) * n_terms, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(a.col, col, sizeof(int) * std::max(1, off[n_terms]), cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(a.val, val, sizeof(double2) * std::max(1, off[n_terms]), cudaMemcpyHostToDevice));
+  a.rp.assign(row_ptr, row_ptr + (size_t)n_terms * (nr + 1));
+  a.col.assign(col, col + off[n_terms]);
+  a.val.assign(val, val + 2 * (size_t)off[n_terms]);
+  F2_CK((ell_upload<double2, double>(a, nr, a.ell)));
   // dense rho_x factors on the tensor cores: the real embedding of c_t R_t, digit-sliced once
   a.dense.assign(n_terms, wg::OzakiRowsDev{});
   a.dense_mask = 0;
@@ -1894,12 +1977,12 @@ int wg2d_apply_repeat(wg2d_problem* h, int n, double* ms, double* parts_ms) {
 
 
 static void free32(wg2d_problem* h) {
-  void* ptrs[] = {h->blocks32[0], h->blocks32[1], h->coef32[0], h->coef32[1], h->val32[0], h->val32[1], h->interp32,
+  for (EllTerms<float2>& e : h->ell32) free_ell(e);
+  void* ptrs[] = {h->blocks32[0], h->blocks32[1], h->coef32[0], h->coef32[1], h->interp32,
                   h->proj32, h->cap32, h->dV32, h->Uq32, h->Rq32, h->G32, h->V32, h->Z32, h->w32, h->Vh32, h->vj32};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   h->blocks32[0] = h->blocks32[1] = h->coef32[0] = h->coef32[1] = nullptr;
-  h->val32[0] = h->val32[1] = nullptr;
   h->interp32 = h->proj32 = h->cap32 = h->dV32 = nullptr;
   h->Uq32 = h->Rq32 = h->G32 = h->V32 = h->Z32 = h->w32 = h->vj32 = nullptr;
   h->Vh32 = nullptr;
@@ -1932,14 +2015,10 @@ static int ensure32(wg2d_problem* h) {
     if (!ax.T) continue;
     const int nk = a == 0 ? h->s.nk_x : h->s.nk_y, ne = a == 0 ? h->s.n_el_x : h->s.n_el_y;
     const int nr = a == 0 ? h->nrx : h->nry;
-    int nnz = 0;
-    std::vector<int> rp((size_t)ax.T * (nr + 1));
-    F2_CK(cudaMemcpy(rp.data(), ax.rp, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost));
-    for (int t = 0; t < ax.T; ++t) nnz += rp[(size_t)t * (nr + 1) + nr];
     int rc = conv(&h->blocks32[a], ax.blocks, (long long)ax.T * ne * 3 * nk * nk);
     if (!rc) rc = conv(&h->coef32[a], ax.dcoef, ax.T);
-    if (!rc) rc = conv(reinterpret_cast<float**>(&h->val32[a]), reinterpret_cast<const double*>(ax.val), 2LL * nnz);
     if (rc) return rc;
+    F2_CK((ell_upload<float2, float>(ax, nr, h->ell32[a])));
   }
   const long long slab = (long long)h->nel * h->nq;
   int rc = conv(&h->interp32, h->interp, (long long)h->nq * h->nloc);
@@ -1950,9 +2029,9 @@ static int ensure32(wg2d_problem* h) {
   F2_CK(dalloc(&h->Uq32, slab * h->nrel));
   F2_CK(dalloc(&h->Rq32, slab * h->nrel));
   F2_CK(dalloc(&h->G32, (size_t)std::max(1, std::max(h->ax[0].T, h->ax[1].T)) * h->n));
-  if (h->nrx * kRelxCols * sizeof(float2) > 48 * 1024)
+  if (h->nrx * kColPitch<float2> * sizeof(float2) > 48 * 1024)
     F2_CK(cudaFuncSetAttribute(f2d_relx_kernel<float2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(h->nrx * kRelxCols * sizeof(float2))));
+                               (int)(h->nrx * kColPitch<float2> * sizeof(float2))));
   F2_CK(cudaStreamSynchronize(h->stream));
   h->d32_ready = true;
   return WG_OK;
@@ -1964,7 +2043,7 @@ OpData<float2, float> op32(wg2d_problem* h) {
   OpData<float2, float> d;
   for (int a = 0; a < 2; ++a) {
     d.blocks[a] = h->blocks32[a];
-    d.val[a] = h->val32[a];
+    d.ell[a] = h->ell32[a];
     d.coef[a] = h->coef32[a];
   }
   d.interp = h->interp32;
