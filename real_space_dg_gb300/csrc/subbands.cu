@@ -215,7 +215,9 @@ __global__ void __launch_bounds__(128) subband_coarse_kernel(const double* __res
     const int cz = lane < 2 ? coarse_count(a, b2, ny, lane == 0 ? -zero : zero, pivmin) : 0;
     const int na = __shfl_sync(0xffffffffu, cz, 0), nb = __shfl_sync(0xffffffffu, cz, 1);
     const int c0 = max(0, na - nm), c1 = min(ny, nb + nm), nc = c1 - c0;
-    bad = nb - na > 1;
+    // more candidates than the window holds (a potential far above the other levels leaves all of them within the
+    // band around 0): nothing is located, the slice goes to the bisection
+    bad = nb - na != 0 && nb - na != 1;
     for (int cb = 0; cb < nc && !bad; cb += 32) {
       const int n = min(32, nc - cb), g = 32 / n, c = lane / g, j = lane % g;
       const bool mine = c < n;
@@ -239,16 +241,16 @@ __global__ void __launch_bounds__(128) subband_coarse_kernel(const double* __res
       if (mine && j == 0) lam[cb + c] = 0.5f * (lo + hi);
     }
     __syncwarp();
-    // the nm of smallest magnitude: grow a window outwards from the sign change
-    int lo = -1, hi = 0;
-    while (hi < nc && lam[hi] < 0.f) ++hi;
-    lo = hi - 1;
-    for (int t = 0; t < nm && !bad; ++t) {
-      if (hi < nc && (lo < 0 || fabsf(lam[hi]) <= fabsf(lam[lo]))) ++hi;
-      else --lo;
-    }
-    // the last one taken and the first one left out on the other side: a tie in FP32 is settled by FP64 counts
     if (!bad) {
+      // the nm of smallest magnitude: grow a window outwards from the sign change
+      int lo = -1, hi = 0;
+      while (hi < nc && lam[hi] < 0.f) ++hi;
+      lo = hi - 1;
+      for (int t = 0; t < nm; ++t) {
+        if (hi < nc && (lo < 0 || fabsf(lam[hi]) <= fabsf(lam[lo]))) ++hi;
+        else --lo;
+      }
+      // the last one taken and the first one left out on the other side: a tie in FP32 is settled by FP64 counts
       const float margin = 2 * kCoarseMargin * gnorm;
       const bool low = lo >= 0 && hi - 1 > lo && lam[hi - 1] > 0.f && fabsf(lam[lo]) - lam[hi - 1] < margin;
       const bool high = hi < nc && lo + 1 < hi && lam[lo + 1] < 0.f && fabsf(lam[hi]) - fabsf(lam[lo + 1]) < margin;

@@ -120,3 +120,19 @@ def test_near_ties(built_lib, nm, ny):
             assert np.abs(np.sort(E[0, ix]) - keep).max() <= tol, (ix, gaps[ix])
         else:
             assert np.abs(np.sort(np.abs(E[0, ix])) - np.sort(np.abs(keep))).max() <= tol + gaps[ix] * rad
+
+
+@pytest.mark.parametrize("ny,nm,wall", [(300, 32, 1e6), (300, 32, 1e7), (64, 4, 1e7), (300, 32, 1e12), (1024, 8, 1e8)])
+def test_wall_above_the_band(built_lib, ny, nm, wall):
+    """One row so far above the other levels that most or all of them lie within the counts' uncertainty around 0 (4e-6
+    of the radius), up to ny candidates for 2 nm + 1 places: such slices go to the bisection.  The last row has no
+    wall; both against the dense solve."""
+    dy = 0.1
+    V = _well(ny, 2, dy)
+    V[0, ny // 3] = wall
+    E, Vs = _solve(np.full((1, 2, ny), 0.3), V, dy, nm)
+    for ix in range(2):
+        w = np.linalg.eigvalsh(S.transversal_hamiltonian(np.full(ny, 0.3), V[ix], dy))
+        want = np.sort(np.sort(np.abs(w))[:nm])
+        assert np.abs(np.sort(np.abs(E[0, ix])) - want).max() <= 16 * 2.3e-16 * np.abs(w).max()
+    assert np.all(np.isfinite(Vs))
