@@ -111,8 +111,11 @@ __device__ __forceinline__ void tmem_ld8x2(uint32_t t0, uint32_t t1, float (&v)[
   }
 }
 
+constexpr int kZeroExp = -4000;    // exponent of a row or column of zeros: it never sets the common unit
+constexpr int kNanExp = 1 << 20;   // of a column with an infinity or NaN: it always does, and its results are NaN
+
 // a * 2^e as the nearest double (ties to even), integer instructions only, no branch (lanes take every side of one);
-// results below the normal range flush to zero.
+// results below the normal range flush to zero, those of a column with kNanExp are NaN.
 __device__ __forceinline__ double fixed_to_double(long long a, int e) {
   const unsigned long long sign = (unsigned long long)a & (1ull << 63);
   unsigned long long u = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
@@ -124,6 +127,7 @@ __device__ __forceinline__ double fixed_to_double(long long a, int e) {
   unsigned long long bits = ((unsigned long long)(unsigned)(ex - 1) << 52) + mant;
   bits = ex >= 0x7FF || bits >= (0x7FFull << 52) ? 0x7FFull << 52 : bits;
   bits = ex <= 0 || a == 0 ? 0ull : bits;
+  bits = e >= kNanExp / 2 ? 0x7FF8ull << 48 : bits;
   return __longlong_as_double((long long)(sign | bits));
 }
 
@@ -358,7 +362,6 @@ __device__ __forceinline__ void pair_align(long long& a, int& ea, long long& b, 
   b = (b + ((1ll << sb) >> 1)) >> sb;
   ea = max(ea, eb);
 }
-constexpr int kZeroExp = -4000;   // exponent of a row or column of zeros: it never sets the common unit
 
 // The pair of results of one node from A and B (units 2^(ea + xa), 2^(eb + xb)), as integers of a common unit with one
 // conversion per result: the FP64 additions of the pairs cost 64 cycles of an SM quarter each.  Not inlined: eight copies
@@ -589,16 +592,17 @@ __global__ void __launch_bounds__(128 * kSlicePairNodes) slice_pairs_kernel(
     mx = t > mx ? t : mx;
   }
   const int m = mx == 0 ? 0 : (int)((mx >> 52) & 0x7FF) - 1023 + 1;   // max|x| < 2^m
+  const bool finite = mx < 0x7FFull << 52, digits = mx != 0 && finite;
   const long long Ncol2 = 2 * ncols, slice_stride = 2 * Ncol2 * (long long)Kout;
   const long long r = (o >> 1) * Ncol2 + 2 * c + (o & 1);
-  if (lane == 0) e_out[r] = mx == 0 ? kZeroExp : m + 1;
+  if (lane == 0) e_out[r] = mx == 0 ? kZeroExp : finite ? m + 1 : kNanExp;
   __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(slices + r * Kout);
 #pragma unroll
   for (int t = 0; t < PASSES; ++t) {
     const int k = 32 * t + lane;
     if (2 * k >= Kout) continue;
-    long long F0 = round_scaled<PAIR_BITS>(v[t][0], m, mx != 0);
-    long long F1 = round_scaled<PAIR_BITS>(v[t][1], m, mx != 0);
+    long long F0 = round_scaled<PAIR_BITS>(v[t][0], m, digits);
+    long long F1 = round_scaled<PAIR_BITS>(v[t][1], m, digits);
 #pragma unroll
     for (int p = S - 1; p > 0; --p) {
       const int d0 = (int)(((F0 + 64) & 127) - 64), d1 = (int)(((F1 + 64) & 127) - 64);

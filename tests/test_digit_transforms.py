@@ -1,0 +1,39 @@
+"""The FP64 transforms as digit products on the tensor cores: non-finite inputs, the choice between them and the native
+kernels, and what they do where memory or the grid is short."""
+import numpy as np
+import pytest
+
+from conftest import small_rtd
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(n_el, nk, nxi, order, batch=1, **kw):
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order, n_xi=nxi)
+    P = Problem1D(n_el=n_el, n_local=order + 1, nk=nk, n_xi=nxi, l_xi=spec.l_xi_m, batch=batch, **kw)
+    for b in range(batch):
+        P.set_potential(b, mat["x"], E * (1 + 0.1 * b), m, spec.m_rel, spec.temp_k, efl, efr)
+    return P
+
+
+@pytest.mark.parametrize("kind", [dict(fp64_tc=True), dict(precision="mixed")])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf, complex(0.0, np.nan)])
+@pytest.mark.parametrize("n_el,nk,nxi,order,at", [(4, 32, 32, 1, 0), (5, 64, 72, 2, 40), (3, 260, 512, 1, 259)])
+def test_non_finite_inputs(built_lib, n_el, nk, nxi, order, at, value, kind):
+    """One infinity or NaN at wave number `at` of one node of the middle element: the operator is non-finite exactly where
+    it is with the native kernels (NaN where a NaN makes it so), and the rest agrees (1e-12 of |A x|, as without it)."""
+    out = []
+    for kw in (dict(), kind):
+        with _problem(n_el, nk, nxi, order, **kw) as P:
+            rng = np.random.default_rng(nk)
+            x = rng.normal(size=P.N) + 1j * rng.normal(size=P.N)
+            x[(n_el // 2 * (order + 1) + 1) * nk + at] = value
+            out.append(P.apply(x))
+    want, got = out
+    finite = np.isfinite(want)
+    assert 0 < finite.sum() < want.size
+    assert np.array_equal(np.isfinite(got), finite)
+    if np.isnan(value):
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.linalg.norm(got[finite] - want[finite]) <= 1e-12 * np.linalg.norm(want[finite])
