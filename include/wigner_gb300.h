@@ -409,6 +409,9 @@ int wg_debug_gemm_bf16(const float* A, const float* B, float* C, int M, int N, i
  * error flag, as a GEMM whose copies never land would; the context stays usable.  No counterpart in
  * the reference. */
 int wg_debug_wait_timeout(long long spin_limit);
+/* Diagnostic: raises the handle's error flag as such a wait would; its later solves, applies and transients return
+ * WG_ERR_TIMEOUT.  WG_ERR_ARG where the handle has no tensor-core kernels. */
+int wg_debug_mark_timeout(wg_problem* h);
 /* Diagnostic: C = A * B in FP64 emulated on the tensor cores (6-bit digit slices,
  * exact BF16 products, grouped FP32 accumulation, recombination in 64-bit integer
  * fixed point, one rounding to FP64), the

@@ -600,12 +600,8 @@ int wg_apply(wg_problem* h, const double* x, double* y) {
   else API_CK(&P, wg::launch_apply(P, P.z, P.w));
   API_CK(&P, cudaMemcpyAsync(y, P.w, sizeof(double2) * n, cudaMemcpyDeviceToHost, P.stream));
   API_CK(&P, cudaStreamSynchronize(P.stream));
-  if (P.mx.err) {
-    int herr = 0;
-    API_CK(&P, cudaMemcpy(&herr, P.mx.err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (herr) return fail(&P, WG_ERR_TIMEOUT, "wg_apply: tensor-core GEMM barrier wait timed out");
-  }
-  return WG_OK;
+  const int rc = wg::tc_status(P, "wg_apply");
+  return rc ? fail(&P, rc, P.err) : WG_OK;
 }
 
 int wg_apply_lowprec(wg_problem* h, const double* x, double* y) {
@@ -617,10 +613,8 @@ int wg_apply_lowprec(wg_problem* h, const double* x, double* y) {
   API_CK(&P, wg::apply_mixed_f64(P, P.z, P.w));
   API_CK(&P, cudaMemcpyAsync(y, P.w, sizeof(double2) * n, cudaMemcpyDeviceToHost, P.stream));
   API_CK(&P, cudaStreamSynchronize(P.stream));
-  int herr = 0;
-  API_CK(&P, cudaMemcpy(&herr, P.mx.err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (herr) return fail(&P, WG_ERR_TIMEOUT, "wg_apply_lowprec: tensor-core GEMM barrier wait timed out");
-  return WG_OK;
+  const int rc = wg::tc_status(P, "wg_apply_lowprec");
+  return rc ? fail(&P, rc, P.err) : WG_OK;
 }
 
 int wg_precondition(wg_problem* h, const double* r, double* z) {
@@ -712,6 +706,16 @@ int wg_debug_gemm_bf16(const float* A, const float* B, float* C, int M, int N, i
   return WG_OK;
 }
 
+int wg_debug_mark_timeout(wg_problem* h) {
+  if (!h) return fail(nullptr, WG_ERR_ARG, "null handle");
+  wg::Problem& P = h->P;
+  if (!P.mx.err) return fail(&P, WG_ERR_ARG, "wg_debug_mark_timeout: the handle has no tensor-core kernels");
+  const int one = 1;
+  API_CK(&P, cudaMemcpyAsync(P.mx.err, &one, sizeof(int), cudaMemcpyHostToDevice, P.stream));
+  API_CK(&P, cudaStreamSynchronize(P.stream));
+  return WG_OK;
+}
+
 int wg_debug_wait_timeout(long long spin_limit) {
   if (spin_limit < 1 || spin_limit > (1ll << 24))
     return fail(nullptr, WG_ERR_ARG, "wg_debug_wait_timeout: spin_limit must be in 1 .. 2^24");
@@ -742,6 +746,7 @@ int wg_apply_repeat(wg_problem* h, int which, int n, double* ms) {
   wg::Problem& P = h->P;
   if (which > 0 && P.precision != WG_PREC_MIXED)
     return fail(&P, WG_ERR_ARG, "wg_apply_repeat: the low-precision and tensor-core FP64 operators need a mixed handle");
+  if (const int rc = wg::tc_status(P, "wg_apply_repeat")) return fail(&P, rc, P.err);
   cudaEvent_t a = nullptr, b = nullptr;
   API_CK(&P, cudaEventCreate(&a));
   API_CK(&P, cudaEventCreate(&b));
@@ -763,6 +768,7 @@ int wg_apply_repeat(wg_problem* h, int which, int n, double* ms) {
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   API_CK(&P, e);
+  if (const int rc = wg::tc_status(P, "wg_apply_repeat")) return fail(&P, rc, P.err);
   *ms = t / n;
   return WG_OK;
 }

@@ -343,6 +343,9 @@ cudaError_t launch_stencil_f64(Problem& P, const double2* xh, double2* yh, const
 // residual that only has to resolve a loose tolerance, ~2^(-7 nd)).  potential_only: y = G x (launch_apply_pre).
 cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const int* mask = nullptr, int nd = 8,
                                 const int* nd_pp = nullptr, bool potential_only = false);
+// After the stream's work: WG_ERR_TIMEOUT (and P.err) when a bounded wait of the handle's tensor-core kernels has run
+// out.  They leave their outputs unwritten from then on, so every entry point that used them asks.
+int tc_status(Problem& P, const char* who);
 int debug_gemm_f64_tc(const double* A, const double* B, double* C, int M, int N, int K, std::string& err, int nd = 8);
 // Rebuild potential-dependent data (Vw weights, contact inflow rhs) of problems [b0, b1).
 // mask (device, optional): problems b with mask[b] == 0 are left untouched.

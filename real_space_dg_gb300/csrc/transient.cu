@@ -248,6 +248,8 @@ int transient_run(Problem& P, const wg_transient_opts& o, double* n_hist, double
     for (int b = 0; b < B; ++b) info[b].steps = t;
   }
   TK(cudaStreamSynchronize(P.stream));
+  // the applies of RK4 and of the Crank-Nicolson right-hand side (the step solves ask by themselves)
+  if (const int rc = tc_status(P, "wg_transient_run")) return rc;
   if (hist) {
     const size_t slab = (size_t)B * ncol;
     std::vector<double> h((size_t)irec * 2 * slab);

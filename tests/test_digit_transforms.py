@@ -37,3 +37,25 @@ def test_non_finite_inputs(built_lib, n_el, nk, nxi, order, at, value, kind):
     if np.isnan(value):
         assert np.array_equal(np.isnan(got), np.isnan(want))
     assert np.linalg.norm(got[finite] - want[finite]) <= 1e-12 * np.linalg.norm(want[finite])
+
+
+@pytest.mark.parametrize("kind", [dict(fp64TensorCores=True), dict(precision="mixed")])
+@pytest.mark.parametrize("method", ["rk4", "cn"])
+def test_timeouts_reach_the_transient(built_lib, kind, method):
+    """A wait of the products that ran out (its flag raised from the host; no kernel runs with it) ends a transient and
+    a timing run with an error, as it does a solve: the state after it is not the integrated one."""
+    from real_space_dg_gb300 import WignerError, _lib, devices
+    from real_space_dg_gb300.rtd import RTDSweep
+    mat = small_rtd(n_el=10, nk=32, order=2)[1]
+    S = RTDSweep(dict(mat, dy_norm_nm=devices.density_normalisation_nm(mat)), 1, dict(transportMaxCycles=60, **kind))
+    try:
+        S.set(0, 0.05)
+        assert S.run()[0] == 0
+        assert S.transient(1e-17, 2, method)[0] == 0 and S.P.apply_time("fp64", 1) > 0
+        assert S.lib.wg_debug_mark_timeout(S.P.h) == _lib.WG_OK
+        for call in (lambda: S.transient(1e-17, 0, method), lambda: S.P.apply_time("fp64", 1)):
+            with pytest.raises(WignerError) as e:
+                call()
+            assert e.value.status == _lib.WG_ERR_TIMEOUT
+    finally:
+        S.close()
