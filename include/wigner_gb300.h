@@ -87,7 +87,7 @@ typedef struct {
   int fp64_tc;       /* FP64 handles: 1 = the two Phi transforms as FP64 products emulated on the tensor cores (eight
                         7-bit digits, 56 bits of a column's largest entry: the error of native FP64 sums or less; 2 Nk
                         and 2 N_xi <= 1024, multiples of 4); 0 (default) = native FP64, or the same digits where they are
-                        faster (n_el n_local Nk N_xi >= 3e7) and their buffers fit the admission budget */
+                        faster (n_el n_local Nk N_xi >= 3e7) and their buffers fit the admission budget; -1 = native FP64 */
   int inner_basis_fp32; /* mixed form: 1 keeps the inner Krylov basis in FP32; 0 (default) stores it in FP16
                            with FP32 arithmetic (the preconditioner works on the stored FP16 vector; the FP64
                            refinement keeps the accuracy; C2: the same inner iteration counts, half the basis

@@ -228,7 +228,7 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
   const int mp1 = P.restart + 1;
   const int pst = P.restart_max + 1;
   // memory estimate before allocating (GmresMemoryLimit analogue)
-  P.fp64_tc = prm->fp64_tc != 0 && P.precision == WG_PREC_FP64;
+  P.fp64_tc = prm->fp64_tc > 0 && P.precision == WG_PREC_FP64;
   P.inner_basis16 = prm->inner_basis_fp32 == 0;
   const double est = wg::estimate_bytes(s, batch, P.restart, P.restart_inner, P.precision, P.fp64_tc,
                                         P.inner_basis16);
@@ -374,7 +374,7 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
   }
   // FP64 transforms as digit products where they are faster: only within the admission budget, and while their
   // buffers are a small part of the memory left (a later handle would have fitted before)
-  if (P.precision == WG_PREC_FP64 && !P.fp64_tc && wg::ozaki_pays(s)) {
+  if (P.precision == WG_PREC_FP64 && prm->fp64_tc == 0 && wg::ozaki_pays(s)) {
     const double extra = wg::ozaki_bytes(s, P.ncols);
     size_t free_b = 0, total_b = 0;
     if ((P.mem_budget <= 0 || est + extra <= P.mem_budget) && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
@@ -402,7 +402,7 @@ int wg_problem_bytes(const wg_params* prm, int batch, double* bytes) {
       wg::build_shape_light(s, prm->n_el, prm->n_local, prm->nk, prm->n_xi, prm->l_xi, prm->m_diff, prm->mpc);
   if (!e.empty()) return fail(nullptr, WG_ERR_ARG, "wg_problem_bytes: " + e);
   const int restart = prm->restart > 0 ? prm->restart : 50, inner = prm->inner_restart > 0 ? prm->inner_restart : 40;
-  *bytes = wg::estimate_bytes(s, batch, restart, inner, prm->precision, prm->fp64_tc != 0,
+  *bytes = wg::estimate_bytes(s, batch, restart, inner, prm->precision, prm->fp64_tc > 0,
                               prm->inner_basis_fp32 == 0);
   return WG_OK;
 }

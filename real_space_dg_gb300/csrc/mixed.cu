@@ -998,8 +998,6 @@ cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const 
   return cudaGetLastError();
 }
 
-// Stand-alone digit-sliced FP64 GEMM for diagnostics: C = A B with A row-major M x K,
-// B column-major K x N, C column-major M x N (host FP64 buffers), K <= 1024, K % 8 == 0.
 int tc_status(Problem& P, const char* who) {
   if (!P.mx.err) return WG_OK;
   int herr = 0;
@@ -1014,6 +1012,8 @@ int tc_status(Problem& P, const char* who) {
   return WG_ERR_TIMEOUT;
 }
 
+// Stand-alone digit-sliced FP64 GEMM for diagnostics: C = A B with A row-major M x K,
+// B column-major K x N, C column-major M x N (host FP64 buffers), K <= 1024, K % 8 == 0.
 int debug_gemm_f64_tc(const double* A, const double* B, double* C, int M, int N, int K, std::string& err, int nd) {
   if (M < 1 || N < 1 || K < 64 || K % 8 || K > oz::MAX_K) {
     err = "debug FP64 GEMM needs 64 <= K <= 1024 and K % 8 == 0";

@@ -25,6 +25,9 @@ class Problem1D:
     Mirrors the function-handle seams of the reference: ``apply`` is
     sysInfo.apply (get_SysM_full2D.m:80), ``precondition`` is
     preconditioner.apply (get_LineTransversePreconditioner_full2D.m:113).
+
+    ``fp64_tc`` (FP64 handles): True takes the transforms as digit products on the tensor cores, -1 the native FP64
+    kernels, False (default) whichever is faster at the shape.
     """
 
     def __init__(self, n_el, n_local, nk, n_xi=None, l_xi=30e-9, batch=1, precision="fp64", restart=50,
@@ -34,7 +37,8 @@ class Problem1D:
         prm = _lib.WgParams(int(n_el), int(n_local), int(nk), int(n_xi or nk), float(l_xi), float(m_diff),
                             float(mpc), PRECISIONS[precision] if isinstance(precision, str) else int(precision),
                             int(restart), float(mem_budget_bytes), int(inner_restart), float(inner_tol),
-                            float(reorth), float(inner_reorth), 1 if fp64_tc else 0, 1 if inner_basis_fp32 else 0)
+                            float(reorth), float(inner_reorth), -1 if fp64_tc == -1 else 1 if fp64_tc else 0,
+                            1 if inner_basis_fp32 else 0)
         h = C.c_void_p()
         st = self.lib.wg_problem_create(C.byref(prm), int(batch), C.byref(h))
         if st != _lib.WG_OK:
@@ -147,8 +151,8 @@ class Problem1D:
         return y
 
     def apply_time(self, which="fp64", n=20):
-        """Mean device time [ms] of one operator apply on the resident state: ``fp64``,
-        ``lowprec`` (mixed inner operator) or ``fp64_tc`` (mixed FP64 operator)."""
+        """Mean device time [ms] of one operator apply on the resident state: ``fp64`` (of an FP64 handle
+        the kernels that ``fp64_tc`` chose), ``lowprec`` (mixed inner operator) or ``fp64_tc`` (mixed FP64 operator)."""
         code = {"fp64": 0, "lowprec": 1, "fp64_tc": 2}[which]
         ms = C.c_double()
         self._check(self.lib.wg_apply_repeat(self.h, code, int(n), C.byref(ms)))

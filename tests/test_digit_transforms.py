@@ -59,3 +59,25 @@ def test_timeouts_reach_the_transient(built_lib, kind, method):
             assert e.value.status == _lib.WG_ERR_TIMEOUT
     finally:
         S.close()
+
+
+@pytest.mark.parametrize("fp64_tc,emulated", [(False, True), (True, True), (-1, False)])
+def test_the_caller_chooses(built_lib, fp64_tc, emulated):
+    """Above 3e7 entries and nodes the default takes the digit products; both kinds can be asked for, here and in the
+    options of a sweep."""
+    from real_space_dg_gb300 import devices
+    from real_space_dg_gb300.rtd import RTDSweep
+    with _problem(58, 512, 512, 3, fp64_tc=fp64_tc) as P:
+        P.profile(on=True, reset=True)
+        P.apply(np.ones(P.N))
+        prof = P.profile(on=False, reset=True)
+        assert (prof["gemm_f64_tc"][2] > 0) == emulated and (prof["gemm_f64"][2] == 0) == emulated
+    mat = small_rtd(n_el=58, nk=512, order=3, n_xi=512)[1]
+    S = RTDSweep(dict(mat, dy_norm_nm=devices.density_normalisation_nm(mat)), 1, dict(fp64TensorCores=fp64_tc))
+    try:
+        S.set(0, 0.0)
+        S.P.profile(on=True, reset=True)
+        S.P.apply(np.ones(S.P.N))
+        assert (S.P.profile(on=False, reset=True)["gemm_f64_tc"][2] > 0) == emulated
+    finally:
+        S.close()
