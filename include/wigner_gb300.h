@@ -87,7 +87,8 @@ typedef struct {
   int fp64_tc;       /* FP64 handles: 1 = the two Phi transforms as FP64 products emulated on the tensor cores (eight
                         7-bit digits, 56 bits of a column's largest entry: the error of native FP64 sums or less; 2 Nk
                         and 2 N_xi <= 1024, multiples of 4); 0 (default) = native FP64, or the same digits where they are
-                        faster (n_el n_local Nk N_xi >= 3e7) and their buffers fit the admission budget; -1 = native FP64 */
+                        faster (n_el n_local Nk N_xi >= 3e7; with a buffer of their own where the admission budget and the
+                        free memory allow it, in the handle's fields otherwise: the same results); -1 = native FP64 */
   int inner_basis_fp32; /* mixed form: 1 keeps the inner Krylov basis in FP32; 0 (default) stores it in FP16
                            with FP32 arithmetic (the preconditioner works on the stored FP16 vector; the FP64
                            refinement keeps the accuracy; C2: the same inner iteration counts, half the basis
@@ -125,7 +126,8 @@ typedef struct wg_problem wg_problem;
 int wg_problem_create(const wg_params* prm, int batch, wg_problem** out);
 int wg_problem_destroy(wg_problem* h);
 /* Device bytes a handle of `batch` problems would allocate (the admission estimate
- * of wg_problem_create, GmresMemoryLimit analogue of solve_transport_DG_full2D.m:198). */
+ * of wg_problem_create, GmresMemoryLimit analogue of solve_transport_DG_full2D.m:198);
+ * optional buffers are counted unless they exceed prm->mem_budget_bytes. */
 int wg_problem_bytes(const wg_params* prm, int batch, double* bytes);
 const char* wg_last_error(const wg_problem* h);
 /* Library-level last error (for failures before a handle exists). */

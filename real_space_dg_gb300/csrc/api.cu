@@ -102,6 +102,11 @@ double estimate_bytes(const Shape& s, int batch, int restart, int restart_inner,
   return est;
 }
 
+// FP64 handles that take digit products without being asked to.
+static bool auto_digits(const wg_params& prm, const Shape& s) {
+  return prm.precision == WG_PREC_FP64 && prm.fp64_tc == 0 && ozaki_pays(s);
+}
+
 // k-line factors of the flux part of A + sigma I, per problem b and wave number k:
 // D_b(k) = (k K1 + |k| K2 + (sigma / qd_b) I)^-1 and h = D_b(k) * upwind coupling column
 // (the line operator of get_LineTransversePreconditioner_full2D.m:174-197 in 1D; the
@@ -228,9 +233,10 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
   const int mp1 = P.restart + 1;
   const int pst = P.restart_max + 1;
   // memory estimate before allocating (GmresMemoryLimit analogue)
-  P.fp64_tc = prm->fp64_tc > 0 && P.precision == WG_PREC_FP64;
+  const bool auto_tc = wg::auto_digits(*prm, s);
+  P.fp64_tc = P.precision == WG_PREC_FP64 && (prm->fp64_tc > 0 || auto_tc);
   P.inner_basis16 = prm->inner_basis_fp32 == 0;
-  const double est = wg::estimate_bytes(s, batch, P.restart, P.restart_inner, P.precision, P.fp64_tc,
+  const double est = wg::estimate_bytes(s, batch, P.restart, P.restart_inner, P.precision, prm->fp64_tc > 0,
                                         P.inner_basis16);
   if (P.mem_budget > 0 && est > P.mem_budget) {
     delete h;
@@ -364,27 +370,27 @@ int wg_problem_create(const wg_params* prm, int batch, wg_problem** out) {
   API_CK(&P, cudaMemsetAsync(P.xq, 0, sizeof(double) * batch * s.n_el * wg::kNqx, P.stream));
   API_CK(&P, cudaStreamSynchronize(P.stream));
   if (P.precision == WG_PREC_MIXED || P.fp64_tc) {
-    const int mr = P.precision == WG_PREC_MIXED ? wg::mixed_alloc(P) : wg::ozaki_alloc(P);
+    // digits that the library chose have a buffer of their own only within the admission budget, and while it is a small
+    // part of the memory left (a later handle would have fitted before)
+    bool own = true;
+    if (auto_tc) {
+      const double extra = wg::ozaki_buffer_bytes(s, P.ncols);
+      size_t free_b = 0, total_b = 0;
+      own = (P.mem_budget <= 0 || est + extra <= P.mem_budget) && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+            16.0 * extra <= (double)free_b;
+    }
+    int mr = P.precision == WG_PREC_MIXED ? wg::mixed_alloc(P) : wg::ozaki_alloc(P, own);
+    if (mr == WG_ERR_OOM && auto_tc && own) {
+      cudaGetLastError();
+      wg::mixed_free(P);
+      P.err.clear();
+      mr = wg::ozaki_alloc(P, false);
+    }
     if (mr != WG_OK) {
       std::string msg = "wg_problem_create: " + P.err;
       free_all(P);
       delete h;
       return fail(nullptr, mr, msg);
-    }
-  }
-  // FP64 transforms as digit products where they are faster: only within the admission budget, and while their
-  // buffers are a small part of the memory left (a later handle would have fitted before)
-  if (P.precision == WG_PREC_FP64 && prm->fp64_tc == 0 && wg::ozaki_pays(s)) {
-    const double extra = wg::ozaki_bytes(s, P.ncols);
-    size_t free_b = 0, total_b = 0;
-    if ((P.mem_budget <= 0 || est + extra <= P.mem_budget) && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-        16.0 * extra <= (double)free_b) {
-      P.fp64_tc = wg::ozaki_alloc(P) == WG_OK && P.mx.ozaki;
-      if (!P.fp64_tc) {
-        cudaGetLastError();
-        wg::mixed_free(P);
-        P.err.clear();
-      }
     }
   }
   P.hp.resize(batch);
@@ -404,6 +410,8 @@ int wg_problem_bytes(const wg_params* prm, int batch, double* bytes) {
   const int restart = prm->restart > 0 ? prm->restart : 50, inner = prm->inner_restart > 0 ? prm->inner_restart : 40;
   *bytes = wg::estimate_bytes(s, batch, restart, inner, prm->precision, prm->fp64_tc > 0,
                               prm->inner_basis_fp32 == 0);
+  const double extra = wg::auto_digits(*prm, s) ? wg::ozaki_buffer_bytes(s, (long long)batch * s.n_el * s.nK) : 0.0;
+  if (prm->mem_budget_bytes <= 0 || *bytes + extra <= prm->mem_budget_bytes) *bytes += extra;
   return WG_OK;
 }
 

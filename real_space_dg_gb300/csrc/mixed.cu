@@ -130,19 +130,26 @@ int pair_row(int K) { return std::max(oz::BK, (K / 2 + 7) & ~7); }
 // Y = Phi X (MODE 0) or Y = i Phi^H X (MODE 1) on the tensor cores: slicing and gemm_pairs_kernel.  X: K complex entries
 // per column, Y: M.
 template <int MODE>
-cudaError_t launch_pairs(Problem& P, const CUtensorMap& a, const CUtensorMap& b, const int* ea, const double2* X,
-                         double2* Y, int K, int M, const int* mask, int nd, const int* nd_pp) {
+cudaError_t launch_pairs(Problem& P, const double2* X, double2* Y, int K, int M, const int* mask, int nd,
+                         const int* nd_pp) {
   static const cudaError_t attr = cudaFuncSetAttribute(oz::gemm_pairs_kernel<MODE>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, oz::SMEM_BYTES);
   if (attr != cudaSuccess) return attr;
   if (nd < 1 || nd > oz::S) return cudaErrorInvalidValue;
   const int npp = (int)(P.ncols / P.batch), Kp = pair_row(K);
   auto slice = Kp <= 64 ? oz::slice_pairs_kernel<1> : Kp <= 128 ? oz::slice_pairs_kernel<2> : oz::slice_pairs_kernel<4>;
-  slice<<<(unsigned)((P.ncols + oz::kSlicePairNodes - 1) / oz::kSlicePairNodes), 128 * oz::kSlicePairNodes, 0, P.stream>>>(
-      X, K, P.ncols, P.mx.ob, P.mx.eb, mask, npp, Kp, nd, nd_pp);
-  const dim3 grid((M / 2 + oz::BM - 1) / oz::BM, (unsigned)((2 * P.ncols + oz::BN - 1) / oz::BN));
-  oz::gemm_pairs_kernel<MODE><<<grid, oz::THREADS, oz::SMEM_BYTES, P.stream>>>(
-      a, b, ea, P.mx.eb, Y, M, 2 * P.ncols, Kp, P.mx.err, mask, 2 * npp, nd, nd_pp);
+  MixedBuffers& B = P.mx;
+  const long long slab = B.oslab[MODE];
+  if (slab < P.ncols && (mask || nd_pp)) return cudaErrorNotSupported;   // the mixed form has its own buffer
+  const dim3 grid((M / 2 + oz::BM - 1) / oz::BM, (unsigned)((2 * slab + oz::BN - 1) / oz::BN));
+  for (long long c = 0; c < P.ncols; c += slab) {
+    const long long c0 = std::min(c, P.ncols - slab);   // columns of the last two passes may overlap: the same results
+    slice<<<(unsigned)((slab + oz::kSlicePairNodes - 1) / oz::kSlicePairNodes), 128 * oz::kSlicePairNodes, 0, P.stream>>>(
+        X + c0 * K, K, slab, B.od[MODE], B.eb, mask, npp, Kp, nd, nd_pp);
+    oz::gemm_pairs_kernel<MODE><<<grid, oz::THREADS, oz::SMEM_BYTES, P.stream>>>(
+        MODE == 0 ? B.tmOA1 : B.tmOA2, B.tmOB[MODE], MODE == 0 ? B.ea1 : B.ea2, B.eb, Y + c0 * M, M, 2 * slab, Kp, B.err,
+        mask, 2 * npp, nd, nd_pp);
+  }
   return cudaGetLastError();
 }
 
@@ -709,15 +716,15 @@ int mixed_alloc(Problem& P) {
   return ozaki_alloc(P);
 }
 
-double ozaki_bytes(const Shape& s, long long ncols) {
-  const double kmax = std::max(pair_row(s.nk), pair_row(s.nxi));
-  return 2.0 * oz::S * 4 * (double)ncols * kmax + 16.0 * ncols + 2.0 * oz::S * 2 * kmax * std::max(s.nk, s.nxi);
+double ozaki_buffer_bytes(const Shape& s, long long ncols) {
+  return 2.0 * oz::S * 4 * (double)ncols * std::max(pair_row(s.nk), pair_row(s.nxi));
 }
 
 // FP64 handles whose transforms are faster as products of digits: a CTA of gemm_pairs_kernel takes 36 us whatever
 // the number of nodes up to 32 an SM, the native kernel 2 us per 10^6 table entries and nodes of one problem.
 // 960 nodes of 256 x 256 (6.3e7): 125 -> 47 us, two problems 224 -> 51 us; 240 nodes (1.6e7): 42 us native, 41 us; 960 of
-// 128 x 128 (1.6e7): 41 and 35 us.  A rule on one problem, so that its results do not depend on the batch it is in.  The
+// 128 x 128 (1.6e7): 41 and 35 us.  A rule on one problem alone: results depend neither on the batch it is in nor on the
+// memory left, which only decides whether the digits have a buffer of their own (ozaki_alloc).  The
 // digits keep 56 bits of a column's largest entry: the rounding error of the operator on 116 to 240 elements, Nk = 200 to 512,
 // fell from 1.6e-16 .. 1.0e-15 (native sums) to 1.3e-16 .. 2.3e-16 of |A x|.
 bool ozaki_pays(const Shape& s) {
@@ -725,7 +732,11 @@ bool ozaki_pays(const Shape& s) {
          (double)s.n_el * s.nK * s.nk * s.nxi >= 3e7;
 }
 
-int ozaki_alloc(Problem& P) {
+// Without a buffer of its own a transform's digits take the place of the field that it neither reads nor writes: yh while
+// x -> xh, xh while yh -> y.  A field holds 16 N_xi bytes per column and the digits take 64 pair_row(K), so two or three
+// passes over the columns do.  The products of a column are the same, so the bits are.  One apply with the buffer, without
+// it and native: 122, 198 and 281 us (960 nodes of 256 x 256), 393, 409 and 1,911 us (7,680 nodes).
+int ozaki_alloc(Problem& P, bool own) {
   MixedBuffers& M = P.mx;
   const Shape& s = P.s;
   const int nk = s.nk, nxi = s.nxi;
@@ -764,10 +775,19 @@ int ozaki_alloc(Problem& P) {
     C2(cudaMalloc(&M.oa2, sizeof(bf16) * d2.size()));
     C2(cudaMalloc(&M.ea1, sizeof(int) * e1.size()));
     C2(cudaMalloc(&M.ea2, sizeof(int) * e2.size()));
-    C2(cudaMalloc(&M.ob, sizeof(bf16) * (size_t)oz::S * 4 * P.ncols * kmax));
     C2(cudaMalloc(&M.eb, sizeof(int) * (size_t)4 * P.ncols));
-    // columns of masked problems are not re-sliced: keep them finite from the start
-    C2(cudaMemset(M.ob, 0, sizeof(bf16) * (size_t)oz::S * 4 * P.ncols * kmax));
+    for (int t = 0; t < 2; ++t) {
+      const long long fit = 16ll * nxi * P.ncols / (2 * oz::S * 4 * (t ? K2 : K1));
+      const long long passes = own || fit < 1 ? 1 : (P.ncols + fit - 1) / fit;
+      M.oslab[t] = (P.ncols + passes - 1) / passes;
+      M.od[t] = reinterpret_cast<bf16*>(t ? P.xh : P.yh);
+    }
+    if (own) {
+      C2(cudaMalloc(&M.ob, sizeof(bf16) * (size_t)oz::S * 4 * P.ncols * kmax));
+      // columns of masked problems are not re-sliced: keep them finite from the start
+      C2(cudaMemset(M.ob, 0, sizeof(bf16) * (size_t)oz::S * 4 * P.ncols * kmax));
+      M.od[0] = M.od[1] = M.ob;
+    }
     C2(cudaMemset(M.eb, 0, sizeof(int) * (size_t)4 * P.ncols));
     C2(cudaMemcpy(M.oa1, d1.data(), sizeof(bf16) * d1.size(), cudaMemcpyHostToDevice));
     C2(cudaMemcpy(M.oa2, d2.data(), sizeof(bf16) * d2.size(), cudaMemcpyHostToDevice));
@@ -778,9 +798,10 @@ int ozaki_alloc(Problem& P) {
       return ce == cudaErrorMemoryAllocation ? WG_ERR_OOM : WG_ERR_CUDA;
     }
     P.device_bytes += 2.0 * (d1.size() + d2.size()) + 4.0 * (e1.size() + e2.size()) +
-                      2.0 * oz::S * 4 * P.ncols * kmax + 16.0 * P.ncols;
+                      (own ? ozaki_buffer_bytes(s, P.ncols) : 0.0) + 16.0 * P.ncols;
     ok = make_map3(&M.tmOA1, M.oa1, 2 * hs, K1, oz::BM) && make_map3(&M.tmOA2, M.oa2, 2 * hk, K2, oz::BM) &&
-         make_map3(&M.tmOB1, M.ob, 4 * P.ncols, K1, oz::BN) && make_map3(&M.tmOB2, M.ob, 4 * P.ncols, K2, oz::BN);
+         make_map3(&M.tmOB[0], M.od[0], 4 * M.oslab[0], K1, oz::BN) &&
+         make_map3(&M.tmOB[1], M.od[1], 4 * M.oslab[1], K2, oz::BN);
     if (!ok) {
       P.err = "cuTensorMapEncodeTiled failed for the FP64 tensor-core operands";
       return WG_ERR_CUDA;
@@ -984,13 +1005,13 @@ cudaError_t launch_apply_f64_tc(Problem& P, const double2* x, double2* y, const 
   const double prod_flops = 2.0 * (2.0 * s.nxi) * (2.0 * s.nk) * ncols / 4;
   cudaEvent_t ev = prof_begin(P, PROF_GEMM_F64TC, 2, 8.0 * P.N * P.batch + 16.0 * s.nxi * ncols, prod_flops, mask,
                               nd, nd_pp);
-  e = launch_pairs<0>(P, M.tmOA1, M.tmOB1, M.ea1, x, P.xh, s.nk, s.nxi, mask, nd, nd_pp);
+  e = launch_pairs<0>(P, x, P.xh, s.nk, s.nxi, mask, nd, nd_pp);
   prof_end(P, PROF_GEMM_F64TC, ev);
   if (e != cudaSuccess) return e;
   e = launch_stencil_f64(P, P.xh, P.yh, mask);
   if (e != cudaSuccess) return e;
   ev = prof_begin(P, PROF_GEMM_F64TC, 2, 8.0 * s.nxi * ncols + 16.0 * P.N * P.batch, prod_flops, mask, nd, nd_pp);
-  e = launch_pairs<1>(P, M.tmOA2, M.tmOB2, M.ea2, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp);
+  e = launch_pairs<1>(P, P.yh, y, s.nxi, s.nk, mask, nd, nd_pp);
   prof_end(P, PROF_GEMM_F64TC, ev);
   if (e != cudaSuccess) return e;
   if (!potential_only) e = launch_flux_f64(P, x, y, mask, true);

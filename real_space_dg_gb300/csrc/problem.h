@@ -113,7 +113,11 @@ struct MixedBuffers {
   int* ea2 = nullptr;                // [Nk]
   __nv_bfloat16* ob = nullptr;       // [S][4 ncols][largest pair row] digits of the state's mirror sums and differences
   int* eb = nullptr;                 // [4 ncols] column exponents
-  CUtensorMap tmOA1, tmOA2, tmOB1, tmOB2;
+  // digits of the two transforms: ob, or where that is not had (ozaki_alloc) the field each of them does not use, which
+  // holds oslab columns at a time
+  __nv_bfloat16* od[2] = {};
+  long long oslab[2] = {};
+  CUtensorMap tmOA1, tmOA2, tmOB[2];
 };
 
 // Kernel classes timed and counted by the profiler.
@@ -360,9 +364,10 @@ int gmres_solve_fp64(Problem& P, const wg_solve_opts& o, bool warm, wg_solve_inf
 std::string mixed_check_shape(const Shape& s);
 double mixed_bytes(const Shape& s, int batch, int restart, bool basis16);
 int mixed_alloc(Problem& P);
-// Digit slices of Phi, state slice buffer and tensor maps of the FP64 emulation (any precision).
-int ozaki_alloc(Problem& P);
-double ozaki_bytes(const Shape& s, long long ncols);
+// Digit slices of Phi, state slice buffer and tensor maps of the FP64 emulation (any precision).  own = false (FP64
+// handles): without the state slice buffer of ozaki_buffer_bytes.
+int ozaki_alloc(Problem& P, bool own = true);
+double ozaki_buffer_bytes(const Shape& s, long long ncols);
 bool ozaki_pays(const Shape& s);
 void mixed_free(Problem& P);
 cudaError_t mixed_sync_weights(Problem& P);

@@ -407,7 +407,12 @@ int wg_server_submit(wg_server* S, const wg_request* r, long long* id) {
     K->index = (int)S->classes.size() - 1;
     K->prm = d.prm;
     double b2 = 0;
-    wg_problem_bytes(&d.prm, 2, &b2);
+    if (probe > S->o.mem_budget_bytes) {   // one slot fits without the optional buffers or not at all
+      K->prm.mem_budget_bytes = 1.0;
+      wg_problem_bytes(&K->prm, 1, &probe);
+    }
+    wg_problem_bytes(&K->prm, 2, &b2);
+    if (K->prm.mem_budget_bytes > 0) K->prm.mem_budget_bytes = S->o.mem_budget_bytes;
     K->bytes1 = probe;
     K->bytes_per_slot = b2 - probe;
   }

@@ -81,3 +81,57 @@ def test_the_caller_chooses(built_lib, fp64_tc, emulated):
         assert (S.P.profile(on=False, reset=True)["gemm_f64_tc"][2] > 0) == emulated
     finally:
         S.close()
+
+
+def _bytes(budget, **shape):
+    import ctypes as C
+    from real_space_dg_gb300 import _lib
+    prm = _lib.WgParams(shape["n_el"], shape["order"] + 1, shape["nk"], shape["nxi"], 30e-9, 0.0, 1.0, _lib.WG_PREC_FP64,
+                        20, budget)
+    out = C.c_double()
+    assert _lib.load().wg_problem_bytes(C.byref(prm), shape["batch"], C.byref(out)) == _lib.WG_OK
+    return out.value
+
+
+@pytest.mark.parametrize("n_el,nk,nxi,order,batch", [(116, 256, 256, 3, 1), (153, 256, 260, 2, 2), (59, 508, 512, 3, 1),
+                                                     (2000, 60, 132, 1, 1)])
+def test_results_do_not_depend_on_memory_or_batch(built_lib, n_el, nk, nxi, order, batch):
+    """The same bits with a buffer for all digits, with an admission budget that leaves no room for one (the digits then
+    take two or three passes, the last one overlapping) and alone in a batch; the estimate
+    counts the buffer."""
+    shape = dict(n_el=n_el, nk=nk, nxi=nxi, order=order, batch=batch)
+    full, least = _bytes(0.0, **shape), _bytes(1.0, **shape)
+    assert least < full
+    rng = np.random.default_rng(nk)
+    out, held = [], []
+    for budget in (0.0, least):
+        with _problem(**shape, mem_budget_bytes=budget, restart=20) as P:
+            if not out:
+                x = rng.normal(size=P.N * batch) + 1j * rng.normal(size=P.N * batch)
+            P.profile(on=True, reset=True)
+            out.append(P.apply(x))
+            assert P.profile(on=False, reset=True)["gemm_f64_tc"][2] > 0
+            held.append(P.device_bytes)
+    assert held[0] - held[1] == full - least
+    assert np.array_equal(out[0], out[1])
+    with _problem(n_el, nk, nxi, order, restart=20) as P:      # problem 0 of the batch has the unscaled potential
+        assert np.array_equal(P.apply(x[:P.N]), out[0][:P.N])
+        P.set_rhs(0, x[:P.N])
+        st, info = P.solve(tol=1e-3, maxit=1)
+    with _problem(n_el, nk, nxi, order, restart=20, mem_budget_bytes=_bytes(1.0, **dict(shape, batch=1))) as P:
+        P.set_rhs(0, x[:P.N])
+        assert P.solve(tol=1e-3, maxit=1)[1][0]["iterations"] == info[0]["iterations"]
+
+
+def test_served_without_room_for_the_digits(built_lib):
+    """A server whose budget holds one slot of a large FP64 shape without the digits' buffer, and not with it."""
+    from real_space_dg_gb300 import devices
+    from real_space_dg_gb300.serve import Server
+    spec, mat, *_ = small_rtd(n_el=58, nk=512, order=3, n_xi=512)
+    mat = dict(mat, dy_norm_nm=devices.density_normalisation_nm(mat))
+    least, full = (_bytes(b, n_el=58, nk=512, nxi=512, order=3, batch=1) for b in (1.0, 0.0))
+    with Server(dict(precision="fp64", restart=20, maxIterations=2, transportTolerance=1e-6),
+                mem_budget_bytes=0.5 * (least + full), max_slots=2) as S:
+        r = S.wait(S.submit(mat, 0.0), timeout=60)
+        assert r["state"] == "done" and np.all(np.isfinite(r["n"])), r["error"]
+        assert least <= S.stats()["device_bytes_peak"] <= 0.5 * (least + full)
