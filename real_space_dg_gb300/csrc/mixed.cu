@@ -141,12 +141,12 @@ cudaError_t launch_pairs(Problem& P, const double2* X, double2* Y, int K, int M,
   MixedBuffers& B = P.mx;
   const long long slab = B.oslab[MODE];
   if (slab < P.ncols && (mask || nd_pp)) return cudaErrorNotSupported;   // the mixed form has its own buffer
-  const dim3 grid((M / 2 + oz::BM - 1) / oz::BM, (unsigned)((2 * slab + oz::BN - 1) / oz::BN));
+  const long long grid = (M / 2 + oz::BM - 1) / oz::BM * ((2 * slab + oz::BN - 1) / oz::BN);
   for (long long c = 0; c < P.ncols; c += slab) {
     const long long c0 = std::min(c, P.ncols - slab);   // columns of the last two passes may overlap: the same results
     slice<<<(unsigned)((slab + oz::kSlicePairNodes - 1) / oz::kSlicePairNodes), 128 * oz::kSlicePairNodes, 0, P.stream>>>(
         X + c0 * K, K, slab, B.od[MODE], B.eb, mask, npp, Kp, nd, nd_pp);
-    oz::gemm_pairs_kernel<MODE><<<grid, oz::THREADS, oz::SMEM_BYTES, P.stream>>>(
+    oz::gemm_pairs_kernel<MODE><<<(unsigned)grid, oz::THREADS, oz::SMEM_BYTES, P.stream>>>(
         MODE == 0 ? B.tmOA1 : B.tmOA2, B.tmOB[MODE], MODE == 0 ? B.ea1 : B.ea2, B.eb, Y + c0 * M, M, 2 * slab, Kp, B.err,
         mask, 2 * npp, nd, nd_pp);
   }

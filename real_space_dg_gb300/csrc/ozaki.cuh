@@ -388,9 +388,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_pairs_kernel(
     const int* __restrict__ mask, int cols_per_problem, int nd, const int* __restrict__ nd_pp) {
   // Ncol2, cols_per_problem: real columns (two per node).  nd (1 .. S): leading digits used of each operand; nd_pp
   // (optional): digits per problem, the tile takes the largest of its problems.  A column tile whose
-  // problems are all inactive has nothing to compute.
+  // problems are all inactive has nothing to compute.  Grid: all tiles in x, row tiles first (columns in y end at 65,535
+  // tiles, two million nodes).
+  const int hm = M / 2, row_tiles = (hm + BM - 1) / BM, m0 = (int)(blockIdx.x % row_tiles) * BM;
+  const long long n0 = (long long)(blockIdx.x / row_tiles) * BN;
   if (mask || nd_pp) {
-    const long long c0 = (long long)blockIdx.y * BN, c1 = min(Ncol2, c0 + BN) - 1;
+    const long long c0 = n0, c1 = min(Ncol2, c0 + BN) - 1;
     bool any = false;
     int ndt = 1;
     for (long long b = c0 / cols_per_problem; b <= c1 / cols_per_problem; ++b) {
@@ -411,8 +414,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_pairs_kernel(
   uint64_t* drained = done + 2;          // plane 0 has been read out of TMEM
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int hm = M / 2, m0 = blockIdx.x * BM;
-  const long long n0 = (long long)blockIdx.y * BN;
   const int nkb = (K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {

@@ -135,3 +135,20 @@ def test_served_without_room_for_the_digits(built_lib):
         r = S.wait(S.submit(mat, 0.0), timeout=60)
         assert r["state"] == "done" and np.all(np.isfinite(r["n"])), r["error"]
         assert least <= S.stats()["device_bytes_peak"] <= 0.5 * (least + full)
+
+
+@pytest.mark.parametrize("kind", [dict(fp64_tc=True), dict(precision="mixed", inner_restart=2)])
+def test_more_nodes_than_grid_rows(built_lib, kind):
+    """2,098,800 nodes, more than 65,535 tiles of 32: the last problem of the handle against the same problem alone."""
+    n_el, nk, order, batch = 990, 32 if "precision" in kind else 8, 3, 530
+    from real_space_dg_gb300 import Problem1D
+    spec, mat, E, efl, efr, m = small_rtd(n_el=n_el, nk=nk, order=order)
+    rng = np.random.default_rng(0)
+    out = []
+    for b in (batch, 1):
+        with Problem1D(n_el=n_el, n_local=order + 1, nk=nk, l_xi=spec.l_xi_m, batch=b, restart=2, **kind) as P:
+            P.set_potential(b - 1, mat["x"], E, m, spec.m_rel, spec.temp_k, efl, efr)
+            x = np.zeros((b, P.N), dtype=complex)
+            x[-1] = rng.normal(size=P.N) + 1j * rng.normal(size=P.N) if not out else out[0][0]
+            out.append((x[-1].copy(), P.apply(x).reshape(b, -1)[-1].copy()))
+    assert np.array_equal(out[0][1], out[1][1]) and np.linalg.norm(out[1][1]) > 0
