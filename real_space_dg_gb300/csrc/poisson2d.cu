@@ -88,7 +88,8 @@ __device__ void block_reduce(const double (&v)[N], double (*red)[8], double* out
   }
 }
 
-// Buffers of one step (all problems): n, v, F [B][nun]; r, y, d [B][nx][NU]; the blocks of the reduction and
+// Buffers of one step (the B problems of a group, launch_step): n, v, F [B][nun]; r, y, d [B][nx][NU]; the blocks of
+// the reduction and
 // the block partials of the reductions over nodes.
 struct P2Work {
   double *n, *v, *F, *r, *y, *d;
@@ -593,12 +594,16 @@ cudaError_t keep(wg_poisson2d* h, T** d, const std::vector<T>& v) {
   return e;
 }
 
-cudaError_t launch_step(wg_poisson2d* h, const double* src, int is_dg, const double* phi0, const double* bc,
-                        int newton, double alpha, double* phi, double* dens, cudaStream_t st) {
+// Problems per group of launches: the grids' second dimension and the reduction's blocks (3 nx NU^2 doubles per
+// problem) stay bounded for any batch.  A group of this size fills the chip at every level.
+constexpr int kP2Group = 1024;
+
+cudaError_t launch_group(wg_poisson2d* h, int B, const double* src, int is_dg, const double* phi0, const double* bc,
+                         int newton, double alpha, double* phi, double* dens, wg_poisson2d_info* info,
+                         cudaStream_t st) {
   const double q_kt = kQ * kQ / (kKB * h->d.temp);
   const P2Dev& P = h->P;
   const P2Work& w = h->w;
-  const unsigned B = (unsigned)h->d.batch;
   const dim3 nodes((unsigned)((P.nu * P.nx + kP2Threads - 1) / kP2Threads), B);
   int top = 1;
   while (P.nx / (2 * top) >= 1) top *= 2;
@@ -631,8 +636,19 @@ cudaError_t launch_step(wg_poisson2d* h, const double* src, int is_dg, const dou
       return cudaErrorInvalidValue;
   }
 #undef WG_P2_CASE
-  poisson2d_finish_kernel<<<nodes, kP2Threads, 0, st>>>(P, w, h->NU, phi0, newton, q_kt, alpha, phi, dens, h->info);
+  poisson2d_finish_kernel<<<nodes, kP2Threads, 0, st>>>(P, w, h->NU, phi0, newton, q_kt, alpha, phi, dens, info);
   return cudaGetLastError();
+}
+
+cudaError_t launch_step(wg_poisson2d* h, const double* src, int is_dg, const double* phi0, const double* bc,
+                        int newton, double alpha, double* phi, double* dens, cudaStream_t st) {
+  const size_t full = (size_t)h->P.nx * h->P.ny, un = (size_t)h->P.nx * h->P.nu,
+               ns = is_dg ? (size_t)h->P.ndx * h->P.ndy : full;
+  cudaError_t e = cudaSuccess;
+  for (int b = 0; b < h->d.batch && e == cudaSuccess; b += kP2Group)
+    e = launch_group(h, std::min(kP2Group, h->d.batch - b), src + b * ns, is_dg, phi0 + b * full, bc + b * un, newton,
+                     alpha, phi + b * full, dens + b * full, h->info + b, st);
+  return e;
 }
 
 }  // namespace
@@ -768,9 +784,9 @@ int wg_poisson2d_create(const wg_poisson2d_desc* d, const double* eps_r, const u
   if (e == cudaSuccess) e = cudaMalloc(&h->phi, sz);
   if (e == cudaSuccess) e = cudaMalloc(&h->dens, sz);
   {
-    const size_t bb = (size_t)h->NU * h->NU, half = (size_t)B * (nx / 2) * bb, even = (size_t)B * ((nx + 1) / 2) * bb,
-                 col = (size_t)B * nx * h->NU, un = (size_t)B * nun,
-                 part = (size_t)B * kP2Part * ((nun + kP2Threads - 1) / kP2Threads);
+    const size_t G = std::min(B, kP2Group), bb = (size_t)h->NU * h->NU, half = G * (nx / 2) * bb,
+                 even = G * ((nx + 1) / 2) * bb, col = G * nx * h->NU, un = G * nun,
+                 part = G * kP2Part * ((nun + kP2Threads - 1) / kP2Threads);
     double** const ptr[] = {&h->w.n, &h->w.v, &h->w.F, &h->w.r, &h->w.y, &h->w.d,    &h->w.D,
                             &h->w.L, &h->w.U, &h->w.XL, &h->w.XU, &h->w.Dinv, &h->w.part};
     const size_t len[] = {un, un, un, col, col, col, half, half, half, half, half, even, part};
@@ -782,8 +798,8 @@ int wg_poisson2d_create(const wg_poisson2d_desc* d, const double* eps_r, const u
       *ptr[i] = h->work + at0;
       at0 += len[i];
     }
-    if (e == cudaSuccess) e = cudaMalloc(&h->w.count, (size_t)B * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(h->w.count, 0, (size_t)B * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&h->w.count, G * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(h->w.count, 0, G * sizeof(int));
   }
   if (e == cudaSuccess) e = cudaMalloc(&h->info, (size_t)B * sizeof(wg_poisson2d_info));
   if (e != cudaSuccess) {

@@ -50,3 +50,26 @@ def test_fixed_nodes_inside(built_lib, method):
 @pytest.mark.parametrize("nx", [2, 6, 40])
 def test_neumann_ends(built_lib, nx):
     _check(grid(nx=nx, ny=5, seed=nx, poisson=dict(xBoundary="neumann")), 0.0, "newton-raphson")
+
+
+@pytest.mark.parametrize("batch,cfg", [(1025, dict(nx=19, ny=6)), (2050, dict(nx=9, ny=14, periodic=True)),
+                                       (65_600, dict(nx=3, ny=2))])
+def test_any_number_of_bias_points(built_lib, batch, cfg):
+    """Batches beyond a group of launches and beyond a grid's second dimension: the points around the groups' edges
+    have the bits that they have alone."""
+    from real_space_dg_gb300.poisson2d import Poisson2D
+    mat = grid(seed=batch, **cfg)
+    nx, ny = mat["Nx"], mat["Ny"]
+    rng = np.random.default_rng(batch)
+    n = density(mat) * rng.uniform(0.5, 1.5, (batch, 1, 1))
+    phi0 = 0.05 * rng.normal(size=(batch, nx, ny))
+    if cfg.get("periodic"):
+        phi0[..., -1] = phi0[..., 0]
+    bias = rng.uniform(0.0, 0.4, batch)
+    with Poisson2D(mat, batch=batch) as op:
+        phi, dens, info = op.solve(n, phi0, bias, method="newton-raphson")
+    assert all(i["converged"] for i in info)
+    with Poisson2D(mat) as op:
+        for b in (0, 1, 1023, 1024, batch - 1):
+            p1, d1, i1 = op.solve(n[b], phi0[b], bias[b], method="newton-raphson")
+            assert np.array_equal(p1, phi[b]) and np.array_equal(d1, dens[b]) and i1 == info[b]
