@@ -425,6 +425,9 @@ int wg_debug_gemm_f64_tc(const double* A, const double* B, double* C, int M, int
  * as the mixed form's residual uses for loose tolerances. */
 int wg_debug_gemm_f64_tc_digits(const double* A, const double* B, double* C, int M, int N, int K, int nd);
 
+/* Diagnostic: y = 1 / x by the reciprocal that the pivots of the subband and Poisson kernels use (host arrays of n). */
+int wg_debug_rcp(const double* x, double* y, long long n);
+
 /* Diagnostic: apply the operator n times to the resident state on the device and
  * return the mean time of one apply in *ms.  which = 0: the FP64 operator;
  * 1: the mixed form's low-precision operator (BF16 transforms, FP32 flux and

@@ -32,7 +32,10 @@
 #include <string>
 #include <vector>
 
+#include "recip.cuh"
 #include "wigner_gb300.h"
+
+using wg::fast_rcp;
 
 namespace {
 
@@ -89,8 +92,7 @@ __device__ void block_reduce(const double (&v)[N], double (*red)[8], double* out
 }
 
 // Buffers of one step (the B problems of a group, launch_step): n, v, F [B][nun]; r, y, d [B][nx][NU]; the blocks of
-// the reduction and
-// the block partials of the reductions over nodes.
+// the reduction and the block partials of the reductions over nodes.
 struct P2Work {
   double *n, *v, *F, *r, *y, *d;
   double *D, *L, *U;      // [B][nx / 2][NU][NU]: the odd columns' blocks of the current level
@@ -207,15 +209,6 @@ struct ReduceShape {
   static constexpr int TPR = (W + CPT - 1) / CPT;             // threads per row
   static constexpr int THREADS = (NU * TPR + 31) / 32 * 32;
 };
-
-// 1 / x to rounding level: the hardware's approximation (rcp.approx.ftz.f64, about 20 bits) and a third-order
-// Newton step r (1 + e + e^2), e = 1 - x r.
-__device__ __forceinline__ double fast_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
 
 // [D | rest] -> D^-1 rest in registers, no pivoting; dg[i]: 1 / the pivot of row i.
 template <int NU, int NB>

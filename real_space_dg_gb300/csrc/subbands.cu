@@ -39,7 +39,10 @@
 #include <cmath>
 #include <string>
 
+#include "recip.cuh"
 #include "wigner_gb300.h"
+
+using wg::fast_rcp;
 
 namespace {
 
@@ -116,14 +119,6 @@ __device__ __forceinline__ int coarse_count(const float* a, const float* b2, int
   return c;
 }
 
-// 1 / x to rounding level: the hardware's approximation (rcp.approx.ftz.f64, about 20 bits) and one third-order
-// Newton step r (1 + e + e^2), e = 1 - x r (error e^3).
-__device__ __forceinline__ double fast_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
 __device__ __forceinline__ unsigned long long abs_bits(double x) {
   return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
 }
@@ -672,6 +667,11 @@ __global__ void __launch_bounds__(256) subband_cleanup_kernel(double* __restrict
     for (int i = lane; i < ny; i += 32) v[i] = -v[i];
 }
 
+__global__ void rcp_kernel(const double* __restrict__ x, double* __restrict__ y, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) y[i] = fast_rcp(x[i]);
+}
+
 size_t slice_smem(int ny) { return (size_t)slice_doubles(ny) * sizeof(double); }
 
 int warps_per_block(int ny) {
@@ -693,6 +693,21 @@ struct wg_subbands {
 };
 
 extern "C" {
+
+int wg_debug_rcp(const double* x, double* y, long long n) {
+  if (!x || !y || n < 1 || n > (1ll << 28)) return WG_ERR_ARG;
+  double* d = nullptr;
+  const size_t sz = (size_t)n * sizeof(double);
+  cudaError_t e = cudaMalloc(&d, 2 * sz);
+  if (e == cudaSuccess) e = cudaMemcpy(d, x, sz, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    rcp_kernel<<<(unsigned)((n + 255) / 256), 256>>>(d, d + n, n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(y, d + n, sz, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? WG_OK : WG_ERR_CUDA;
+}
 
 int wg_subbands_create(int batch, int n_valleys, int nx, int ny, int n_modes, wg_subbands** out) {
   if (!out) return WG_ERR_ARG;
