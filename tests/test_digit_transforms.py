@@ -152,3 +152,27 @@ def test_more_nodes_than_grid_rows(built_lib, kind):
             x[-1] = rng.normal(size=P.N) + 1j * rng.normal(size=P.N) if not out else out[0][0]
             out.append((x[-1].copy(), P.apply(x).reshape(b, -1)[-1].copy()))
     assert np.array_equal(out[0][1], out[1][1]) and np.linalg.norm(out[1][1]) > 0
+
+
+@pytest.mark.parametrize("kind", ["normal", "decades in k", "decades over elements"])
+@pytest.mark.parametrize("n_el,nk,nxi,order", [(6, 16, 16, 1), (4, 36, 52, 2), (5, 64, 64, 3), (40, 60, 64, 1)])
+def test_all_digits_count(built_lib, n_el, nk, nxi, order, kind):
+    """The potential term (the flux is made negligible by a heavy m_diff) against the native kernels, per element.  Native
+    sums of up to 32 pairs carry about sqrt(32) / 2 roundings, 3e-16 a transform, the digits one, so both transforms
+    differ by about 5e-16 of the result: 8e-16 is allowed.  The largest entry of a column in units of its rms is about 3,
+    so seven digits of 7 bits (2^-50 of it per entry) are off by 1.5e-15 a transform at least (1.8e-14 measured)."""
+    rng = np.random.default_rng(nk)
+    out = []
+    for tc in (-1, True):
+        with _problem(n_el, nk, nxi, order, fp64_tc=tc, m_diff=1e-22) as P:
+            if not out:
+                x = rng.normal(size=(n_el, order + 1, nk)) + 1j * rng.normal(size=(n_el, order + 1, nk))
+                if kind == "decades in k":
+                    x *= 10.0 ** rng.uniform(-12, 0, (1, 1, nk))
+                if kind == "decades over elements":
+                    x *= 10.0 ** rng.uniform(-100, 100, (n_el, 1, 1))
+                    x[1::2] = 0.0     # the flux takes one node of a neighbour
+            out.append(P.apply(x.ravel()).reshape(n_el, -1))
+    want, got = out
+    on = np.linalg.norm(want, axis=1) > 0 if kind != "decades over elements" else np.arange(n_el) % 2 == 0
+    assert np.all(np.linalg.norm((got - want)[on], axis=1) <= 8e-16 * np.linalg.norm(want[on], axis=1))

@@ -140,3 +140,53 @@ def test_transient_dropin_from_init_matches_oracle(built_lib):
     assert np.array_equal(DG["n_over_t"][:, 0, 1], DG["n_all"][:, 50])
     assert np.array_equal(DG["j_over_t"][:, 3], DG["j_all"][:, 15])
     assert rel(DG["rho_INIT"][0], ref["rho"]) < 1e-9
+
+
+@pytest.mark.gpu
+def test_shifted_steps_with_an_odd_number_of_wave_numbers(built_lib):
+    """Crank-Nicolson with Nk = 33: the shift gives the wave number 0 a line block of its own, so the step solves'
+    preconditioner inverts it too, which the stationary one does not.  From the device's stationary state against the
+    oracle (1e-8 as for even Nk), and back on the stationary operator."""
+    from real_space_dg_gb300 import devices
+    spec, mat, *_ = small_rtd(n_el=10, nk=33, order=2)
+    dy = devices.density_normalisation_nm(mat)
+    S = _gpu_sweep(mat, dy, 1)
+    try:
+        rho0, phi0 = S.P.rho(0), S.get(0)[0]
+        S.step_bias(0, 0.15)
+        st, info, n, j = S.transient(1e-15, 8, "cn", scale_a=2e-10, refresh_every=5, refresh_first=3, tol=1e-12,
+                                     maxit=40)
+        assert st == 0
+        assert S.P.solve(tol=1e-10, maxit=60)[0] == 0
+    finally:
+        S.close()
+    ref = transient1d.transient(mat, rho0, phi0, 0.15, 1e-15, 8, dy_nm=dy, method="cn", scale_a=2e-10,
+                                scale_rhs=2e-10, refresh_every=5, refresh_first=3)
+    for t in range(8):
+        assert rel(n[t, 0], ref["n"][t]) < 1e-8 and rel(j[t, 0], ref["j"][t]) < 1e-8, t
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("method,dt", [("cn", 1e-15), ("rk4", 1e-18)])
+def test_large_fp64_transient_on_both_kinds_of_transforms(built_lib, method, dt):
+    """An FP64 handle above the size from which its transforms are digit products (potential part alone in the shifted
+    step solves) against native FP64: both within the step solves' 1e-12, compared at the 1e-8 of this file (RK4: 1e-9)."""
+    from real_space_dg_gb300 import devices
+    from real_space_dg_gb300.rtd import RTDSweep
+    spec, mat, *_ = small_rtd(n_el=58, nk=512, order=3, n_xi=512)
+    mat = dict(mat, dy_norm_nm=devices.density_normalisation_nm(mat))
+    out = []
+    for tc in (False, -1):
+        S = RTDSweep(mat, 2, dict(fp64TensorCores=tc, restart=30))
+        try:
+            for b, v in enumerate((0.05, 0.1)):
+                S.set(b, v)
+                S.step_bias(b, v + 0.05)
+            st, info, n, j = S.transient(dt, 4, method, refresh_every=2, refresh_first=2, tol=1e-12, maxit=40)
+            assert st == 0
+            out.append((n, j))
+        finally:
+            S.close()
+    tol = 1e-8 if method == "cn" else 1e-9
+    assert rel(out[0][0], out[1][0]) < tol and rel(out[0][1], out[1][1]) < tol
+    assert np.linalg.norm(out[1][0]) > 0
