@@ -1232,6 +1232,13 @@ int fail(wg2d_problem* h, int code, const std::string& msg) {
     if (e_ != cudaSuccess) return fail(h, WG_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e_) + " at " #expr); \
   } while (0)
 
+// The limit of dynamic shared memory belongs to the kernel, not to a handle: set to the largest block's, so that a later
+// handle of a smaller shape does not lower it for the ones that are there.
+template <typename F>
+cudaError_t lift_smem(F* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
 template <typename T>
 cudaError_t dalloc(T** p, size_t n) {
   return cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * (n ? n : 1));
@@ -1513,9 +1520,7 @@ int wg2d_create(const wg2d_shape* s, wg2d_problem** out) {
   if (e == cudaSuccess) e = cudaMemset(h->tc_err, 0, sizeof(int));
   for (cudaEvent_t& ev : h->ev)
     if (e == cudaSuccess) e = cudaEventCreate(&ev);
-  if (e == cudaSuccess && h->nrx * kColPitch<double2> * sizeof(double2) > 48 * 1024)
-    e = cudaFuncSetAttribute(f2d_relx_kernel<double2, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(h->nrx * kColPitch<double2> * sizeof(double2)));
+  if (e == cudaSuccess) e = lift_smem(f2d_relx_kernel<double2, double>);
   if (e != cudaSuccess) {
     wg2d_destroy(h);
     return e == cudaErrorMemoryAllocation ? WG_ERR_OOM : WG_ERR_CUDA;
@@ -1781,17 +1786,13 @@ static cudaError_t xline_maps(wg2d_problem* h, const T* xinv, const T* xcpl) {
   return cudaGetLastError();
 }
 
-// Shared memory of the preconditioner's kernels of one precision beyond the default limit.
+// The preconditioner's kernels of one precision beyond the default limit of shared memory.
 template <typename T>
-static cudaError_t precond_attributes(wg2d_problem* h) {
-  const int tsm = (int)tx_smem(h->nT, sizeof(T)), msm = (int)(sizeof(T) * kColPitch<T> * modal_rows(h->nrx));
-  cudaError_t e = cudaFuncSetAttribute(f2d_transverse_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(f2d_transverse_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
-  if (e == cudaSuccess && msm > 48 * 1024)
-    e = cudaFuncSetAttribute(f2d_modal_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, msm);
-  if (e == cudaSuccess && msm > 48 * 1024)
-    e = cudaFuncSetAttribute(f2d_modal_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, msm);
+static cudaError_t precond_attributes() {
+  cudaError_t e = lift_smem(f2d_transverse_kernel<T, true>);
+  if (e == cudaSuccess) e = lift_smem(f2d_transverse_kernel<T, false>);
+  if (e == cudaSuccess) e = lift_smem(f2d_modal_kernel<T, true>);
+  if (e == cudaSuccess) e = lift_smem(f2d_modal_kernel<T, false>);
   return e;
 }
 
@@ -2029,9 +2030,7 @@ static int ensure32(wg2d_problem* h) {
   F2_CK(dalloc(&h->Uq32, slab * h->nrel));
   F2_CK(dalloc(&h->Rq32, slab * h->nrel));
   F2_CK(dalloc(&h->G32, (size_t)std::max(1, std::max(h->ax[0].T, h->ax[1].T)) * h->n));
-  if (h->nrx * kColPitch<float2> * sizeof(float2) > 48 * 1024)
-    F2_CK(cudaFuncSetAttribute(f2d_relx_kernel<float2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(h->nrx * kColPitch<float2> * sizeof(float2))));
+  F2_CK((lift_smem(f2d_relx_kernel<float2, float>)));
   F2_CK(cudaStreamSynchronize(h->stream));
   h->d32_ready = true;
   return WG_OK;
@@ -2155,7 +2154,7 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
     if (rc) return rc;
     F2_CK(dalloc(&h->pa32, h->n));
     F2_CK(dalloc(&h->pb32, h->n));
-    F2_CK(precond_attributes<float2>(h));
+    F2_CK(precond_attributes<float2>());
     F2_CK(xline_maps(h, h->xinv32, h->xcpl32));
     h->pre32 = true;
     h->pre_ready = true;
@@ -2169,7 +2168,7 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
   F2_CK(cudaMemcpy(h->xinv, x_inverse, sizeof(double2) * nx, cudaMemcpyHostToDevice));
   F2_CK(cudaMemcpy(h->xcpl, x_coupling, sizeof(double2) * nx, cudaMemcpyHostToDevice));
   F2_CK(cudaMemcpy(h->tinv, ti.data(), sizeof(double2) * nt, cudaMemcpyHostToDevice));
-  F2_CK(precond_attributes<double2>(h));
+  F2_CK(precond_attributes<double2>());
   F2_CK(xline_maps(h, h->xinv, h->xcpl));
   if (h->s.tensor_cores) {
     int rc = wg::ozaki_rows_upload(embed(U, nr, 1.0, true), 2 * nr, 2 * nr, h->UH, h->err);

@@ -733,9 +733,9 @@ int wg_subbands_create(int batch, int n_valleys, int nx, int ny, int n_modes, wg
   if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&h->kfirst, slices * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&h->fallback, (2 * slices + 1) * sizeof(int));
-  if (e == cudaSuccess && warps_per_block(ny) * slice_smem(ny) > 48 * 1024)
-    e = cudaFuncSetAttribute(subband_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(warps_per_block(ny) * slice_smem(ny)));
+  // the largest block's limit: it belongs to the kernel, and a later handle must not lower it for this one
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(subband_bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
   if (e != cudaSuccess) {
     wg_subbands_destroy(h);
     cudaGetLastError();
