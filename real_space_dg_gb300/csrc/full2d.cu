@@ -1232,6 +1232,13 @@ int fail(wg2d_problem* h, int code, const std::string& msg) {
     if (e_ != cudaSuccess) return fail(h, WG_ERR_CUDA, std::string("CUDA: ") + cudaGetErrorString(e_) + " at " #expr); \
   } while (0)
 
+// Upload that is complete on return: a copy from pageable memory may return with its last part still on the way, and the
+// handles' streams do not wait for the default stream.
+cudaError_t h2d(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // The limit of dynamic shared memory belongs to the kernel, not to a handle: set to the largest block's, so that a later
 // handle of a smaller shape does not lower it for the ones that are there.
 template <typename F>
@@ -1280,9 +1287,9 @@ cudaError_t ell_upload(const wg2d_problem::Axis& a, int nr, EllTerms<T>& out) {
   cudaError_t e = dalloc(&out.col, col.size());
   if (e == cudaSuccess) e = dalloc(&out.val, val.size());
   if (e == cudaSuccess) e = dalloc(&out.count, count.size());
-  if (e == cudaSuccess) e = cudaMemcpy(out.col, col.data(), sizeof(int) * col.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(out.val, val.data(), sizeof(T) * val.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(out.count, count.data(), sizeof(int) * count.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = h2d(out.col, col.data(), sizeof(int) * col.size());
+  if (e == cudaSuccess) e = h2d(out.val, val.data(), sizeof(T) * val.size());
+  if (e == cudaSuccess) e = h2d(out.count, count.data(), sizeof(int) * count.size());
   return e;
 }
 
@@ -1517,7 +1524,7 @@ int wg2d_create(const wg2d_shape* s, wg2d_problem** out) {
   if (e == cudaSuccess) e = dalloc(&h->vy, h->nvert);
   if (e == cudaSuccess) e = dalloc(&h->cap, h->nrel);
   if (e == cudaSuccess) e = dalloc(&h->tc_err, 1);
-  if (e == cudaSuccess) e = cudaMemset(h->tc_err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->tc_err, 0, sizeof(int), h->stream);
   for (cudaEvent_t& ev : h->ev)
     if (e == cudaSuccess) e = cudaEventCreate(&ev);
   if (e == cudaSuccess) e = lift_smem(f2d_relx_kernel<double2, double>);
@@ -1579,8 +1586,8 @@ int wg2d_set_transport(wg2d_problem* h, int axis, int n_terms, const double* coe
   const size_t nb = (size_t)n_terms * n_el * 3 * nk * nk;
   F2_CK(dalloc(&a.blocks, nb));
   F2_CK(dalloc(&a.dcoef, n_terms));
-  F2_CK(cudaMemcpy(a.blocks, center_blocks, sizeof(double) * nb, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(a.dcoef, coef, sizeof(double) * n_terms, cudaMemcpyHostToDevice));
+  F2_CK(h2d(a.blocks, center_blocks, sizeof(double) * nb));
+  F2_CK(h2d(a.dcoef, coef, sizeof(double) * n_terms));
   a.rp.assign(row_ptr, row_ptr + (size_t)n_terms * (nr + 1));
   a.col.assign(col, col + off[n_terms]);
   a.val.assign(val, val + 2 * (size_t)off[n_terms]);
@@ -1885,7 +1892,7 @@ int wg2d_set_transport_masks(wg2d_problem* h, int axis, int n_terms, const unsig
   if (!masks) return WG_OK;
   const size_t nm = (size_t)n_terms * h->nY;
   F2_CK(cudaMalloc(&a.ymask, nm));
-  F2_CK(cudaMemcpy(a.ymask, masks, nm, cudaMemcpyHostToDevice));
+  F2_CK(h2d(a.ymask, masks, nm));
   // a masked term leaves the dense tensor-core path (which applies a term on every column)
   for (int t = 0; t < n_terms; ++t) {
     bool all = true;
@@ -1922,9 +1929,9 @@ int wg2d_set_hard_wall(wg2d_problem* h, const unsigned char* active, const doubl
   F2_CK(dalloc(&h->wall_T32, nt));
   F2_CK(dalloc(&h->wall_u, h->n));
   F2_CK(dalloc(&h->wall_u32, h->n));
-  F2_CK(cudaMemcpy(h->wall_act, active, na, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(h->wall_T, projection, sizeof(double) * nt, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(h->wall_T32, t32.data(), sizeof(float) * nt, cudaMemcpyHostToDevice));
+  F2_CK(h2d(h->wall_act, active, na));
+  F2_CK(h2d(h->wall_T, projection, sizeof(double) * nt));
+  F2_CK(h2d(h->wall_T32, t32.data(), sizeof(float) * nt));
   h->wall_scale = scale;
   h->wall = true;
   return WG_OK;
@@ -2121,7 +2128,7 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
     if (h->x_chunks > 1) F2_CK(dalloc(&h->xmaps, (size_t)nr * h->x_chunks * nk * nk));
   }
   F2_CK(dalloc(&h->fwd, nr));
-  F2_CK(cudaMemcpy(h->fwd, forward, sizeof(int) * nr, cudaMemcpyHostToDevice));
+  F2_CK(h2d(h->fwd, forward, sizeof(int) * nr));
   // U^H and U / sigma as complex [nr][nr], transposed; the transverse inverses transposed per mode
   const size_t nu = (size_t)nr * (modal_rows(nr) + 4);   // zero rows past nr
   std::vector<double> uh(2 * nu, 0.0), us(2 * nu, 0.0), ti(2 * nt);
@@ -2143,7 +2150,7 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
       std::vector<float> f(2 * count);
       for (size_t i = 0; i < 2 * count; ++i) f[i] = (float)src[i];
       F2_CK(dalloc(dst, count));
-      F2_CK(cudaMemcpy(*dst, f.data(), sizeof(float) * f.size(), cudaMemcpyHostToDevice));
+      F2_CK(h2d(*dst, f.data(), sizeof(float) * f.size()));
       return WG_OK;
     };
     int rc = up32(&h->xinv32, x_inverse, nx);
@@ -2165,9 +2172,9 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
   F2_CK(dalloc(&h->tinv, nt));
   F2_CK(dalloc(&h->pa, h->n));
   F2_CK(dalloc(&h->pb, h->n));
-  F2_CK(cudaMemcpy(h->xinv, x_inverse, sizeof(double2) * nx, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(h->xcpl, x_coupling, sizeof(double2) * nx, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(h->tinv, ti.data(), sizeof(double2) * nt, cudaMemcpyHostToDevice));
+  F2_CK(h2d(h->xinv, x_inverse, sizeof(double2) * nx));
+  F2_CK(h2d(h->xcpl, x_coupling, sizeof(double2) * nx));
+  F2_CK(h2d(h->tinv, ti.data(), sizeof(double2) * nt));
   F2_CK(precond_attributes<double2>());
   F2_CK(xline_maps(h, h->xinv, h->xcpl));
   if (h->s.tensor_cores) {
@@ -2178,8 +2185,8 @@ int wg2d_set_preconditioner(wg2d_problem* h, const double* U, double sigma, cons
   } else {
     F2_CK(dalloc(&h->UHd, nu));
     F2_CK(dalloc(&h->Usd, nu));
-    F2_CK(cudaMemcpy(h->UHd, uh.data(), sizeof(double) * uh.size(), cudaMemcpyHostToDevice));
-    F2_CK(cudaMemcpy(h->Usd, us.data(), sizeof(double) * us.size(), cudaMemcpyHostToDevice));
+    F2_CK(h2d(h->UHd, uh.data(), sizeof(double) * uh.size()));
+    F2_CK(h2d(h->Usd, us.data(), sizeof(double) * us.size()));
   }
   h->pre_ready = true;
   return WG_OK;
@@ -2626,8 +2633,8 @@ int wg2d_set_observables(wg2d_problem* h, const wg2d_observables_desc* d, const 
   F2_CK(dalloc(&h->obs_W, nty * h->nY));
   F2_CK(dalloc(&h->obs_wj, nty));
   F2_CK(dalloc(&h->obs_out, (size_t)3 * h->nX * h->nY + (size_t)3 * h->nX * nty + h->nX));
-  F2_CK(cudaMemcpy(h->obs_W, W, sizeof(double) * nty * h->nY, cudaMemcpyHostToDevice));
-  F2_CK(cudaMemcpy(h->obs_wj, wj, sizeof(double) * nty, cudaMemcpyHostToDevice));
+  F2_CK(h2d(h->obs_W, W, sizeof(double) * nty * h->nY));
+  F2_CK(h2d(h->obs_wj, wj, sizeof(double) * nty));
   h->obs = *d;
   h->obs_ready = true;
   return WG_OK;

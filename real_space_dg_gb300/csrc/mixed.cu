@@ -793,6 +793,7 @@ int ozaki_alloc(Problem& P, bool own) {
     C2(cudaMemcpy(M.oa2, d2.data(), sizeof(bf16) * d2.size(), cudaMemcpyHostToDevice));
     C2(cudaMemcpy(M.ea1, e1.data(), sizeof(int) * e1.size(), cudaMemcpyHostToDevice));
     C2(cudaMemcpy(M.ea2, e2.data(), sizeof(int) * e2.size(), cudaMemcpyHostToDevice));
+    C2(cudaStreamSynchronize(cudaStreamLegacy));   // P.stream does not wait for the default stream
     if (ce != cudaSuccess) {
       P.err = std::string("FP64 tensor-core buffers: ") + cudaGetErrorString(ce);
       return ce == cudaErrorMemoryAllocation ? WG_ERR_OOM : WG_ERR_CUDA;
@@ -1110,6 +1111,7 @@ int ozaki_rows_upload(const std::vector<double>& A, int M, int K, OzakiRowsDev& 
   if (ce == cudaSuccess) ce = cudaMalloc(&out.e, sizeof(int) * e.size());
   if (ce == cudaSuccess) ce = cudaMemcpy(out.dig, dig.data(), sizeof(bf16) * dig.size(), cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMemcpy(out.e, e.data(), sizeof(int) * e.size(), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(cudaStreamLegacy);   // the caller's stream does not wait for it
   if (ce != cudaSuccess) {
     err = std::string("emulated GEMM rows: ") + cudaGetErrorString(ce);
     ozaki_free(out);

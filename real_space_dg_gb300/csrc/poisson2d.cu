@@ -555,6 +555,8 @@ template <typename T>
 cudaError_t upload(T** d, const std::vector<T>& h) {
   cudaError_t e = cudaMalloc(d, std::max<size_t>(1, h.size()) * sizeof(T));
   if (e == cudaSuccess && !h.empty()) e = cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+  // the copy may return with its last part on the way, and the streams that read it do not wait for the default stream
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
   return e;
 }
 
@@ -793,6 +795,7 @@ int wg_poisson2d_create(const wg_poisson2d_desc* d, const double* eps_r, const u
     }
     if (e == cudaSuccess) e = cudaMalloc(&h->w.count, G * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(h->w.count, 0, G * sizeof(int));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
   }
   if (e == cudaSuccess) e = cudaMalloc(&h->info, (size_t)B * sizeof(wg_poisson2d_info));
   if (e != cudaSuccess) {

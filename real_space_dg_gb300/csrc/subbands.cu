@@ -731,6 +731,7 @@ int wg_subbands_create(int batch, int n_valleys, int nx, int ny, int n_modes, wg
   if (e == cudaSuccess) e = cudaMalloc(&h->dm, slices * n_modes * ny * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&h->err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // the solves' streams do not wait for it
   if (e == cudaSuccess) e = cudaMalloc(&h->kfirst, slices * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&h->fallback, (2 * slices + 1) * sizeof(int));
   // the largest block's limit: it belongs to the kernel, and a later handle must not lower it for this one
