@@ -80,30 +80,42 @@ bool make_map3(CUtensorMap* m, const void* base, long long rows, int K, int box_
 // Digits of the rows of a row-major M x K FP64 matrix (host), the split of slice_columns_kernel (bits = 6) and
 // slice_pairs_kernel (7): row r with max|a| < 2^m has F = round(a 2^(bits S-1-m)) written
 // in balanced digits, a = 2^e[r] sum_p t_p 2^(-bits(p+1)), e[r] = m + 1.
+// Runs at every creation of a handle with such tables: one multiplication per entry and a table of the digits' values
+// (conversions and ldexp per digit had taken twice as long, 4.3 ms of a handle with Nk = 512).
 void slice_rows_host(const std::vector<double>& A, int M, int K, std::vector<bf16>& dig, std::vector<int>& e,
                      int bits = oz::BETA) {
   const long long half = 1ll << (bits - 1), digit = (1ll << bits) - 1;
-  dig.assign((size_t)oz::S * M * K, __float2bfloat16(0.f));
+  static const std::vector<bf16> values = [] {
+    std::vector<bf16> v;
+    for (int d = -64; d <= 64; ++d) v.push_back(__float2bfloat16((float)d));
+    return v;
+  }();
+  const bf16* value = values.data() + 64;
+  const size_t plane = (size_t)M * K;
+  dig.assign(oz::S * plane, value[0]);
   e.assign(M, 0);
   for (int r = 0; r < M; ++r) {
+    const double* row = &A[(size_t)r * K];
     double mx = 0;
-    for (int k = 0; k < K; ++k) mx = std::max(mx, std::fabs(A[(size_t)r * K + k]));
+    for (int k = 0; k < K; ++k) mx = std::max(mx, std::fabs(row[k]));
     if (mx == 0) continue;
     int m;
     std::frexp(mx, &m);   // mx = f 2^m, 0.5 <= f < 1
     e[r] = m + 1;
+    const int shift = bits * oz::S - 1 - m;
+    const double scale = std::ldexp(1.0, std::min(shift, 1000));   // a power of two: the product is exact
     for (int k = 0; k < K; ++k) {
-      const double a = A[(size_t)r * K + k];
       // 6 bits: |a| 2^(6S-1-m) < 2^47, adding one half is exact; 7 bits: up to 2^55, an integer from 2^52 on
-      const double scaled = std::ldexp(std::fabs(a), bits * oz::S - 1 - m);
+      const double scaled = shift <= 1000 ? std::fabs(row[k]) * scale : std::ldexp(std::fabs(row[k]), shift);
       long long F = bits == oz::BETA ? (long long)std::floor(scaled + 0.5) : std::llrint(scaled);
-      if (a < 0) F = -F;
+      if (row[k] < 0) F = -F;
+      bf16* out = &dig[(size_t)r * K + k];
       for (int p = oz::S - 1; p > 0; --p) {
         const long long d = ((F + half) & digit) - half;
-        dig[((size_t)p * M + r) * K + k] = __float2bfloat16((float)d);
+        out[p * plane] = value[d];
         F = (F - d) >> bits;
       }
-      dig[(size_t)r * K + k] = __float2bfloat16((float)F);
+      *out = value[F];
     }
   }
 }
