@@ -838,11 +838,12 @@ cudaError_t mixed_sync_weights(Problem& P) {
   const int ne = s.nxi + 1, ne4 = P.mx.ne4, np = pair_count(s.nK);
   const long long rows = (long long)P.batch * s.n_el;
   const long long nb = rows * np * ne4, ni = (long long)s.nK * s.nK * ne4;
-  P.prof.launches[PROF_OTHER] += 6;
+  P.prof.launches[PROF_OTHER] += P.mx.fused ? 6 : 5;
   pack_weights_kernel<<<(unsigned)((nb + 255) / 256), 256, 0, P.stream>>>(P.beta, P.mx.beta, rows, s.nK, np, false,
                                                                           ne, ne4);
-  pack_weights_kernel<<<(unsigned)((ni + 255) / 256), 256, 0, P.stream>>>(P.betai, P.mx.betai, 1, s.nK,
-                                                                          s.nK * s.nK, true, ne, ne4);
+  if (P.mx.fused)   // the stencil kernel takes the absorbing part as a product (cap, capk)
+    pack_weights_kernel<<<(unsigned)((ni + 255) / 256), 256, 0, P.stream>>>(P.betai, P.mx.betai, 1, s.nK,
+                                                                            s.nK * s.nK, true, ne, ne4);
   d2f_kernel<<<(P.batch + 255) / 256, 256, 0, P.stream>>>(P.qd, P.mx.qd, P.batch);
   d2f_kernel<<<(unsigned)((s.nk + 255) / 256), 256, 0, P.stream>>>(P.kvec, P.mx.kvec, s.nk);
   const long long nd = (long long)P.batch * s.nk * s.nK * s.nK, nh = (long long)P.batch * s.nk * s.nK;
