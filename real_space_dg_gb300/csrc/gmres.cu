@@ -185,14 +185,11 @@ __device__ __forceinline__ R warp_sum8(R (&v)[8]) {
 // reduces the partials into the Hessenberg column.  The warps drop their sums of four vectors (real and
 // imaginary parts: 8 values) in shared memory and the block adds them at the end.
 //
-// FP32 vectors, basis of VB (FP16 or FP32): one block per (`quads` groups of four elements, problem), all blocks
-// resident at once (gs_quads); 2,048 elements of w at a time stay in registers, two basis vectors are loaded
-// (16 bytes per load) while two are summed.  Bound by HBM; with few vectors by the fixed latencies of a block (w, the
-// fence and the ticket), which every further wave of blocks paid again.
-// 16 problems of 245,760 unknowns: 25 -> 18 us with one vector, 82 -> 75 us with 20 (346 MB); 4 of 368,640, over a
-// solve: 21.1 -> 18.0 us.  (Tried and slower: the copies through a shared-memory ring, and this kernel and the update in
+// FP32 vectors, basis of VB (FP16 or FP32): one block per (`quads` groups of four elements, problem; dot_quads); 2,048
+// elements of w at a time stay in registers, two basis vectors are loaded (16 bytes per load) while two are summed.
+// Bound by HBM; with few vectors by the fixed latencies of a block (w, the fence and the ticket), which every further
+// wave of blocks pays again.  (Tried and slower: the copies through a shared-memory ring, and this kernel and the update in
 // one launch by problem so that the basis stays in the L2: 150 us against 141 us for both.)
-constexpr int kMdChunk = 2048;
 template <typename VB>
 __global__ void __launch_bounds__(256, 3) multidot32_kernel(const VB* __restrict__ V, const float2* __restrict__ w,
                                                             double2* __restrict__ partial,
@@ -362,10 +359,8 @@ __device__ void update_tail(Acc& a, const int b, double* __restrict__ nrm_partia
 
 // w -= sum_i V_i hcol_i, FP32 vectors: 128 threads of four consecutive complex values, the loads of eight
 // basis vectors in flight per thread (16 bytes each of an FP16 basis), the next four before the last four are used.
-// Bound by HBM.  One wave of blocks as in the multi-dot; the problems in the reverse of its order, so that the
-// basis vectors that one of the two reads last are the first of the other while they are in the L2.
-// 16 problems of 245,760 unknowns: 29 -> 21 us with one vector, 105 -> 64 us with 20; 4 of 368,640, over a solve:
-// 22.0 -> 18.8 us.
+// Bound by HBM.  The problems in the reverse of the multi-dot's order, so that the basis vectors that one of the two
+// reads last are the first of the other while they are in the L2.
 constexpr int kUp32Threads = 128;
 template <int MODE, typename VB>
 __global__ void __launch_bounds__(kUp32Threads, 8) gs_update32_kernel(const VB* __restrict__ V,
@@ -596,8 +591,7 @@ int arnoldi_step(Problem& P, VB* V, T* w, int k, int m, bool pre, Prec prec, App
   const int nv = k + 1;
   const double vec = (double)N * B * sizeof(T), vecb = (double)N * B * sizeof(VB);
   constexpr bool f32 = std::is_same<T, float2>::value;
-  // FP32: one wave of blocks
-  const int mq = gs_quads(N, B, 3, kMdChunk / 4), uq = gs_quads(N, B, 8, kUp32Threads);
+  const int mq = dot_quads(N), uq = update_quads(N);
   const int mblk = (int)((N / 4 + mq - 1) / mq);
   const int nblk = f32 ? (int)((N / 4 + uq - 1) / uq) : (int)((N + 255) / 256);
   const dim3 gu(nblk, B);

@@ -341,16 +341,13 @@ __global__ void __launch_bounds__(kFusedThreads<R>) kline_fused_kernel(
     }
 }
 
-// Lines per block of the fused form: about 256 threads, and no fewer lines than make 64-byte rows; fewer lines
-// while the grid leaves SMs idle.  0 where the two-kernel form is taken (long chunks, or too many of them).
+// Lines per block of the fused form: those that make 64-byte rows (with more, a block's 256 threads are reached at a few
+// chunks, and a lone problem leaves SMs idle).  The scan's order follows from it, so it does not depend on the
+// batch.  0 where the two-kernel form is taken (long chunks, or too many of them).
 template <typename R, int NK>
-inline int fused_lines(int n_el, int nk, int batch, int L) {
-  constexpr int least = 64 / (2 * (int)sizeof(R));
-  const int nc = (n_el + L - 1) / L;
-  if (L > FusedLen<R, NK>::value || nc * least > kFusedThreads<R>) return 0;
-  int kl = 32;
-  while (kl > least && (kl * nc > 256 || (long long)((nk + kl - 1) / kl) * batch < 152)) kl /= 2;
-  return kl;
+inline int fused_lines(int n_el, int L) {
+  constexpr int lines = 64 / (2 * (int)sizeof(R));
+  return L > FusedLen<R, NK>::value || (n_el + L - 1) / L * lines > kFusedThreads<R> ? 0 : lines;
 }
 
 // Elements per chunk L.  The default: about 32 chunks per line (the incoming-state fold

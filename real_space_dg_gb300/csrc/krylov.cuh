@@ -230,12 +230,12 @@ __global__ void backsolve_kernel(const double2* __restrict__ H, const double2* _
     }
 }
 
-// Groups of four elements per block of the FP32 Gram-Schmidt kernels: one wave of `per_sm` blocks on each SM
-// for the batch, at least `least` groups, whole warps.
-inline int gs_quads(long long N, int B, int per_sm, int least) {
-  const long long blocks = std::max(1, 152 * per_sm / B), q = (N / 4 + blocks - 1) / blocks;
-  return (int)std::max<long long>(least, (q + 31) / 32 * 32);
-}
+// Groups of four elements per block of the FP32 Gram-Schmidt kernels, a rule on the size of one problem alone: a problem's
+// sums, and with them its bits, do not depend on the batch it is in.  Pieces of 4,096 and 2,048 elements against
+// one wave of blocks for the batch, whole solves: 8 problems of 153,600 unknowns 26.7 and 26.6 ms, 16 of 245,760 63.4
+// and 64.0, eight concurrent handles of 2 such 211 and 204, 4 of 368,640 67.9 and 67.5.  Half of both: 27.1, 64.0, 206, 69.3.
+inline int dot_quads(long long N) { return N >= 1 << 17 ? 1024 : 512; }
+inline int update_quads(long long N) { return N >= 1 << 17 ? 512 : N >= 1 << 16 ? 256 : 128; }
 
 }  // namespace
 }  // namespace wg

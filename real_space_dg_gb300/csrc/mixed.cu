@@ -586,7 +586,7 @@ cudaError_t precond_mixed_nk(Problem& P, const float2* r, long long r_stride, fl
   float* ma = static_cast<float*>(P.kmap_a);
   float2* ms = static_cast<float2*>(P.kmap_s);
   const double written = (z ? 8.0 : 0.0) + (zb ? 4.0 : 0.0) + (rout ? (double)sizeof(O) : 0.0);
-  if (const int KL = kline::fused_lines<float, NK>(P.s.n_el, P.s.nk, P.batch, L)) {
+  if (const int KL = kline::fused_lines<float, NK>(P.s.n_el, L)) {
     const int th = (KL * nc + 31) / 32 * 32;
     cudaEvent_t fe = prof_begin(P, PROF_PRECOND, 1, (8.0 + written) * P.N * P.batch, 0, mask);
     kline::kline_fused_kernel<NK, float, O><<<dim3((P.s.nk + KL - 1) / KL, P.batch), th, 12 * KL * (th / 32), P.stream>>>(

@@ -514,7 +514,7 @@ cudaError_t precond_nk(Problem& P, const double2* r, long long r_stride, double2
   const dim3 block(32, kline::kChunksPerBlock);
   double* ma = static_cast<double*>(P.kmap_a);
   double2* ms = static_cast<double2*>(P.kmap_s);
-  if (const int KL = kline::fused_lines<double, NK>(P.s.n_el, P.s.nk, P.batch, L)) {
+  if (const int KL = kline::fused_lines<double, NK>(P.s.n_el, L)) {
     const int th = (KL * nc + 31) / 32 * 32;
     cudaEvent_t fe = prof_begin(P, PROF_PRECOND, 1, (32.0 + (rout ? 16.0 : 0.0)) * P.N * P.batch);
     kline::kline_fused_kernel<NK, double><<<dim3((P.s.nk + KL - 1) / KL, P.batch), th, 24 * KL * (th / 32), P.stream>>>(
