@@ -196,16 +196,19 @@ __device__ __forceinline__ double right_entry(const P2Dev& P, int c, int i) {
 // are diagonal and come from the stencil), then an even k eliminates: [X_L X_U y] = D^-1 [L U r]; an odd k stores
 // the folded blocks.  Thread (i, q) keeps row i, columns q + t TPR of the augmented matrix in registers.
 //
-// A warp's FP64 instruction takes its SM quarter's pipe for 64 cycles and returns after as many, so a block is
-// four warps (one per quarter) at up to 16 rows, and what counts in a latter level, where a handful of blocks run,
-// is instructions per pivot: CPT updates, one product, and the reciprocal (4, by the pivot's warp alone).  Both
-// neighbours in one block (eliminating a shared one twice) and 1 / x by division took 93, 82 and 44 us at levels 0, 1
-// and 2 of 16 bias points on 361 columns of 12 rows, 436 us for the whole step; here the step takes 346 us (one
-// point on 97 columns of 11 rows: 179 -> 148 us).
+// A warp's FP64 instruction takes its SM quarter's pipe for 64 cycles and returns after as many, so a block has few warps, and
+// what counts in a latter level, where a handful of blocks run, is instructions per pivot: CPT updates, one
+// product, and the reciprocal (4, by the pivot's warp alone).  Both neighbours in one block (eliminating a shared one twice)
+// and 1 / x by division took 93, 82 and 44 us at levels 0, 1 and 2 of 16 bias points on 361 columns of 12 rows, 436 us for
+// the whole step; here it takes 324 us.
+// Columns per thread by width, whole step in us, 16 points of 361 columns and one of 97 (chosen first): 4 rows 122 and 78
+// with 4 columns, 123 and 81 with 3; 8 rows 192 and 91 with 3, 203 and 109 with 4; 12 rows 324 and 122, 336 and 138; 16 rows 523
+// and 157, 538 and 168; 24 rows 1,325 and 369 with 8, 1,419 and 338 with 4; 32 rows 2,896 and 636, 3,541 and 723.  That is 1,
+// 3, 5, 9, 8 and 13 warps a block, one to six at level 0 up to 16 rows.
 template <int NU, int NB>
 struct ReduceShape {
   static constexpr int W = NB * NU + 1;                       // augmented width: NB blocks and r
-  static constexpr int CPT = NU >= 24 ? 8 : (NB == 2 && NU == 12 ? 3 : 4);   // columns per thread
+  static constexpr int CPT = NU >= 24 ? 8 : NU >= 8 ? 3 : 4;   // columns per thread
   static constexpr int TPR = (W + CPT - 1) / CPT;             // threads per row
   static constexpr int THREADS = (NU * TPR + 31) / 32 * 32;
 };
@@ -661,7 +664,7 @@ int wg_poisson2d_create(const wg_poisson2d_desc* d, const double* eps_r, const u
   const int periodic = d->periodic_y ? 1 : 0;
   if (periodic && ny < 3) return WG_ERR_ARG;                       // RTD:PoissonPeriodicMaterial
   const int nu = ny - periodic;
-  if (nu > 32) return WG_ERR_ARG;                                   // the warp-row block sweep
+  if (nu > 32) return WG_ERR_ARG;                                   // the widest blocks of the reduction
   const size_t full = (size_t)nx * ny;
   double emax = 0.0;
   for (size_t k = 0; k < full; ++k) {
