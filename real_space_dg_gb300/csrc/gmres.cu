@@ -188,8 +188,10 @@ __device__ __forceinline__ R warp_sum8(R (&v)[8]) {
 // FP32 vectors, basis of VB (FP16 or FP32): one block per (`quads` groups of four elements, problem; dot_quads); 2,048
 // elements of w at a time stay in registers, two basis vectors are loaded (16 bytes per load) while two are summed.
 // Bound by HBM; with few vectors by the fixed latencies of a block (w, the fence and the ticket), which every further
-// wave of blocks pays again.  (Tried and slower: the copies through a shared-memory ring, and this kernel and the update in
-// one launch by problem so that the basis stays in the L2: 150 us against 141 us for both.)
+// wave of blocks pays again.  16 problems of 245,760 unknowns, 21 vectors: 73 us, 5.0 TB/s (82 us with 20 vectors where a
+// block took one chunk of 2,048 elements and reduced it vector by vector).  Tried and slower: the copies through a
+// shared-memory ring, and this kernel and the update in one launch by problem so that the basis stays in the L2 (150 us
+// against 141 us for both).
 template <typename VB>
 __global__ void __launch_bounds__(256, 3) multidot32_kernel(const VB* __restrict__ V, const float2* __restrict__ w,
                                                             double2* __restrict__ partial,
@@ -360,7 +362,8 @@ __device__ void update_tail(Acc& a, const int b, double* __restrict__ nrm_partia
 // w -= sum_i V_i hcol_i, FP32 vectors: 128 threads of four consecutive complex values, the loads of eight
 // basis vectors in flight per thread (16 bytes each of an FP16 basis), the next four before the last four are used.
 // Bound by HBM.  The problems in the reverse of the multi-dot's order, so that the basis vectors that one of the two
-// reads last are the first of the other while they are in the L2.
+// reads last are the first of the other while they are in the L2.  16 problems of 245,760 unknowns, 21 vectors: 70 us,
+// 5.5 TB/s (105 us with 20 vectors at 512 elements a block).
 constexpr int kUp32Threads = 128;
 template <int MODE, typename VB>
 __global__ void __launch_bounds__(kUp32Threads, 8) gs_update32_kernel(const VB* __restrict__ V,

@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(32 * kChunksPerBlock) kline_apply_kernel(
 
 // Maps, fold and sweep in one launch: thread (line jl, chunk c) of a block of KL lines and all nchunk chunks.  The loads
 // of a thread's whole chunk are in flight together (the two-kernel form had one element's at a time, 1.4 TB/s in
-// its second kernel, and read r twice).  Bound by HBM: r once, z or its BF16 copy and the basis vector written.
+// its second kernel, and read r twice): r once, z or its BF16 copy and the basis vector written.  FP32: bound by the loads
+// that 1.7 waves of blocks keep in flight (63 MB in 18 us, 3.4 TB/s); FP64: by its pipe (55% busy) and the chain of a chunk.
 // 16 problems of 240 elements, Nk = 256, nK = 4, FP16 basis: 32 -> 18 us; 4 of 180 elements, Nk = 512:
 // 18.5 -> 10.7 us; FP64, 2 problems of 240 elements (FP64 pipe, 16 us of sums): 41 -> 31 us.
 template <typename R, int NK> struct FusedLen {   // registers bound it: 32 complex FP32 values, 16 FP64

@@ -550,7 +550,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_pairs_kernel(
 
 // Digits of E and O of every node's complex column (K entries, K even and at most 512), one warp per real column (E re,
 // E im, O re, O im of a node: four warps share its loads through the L1; one warp per node left a chain of 1,900
-// instructions, 14 us at 1,920 nodes of 256 entries against 11), two consecutive pairs per lane and pass; the column
+// instructions, 14 us at 1,920 nodes of 256 entries against 11; bound by the FP64 additions, the pipe is 76% busy), two
+// consecutive pairs per lane and pass; the column
 // stays in registers between its maximum and its digits.  Rows of Kout entries (>= K / 2, zero-padded).  nd, nd_pp:
 // the digits gemm_pairs_kernel reads for the node's tile.  PASSES of 64 entries cover Kout (1, 2 or 4).
 constexpr int kSlicePairNodes = 2;   // per block of eight warps
