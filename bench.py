@@ -162,11 +162,10 @@ def make_workload(batch):
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one timed gemm_f64_tc event of the mixed form (digit
-# slicing + emulated GEMM; the mean of the C = AB and C += AB launches) per state column (element x node), from
-# ncu captures of residuals at 5 digits (profiles/gemm_ozaki_c2_batch8_mixed.md): the GEMMs at batch 8 (7,680
-# columns) 44.5 and 75.8 MB, the slicing at a 2-problem handle (1,920 columns) 7.9 MB (its digit writes stay in
-# L2).  The traffic grows with the columns, so a launch of the bench's batch scales by its columns.
-OZAKI_TRAFFIC_PER_COLUMN = 7.89e6 / 1920 + 0.5 * (44.53e6 + 75.75e6) / 7680
+# slicing + digit products of one transform) per state column (element x node), from ncu captures of a residual at
+# seven digits, 15,360 columns of 256 entries: slicing 62.9 + 53.6 MB, products 110.9 + 25.9 MB.  The traffic grows
+# with the columns, so a launch of the bench's batch scales by its columns.
+OZAKI_TRAFFIC_PER_COLUMN = (62.9e6 + 53.6e6 + 110.9e6 + 25.9e6) / 15360
 FP64_NOMINAL_TFLOPS = 1.25   # no FP64 peak is measured on this machine: nominal GB300 FP64 (CUDA cores)
 
 
@@ -1086,8 +1085,8 @@ def run_subbands(args):
     """f4: the transverse subband eigensolve of the mode-space set-up (solve_subbands.m) for the
     C4 gate sweep with the confinement direction resolved: per gate point 2 valleys x 401
     slices of the 5 nm body between 1 nm oxides (Ny = 71, dy = 0.1 nm), the 8 eigenpairs of
-    smallest magnitude per slice.  One step solves all 32 gate points as one batch (one
-    launch of the slice kernel and one of the sign clean-up) from potentials resident on the
+    smallest magnitude per slice.  One step solves all 32 gate points as one batch (four
+    launches: location, refinement, bisection, sign clean-up) from potentials resident on the
     device; e2e runs the same batch through SubbandSolver.solve with host arrays (copies in
     and out timed)."""
     import torch
@@ -1137,14 +1136,10 @@ def run_subbands(args):
         sol.status(stream.cuda_stream)
     slices = G * nv * nx
     value = slices * args.steps / (ms / 1000.0)
-    # per slice, FP64 only: Sturm counts of ny entries (2 subtractions, 1 division, 1 compare) -- 1 + the
-    # 2 bracket checks + 32 / nm lanes per candidate x the multisection steps from the FP32 bracket
-    # (4e-5 of the spectral radius) down to eps x nm candidates (all eigenvalues positive here) -- and
-    # the 5 passes of the twisted factorisation per mode (~14 flops per entry); the coarse FP32
-    # multisection runs on the FP32 pipe and is not counted
-    g = 32 // nm
-    steps64 = int(np.ceil(np.log(4e-5 / 2.2e-16) / np.log(g + 1)))
-    flops_slice = ((3 + steps64 * g * nm) * 4 + 14 * nm) * ny
+    # per slice, FP64 only: the refinement takes about 69 FP64 instructions per mode and node (a profile of
+    # this workload: three factorisations of two recurrences with their reciprocals, and the vector),
+    # counted as FMAs; the FP32 location is not counted
+    flops_slice = 2 * 69 * nm * ny
     achieved = flops_slice * value / 1e12
     out = {"metric": "transverse subband eigensolves (slices/s, %d eigenpairs of smallest magnitude per slice)" % nm,
            "value": round(value, 1), "unit": "slices/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
@@ -1153,12 +1148,12 @@ def run_subbands(args):
            "config": {"workload": "f4 subbands: %d gate points x %d valleys x %d slices, Ny = %d (5 nm body + 2 x 1 nm "
                                   "oxide, dy = 0.1 nm), %d modes" % (G, nv, nx, ny, nm),
                       "l2": "256 MB buffer written between timed steps"},
-           "gpu_launches": 2 * args.steps,
+           "gpu_launches": 4 * args.steps,     # location, refinement, bisection, sign clean-up
            "roofline": {"bound": "fp64", "achieved": round(achieved, 4), "peak": 1.25, "unit": "TFLOP/s",
                         "frac": round(achieved / 1.25, 4), "traffic": None,
-                        "peak_source": "nominal GB300 FP64 1.25 TFLOP/s (no measured FP64 peak); flops estimated "
-                                       "from the Sturm counts and eigenvector passes, a division counted as "
-                                       "one (it is ~10 FP64 instructions)"},
+                        "peak_source": "nominal GB300 FP64 1.25 TFLOP/s (no measured FP64 peak); the "
+                                       "refinement's FP64 instructions (69 per mode and node, profiled) counted as "
+                                       "FMAs"},
            "clocks": clk}
     if not args.no_e2e:
         sol.solve(me_all, V_all, SUBBANDS["dy_nm"])
@@ -1291,11 +1286,16 @@ def run_poisson2d(args):
         clk = clocks.stop()
     value = B * args.steps / (ms / 1000.0)
     nu = ny - 1
-    # per bias point: the block sweep (nx Gauss-Jordan inversions of 16 x 16 padded blocks, 2 NU^3
-    # flops each, plus the Schur updates and the two block matvecs) and ~60 flops per node for the
-    # projection, residuals and diagnostics
-    NU = 16
-    flops = nx * (2 * NU ** 3 + 4 * NU * NU) + 60 * nx * ny
+    # per bias point: block cyclic reduction (blocks of NU = 12 rows; level 0 eliminates half of the columns,
+    # 2 NU^2 (2 NU + 1) flops each; level l folds nx / 2^l columns, four products of 2 NU^3 from
+    # level 2 on, and eliminates half of them, 2 NU^2 (3 NU + 1)), the back substitution and ~60 flops per node
+    # for the projection, residuals and diagnostics
+    NU = 12
+    levels = int(np.log2(nx))
+    flops = (nx + 1) // 2 * 2 * NU ** 2 * (2 * NU + 1) + nx * 4 * NU ** 2 + 60 * nx * ny
+    for lv in range(1, levels + 1):
+        flops += (nx >> lv) * ((6 * NU ** 2 if lv == 1 else 8 * NU ** 3) + NU ** 2 * (3 * NU + 1))
+    launches = 3 + levels + (2 if levels >= 3 else 1)   # assemble, invert, finish; a reduction per level; back
     out = {"metric": "2D Poisson steps/s (DG density projection + approximate-Newton update, %d x %d grid)" % (nx, ny),
            "value": round(value, 2), "unit": "bias_point_steps/s", "n_gpus": 1, "steps": args.steps,
            "warmup": args.warmup, "ms_per_step": round(ms / args.steps, 4), "higher_is_better": True,
@@ -1304,11 +1304,12 @@ def run_poisson2d(args):
            "config": {"workload": "f3 Poisson step: %d bias points per call, material grid %d x %d (periodic Y, %d "
                                   "unique rows), DG axes 120 x 2 elements p=2" % (B, nx, ny, nu),
                       "l2": "256 MB buffer written between timed steps"},
-           "gpu_launches": args.steps,
+           "gpu_launches": launches * args.steps,
            "roofline": {"bound": "latency", "achieved": round(flops * value / 1e12, 5), "peak": 1.25,
                         "unit": "TFLOP/s", "frac": round(flops * value / 1e12 / 1.25, 5), "traffic": None,
-                        "peak_source": "nominal GB300 FP64 1.25 TFLOP/s; one warp per bias point runs the "
-                                       "sequential block sweep (latency-bound by construction)"},
+                        "peak_source": "nominal GB300 FP64 1.25 TFLOP/s; the first levels of the block cyclic "
+                                       "reduction are FP64 work, the later ones the latency of one block's "
+                                       "inversion"},
            "clocks": clk}
     if not args.no_e2e:
         op.solve(nDG, phi0, bias, method="newton-raphson", dg=True)
