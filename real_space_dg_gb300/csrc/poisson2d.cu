@@ -594,6 +594,10 @@ cudaError_t keep(wg_poisson2d* h, T** d, const std::vector<T>& v) {
 
 // Problems per group of launches: the grids' second dimension and the reduction's blocks (3 nx NU^2 doubles per
 // problem) stay bounded for any batch.  A group of this size fills the chip at every level.
+// With the chip full, operations count, and the reduction has three times those of a sweep over the columns: one warp per
+// point sweeping would be faster from about 300 points of 32 rows, 450 of 24, 650 of 16 and 1,000 of 12 on (1,024 points
+// of 361 columns: 60, 35, 16.7 and 10.5 ms against 141, 57, 21.1 and 10.9; 5.6 against 5.0 at 8 rows).  Not taken, since a
+// point's bits would depend on the batch it is in.
 constexpr int kP2Group = 1024;
 
 cudaError_t launch_group(wg_poisson2d* h, int B, const double* src, int is_dg, const double* phi0, const double* bc,
